@@ -10,7 +10,7 @@
 //
 //   1 table    queue over problems: up to kBMaxS keys sampled into shared
 //              memory, the problem's splitter table built by build_lut_cta
-//              (the single-vector builder) with 2^nsl_bits <= kBSlices slices;
+//              (the single-vector builder) with 2^nsl_bits slices, nsl_bits <= b_slice_bits;
 //              the tile phases hold it in shared memory once per bank.
 //   2 hist     queue over (problem, tile) items: a tile is a contiguous range
 //              of one problem; its shared-memory histogram becomes one row of
@@ -64,9 +64,18 @@ constexpr int kBThreads = 512;
 // the table once per bank (entry j of lane l's copy at word 32 j + l), so a
 // warp's 32 lookups take one shared-memory wavefront whatever slices its keys
 // hit (a single copy of up to 4096 slices took two to three)
-constexpr uint32_t kBSliceBits = 7;
-constexpr uint32_t kBSlices = 1u << kBSliceBits;
-constexpr uint32_t kBRepLut = (kBSlices + 1) * 32;  // words of the per-bank table
+// (4-byte keys).  8-byte keys: 4 copies of up to 2^10 slices in the same space
+// (entry j of copy c at word 4 j + c), because a double's span covers every
+// exponent between its largest magnitude and zero (see sv_bits): 2^7 slices
+// were 16 binades wide.
+template <class K>
+__host__ __device__ constexpr uint32_t b_slice_bits() {
+  return sizeof(K) == 4 ? 7u : 10u;
+}
+constexpr uint32_t kBRepLut = ((1u << 7) + 1) * 32;  // words of the copies: 32 of 2^7 + 1 entries
+static_assert(((1u << b_slice_bits<uint64_t>()) + 1) * sv_copies<uint64_t>() <= kBRepLut &&
+                  ((1u << b_slice_bits<uint32_t>()) + 1) * sv_copies<uint32_t>() <= kBRepLut,
+              "the table's copies fit their shared memory");
 // shared-memory words in front of the tile phases' histogram / cursors
 constexpr uint32_t kBTileLut = kBRepLut > kLutPadded ? kBRepLut : kLutPadded;
 constexpr int kBSpt = (int)kLutIdx / kBThreads;  // slices per thread in the table build
@@ -249,15 +258,15 @@ __device__ __forceinline__ uint32_t queue_pop(uint32_t *q, uint32_t *s_item) {
 // permutation inside every group of 32 entries.
 __device__ __forceinline__ uint32_t swz(uint32_t x) { return x ^ ((x >> 5) & 31u); }
 
-// bucket_of with the splitter table held once per bank: lane_lut = table +
-// (lane index), entry j at lane_lut[32 j]
+// bucket_of with the splitter table's copies (as bucket_of_rep, with a slice
+// count of the problem's own): entry j at lane_lut[j * copies]
 template <class K>
 __device__ __forceinline__ uint32_t bucket_of_lane(K key, K base, uint32_t shift,
                                                    const uint32_t *lane_lut, uint32_t nsl) {
   const K d = key - base;  // wraps for key < base; that result is discarded
   const K idx = d >> shift;
   const uint32_t j = idx < (K)nsl ? (uint32_t)idx : nsl;
-  const uint32_t e = lane_lut[32 * j];
+  const uint32_t e = lane_lut[j << sv_copy_bits<K>()];
   const uint32_t b = (uint32_t)((int32_t)e >> 7) + shr_clamp(d, e & 127u);
   return key < base ? 0u : b;
 }
@@ -719,7 +728,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
   // ---------------- phase 2: one histogram row per tile
   if (tid == 0) s_cur = 0xFFFFFFFFu;  // problem whose table is in shared memory
   uint32_t *lut = sm;                     // the plan phase's single copy
-  const uint32_t *lane_lut = sm + (tid & 31);  // the tile phases' per-bank copies
+  const uint32_t *lane_lut = sv_lane_table<K>(sm);  // the tile phases' copies
   uint32_t *hist = sm + kBTileLut;
   K *rep = reinterpret_cast<K *>(hist + kBMaxNb);
   K *reps = reinterpret_cast<K *>(A.reps);
@@ -731,7 +740,8 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       const BHdr H = load_hdr(A.hdrs + tl.prob);
       const uint32_t nsl = 1u << P.nsl_bits;
       if (s_cur != tl.prob)
-        for (uint32_t w = tid; w < (nsl + 1) * 32; w += nt) sm[w] = __ldcg(A.luts + P.lut_off + (w >> 5));
+        for (uint32_t w = tid; w < (nsl + 1) * sv_copies<K>(); w += nt)
+          sm[w] = __ldcg(A.luts + P.lut_off + (w >> sv_copy_bits<K>()));
       for (uint32_t b = tid; b < ((H.nb + 31) & ~31u); b += nt) {
         hist[b] = 0;
         if (H.dup) rep[b] = KeyMax<K>::v;
@@ -1066,7 +1076,8 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       const BHdr H = load_hdr(A.hdrs + tl.prob);
       const uint32_t nsl = 1u << P.nsl_bits;
       if (s_cur != tl.prob)
-        for (uint32_t w = tid; w < (nsl + 1) * 32; w += nt) sm[w] = __ldcg(A.luts + P.lut_off + (w >> 5));
+        for (uint32_t w = tid; w < (nsl + 1) * sv_copies<K>(); w += nt)
+          sm[w] = __ldcg(A.luts + P.lut_off + (w >> sv_copy_bits<K>()));
       for (uint32_t b = tid; b < ((H.nb + 31) & ~31u); b += nt) cursor[b] = kInactive;
       __syncthreads();
       if (tid == 0) s_cur = tl.prob;

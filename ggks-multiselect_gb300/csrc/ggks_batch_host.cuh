@@ -91,12 +91,12 @@ int select_batch(Context &ctx, const BatchInput &in, T *d_out_user, T *h_out, cu
     b.x = in.vecs[p];
     b.n = in.n[p];
     // buckets: about n / div elements each, a power of two in [4, kBMaxNb];
-    // half as many slices, at most kBSlices (the table needs nb_max >=
-    // slices + 2; the tile phases hold it once per bank)
+    // half as many slices, at most 2^b_slice_bits (the table needs nb_max >=
+    // slices + 2)
     uint32_t nbm = pow2_ceil_u32((b.n + tune.div - 1) / tune.div);
     nbm = std::min(kBMaxNb, std::max(4u, nbm));
     uint32_t nsl_bits = 0;
-    while ((2u << nsl_bits) < nbm && nsl_bits < kBSliceBits) ++nsl_bits;
+    while ((2u << nsl_bits) < nbm && nsl_bits < b_slice_bits<K>()) ++nsl_bits;
     b.nb_max = nbm;
     b.nsl_bits = nsl_bits;
     b.S = (uint32_t)std::min<uint64_t>(b.n, kBMaxS);

@@ -68,16 +68,44 @@ constexpr uint32_t kLutPadded = (kLutEntries + 3) & ~3u;  // 16-byte multiple
 // at most 2^15 buckets per slice, and 2^(24 - slice bits) so that a packed
 // table entry's first-bucket offset fits its signed 25-bit field
 constexpr int kMaxSubBits = 15;
-// The single-vector path's table: 2^9 slices.  Its streaming passes keep the
-// table in shared memory once per bank -- entry j of copy l at word 32 j + l,
-// read by lane l only -- so that a warp's 32 lookups take one wavefront
-// whatever slices its keys fall in (one shared copy costs about three: the
-// lanes' distinct entries pile up in a few banks).  2^9 slices keep the 32
-// copies at 64 KB beside the 128 KB histogram.  The sample is still binned in
-// 2^12 fine slices, which place the speculative windows (see build_lut_cta).
-constexpr int kSvBits = 9;
-constexpr uint32_t kSvSlices = 1u << kSvBits;
-constexpr uint32_t kRepWords = (kSvSlices + 1) * 32;  // 32 copies of the 2^9 + 1 entries
+// The single-vector path's table (sv_bits<K>: 2^9 slices for 4-byte keys, 2^12
+// for 8-byte ones).  Its streaming passes keep the table in shared memory in
+// sv_copies<K> interleaved copies -- entry j of copy c at word j * copies + c,
+// read by the lanes l with l mod copies = c:
+//   4-byte keys: one copy per bank (32), so that a warp's 32 lookups take one
+//     wavefront whatever slices its keys fall in (one shared copy costs about
+//     three: the lanes' distinct entries pile up in a few banks); 2^9 slices
+//     keep the copies at 64 KB beside the 128 KB histogram;
+//   8-byte keys: 4 copies of 2^12 slices in the same 64 KB.  A double's key
+//     span covers both signs and every exponent between the largest magnitude
+//     and zero, about 2090 binades for +-1e6, of which the elements fill some
+//     30: 2^9 slices are 4 binades wide, so that the widest-filled binade got
+//     a quarter of its slice's buckets (2^27 uniform in +-1e6, 1001 k's: 14.9 M
+//     survivors where equal buckets would hold 4.1 M).  2^12 slices are half a
+//     binade.  A pass over 8-byte keys has half the lookups per byte, so their
+//     extra wavefronts (eight lanes on eight banks per copy) are affordable.
+// The sample is binned in 2^12 fine slices, which place the speculative
+// windows (see build_lut_cta).
+template <class K>
+__host__ __device__ constexpr int sv_bits() {
+  return sizeof(K) == 4 ? 9 : 12;
+}
+template <class K>
+__host__ __device__ constexpr uint32_t sv_slices() {
+  return 1u << sv_bits<K>();
+}
+template <class K>
+__host__ __device__ constexpr uint32_t sv_copy_bits() {
+  return sizeof(K) == 4 ? 5u : 2u;
+}
+template <class K>
+__host__ __device__ constexpr uint32_t sv_copies() {
+  return 1u << sv_copy_bits<K>();
+}
+constexpr uint32_t kRepWords = ((1u << 9) + 1) * 32;  // words of the copies: 32 of 2^9 + 1 entries
+static_assert((sv_slices<uint64_t>() + 1) * sv_copies<uint64_t>() <= kRepWords &&
+                  (sv_slices<uint32_t>() + 1) * sv_copies<uint32_t>() <= kRepWords,
+              "the table's copies fit their shared memory");
 constexpr uint32_t kMaxNb = 32768;  // buckets of one vector: shared-memory histogram limit (u32)
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 constexpr uint32_t kInactive = 0x80000000u;  // compaction cursor of an inactive bucket
@@ -426,24 +454,32 @@ __device__ __forceinline__ uint32_t bucket_of(K key, K base, uint32_t shift, con
   return key < base ? 0u : b;
 }
 
-// bucket_of on the single-vector table (kSvSlices slices) replicated once per
-// bank in shared memory: lane_lut = table + (lane index), entry j at
-// lane_lut[32 j], so the lanes of a warp never share a bank.
+// bucket_of on the single-vector table (sv_slices<K>() slices) held in copies in
+// shared memory: lane_lut = sv_lane_table(table), entry j at
+// lane_lut[j * copies].
 template <class K>
 __device__ __forceinline__ uint32_t bucket_of_rep(K key, K base, uint32_t shift,
                                                   const uint32_t *lane_lut) {
   const K d = key - base;  // wraps for key < base; that result is discarded
   const K idx = d >> shift;
-  const uint32_t j = idx < (K)kSvSlices ? (uint32_t)idx : kSvSlices;
-  const uint32_t e = lane_lut[j << 5];
+  const uint32_t j = idx < (K)sv_slices<K>() ? (uint32_t)idx : sv_slices<K>();
+  const uint32_t e = lane_lut[j << sv_copy_bits<K>()];
   const uint32_t b = (uint32_t)((int32_t)e >> 7) + shr_clamp(d, e & 127u);
   return key < base ? 0u : b;
 }
 
-// Copies the single-vector table (kSvSlices + 1 entries, global) into shared
-// memory once per bank (kRepWords words); the caller synchronises.
+// this lane's copy of the table
+template <class K>
+__device__ __forceinline__ const uint32_t *sv_lane_table(const uint32_t *rep) {
+  return rep + (threadIdx.x & (sv_copies<K>() - 1u));
+}
+
+// Copies the single-vector table (sv_slices<K>() + 1 entries, global) into its
+// copies in shared memory; the caller synchronises.
+template <class K>
 __device__ __forceinline__ void load_rep_table(uint32_t *rep, const uint32_t *__restrict__ lut_g) {
-  for (uint32_t i = threadIdx.x; i < kRepWords; i += blockDim.x) rep[i] = __ldg(lut_g + (i >> 5));
+  for (uint32_t i = threadIdx.x; i < (sv_slices<K>() + 1) * sv_copies<K>(); i += blockDim.x)
+    rep[i] = __ldg(lut_g + (i >> sv_copy_bits<K>()));
 }
 
 __device__ __forceinline__ uint32_t lut_pack(int32_t C, uint32_t rs) {
@@ -1005,11 +1041,11 @@ __global__ void __launch_bounds__(1024) k_lut(const K *__restrict__ samples, uin
   __syncthreads();
   if (!s_last) return;
 
-  // the table has kSvSlices slices; the fine counts (this CTA's ccnt is free
+  // the table has sv_slices<K>() slices; the fine counts (this CTA's ccnt is free
   // now) place the speculative windows
   __syncthreads();
   const SpecArgs sa{ctrl, n, cand_cap, G};
-  build_lut_cta<K, 4, false>(samples, S, kmin, kmax, nb_max, lut, hdr, kSvBits, slice_cnt,
+  build_lut_cta<K, 4, false>(samples, S, kmin, kmax, nb_max, lut, hdr, sv_bits<K>(), slice_cnt,
                              (int64_t)__ldcg(&ctrl->same_key), &sa, dup_nb_cap<K>(nb_max), ccnt);
   if (tid == 0) {
     ctrl->nb = hdr->nb;
@@ -1303,14 +1339,14 @@ __global__ void __launch_bounds__(1024, 1)
   pdl_start();
   using K = typename Traits<T>::K;
   extern __shared__ uint4 smem_raw[];
-  uint32_t *rep_lut = reinterpret_cast<uint32_t *>(smem_raw);  // one copy per bank
+  uint32_t *rep_lut = reinterpret_cast<uint32_t *>(smem_raw);  // the table's copies
   uint32_t *hist = (rep_lut + kRepWords);
-  const uint32_t *lut = rep_lut + (threadIdx.x & 31);  // this lane's copy
+  const uint32_t *lut = sv_lane_table<K>(rep_lut);  // this lane's copy
   __shared__ uint32_t s_wcnt[kCandWarps];
   __shared__ uint32_t s_tab[kCandWarps * kCandChunksPerWarp];
   if (ctrl->status & ST_FATAL) return;
   const LutHeader<K> h = *hdr;
-  load_rep_table(rep_lut, lut_g);
+  load_rep_table<K>(rep_lut, lut_g);
   const uint32_t dcap = dup_nb_cap<K>(nb_max);
   const bool track = reps != nullptr && h.dup && dcap != 0 && h.nb <= dcap;
   K *rep = track ? reinterpret_cast<K *>(hist + dcap) : nullptr;
@@ -1933,8 +1969,8 @@ __global__ void __launch_bounds__(1024, 1)
   const bool dtrack = bsingle != nullptr && bkey != nullptr && h.dup && dcap != 0 && nb <= dcap;
   for (uint32_t q = s0; q < s1; ++q) {
     const uint32_t b = segb_smem ? s_segb[q] : __ldcg(seg_bucket + q);
-    const K klo = bucket_lo<K>(b, h.base, h.shift, lut, kSvSlices);
-    const K knext = (b + 1 < nb) ? bucket_lo<K>(b + 1, h.base, h.shift, lut, kSvSlices) : K(0);
+    const K klo = bucket_lo<K>(b, h.base, h.shift, lut, sv_slices<K>());
+    const K knext = (b + 1 < nb) ? bucket_lo<K>(b + 1, h.base, h.shift, lut, sv_slices<K>()) : K(0);
     // single key iff the next bucket starts one key later; the start of the
     // top entry's bucket can wrap past the key width, and then bucket b runs
     // up to the largest key
@@ -2146,7 +2182,7 @@ __device__ __forceinline__ void compact_body(const T *__restrict__ x, uint64_t n
   }
 }
 
-// dynamic shared memory of k_compact: the table once per bank, then one
+// dynamic shared memory of k_compact: the table's copies, then one
 // cursor per bucket
 __host__ __device__ constexpr size_t compact_smem_bytes(uint32_t nb_max) {
   return (size_t)(kRepWords + nb_max) * sizeof(uint32_t);
@@ -2194,9 +2230,9 @@ __global__ void __launch_bounds__(1024, 1)
   pdl_start();
   using K = typename Traits<T>::K;
   extern __shared__ uint4 smem_raw[];
-  uint32_t *rep_lut = reinterpret_cast<uint32_t *>(smem_raw);  // one copy per bank
+  uint32_t *rep_lut = reinterpret_cast<uint32_t *>(smem_raw);  // the table's copies
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t *lut = rep_lut + lane;  // this lane's copy
+  const uint32_t *lut = sv_lane_table<K>(rep_lut);  // this lane's copy
   uint32_t *cursor = rep_lut + kRepWords;  // per bucket
   __shared__ bool s_bad;
   __shared__ bool s_spec_miss;
@@ -2207,7 +2243,7 @@ __global__ void __launch_bounds__(1024, 1)
   if ((ctrl->status & (ST_FATAL | ST_OVERFLOW)) || ctrl->total_surv == 0) return;
   const LutHeader<K> h = *hdr;
   const uint32_t c = blockIdx.x;
-  load_rep_table(rep_lut, lut_g);
+  load_rep_table<K>(rep_lut, lut_g);
   const uint32_t num_slots = ctrl->num_slots;
   const bool spec = cand != nullptr && h.spec != 0;
   for (uint32_t b = threadIdx.x; b < h.nb; b += blockDim.x) cursor[b] = kInactive;

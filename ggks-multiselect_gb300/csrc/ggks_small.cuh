@@ -11,9 +11,9 @@
 //
 //   A  every CTA samples the same keys (pairs of neighbouring elements at
 //      hashed positions) and builds the same table with build_lut_cta, the
-//      single-vector builder (512 slices, kSmNb buckets): no CTA waits for
+//      single-vector builder (sv_slices slices, kSmNb buckets): no CTA waits for
 //      another's table.
-//   B  every CTA holds the table once per bank and counts its contiguous
+//   B  every CTA holds the table's copies and counts its contiguous
 //      share of the vector into one shared-memory word per bucket.
 //   C  bucket b is owned by thread b % 1024 of CTA b / 1024: it sums the
 //      bucket's counts over the cluster; a block scan and the CTAs' totals
@@ -94,7 +94,7 @@ constexpr uint64_t kSmMaxN = 1ull << 20;
 constexpr uint64_t kSmMaxTopkN = 1ull << 18;
 constexpr uint32_t ST_SMALL_MISS = 64u;           // run the pipeline instead
 
-// dynamic shared memory: the table once per bank, then one word per bucket --
+// dynamic shared memory: the table's copies, then one word per bucket --
 // its count after the histogram phase, its compaction cursor after the plan
 // (inactive cursors carry bit 31).  CTA 0's samples (phase A) lie over the
 // bucket words; the finishers' scratch (phase F) over both.
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   extern __shared__ uint4 smem_raw[];
   uint32_t *rep = reinterpret_cast<uint32_t *>(smem_raw);
   uint32_t *hc = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(smem_raw) + kSmHcOff);
-  __shared__ uint32_t s_tab[kSvSlices + 1];  // the splitter table
+  __shared__ uint32_t s_tab[sv_slices<K>() + 1];  // the splitter table
   __shared__ LutHeader<K> s_hdr;
   __shared__ K redk[33];
   __shared__ uint32_t red32[33];
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
     hi = block_reduce(hi, [](K u, K v) { return u > v ? u : v; }, redk);
     GGKS_SMALL_STAMP(1);
     build_lut_cta<K, (int)(kLutIdx / kSmThreads), true>(samples, S, lo, hi, kSmNb, s_tab, &s_hdr,
-                                                        kSvBits);
+                                                        sv_bits<K>());
   }
   __syncthreads();
   GGKS_SMALL_STAMP(2);
@@ -264,10 +264,11 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   // ---------------- B: histogram of this CTA's share
   for (uint32_t b = tid; b < kSmNb; b += kSmThreads) hc[b] = 0;
   __syncthreads();
-  for (uint32_t i = tid; i < kRepWords; i += kSmThreads) rep[i] = s_tab[i >> 5];
+  for (uint32_t i = tid; i < (sv_slices<K>() + 1) * sv_copies<K>(); i += kSmThreads)
+    rep[i] = s_tab[i >> sv_copy_bits<K>()];
   const LutHeader<K> h = s_hdr;
   const uint64_t a0 = n * r / kSmCtas, a1 = n * (r + 1) / kSmCtas;
-  const uint32_t *lut = rep + lane;
+  const uint32_t *lut = sv_lane_table<K>(rep);
   __syncthreads();
   for_range<T>(x, a0, a1, [&](K k, bool) {
     atomicAdd(&hc[bucket_of_rep<K>(k, h.base, h.shift, lut)], 1u);
@@ -386,8 +387,8 @@ __global__ void __launch_bounds__(kSmThreads, 1)
     const uint32_t nsmall = s_nsmall, nlarge = s_nlarge;
     // key range of bucket gb: from its first key to the next bucket's
     auto range = [&](uint32_t gb, K *klo, K *khi) {
-      const K lo = bucket_lo<K>(gb, h.base, h.shift, s_tab, kSvSlices);
-      const K nx = gb + 1 < h.nb ? bucket_lo<K>(gb + 1, h.base, h.shift, s_tab, kSvSlices) : K(0);
+      const K lo = bucket_lo<K>(gb, h.base, h.shift, s_tab, sv_slices<K>());
+      const K nx = gb + 1 < h.nb ? bucket_lo<K>(gb + 1, h.base, h.shift, s_tab, sv_slices<K>()) : K(0);
       *klo = lo;
       *khi = nx > lo ? nx - K(1) : KeyMax<K>::v;
     };
