@@ -475,11 +475,51 @@ __device__ __forceinline__ const uint32_t *sv_lane_table(const uint32_t *rep) {
 }
 
 // Copies the single-vector table (sv_slices<K>() + 1 entries, global) into its
-// copies in shared memory; the caller synchronises.
+// copies in shared memory, by a CTA of 1024 threads: each entry is read once
+// per CTA, coalesced, in one round of loads (every CTA reads the same few
+// kilobytes at the same time: a gather that asked L2 for each warp's own
+// sectors cost 2-4 us), and the copies are written with 16-byte stores.  tab:
+// sv_slices<K>() + 1 shared words (sv_copies 32; else unused).  Ends with a
+// barrier for the caller's shared memory.
 template <class K>
-__device__ __forceinline__ void load_rep_table(uint32_t *rep, const uint32_t *__restrict__ lut_g) {
-  for (uint32_t i = threadIdx.x; i < (sv_slices<K>() + 1) * sv_copies<K>(); i += blockDim.x)
-    rep[i] = __ldg(lut_g + (i >> sv_copy_bits<K>()));
+__device__ __forceinline__ void load_rep_table(uint32_t *rep, const uint32_t *__restrict__ lut_g,
+                                               uint32_t *tab) {
+  constexpr uint32_t kEnt = sv_slices<K>() + 1;
+  constexpr uint32_t kPer = (kEnt + 1023) / 1024;
+  uint32_t e[kPer];
+#pragma unroll
+  for (uint32_t i = 0; i < kPer; ++i) {
+    const uint32_t j = threadIdx.x + 1024 * i;
+    e[i] = j < kEnt ? __ldcg(lut_g + j) : 0u;
+  }
+  if constexpr (sv_copies<K>() == 4) {
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i) {
+      const uint32_t j = threadIdx.x + 1024 * i;
+      if (j < kEnt) reinterpret_cast<uint4 *>(rep)[j] = make_uint4(e[i], e[i], e[i], e[i]);
+    }
+  } else {
+    constexpr uint32_t kVecs = sv_copies<K>() / 4;  // 16-byte stores per entry
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i)
+      if (threadIdx.x + 1024 * i < kEnt) tab[threadIdx.x + 1024 * i] = e[i];
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = 0; i < (kEnt * kVecs + 1023) / 1024; ++i) {
+      const uint32_t q = threadIdx.x + 1024 * i;
+      if (q < kEnt * kVecs) {
+        const uint32_t v = tab[q / kVecs];
+        reinterpret_cast<uint4 *>(rep)[q] = make_uint4(v, v, v, v);
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// Fills nb_max words (a multiple of 4, 16-byte aligned) of shared memory.
+__device__ __forceinline__ void fill_words(uint32_t *a, uint32_t words, uint32_t v) {
+  for (uint32_t i = threadIdx.x; i < words / 4; i += blockDim.x)
+    reinterpret_cast<uint4 *>(a)[i] = make_uint4(v, v, v, v);
 }
 
 __device__ __forceinline__ uint32_t lut_pack(int32_t C, uint32_t rs) {
@@ -1336,7 +1376,12 @@ __global__ void __launch_bounds__(1024, 1)
            const Ctrl *ctrl, T *__restrict__ copy_to, typename Traits<T>::K *__restrict__ cand,
            uint32_t *__restrict__ cand_cnt, uint32_t *__restrict__ cand_tab,
            uint32_t *cand_next, typename Traits<T>::K *__restrict__ reps) {
-  pdl_start();
+  // Clearing the counts needs nothing of the kernels before: it runs ahead of
+  // the dependency wait, while they finish.  After the wait the header and the
+  // table come in one round of loads.  (10 M floats: this and the 16-byte row
+  // stores below took the pass from 21 to 19 us, of which 7 are the
+  // streaming itself.)
+  pdl_trigger();
   using K = typename Traits<T>::K;
   extern __shared__ uint4 smem_raw[];
   uint32_t *rep_lut = reinterpret_cast<uint32_t *>(smem_raw);  // the table's copies
@@ -1344,18 +1389,21 @@ __global__ void __launch_bounds__(1024, 1)
   const uint32_t *lut = sv_lane_table<K>(rep_lut);  // this lane's copy
   __shared__ uint32_t s_wcnt[kCandWarps];
   __shared__ uint32_t s_tab[kCandWarps * kCandChunksPerWarp];
-  if (ctrl->status & ST_FATAL) return;
+  static_assert(sv_slices<uint32_t>() + 1 <= kCandWarps * kCandChunksPerWarp, "s_tab lends its space");
+  fill_words(hist, nb_max, 0u);
+  pdl_wait();
+  const uint32_t status = ctrl->status;
   const LutHeader<K> h = *hdr;
-  load_rep_table<K>(rep_lut, lut_g);
+  load_rep_table<K>(rep_lut, lut_g, s_tab);
+  if (status & ST_FATAL) return;
   const uint32_t dcap = dup_nb_cap<K>(nb_max);
   const bool track = reps != nullptr && h.dup && dcap != 0 && h.nb <= dcap;
   K *rep = track ? reinterpret_cast<K *>(hist + dcap) : nullptr;
-  const uint32_t span = min(bank_span(h.nb), nb_max);
-  for (uint32_t b = threadIdx.x; b < span; b += blockDim.x) {
-    hist[b] = 0;
-    if (track) rep[b] = KeyMax<K>::v;
+  if (track) {  // over cleared counts (load_rep_table ended with a barrier)
+    for (uint32_t b = threadIdx.x; b < min(bank_span(h.nb), nb_max); b += blockDim.x)
+      rep[b] = KeyMax<K>::v;
+    __syncthreads();
   }
-  __syncthreads();
   const bool spec = cand != nullptr && h.spec != 0;
   const uint32_t warp = threadIdx.x >> 5;
   CandPool<K> cr;
@@ -1380,10 +1428,15 @@ __global__ void __launch_bounds__(1024, 1)
   }
   __syncthreads();
   uint32_t *row = partials + (uint64_t)blockIdx.x * nb_max;
-  for (uint32_t b = threadIdx.x; b < h.nb; b += blockDim.x) {
-    const uint32_t i = track ? bank_swz(b) : b;
-    row[b] = hist[i];
-    if (track) reps[(uint64_t)blockIdx.x * nb_max + b] = rep[i];
+  if (track) {
+    for (uint32_t b = threadIdx.x; b < h.nb; b += blockDim.x) {
+      const uint32_t i = bank_swz(b);
+      row[b] = hist[i];
+      reps[(uint64_t)blockIdx.x * nb_max + b] = rep[i];
+    }
+  } else {
+    for (uint32_t v = threadIdx.x; v < (h.nb + 3) / 4; v += blockDim.x)
+      reinterpret_cast<uint4 *>(row)[v] = reinterpret_cast<const uint4 *>(hist)[v];
   }
   if (spec) {
     if (threadIdx.x < kCandWarps)
@@ -2227,7 +2280,10 @@ __global__ void __launch_bounds__(1024, 1)
               const typename Traits<T>::K *__restrict__ cand,
               const uint32_t *__restrict__ cand_cnt, const uint32_t *__restrict__ cand_tab,
               uint64_t surv_half) {
-  pdl_start();
+  // the cursors are cleared ahead of the dependency wait (as in k_hist); after
+  // it the control block, the table and each thread's first slot come in one
+  // round of loads (the slot arrays hold nb_max entries)
+  pdl_trigger();
   using K = typename Traits<T>::K;
   extern __shared__ uint4 smem_raw[];
   uint32_t *rep_lut = reinterpret_cast<uint32_t *>(smem_raw);  // the table's copies
@@ -2238,20 +2294,27 @@ __global__ void __launch_bounds__(1024, 1)
   __shared__ bool s_spec_miss;
   __shared__ uint32_t s_wcnt[kCandWarps];
   __shared__ uint32_t s_tab[kCandWarps * kCandChunksPerWarp];
-  // nothing to compact when every slot is a single-key one (answered by the
-  // finisher from its key alone), and then no cursor needs checking either
-  if ((ctrl->status & (ST_FATAL | ST_OVERFLOW)) || ctrl->total_surv == 0) return;
-  const LutHeader<K> h = *hdr;
-  const uint32_t c = blockIdx.x;
-  load_rep_table<K>(rep_lut, lut_g);
-  const uint32_t num_slots = ctrl->num_slots;
-  const bool spec = cand != nullptr && h.spec != 0;
-  for (uint32_t b = threadIdx.x; b < h.nb; b += blockDim.x) cursor[b] = kInactive;
+  static_assert(sv_slices<uint32_t>() + 1 <= kCandWarps * kCandChunksPerWarp, "s_tab lends its space");
+  fill_words(cursor, nb_max, kInactive);
   if (threadIdx.x == 0) {
     s_bad = false;
     s_spec_miss = false;
   }
-  __syncthreads();
+  pdl_wait();
+  const uint32_t status = ctrl->status;
+  const uint64_t total_surv = ctrl->total_surv;
+  const uint32_t num_slots = ctrl->num_slots;
+  const LutHeader<K> h = *hdr;
+  const bool has0 = threadIdx.x < nb_max;
+  const uint32_t sz0 = has0 ? __ldcg(seg_size + threadIdx.x) : 0u;
+  const uint32_t b0 = has0 ? __ldcg(seg_bucket + threadIdx.x) : 0u;
+  const uint64_t off0 = has0 ? __ldcg(seg_off + threadIdx.x) : 0u;
+  load_rep_table<K>(rep_lut, lut_g, s_tab);
+  // nothing to compact when every slot is a single-key one (answered by the
+  // finisher from its key alone), and then no cursor needs checking either
+  if ((status & (ST_FATAL | ST_OVERFLOW)) || total_surv == 0) return;
+  const uint32_t c = blockIdx.x;
+  const bool spec = cand != nullptr && h.spec != 0;
   // a warp whose list is incomplete (its table or the pool ran out) sends the
   // CTA to its tiles
   if (spec) {
@@ -2270,9 +2333,21 @@ __global__ void __launch_bounds__(1024, 1)
       }
     }
   }
-  // flat slots (seg_size 0: a single-key bucket) are answered without survivors
+  // flat slots (seg_size 0: a single-key bucket) are answered without
+  // survivors.  A thread's first slot stays in registers (its bucket and where
+  // its cursor has to end); further slots leave the end in the row.
   uint32_t *row = rows + (uint64_t)c * nb_max;
-  for (uint32_t s = threadIdx.x; s < num_slots; s += blockDim.x) {
+  const bool live0 = threadIdx.x < num_slots && sz0 != 0;
+  uint32_t end0 = 0;
+  if (live0) {
+    const uint32_t cnt = __ldcg(row + b0) & ~kMixed;
+    const uint32_t pre = cnt ? atomicAdd(fill + threadIdx.x, cnt) : 0u;
+    const uint32_t at = (uint32_t)(off0 + pre);
+    cursor[b0] = at;
+    end0 = at + cnt;
+    if (spec && !in_spec(h, b0)) s_spec_miss = true;
+  }
+  for (uint32_t s = threadIdx.x + blockDim.x; s < num_slots; s += blockDim.x) {
     const uint32_t sz = seg_size[s];
     if (sz == 0) continue;
     const uint32_t b = seg_bucket[s];
@@ -2285,7 +2360,7 @@ __global__ void __launch_bounds__(1024, 1)
   }
   __syncthreads();
   const uint32_t cap = (uint32_t)(surv_cap < (uint64_t)kInactive ? surv_cap : kInactive);
-  if (spec && !s_spec_miss && ctrl->total_surv <= surv_half) {
+  if (spec && !s_spec_miss && total_surv <= surv_half) {
     // warp w reads the candidates of the histogram pass's warp w
     const uint32_t w = threadIdx.x >> 5;
     const uint32_t *wt = s_tab + w * kCandChunksPerWarp;
@@ -2323,7 +2398,8 @@ __global__ void __launch_bounds__(1024, 1)
   __syncthreads();
   // every cursor must have reached the end of the CTA's share; anything else
   // means the input changed between the two passes
-  for (uint32_t s = threadIdx.x; s < num_slots; s += blockDim.x) {
+  if (live0 && cursor[b0] != end0) s_bad = true;
+  for (uint32_t s = threadIdx.x + blockDim.x; s < num_slots; s += blockDim.x) {
     if (seg_size[s] == 0) continue;
     const uint32_t b = seg_bucket[s];
     if (cursor[b] != row[b]) s_bad = true;
