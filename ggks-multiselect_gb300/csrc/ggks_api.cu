@@ -157,13 +157,20 @@ cudaError_t ensure_pin(Context &ctx, size_t bytes) {
   if (ctx.pin) {
     cudaFreeHost(ctx.pin);
     ctx.pin = nullptr;
+    ctx.pin_dev = nullptr;
     ctx.pin_bytes = 0;
   }
   size_t want = bytes + bytes / 4 + 4096;
-  void *p = nullptr;
-  cudaError_t e = cudaHostAlloc(&p, want, cudaHostAllocDefault);
+  void *p = nullptr, *d = nullptr;
+  cudaError_t e = cudaHostAlloc(&p, want, cudaHostAllocMapped);
   if (e != cudaSuccess) return e;
+  e = cudaHostGetDevicePointer(&d, p, 0);
+  if (e != cudaSuccess) {
+    cudaFreeHost(p);
+    return e;
+  }
   ctx.pin = static_cast<char *>(p);
+  ctx.pin_dev = static_cast<char *>(d);
   ctx.pin_bytes = want;
   return cudaSuccess;
 }

@@ -203,7 +203,8 @@ struct Req {
   uint32_t out;
 };
 
-// Device control block (lives in the workspace; zeroed once at allocation).
+// Device control block (lives in the workspace; k_sample, the call's first
+// kernel, sets every word of it).
 struct Ctrl {
   uint32_t status;
   uint32_t num_slots;
@@ -213,16 +214,15 @@ struct Ctrl {
   uint32_t same_key;       // far-apart sample pairs holding one key (k_lut)
   uint32_t nb;             // buckets in use
   uint64_t cap_needed;
-  uint64_t kmin_inv;     // ~(smallest sampled key), by atomicMax
-  uint64_t kmax;         // largest sampled key, by atomicMax
-  // rank windows of the call's requests, written by the host into the
-  // uploaded image (0 windows: the requests are spread out or unknown)
+  // rank windows of the call's requests, set by the host (0 windows: the
+  // requests are spread out or unknown)
   uint32_t spec_nwin;
   uint32_t spec_pad;
   uint64_t spec_lo[2], spec_hi[2];  // ascending 0-based ranks, inclusive
   uint32_t spec_on;    // the table keeps candidate buckets (k_lut)
   uint32_t spec_ctas;  // compaction CTAs that read candidates
   uint32_t cand_next;  // candidate chunks handed out (k_hist)
+  uint32_t fin_done;   // last-CTA ticket of k_finish
   uint64_t t_ns[16];   // phase stamps of the small-vector kernel (GGKS_SMALL_TIMING builds)
 };
 
@@ -995,8 +995,10 @@ __device__ void build_lut_cta(const K *samples, uint32_t S, K kmin, K kmax, uint
 }
 
 // Two kernels of ceil(S / 1024) CTAs.  k_sample: each thread gathers one
-// sample (pairs of neighbouring elements at hashed positions) and each CTA
-// folds its min / max into Ctrl.
+// sample (pairs of neighbouring elements at hashed positions), each CTA leaves
+// its samples' smallest and largest key in spans (two keys per CTA), and CTA 0
+// sets the control block to init, which travels in the launch's parameters: no
+// copy or clearing precedes the call's first kernel.
 // k_lut (after it in the stream): each CTA re-reads its 1024 samples, bins
 // them by slice in shared memory against the sample's span, adds its non-zero
 // slice counts to slice_cnt (global, zero on entry) and counts the far-apart
@@ -1011,10 +1013,14 @@ template <class T>
 __global__ void __launch_bounds__(1024) k_sample(const T *__restrict__ x, uint64_t n, uint32_t S,
                                                  uint32_t seed,
                                                  typename Traits<T>::K *__restrict__ samples,
-                                                 Ctrl *ctrl) {
+                                                 typename Traits<T>::K *__restrict__ spans,
+                                                 Ctrl *ctrl, const __grid_constant__ Ctrl init) {
   pdl_start();
   using K = typename Traits<T>::K;
   __shared__ K redk[33];
+  if (blockIdx.x == 0 && threadIdx.x < sizeof(Ctrl) / 4)
+    reinterpret_cast<uint32_t *>(ctrl)[threadIdx.x] =
+        reinterpret_cast<const uint32_t *>(&init)[threadIdx.x];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   K mine_lo = KeyMax<K>::v, mine_hi = 0;
   if (i < S) {
@@ -1035,14 +1041,35 @@ __global__ void __launch_bounds__(1024) k_sample(const T *__restrict__ x, uint64
   mine_lo = block_reduce(mine_lo, [](K p, K q) { return p < q ? p : q; }, redk);
   mine_hi = block_reduce(mine_hi, [](K p, K q) { return p > q ? p : q; }, redk);
   if (threadIdx.x == 0) {
-    atomicMax((unsigned long long *)&ctrl->kmin_inv, (unsigned long long)~(uint64_t)mine_lo);
-    atomicMax((unsigned long long *)&ctrl->kmax, (unsigned long long)mine_hi);
+    spans[2 * blockIdx.x] = mine_lo;
+    spans[2 * blockIdx.x + 1] = mine_hi;
   }
+}
+
+// The sample's smallest and largest key from the parts CTAs' spans (k_sample);
+// every warp reduces them for itself.
+template <class K>
+__device__ __forceinline__ void sample_span(const K *__restrict__ spans, uint32_t parts, K *kmin,
+                                            K *kmax) {
+  K lo = KeyMax<K>::v, hi = 0;
+  for (uint32_t i = threadIdx.x & 31; i < parts; i += 32) {
+    const K a = __ldcg(spans + 2 * i), z = __ldcg(spans + 2 * i + 1);
+    lo = a < lo ? a : lo;
+    hi = z > hi ? z : hi;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const K a = __shfl_xor_sync(0xffffffffu, lo, o), z = __shfl_xor_sync(0xffffffffu, hi, o);
+    lo = a < lo ? a : lo;
+    hi = z > hi ? z : hi;
+  }
+  *kmin = lo;
+  *kmax = hi;
 }
 
 template <class K>
 __global__ void __launch_bounds__(1024) k_lut(const K *__restrict__ samples, uint32_t S,
-                                              Ctrl *ctrl, LutHeader<K> *hdr, uint32_t *lut,
+                                              const K *__restrict__ spans, Ctrl *ctrl, LutHeader<K> *hdr, uint32_t *lut,
                                               uint32_t nb_max, uint32_t *slice_cnt, uint64_t n,
                                               uint32_t cand_cap, uint32_t G) {
   pdl_start();
@@ -1056,8 +1083,8 @@ __global__ void __launch_bounds__(1024) k_lut(const K *__restrict__ samples, uin
   const uint32_t npairs = S / 2 < 4096u ? S / 2 : 4096u;
   const K k = i < S ? __ldcg(samples + i) : K(0);
   const K other = i < npairs ? __ldcg(samples + i + S / 2) : K(0);
-  const K kmin = (K)~__ldcg((const unsigned long long *)&ctrl->kmin_inv);
-  const K kmax = (K)__ldcg((const unsigned long long *)&ctrl->kmax);
+  K kmin, kmax;
+  sample_span<K>(spans, gridDim.x, &kmin, &kmax);
   const int bl = bitlen<K>(kmax - kmin);
   const uint32_t shift = bl > kLutIdxBits ? (uint32_t)(bl - kLutIdxBits) : 0u;
   __syncthreads();
@@ -1859,10 +1886,9 @@ __global__ void __launch_bounds__(1024, 1)
            uint32_t *__restrict__ req_local, Req *__restrict__ klist, uint64_t surv_cap,
            Premap pm, const uint32_t *__restrict__ bsingle = nullptr,
            const typename Traits<InT>::K *__restrict__ bkey = nullptr) {
-  // The requests are complete before the call's first kernel (uploaded, made
-  // by a kernel the plainly launched sample kernel waits for, or left by an
-  // earlier call): with at most one per thread, each thread loads its own
-  // ahead of the dependency wait.
+  // At most one request per thread: the requests were complete before the
+  // call's first launch (in host memory, read here in place, or left by an
+  // earlier call), so each thread loads its own ahead of the dependency wait.
   pdl_trigger();
   const bool own = num_req <= blockDim.x;
   Req my_rq;
@@ -2930,11 +2956,12 @@ __global__ void __launch_bounds__(kFinThreads)
              const uint32_t *__restrict__ seg_size, const K *__restrict__ seg_lo,
              const K *__restrict__ seg_hi, const uint32_t *__restrict__ kstart,
              const uint32_t *__restrict__ kcnt, const Req *__restrict__ klist,
-             uint32_t *__restrict__ deferred, uint32_t bcap, OutT *__restrict__ out) {
+             uint32_t *__restrict__ deferred, uint32_t bcap, OutT *__restrict__ out,
+             Ctrl *__restrict__ host_ctrl) {
   pdl_start();
   extern __shared__ uint4 smem_raw[];
-  if (ctrl->status & (ST_FATAL | ST_OVERFLOW)) return;
-  const uint32_t num_slots = ctrl->num_slots;
+  const uint32_t num_slots =
+      (ctrl->status & (ST_FATAL | ST_OVERFLOW)) ? 0u : ctrl->num_slots;
   for (uint32_t slot = blockIdx.x; slot < num_slots; slot += gridDim.x) {
     const bool done = finish_slot<K, OutT>(surv + seg_off[slot], seg_size[slot], seg_lo[slot],
                                            seg_hi[slot], klist + kstart[slot], kcnt[slot], bcap,
@@ -2943,6 +2970,24 @@ __global__ void __launch_bounds__(kFinThreads)
       const uint32_t d = atomicAdd(&ctrl->deferred_count, 1u);
       deferred[d] = slot;
       atomicOr(&ctrl->status, ST_DEFERRED);
+    }
+  }
+  // The last CTA writes the control block to host memory (host_ctrl, when
+  // given): the host reads it after the stream's synchronisation, no copy
+  // follows the call's last kernel.
+  if (host_ctrl) {
+    __shared__ uint32_t s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      s_last = atomicAdd(&ctrl->fin_done, 1u) == gridDim.x - 1 ? 1u : 0u;
+      __threadfence();
+    }
+    __syncthreads();
+    if (s_last && threadIdx.x < sizeof(Ctrl) / 4) {
+      reinterpret_cast<uint32_t *>(host_ctrl)[threadIdx.x] =
+          __ldcg(reinterpret_cast<const uint32_t *>(ctrl) + threadIdx.x);
+      if (threadIdx.x == 0) ctrl->fin_done = 0;  // the kernel may run again in this call
     }
   }
 }

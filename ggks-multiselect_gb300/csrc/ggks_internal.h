@@ -60,6 +60,8 @@ struct Context {
   size_t dvec_bytes = 0;
   char *pin = nullptr;
   size_t pin_bytes = 0;
+  char *pin_dev = nullptr;  // pin's address for kernels (they read requests and write
+                            // results and status there in place)
 
   std::unique_ptr<Context> child;
   int depth = 0;

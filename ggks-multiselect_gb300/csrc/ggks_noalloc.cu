@@ -46,7 +46,8 @@ constexpr size_t kNaReqs = na_align(kNaSliceCnt + kSliceCntBytes);
 constexpr size_t kNaHdr = na_align(kNaReqs + kNaMaxK * sizeof(Req));
 constexpr size_t kNaLut = na_align(kNaHdr + sizeof(LutHeader<uint32_t>));
 constexpr size_t kNaSamples = na_align(kNaLut + kLutPadded * sizeof(uint32_t));
-constexpr size_t kNaPartials = na_align(kNaSamples + kNaS * sizeof(uint32_t));
+constexpr size_t kNaSpans = na_align(kNaSamples + kNaS * sizeof(uint32_t));
+constexpr size_t kNaPartials = na_align(kNaSpans + 2 * (kNaS / 1024) * sizeof(uint32_t));
 constexpr size_t kNaCounts = na_align(kNaPartials + (size_t)kNaMaxG * kNaNbMax * 4);
 constexpr size_t kNaTtot = na_align(kNaCounts + kNaNbMax * 4);
 constexpr size_t kNaSegBucket = na_align(kNaTtot + kNaNbMax / kScanTile * 4);
@@ -131,6 +132,7 @@ extern "C" int ggks_multiselect_noalloc_f32(const float *d_vec, uint64_t n, cons
   LutHeader<K> *hdr = reinterpret_cast<LutHeader<K> *>(A + kNaHdr);
   uint32_t *lut = reinterpret_cast<uint32_t *>(A + kNaLut);
   K *samples = reinterpret_cast<K *>(A + kNaSamples);
+  K *spans = reinterpret_cast<K *>(A + kNaSpans);
   uint32_t *partials = reinterpret_cast<uint32_t *>(A + kNaPartials);
   uint32_t *bpre = reinterpret_cast<uint32_t *>(A + kNaCounts);  // prefix inside 64-bucket tiles
   uint32_t *ttot = reinterpret_cast<uint32_t *>(A + kNaTtot);
@@ -166,12 +168,14 @@ extern "C" int ggks_multiselect_noalloc_f32(const float *d_vec, uint64_t n, cons
   if (e == cudaSuccess) e = set_smem_max<k_finish<K, float>>(finish_smem_bytes<float>());
   if (e != cudaSuccess) return from_cuda(e);
 
-  // the control block and the slice counts start at zero
-  e = cudaMemsetAsync(A + kNaCtrl, 0, kNaSliceCnt + kSliceCntBytes, s);
+  // the slice counts start at zero; k_sample clears the control block, so the
+  // requests' check of the k's comes after it
+  e = cudaMemsetAsync(A + kNaSliceCnt, 0, kSliceCntBytes, s);
   if (e != cudaSuccess) return from_cuda(e);
+  k_sample<float><<<(S + 1023) / 1024, 1024, 0, s>>>(d_vec, n, S, 0x5EEDu, samples, spans, ctrl,
+                                                     Ctrl{});
   k_na_reqs<<<(num_k + 255) / 256, 256, 0, s>>>(d_k, num_k, n, reqs, ctrl);
-  k_sample<float><<<(S + 1023) / 1024, 1024, 0, s>>>(d_vec, n, S, 0x5EEDu, samples, ctrl);
-  k_lut<K><<<(S + 1023) / 1024, 1024, 0, s>>>(samples, S, ctrl, hdr, lut, kNaNbMax,
+  k_lut<K><<<(S + 1023) / 1024, 1024, 0, s>>>(samples, S, spans, ctrl, hdr, lut, kNaNbMax,
                                                reinterpret_cast<uint32_t *>(A + kNaSliceCnt), n,
                                                0u, G);
   {
@@ -199,7 +203,7 @@ extern "C" int ggks_multiselect_noalloc_f32(const float *d_vec, uint64_t n, cons
     const int smem = finish_smem_bytes<float>();
     k_finish<K, float><<<fin_grid, kFinThreads, smem, s>>>(surv, ctrl, seg_off, seg_size, seg_lo,
                                                           seg_hi, kstart, kcnt, klist, deferred,
-                                                          cap_keys, d_out);
+                                                          cap_keys, d_out, nullptr);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return from_cuda(e);

@@ -53,7 +53,7 @@ struct Plan {
   uint32_t fin_grid = 0;
   uint64_t surv_cap = 0;
   // arena offsets
-  size_t out = 0, ctrl = 0, reqs = 0, hdr = 0, lut = 0, samples = 0, partials = 0,
+  size_t out = 0, ctrl = 0, reqs = 0, hdr = 0, lut = 0, samples = 0, spans = 0, partials = 0,
          bpre = 0, ttot = 0, seg_bucket = 0, seg_off = 0, seg_size = 0, kstart = 0, kcnt = 0, fill = 0,
          kcur = 0, seg_lo = 0, seg_hi = 0, deferred = 0, req_bucket = 0, req_local = 0, klist = 0,
          pm_bits = 0, pm_bcount = 0, pm_bslot = 0, cand_cnt = 0, cand_tab = 0, reps = 0,
@@ -63,7 +63,18 @@ struct Plan {
   uint64_t surv_half = 0;
   uint32_t cand_chunks = 0;
 };
-static_assert(sizeof(Ctrl) <= 256, "the control block travels in one 256-byte image");
+static_assert(sizeof(Ctrl) <= 256 && sizeof(Ctrl) % 4 == 0, "the control block's 256-byte slot");
+// Host k lists of at most kPinReq requests are read by the kernels from pinned
+// host memory (the plan CTA and the small-vector kernel load one per thread),
+// and at most kPinOut results are written there by the finishing kernels; the
+// control block goes up in k_sample's parameters and comes back by k_finish's
+// last CTA.  Such a call puts no copy on the stream.  More requests go up in a
+// copy (several kernels read them, several times), and more results come back
+// in one (their scattered 4- and 8-byte stores would cross the link one by one).
+// (2^20 floats, 101 k's: 72 -> 65 us a call; 5003 floats, 11 k's: 47 -> 43 us;
+// 10 M floats, 257 k's: 96 -> 91 us.)
+constexpr uint32_t kPinReq = 1024;
+constexpr uint32_t kPinOut = 4096;
 
 template <class InT, class OutT>
 static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req) {
@@ -122,6 +133,8 @@ static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req) {
   o = align_up(o + kLutPadded * sizeof(uint32_t), A);
   p.samples = o;
   o = align_up(o + (size_t)p.S * sizeof(K), A);
+  p.spans = o;
+  o = align_up(o + 2 * (size_t)p.sample_grid * sizeof(K), A);
   p.partials = o;
   o = align_up(o + (size_t)p.G * p.nb_max * sizeof(uint32_t), A);
   auto arr = [&](size_t &off, size_t elems, size_t esz) {
@@ -349,19 +362,19 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   Ctrl *ctrl = reinterpret_cast<Ctrl *>(A + p.ctrl);
   Kt *tau = reinterpret_cast<Kt *>(A + p.hdr);
   Kt *samples = reinterpret_cast<Kt *>(A + p.samples);
+  Kt *spans = reinterpret_cast<Kt *>(A + p.spans);
   uint32_t *slice_cnt = reinterpret_cast<uint32_t *>(A);
   Kt *arr = reinterpret_cast<Kt *>(ctx.surv);  // the candidate array
   const uint64_t arr_cap = p.surv_cap;
-  InT *d_out = d_out_user ? d_out_user : reinterpret_cast<InT *>(A + p.out);
+  InT *d_out = d_out_user;
+  // pinned: [out | status]
   const size_t out_span = p.ctrl - p.out;
-  e = ensure_pin(ctx, 256 + out_span + 256);
+  e = ensure_pin(ctx, out_span + 256);
   if (e != cudaSuccess) return from_cuda(e);
-  char *pin_up = ctx.pin;
-  char *pin_down = ctx.pin + 256;
-  Ctrl *h_ctrl = reinterpret_cast<Ctrl *>(pin_down + out_span);
-  std::memset(pin_up, 0, 256);  // a zeroed control block
-  e = cudaMemcpyAsync(ctrl, pin_up, 256, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return from_cuda(e);
+  const bool want_host = host_results != nullptr;
+  static_assert(kPickMax <= kPinOut, "k_pick writes its results in place");
+  if (!d_out_user) d_out = reinterpret_cast<InT *>(ctx.pin_dev);
+  const volatile uint32_t *h_status = reinterpret_cast<const uint32_t *>(ctx.pin + out_span);
   cudaError_t le = cudaSuccess;
   auto L = [&le](cudaError_t r) {
     if (le == cudaSuccess) le = r;
@@ -375,8 +388,9 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   {
     PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
     L(launch(k_sample<InT>, p.sample_grid, 1024, 0, s, ingest ? ingest : d_in, n, p.S, 0x5EEDu,
-             samples, ctrl));
-    L(launch(k_tau<Kt>, p.sample_grid, 1024, 0, s, samples, p.S, ctrl, slice_cnt, n, K, tau));
+             samples, spans, ctrl, Ctrl{}));
+    L(launch(k_tau<Kt>, p.sample_grid, 1024, 0, s, samples, p.S, spans, ctrl, slice_cnt, n, K,
+             tau));
     ctx.stats.launches++;
     ran[GGKS_PASS_SAMPLE] = true;
   }
@@ -390,30 +404,25 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   {
     PassTimer t(ctx, s, GGKS_PASS_FINISH);
     L(launch(k_pick<Kt, InT>, 1, 1024, pick_smem, s, arr, arr_cap, &ctrl->cand_next, tau, K,
-             d_out, ctrl));
+             d_out, ctrl, reinterpret_cast<uint32_t *>(ctx.pin_dev + out_span)));
     ran[GGKS_PASS_FINISH] = true;
   }
   e = le != cudaSuccess ? le : cudaGetLastError();
   if (e != cudaSuccess) return from_cuda(e);
-  const bool want_host = host_results != nullptr;
-  if (want_host && !d_out_user)
-    e = cudaMemcpyAsync(pin_down, A + p.out, out_span + sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
-  else
-    e = cudaMemcpyAsync(h_ctrl, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess && want_host && d_out_user)
-    e = cudaMemcpyAsync(pin_down, d_out, (size_t)K * sizeof(InT), cudaMemcpyDeviceToHost, s);
+  if (want_host && d_out_user)
+    e = cudaMemcpyAsync(ctx.pin, d_out, (size_t)K * sizeof(InT), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return from_cuda(e);
   collect_pass_times(ctx, ran);
-  const Ctrl c = *h_ctrl;
-  if (c.status & ST_FATAL) return (c.status & ST_TIMEOUT) ? GGKS_TIMEOUT : GGKS_INTERNAL;
-  if (c.status & ST_TOPK_MISS) {
+  const uint32_t status = *h_status;
+  if (status & ST_FATAL) return (status & ST_TIMEOUT) ? GGKS_TIMEOUT : GGKS_INTERNAL;
+  if (status & ST_TOPK_MISS) {
     *missed = true;
     ctx.stats.topk_misses++;
     return GGKS_OK;
   }
   ctx.stats.topk_threshold_calls++;
-  if (want_host) *host_results = reinterpret_cast<const InT *>(pin_down);
+  if (want_host) *host_results = reinterpret_cast<const InT *>(ctx.pin);
   return GGKS_OK;
 }
 
@@ -422,9 +431,8 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
 // (kSmMaxTopkN for a top-k) elements.
 // *missed: the kernel met a case it leaves to the pipeline (nothing is
 // answered; the caller runs the pipeline, which writes every output again).
-// Arena: [slice counts | out | ctrl | requests]: the control block and the
-// requests go up in one copy, the outputs and the control block come back in
-// one.
+// Arena: [slice counts | phase stamps | cursors' starts]; pinned host memory,
+// which the kernel reads and writes in place: [out | status | requests].
 template <class InT, class OutT>
 static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src,
                         uint32_t num_req, OutT *d_out_user, const OutT **host_results,
@@ -436,35 +444,34 @@ static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSour
     return GGKS_OK;
   }
   const size_t out_span = align_up((size_t)num_req * sizeof(OutT), 256);
-  const size_t o_out = kSliceCntBytes, o_ctrl = o_out + out_span, o_reqs = o_ctrl + 256;
-  const size_t o_chk = align_up(o_reqs + (size_t)num_req * sizeof(Req), 256);
-  const size_t up_bytes = 256 + (size_t)num_req * sizeof(Req);
+  const size_t o_ctrl = kSliceCntBytes, o_chk = o_ctrl + 256;
   cudaError_t e = ensure_arena(ctx, o_chk + (size_t)kSmNb * kSmCtas * sizeof(uint32_t));
   if (e == cudaSuccess) e = ensure_surv(ctx, (size_t)n * sizeof(K));
-  const size_t down_off = align_up(up_bytes, 256);
-  if (e == cudaSuccess) e = ensure_pin(ctx, down_off + out_span + 256);
+  if (e == cudaSuccess) e = ensure_pin(ctx, out_span + 256 + (size_t)num_req * sizeof(Req));
   if (e != cudaSuccess) return from_cuda(e);
   char *A = ctx.arena;
   Ctrl *ctrl = reinterpret_cast<Ctrl *>(A + o_ctrl);
-  OutT *d_out = d_out_user ? d_out_user : reinterpret_cast<OutT *>(A + o_out);
-  char *pin_up = ctx.pin;
-  char *pin_down = ctx.pin + down_off;
-  Ctrl *h_ctrl = reinterpret_cast<Ctrl *>(pin_down + out_span);
-  // every call ends with a stream synchronisation: no earlier copy still
-  // reads the pinned buffer
-  std::memset(pin_up, 0, 256);
-  Req *hr = reinterpret_cast<Req *>(pin_up + 256);
+  static_assert(kSmMaxReq <= kPinReq && kSmMaxReq <= kPinOut && kSmCtas * 4 <= 256,
+                "requests, results and status in place");
+  OutT *d_out = d_out_user ? d_out_user : reinterpret_cast<OutT *>(ctx.pin_dev);
+  const volatile uint32_t *h_status = reinterpret_cast<const uint32_t *>(ctx.pin + out_span);
+  // every call ends with a stream synchronisation: no earlier kernel still
+  // reads or writes the pinned buffer
+  Req *hr = reinterpret_cast<Req *>(ctx.pin + out_span + 256);
   for (uint32_t i = 0; i < num_req; ++i) {
     hr[i].rank = src.topk ? (uint32_t)(n - 1 - i) : (uint32_t)(n - src.h_k[i]);
     hr[i].out = i;
   }
-  e = cudaMemcpyAsync(ctrl, pin_up, up_bytes, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return from_cuda(e);
+#ifdef GGKS_SMALL_TIMING
+  cudaMemsetAsync(ctrl, 0, sizeof(Ctrl), s);
+#endif
   {
     PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
-    e = launch_small(k_small<InT, OutT>, s, d_in, n, reinterpret_cast<const Req *>(A + o_reqs),
-                     num_req, d_out, reinterpret_cast<K *>(ctx.surv), ctx.surv_bytes / sizeof(K),
-                     reinterpret_cast<uint32_t *>(A + o_chk), ctrl);
+    e = launch_small(k_small<InT, OutT>, s, d_in, n,
+                     reinterpret_cast<const Req *>(ctx.pin_dev + out_span + 256), num_req, d_out,
+                     reinterpret_cast<K *>(ctx.surv), ctx.surv_bytes / sizeof(K),
+                     reinterpret_cast<uint32_t *>(A + o_chk),
+                     reinterpret_cast<uint32_t *>(ctx.pin_dev + out_span), ctrl);
   }
   if (e != cudaSuccess) {
     // a cluster launch the device refuses (its SMs held by other work in a
@@ -474,25 +481,22 @@ static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSour
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices)
       small_state<InT, OutT>()[dev].store(2, std::memory_order_release);
-    e = cudaStreamSynchronize(s);  // the uploaded requests are no longer needed
-    if (e != cudaSuccess) return from_cuda(e);
     *missed = true;
     return GGKS_OK;
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return from_cuda(e);
   const bool want_host = host_results != nullptr;
-  if (want_host && !d_out_user)
-    e = cudaMemcpyAsync(pin_down, A + o_out, out_span + sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
-  else
-    e = cudaMemcpyAsync(h_ctrl, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess && want_host && d_out_user)
-    e = cudaMemcpyAsync(pin_down, d_out, (size_t)num_req * sizeof(OutT), cudaMemcpyDeviceToHost, s);
+  if (want_host && d_out_user)
+    e = cudaMemcpyAsync(ctx.pin, d_out, (size_t)num_req * sizeof(OutT), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return from_cuda(e);
   bool ran[GGKS_NUM_PASSES] = {true, false, false, false, false, false};
   collect_pass_times(ctx, ran);
 #ifdef GGKS_SMALL_TIMING
+  Ctrl tc;
+  const Ctrl *h_ctrl = &tc;
+  cudaMemcpy(&tc, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost);
   fprintf(stderr, "ggks small timing n=%llu req=%u:", (unsigned long long)n, num_req);
   // stamp order: 0 start, 1 sampled, 2 table, 3 histograms, 8 totals, 9 scan,
   // 10 barrier, 11 prefix, 12 requests, 13 cursors, 4 barrier, 5 compacted,
@@ -505,14 +509,15 @@ static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSour
           (double)(h_ctrl->t_ns[0] - ~h_ctrl->t_ns[14]) * 1e-3,
           (double)(h_ctrl->t_ns[15] - h_ctrl->t_ns[7]) * 1e-3);
 #endif
-  if (h_ctrl->status & ST_SMALL_MISS) {
+  uint32_t status = 0;
+  for (uint32_t c = 0; c < kSmCtas; ++c) status |= h_status[c];
+  if (status & ST_SMALL_MISS) {
     *missed = true;
     ctx.stats.small_misses++;
     return GGKS_OK;
   }
-  if (h_ctrl->status & ST_FATAL) return (h_ctrl->status & ST_TIMEOUT) ? GGKS_TIMEOUT : GGKS_INTERNAL;
   ctx.stats.small_calls++;
-  if (want_host) *host_results = reinterpret_cast<const OutT *>(pin_down);
+  if (want_host) *host_results = reinterpret_cast<const OutT *>(ctx.pin);
   return GGKS_OK;
 }
 
@@ -555,6 +560,7 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   LutHeader<K> *hdr = reinterpret_cast<LutHeader<K> *>(A + p.hdr);
   uint32_t *lut = reinterpret_cast<uint32_t *>(A + p.lut);
   K *samples = reinterpret_cast<K *>(A + p.samples);
+  K *spans = reinterpret_cast<K *>(A + p.spans);
   uint32_t *slice_cnt = reinterpret_cast<uint32_t *>(A);
   uint32_t *partials = reinterpret_cast<uint32_t *>(A + p.partials);
   uint32_t *bpre = reinterpret_cast<uint32_t *>(A + p.bpre);  // prefix inside 64-bucket tiles
@@ -579,43 +585,48 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   K *reps = reinterpret_cast<K *>(A + p.reps);
   uint32_t *bsingle = reinterpret_cast<uint32_t *>(A + p.bsingle);
   K *bkey = reinterpret_cast<K *>(A + p.bkey);
-  OutT *d_out = d_out_user ? d_out_user : reinterpret_cast<OutT *>(A + p.out);
-  const bool out_in_arena = d_out_user == nullptr;
-
-  // pinned staging: [ctrl image | host requests] up, [out | pad | ctrl] down
-  const size_t up_bytes = 256 + (src.h_k ? (size_t)num_req * sizeof(Req) : 0);
+  // pinned host memory: [out | control block | requests]
+  const bool want_host = host_results != nullptr;
+  const bool host_reqs = src.h_k || (src.topk && num_req <= kPinReq);
   const size_t out_span = p.ctrl - p.out;  // == align_up(num_req * sizeof(OutT), 256)
-  const size_t down_off = align_up(up_bytes, 256);
-  e = ensure_pin(ctx, down_off + out_span + 256);
+  e = ensure_pin(ctx, out_span + 256 + (host_reqs ? (size_t)num_req * sizeof(Req) : 0));
   if (e != cudaSuccess) return from_cuda(e);
-  char *pin_up = ctx.pin;
-  char *pin_down = ctx.pin + down_off;
-  Ctrl *h_ctrl = reinterpret_cast<Ctrl *>(pin_down + out_span);
-  // every call ends with a stream synchronisation, so no earlier copy still
-  // reads the pinned buffer here
-  std::memset(pin_up, 0, 256);
-  Ctrl *ci = reinterpret_cast<Ctrl *>(pin_up);
-  if (src.h_k) {
-    Req *hr = reinterpret_cast<Req *>(pin_up + 256);
+  Ctrl *h_ctrl = reinterpret_cast<Ctrl *>(ctx.pin + out_span);
+  Ctrl *h_ctrl_dev = reinterpret_cast<Ctrl *>(ctx.pin_dev + out_span);
+  const bool out_in_pin = !d_out_user && want_host && num_req <= kPinOut;
+  const bool out_in_arena = !d_out_user && !out_in_pin;
+  OutT *d_out = d_out_user    ? d_out_user
+                : out_in_pin ? reinterpret_cast<OutT *>(ctx.pin_dev)
+                             : reinterpret_cast<OutT *>(A + p.out);
+  Ctrl ci{};  // the control block's initial words
+  const Req *rq = src.d_reqs ? src.d_reqs : reqs;
+  if (host_reqs) {
+    // every call ends with a stream synchronisation, so nothing of an earlier
+    // one still reads the pinned buffer here
+    Req *hr = reinterpret_cast<Req *>(ctx.pin + out_span + 256);
     for (uint32_t i = 0; i < num_req; ++i) {
-      hr[i].rank = (uint32_t)(n - src.h_k[i]);
+      hr[i].rank = src.h_k ? (uint32_t)(n - src.h_k[i]) : (uint32_t)(n - 1 - i);
       hr[i].out = i;
     }
-    set_windows(ci, hr, num_req, n);
-  } else if (src.topk && num_req && (uint64_t)num_req <= n / 16) {
-    ci->spec_nwin = 1;
-    ci->spec_lo[0] = n - num_req;
-    ci->spec_hi[0] = n - 1;
+    if (src.h_k) set_windows(&ci, hr, num_req, n);
+    if (num_req <= kPinReq) {
+      rq = reinterpret_cast<const Req *>(ctx.pin_dev + out_span + 256);
+    } else {
+      e = cudaMemcpyAsync(reqs, hr, (size_t)num_req * sizeof(Req), cudaMemcpyHostToDevice, s);
+      if (e != cudaSuccess) return from_cuda(e);
+    }
   }
-  e = cudaMemcpyAsync(ctrl, pin_up, up_bytes, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return from_cuda(e);
-  const Req *rq = src.d_reqs ? src.d_reqs : reqs;
+  if (src.topk && num_req && (uint64_t)num_req <= n / 16) {
+    ci.spec_nwin = 1;
+    ci.spec_lo[0] = n - num_req;
+    ci.spec_hi[0] = n - 1;
+  }
   bool ran[GGKS_NUM_PASSES] = {false, false, false, false, false, false};
   cudaError_t le = cudaSuccess;  // the first failed launch
   auto L = [&le](cudaError_t r) {
     if (le == cudaSuccess) le = r;
   };
-  if (src.topk) {
+  if (src.topk && !host_reqs) {
     L(launch(k_make_topk_reqs, (num_req + 255) / 256, 256, 0, s, reqs, n, num_req));
     ctx.stats.launches++;
   }
@@ -624,8 +635,8 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   {
     PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
     L(launch(k_sample<InT>, p.sample_grid, 1024, 0, s, ingest ? ingest : d_in, n, p.S, 0x5EEDu,
-             samples, ctrl));
-    L(launch(k_lut<K>, p.sample_grid, 1024, 0, s, samples, p.S, ctrl, hdr, lut, p.nb_max,
+             samples, spans, ctrl, ci));
+    L(launch(k_lut<K>, p.sample_grid, 1024, 0, s, samples, p.S, spans, ctrl, hdr, lut, p.nb_max,
              slice_cnt, n, p.cand_chunks, p.G));
     ctx.stats.launches++;
     ran[GGKS_PASS_SAMPLE] = true;
@@ -701,7 +712,7 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
       L(set_smem_max<k_finish<K, OutT>>(smem));
       PassTimer t(ctx, s, GGKS_PASS_FINISH);
       L(launch(k_finish<K, OutT>, p.fin_grid, kFinThreads, smem, s, surv, ctrl, seg_off, seg_size,
-               seg_lo, seg_hi, kstart, kcnt, klist, deferred, p.cap_keys, d_out));
+               seg_lo, seg_hi, kstart, kcnt, klist, deferred, p.cap_keys, d_out, h_ctrl_dev));
       ran[GGKS_PASS_FINISH] = true;
     }
   };
@@ -709,19 +720,14 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   e = le != cudaSuccess ? le : cudaGetLastError();
   if (e != cudaSuccess) return from_cuda(e);
 
-  // results and control block come back in one copy when the output is ours
+  // k_finish leaves the control block (and few results) in pinned memory
   auto pull = [&](bool with_out) -> cudaError_t {
-    cudaError_t r;
-    if (with_out && out_in_arena)
-      r = cudaMemcpyAsync(pin_down, A + p.out, out_span + sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
-    else
-      r = cudaMemcpyAsync(h_ctrl, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
-    if (r == cudaSuccess && with_out && !out_in_arena)
-      r = cudaMemcpyAsync(pin_down, d_out, (size_t)num_req * sizeof(OutT), cudaMemcpyDeviceToHost, s);
-    if (r != cudaSuccess) return r;
-    return cudaStreamSynchronize(s);
+    cudaError_t r = cudaSuccess;
+    if (with_out && !out_in_pin)
+      r = cudaMemcpyAsync(ctx.pin, out_in_arena ? reinterpret_cast<const OutT *>(A + p.out) : d_out,
+                          (size_t)num_req * sizeof(OutT), cudaMemcpyDeviceToHost, s);
+    return r != cudaSuccess ? r : cudaStreamSynchronize(s);
   };
-  const bool want_host = host_results != nullptr;
   e = pull(want_host);
   if (e != cudaSuccess) return from_cuda(e);
   collect_pass_times(ctx, ran);
@@ -787,7 +793,7 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   ctx.stats.survivors += h_ctrl->total_surv;
   ctx.stats.spec_calls += h_ctrl->spec_on;
   ctx.stats.spec_ctas += h_ctrl->spec_ctas;
-  if (want_host) *host_results = reinterpret_cast<const OutT *>(pin_down);
+  if (want_host) *host_results = reinterpret_cast<const OutT *>(ctx.pin);
   return GGKS_OK;
 }
 

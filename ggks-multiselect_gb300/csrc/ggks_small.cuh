@@ -36,7 +36,7 @@
 //
 // Anything this layout does not cover -- a bucket whose needed bins do not fit
 // (finish_slot asks for a recursive level), cursors that did not reach their
-// ends (the input changed between the passes) -- sets ST_SMALL_MISS and the
+// ends (the input changed between the passes) -- reports ST_SMALL_MISS and the
 // host runs the pipeline instead; the outputs are then written again.  Every
 // CTA passes every cluster barrier (no early exit), and no CTA reads another's
 // shared memory after the last barrier.
@@ -169,13 +169,16 @@ __device__ __forceinline__ void bitonic_merge_smem(K *s, uint32_t P) {
 // any n below 2^31); reqs: num_req requests
 // (ascending 0-based rank, output index; num_req <= kSmMaxReq); out: outputs;
 // surv: survivor buffer of surv_cap >= n keys; chk: kSmNb * kSmCtas words
-// (each requested bucket's first cursors, for the check); ctrl: status.
-// Launched as one cluster of kSmCtas CTAs of kSmThreads threads.
+// (each requested bucket's first cursors, for the check); host_status: kSmCtas
+// words, every CTA writes its own (0 or ST_SMALL_MISS).  reqs, out and
+// host_status may lie in host memory (read and written in place: the launch is
+// the call's only operation on the stream).  ctrl: phase stamps, in
+// GGKS_SMALL_TIMING builds.  Launched as one cluster of kSmCtas CTAs of kSmThreads threads.
 template <class T, class OutT>
 __global__ void __launch_bounds__(kSmThreads, 1)
     k_small(const T *__restrict__ x, uint64_t n, const Req *__restrict__ reqs, uint32_t num_req,
             OutT *__restrict__ out, typename Traits<T>::K *__restrict__ surv, uint64_t surv_cap,
-            uint32_t *__restrict__ chk, Ctrl *ctrl) {
+            uint32_t *__restrict__ chk, uint32_t *__restrict__ host_status, Ctrl *ctrl) {
   namespace cg = cooperative_groups;
   using K = typename Traits<T>::K;
   cg::cluster_group cl = cg::this_cluster();
@@ -467,7 +470,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
              s_nlarge, mxl, ctot);
   }
 #endif
-  if (tid == 0 && s_miss) atomicOr(&ctrl->status, ST_SMALL_MISS);
+  if (tid == 0) host_status[r] = s_miss ? ST_SMALL_MISS : 0u;
 }
 
 }  // namespace ggks

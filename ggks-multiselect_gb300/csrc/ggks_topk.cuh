@@ -24,7 +24,7 @@
 //             and the K largest out in descending order.
 // Correctness never rests on the prediction: k_pick checks that every
 // candidate was kept and that there are at least K, and that the gathered
-// keys fit; else it flags ST_TOPK_MISS and the caller runs the pipeline.
+// keys fit; else it reports ST_TOPK_MISS and the caller runs the pipeline.
 #pragma once
 
 #include <type_traits>
@@ -41,11 +41,12 @@ constexpr uint32_t kTauBuf = 2048;      // samples of the threshold's fine slice
 // ---------------------------------------------------------------------------
 // k_tau: the threshold from the sample
 // ---------------------------------------------------------------------------
-// Grid: ceil(S / 1024) CTAs of 1024 threads, after k_sample (span in Ctrl).
+// Grid: ceil(S / 1024) CTAs of 1024 threads, after k_sample (spans).
 // slice_cnt (global, kLutIdx words) is zero on entry and left zero.  The last
 // CTA writes tau (0: no useful threshold, which the caller treats as a miss).
 template <class K>
-__global__ void __launch_bounds__(1024) k_tau(const K *__restrict__ samples, uint32_t S, Ctrl *ctrl,
+__global__ void __launch_bounds__(1024) k_tau(const K *__restrict__ samples, uint32_t S,
+                                              const K *__restrict__ spans, Ctrl *ctrl,
                                               uint32_t *slice_cnt, uint64_t n, uint32_t kk,
                                               K *tau) {
   pdl_start();
@@ -58,8 +59,8 @@ __global__ void __launch_bounds__(1024) k_tau(const K *__restrict__ samples, uin
   const uint32_t i = blockIdx.x * blockDim.x + tid;
   for (uint32_t j = tid; j < kLutIdx; j += blockDim.x) ccnt[j] = 0;
   const K k = i < S ? __ldcg(samples + i) : K(0);
-  const K kmin = (K)~__ldcg((const unsigned long long *)&ctrl->kmin_inv);
-  const K kmax = (K)__ldcg((const unsigned long long *)&ctrl->kmax);
+  K kmin, kmax;
+  sample_span<K>(spans, gridDim.x, &kmin, &kmax);
   const int bl = bitlen<K>(kmax - kmin);
   const uint32_t fsh = bl > kLutIdxBits ? (uint32_t)(bl - kLutIdxBits) : 0u;
   __syncthreads();
@@ -336,7 +337,10 @@ __global__ void __launch_bounds__(1024, 1)
 // (coalesced reads).  When C fits the stage (kStage keys) the candidates are
 // copied into shared memory once and every later pass reads them there.
 // Dynamic shared memory: the histogram and the bins' offsets (kPickBins words
-// each), the stage and the sort buffer (kPickCap keys).  out[i] = the (i + 1)-th largest, i < kk.
+// each), the stage and the sort buffer (kPickCap keys).  out[i] = the (i + 1)-th
+// largest, i < kk.  The call's status (ctrl's, with ST_TOPK_MISS on a miss) goes
+// to *host_status, in host memory, as the outputs may: the host reads both after
+// the stream's synchronisation, no copy follows.
 template <class K>
 struct PickShape {
   static constexpr uint32_t kStage = sizeof(K) == 4 ? 36864u : 14336u;
@@ -351,7 +355,7 @@ __host__ __device__ constexpr size_t pick_smem_bytes() {
 template <class K, class OutT>
 __global__ void __launch_bounds__(1024, 1)
     k_pick(const K *__restrict__ arr, uint64_t cap, const uint32_t *len, const K *tau, uint32_t kk,
-           OutT *__restrict__ out, Ctrl *ctrl) {
+           OutT *__restrict__ out, const Ctrl *ctrl, uint32_t *host_status) {
   pdl_start();
   constexpr uint32_t kStage = PickShape<K>::kStage;
   extern __shared__ uint4 smem_raw[];
@@ -363,12 +367,14 @@ __global__ void __launch_bounds__(1024, 1)
   __shared__ K redk[33];
   __shared__ uint32_t s_j, s_above, s_cnt;
   const uint32_t tid = threadIdx.x, nt = blockDim.x;
-  if (ctrl->status & ST_FATAL) return;
+  const uint32_t status = ctrl->status;
+  if (tid == 0) *host_status = status;
+  if (status & ST_FATAL) return;
   const uint32_t C = __ldcg(len);
   const K t = *tau;
   for (uint32_t b = tid; b < kPickBins; b += nt) hist[b] = 0;
   if ((uint64_t)C > cap || C < kk) {  // candidates lost past the capacity, or too few
-    if (tid == 0) atomicOr(&ctrl->status, ST_TOPK_MISS);
+    if (tid == 0) *host_status = status | ST_TOPK_MISS;
     return;
   }
   const bool staged = C <= kStage;
@@ -444,7 +450,7 @@ __global__ void __launch_bounds__(1024, 1)
   const bool single = sh == 0;
   const uint32_t need = single ? above : above + in_j;
   if (need > kPickCap) {
-    if (tid == 0) atomicOr(&ctrl->status, ST_TOPK_MISS);
+    if (tid == 0) *host_status = status | ST_TOPK_MISS;
     return;
   }
   // Bins of at most kPickBinSort keys: each key goes to its bin's place in
