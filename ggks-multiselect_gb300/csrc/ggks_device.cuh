@@ -194,6 +194,7 @@ enum : uint32_t {
   ST_INTERNAL = 8u,  // a consistency check failed (counts do not add up to n)
   ST_BAD_K = 16u,    // a k outside [1, n] (device-side k lists)
   ST_TOPK_MISS = 32u,  // the threshold top-k's candidates fell short: run the pipeline
+  ST_SMALL_MISS = 64u,  // a one-launch kernel left the vector to the next larger path
 };
 constexpr uint32_t ST_FATAL = ST_TIMEOUT | ST_INTERNAL;
 

@@ -13,6 +13,7 @@
 
 #include "ggks_internal.h"
 #include "ggks_small.cuh"
+#include "ggks_tiny.cuh"
 #include "ggks_topk.cuh"
 
 namespace ggks {
@@ -426,7 +427,8 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   return GGKS_OK;
 }
 
-// A small vector in one launch (ggks_small.cuh): host k lists or a top-k of
+// A small vector in one launch (ggks_tiny.cuh: one CTA, where the vector fits
+// its registers; else ggks_small.cuh: one cluster): host k lists or a top-k of
 // at most kSmMaxReq requests on a device vector of at most kSmMaxN
 // (kSmMaxTopkN for a top-k) elements.
 // *missed: the kernel met a case it leaves to the pipeline (nothing is
@@ -439,18 +441,10 @@ static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSour
                         cudaStream_t s, bool *missed) {
   using K = typename Traits<InT>::K;
   *missed = false;
-  if (!small_ready<InT, OutT>()) {
-    *missed = true;
-    return GGKS_OK;
-  }
   const size_t out_span = align_up((size_t)num_req * sizeof(OutT), 256);
   const size_t o_ctrl = kSliceCntBytes, o_chk = o_ctrl + 256;
-  cudaError_t e = ensure_arena(ctx, o_chk + (size_t)kSmNb * kSmCtas * sizeof(uint32_t));
-  if (e == cudaSuccess) e = ensure_surv(ctx, (size_t)n * sizeof(K));
-  if (e == cudaSuccess) e = ensure_pin(ctx, out_span + 256 + (size_t)num_req * sizeof(Req));
+  cudaError_t e = ensure_pin(ctx, out_span + 256 + (size_t)num_req * sizeof(Req));
   if (e != cudaSuccess) return from_cuda(e);
-  char *A = ctx.arena;
-  Ctrl *ctrl = reinterpret_cast<Ctrl *>(A + o_ctrl);
   static_assert(kSmMaxReq <= kPinReq && kSmMaxReq <= kPinOut && kSmCtas * 4 <= 256,
                 "requests, results and status in place");
   OutT *d_out = d_out_user ? d_out_user : reinterpret_cast<OutT *>(ctx.pin_dev);
@@ -462,16 +456,60 @@ static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSour
     hr[i].rank = src.topk ? (uint32_t)(n - 1 - i) : (uint32_t)(n - src.h_k[i]);
     hr[i].out = i;
   }
+  const Req *d_reqs = reinterpret_cast<const Req *>(ctx.pin_dev + out_span + 256);
+  uint32_t *d_status = reinterpret_cast<uint32_t *>(ctx.pin_dev + out_span);
+  const bool want_host = host_results != nullptr;
+  // waits for the launch; statuses: words the kernel leaves in h_status
+  auto finish = [&](uint32_t statuses, bool *miss) -> int {
+    cudaError_t r = cudaGetLastError();
+    if (r == cudaSuccess && want_host && d_out_user)
+      r = cudaMemcpyAsync(ctx.pin, d_out, (size_t)num_req * sizeof(OutT), cudaMemcpyDeviceToHost,
+                          s);
+    if (r == cudaSuccess) r = cudaStreamSynchronize(s);
+    if (r != cudaSuccess) return from_cuda(r);
+    const bool ran[GGKS_NUM_PASSES] = {true, false, false, false, false, false};
+    collect_pass_times(ctx, ran);
+    uint32_t status = 0;
+    for (uint32_t c = 0; c < statuses; ++c) status |= h_status[c];
+    *miss = (status & ST_SMALL_MISS) != 0;
+    if (!*miss) {
+      ctx.stats.small_calls++;
+      if (want_host) *host_results = reinterpret_cast<const OutT *>(ctx.pin);
+    }
+    return GGKS_OK;
+  };
+  // A vector that fits the registers of one CTA: one CTA, unless a requested
+  // bin holds too many keys.
+  if (n <= tiny_max<K>()) {
+    const int smem = (int)tiny_smem_bytes<K>(n);
+    e = set_smem_max<k_tiny<InT, OutT>>((int)tiny_smem_bytes<K>(tiny_max<K>()));
+    if (e != cudaSuccess) return from_cuda(e);
+    {
+      PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
+      k_tiny<InT, OutT><<<1, kTinyThreads, smem, s>>>(d_in, (uint32_t)n, d_reqs, num_req, d_out,
+                                                      d_status);
+    }
+    bool miss = false;
+    const int st = finish(1, &miss);
+    if (st != GGKS_OK || !miss) return st;
+  }
+  if (!small_ready<InT, OutT>()) {
+    *missed = true;
+    return GGKS_OK;
+  }
+  e = ensure_arena(ctx, o_chk + (size_t)kSmNb * kSmCtas * sizeof(uint32_t));
+  if (e == cudaSuccess) e = ensure_surv(ctx, (size_t)n * sizeof(K));
+  if (e != cudaSuccess) return from_cuda(e);
+  char *A = ctx.arena;
+  Ctrl *ctrl = reinterpret_cast<Ctrl *>(A + o_ctrl);
 #ifdef GGKS_SMALL_TIMING
   cudaMemsetAsync(ctrl, 0, sizeof(Ctrl), s);
 #endif
   {
     PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
-    e = launch_small(k_small<InT, OutT>, s, d_in, n,
-                     reinterpret_cast<const Req *>(ctx.pin_dev + out_span + 256), num_req, d_out,
+    e = launch_small(k_small<InT, OutT>, s, d_in, n, d_reqs, num_req, d_out,
                      reinterpret_cast<K *>(ctx.surv), ctx.surv_bytes / sizeof(K),
-                     reinterpret_cast<uint32_t *>(A + o_chk),
-                     reinterpret_cast<uint32_t *>(ctx.pin_dev + out_span), ctrl);
+                     reinterpret_cast<uint32_t *>(A + o_chk), d_status, ctrl);
   }
   if (e != cudaSuccess) {
     // a cluster launch the device refuses (its SMs held by other work in a
@@ -484,15 +522,8 @@ static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSour
     *missed = true;
     return GGKS_OK;
   }
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return from_cuda(e);
-  const bool want_host = host_results != nullptr;
-  if (want_host && d_out_user)
-    e = cudaMemcpyAsync(ctx.pin, d_out, (size_t)num_req * sizeof(OutT), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return from_cuda(e);
-  bool ran[GGKS_NUM_PASSES] = {true, false, false, false, false, false};
-  collect_pass_times(ctx, ran);
+  const int st = finish(kSmCtas, missed);
+  if (st != GGKS_OK) return st;
 #ifdef GGKS_SMALL_TIMING
   Ctrl tc;
   const Ctrl *h_ctrl = &tc;
@@ -509,15 +540,7 @@ static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSour
           (double)(h_ctrl->t_ns[0] - ~h_ctrl->t_ns[14]) * 1e-3,
           (double)(h_ctrl->t_ns[15] - h_ctrl->t_ns[7]) * 1e-3);
 #endif
-  uint32_t status = 0;
-  for (uint32_t c = 0; c < kSmCtas; ++c) status |= h_status[c];
-  if (status & ST_SMALL_MISS) {
-    *missed = true;
-    ctx.stats.small_misses++;
-    return GGKS_OK;
-  }
-  ctx.stats.small_calls++;
-  if (want_host) *host_results = reinterpret_cast<const OutT *>(ctx.pin);
+  if (*missed) ctx.stats.small_misses++;
   return GGKS_OK;
 }
 

@@ -92,7 +92,6 @@ constexpr uint32_t kSmMaxReq = kSmThreads;        // one request per thread
 // even at 2^21); top-k up to 2^18 (the threshold path is faster above)
 constexpr uint64_t kSmMaxN = 1ull << 20;
 constexpr uint64_t kSmMaxTopkN = 1ull << 18;
-constexpr uint32_t ST_SMALL_MISS = 64u;           // run the pipeline instead
 
 // dynamic shared memory: the table's copies, then one word per bucket --
 // its count after the histogram phase, its compaction cursor after the plan
@@ -100,10 +99,12 @@ constexpr uint32_t ST_SMALL_MISS = 64u;           // run the pipeline instead
 // bucket words; the finishers' scratch (phase F) over both.
 constexpr size_t kSmHcOff = (size_t)kRepWords * 4;
 constexpr size_t kSmBytes = kSmHcOff + (size_t)kSmNb * 4;
-// a warp finisher's buffer: a warp sorts at most 256 four-byte keys (a
-// one-warp bitonic network over 1024 keys took about 30 us; larger segments
-// go to the whole-CTA finisher)
-constexpr uint32_t kSmWarpBytes = 1024;
+// a warp finisher's buffer: a warp sorts at most 512 four-byte or 256 eight-byte
+// keys (a one-warp bitonic network over 1024 keys took about 30 us; larger
+// segments go to the whole-CTA finisher, one after the other: with half these
+// keys, 2^20 normal doubles and 1001 k's took 143 us a call, now 92; floats 81,
+// now 78)
+constexpr uint32_t kSmWarpBytes = 2048;
 static_assert(kSmHcOff % 16 == 0, "bucket words' alignment");
 static_assert((size_t)small_samples<uint32_t>() * 4 <= kSmBytes - kSmHcOff, "samples fit");
 static_assert((size_t)small_samples<uint64_t>() * 8 <= kSmBytes - kSmHcOff, "samples fit");
@@ -403,6 +404,25 @@ __global__ void __launch_bounds__(kSmThreads, 1)
       const uint32_t size = size_of(t);
       const Req *rq = s_klist + s_kstart[t];
       const uint32_t m = s_kcnt[t];
+      // few-valued input (h.dup): copies of one key need no sort, one round of
+      // loads tells (2^18 floats of 256 values, 101 k's: 131 -> 67 us a call;
+      // on other input the check would cost 1 us a segment)
+      if (h.dup) {
+        const K first = __ldcg(surv + s_pre[t]);
+        bool same = true;
+        for (uint32_t j0 = tid; j0 < size; j0 += 4 * kSmThreads) {
+          K v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            v[u] = j0 + u * kSmThreads < size ? __ldcg(surv + s_pre[t] + j0 + u * kSmThreads) : first;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) same = same && v[u] == first;
+        }
+        if (__syncthreads_and(same)) {
+          for (uint32_t j = tid; j < m; j += kSmThreads) out[rq[j].out] = Traits<OutT>::value(first);
+          continue;
+        }
+      }
       if (size <= small_sort_cap<K>()) {
         // the whole segment, padded to a power of two with the largest key:
         // 32-key runs sorted in registers, then the CTA's bitonic merges
