@@ -11,22 +11,6 @@
 namespace ggks {
 
 // ---------------------------------------------------------------------------
-// small kernels owned by this unit
-// ---------------------------------------------------------------------------
-// top-k requests: output i receives the (i+1)-th largest, i.e. ascending rank
-// n-1-i (multiselectTimingFunctions.cu:207-209 builds k = 1..K for this)
-__global__ void k_make_topk_reqs(Req *reqs, uint64_t n, uint32_t K) {
-  pdl_start();
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < K) {
-    Req r;
-    r.rank = (uint32_t)(n - 1 - i);
-    r.out = i;
-    reqs[i] = r;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // context and workspace
 // ---------------------------------------------------------------------------
 int from_cuda(cudaError_t e) {
@@ -76,13 +60,7 @@ int context_init(Context &ctx, int device) {
   return from_cuda(e);
 }
 
-// zero: clear the new buffer on `stream` (the stream that uses it), so that
-// the clearing is ordered before that stream's work; a plain cudaMemset would
-// go to the legacy default stream, which a non-blocking stream does not wait
-// for, and could land in the middle of a call while other work keeps the
-// default stream busy.
-static cudaError_t grow(void **p, size_t *have, size_t need, bool zero,
-                        cudaStream_t stream = nullptr) {
+static cudaError_t grow(void **p, size_t *have, size_t need) {
   if (need <= *have && *p) return cudaSuccess;
   size_t want = need + need / 4 + 4096;
   if (*p) {
@@ -96,17 +74,15 @@ static cudaError_t grow(void **p, size_t *have, size_t need, bool zero,
     return e;
   }
   *have = want;
-  if (zero) e = cudaMemsetAsync(*p, 0, want, stream);
-  return e;
+  return cudaSuccess;
 }
 
 cudaError_t ensure_arena(Context &ctx, size_t bytes) {
-  // the arena's head holds state that must start zeroed (slice counts)
   if (bytes <= ctx.arena_bytes && ctx.arena) return cudaSuccess;
   cudaError_t e = cudaStreamSynchronize(ctx.stream);
   if (e != cudaSuccess) return e;
   void *p = ctx.arena;
-  e = grow(&p, &ctx.arena_bytes, bytes, true, ctx.stream);
+  e = grow(&p, &ctx.arena_bytes, bytes);
   ctx.arena = static_cast<char *>(p);
   return e;
 }
@@ -116,7 +92,7 @@ cudaError_t ensure_buffer(Context &ctx, char **p, size_t *have, size_t bytes) {
   cudaError_t e = cudaStreamSynchronize(ctx.stream);
   if (e != cudaSuccess) return e;
   void *v = *p;
-  e = grow(&v, have, bytes, false);
+  e = grow(&v, have, bytes);
   *p = static_cast<char *>(v);
   return e;
 }
@@ -142,14 +118,14 @@ cudaError_t ensure_surv(Context &ctx, size_t bytes) {
   if (bytes <= ctx.surv_bytes && ctx.surv) return cudaSuccess;
   cudaError_t e = cudaStreamSynchronize(ctx.stream);
   if (e != cudaSuccess) return e;
-  return grow(&ctx.surv, &ctx.surv_bytes, bytes, false);
+  return grow(&ctx.surv, &ctx.surv_bytes, bytes);
 }
 
 cudaError_t ensure_dvec(Context &ctx, size_t bytes) {
   if (bytes <= ctx.dvec_bytes && ctx.dvec) return cudaSuccess;
   cudaError_t e = cudaStreamSynchronize(ctx.stream);
   if (e != cudaSuccess) return e;
-  return grow(&ctx.dvec, &ctx.dvec_bytes, bytes, false);
+  return grow(&ctx.dvec, &ctx.dvec_bytes, bytes);
 }
 
 cudaError_t ensure_pin(Context &ctx, size_t bytes) {

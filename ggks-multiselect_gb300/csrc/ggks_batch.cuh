@@ -78,7 +78,10 @@ static_assert(((1u << b_slice_bits<uint64_t>()) + 1) * sv_copies<uint64_t>() <= 
               "the table's copies fit their shared memory");
 // shared-memory words in front of the tile phases' histogram / cursors
 constexpr uint32_t kBTileLut = kBRepLut > kLutPadded ? kBRepLut : kLutPadded;
-constexpr int kBSpt = (int)kLutIdx / kBThreads;  // slices per thread in the table build
+template <class K>
+__host__ __device__ constexpr int kBSpt() {  // slices per thread in the table build
+  return ((1 << b_slice_bits<K>()) + kBThreads - 1) / kBThreads;
+}
 constexpr uint32_t kBMaxNb = 8192;               // bucket budget of one problem
 constexpr uint32_t kBMaxS = 8192;                // samples of one problem (shared memory)
 constexpr int kBPhases = 5;
@@ -677,8 +680,8 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
 #endif
     if (!BCHECK(P.lut_off + (1u << P.nsl_bits) < A.lut_words && P.S <= kBMaxS, 1, p, P.lut_off))
       continue;
-    build_lut_cta<K, kBSpt, true>(samples, P.S, lo, hi, P.nb_max, A.luts + P.lut_off, &s_hdr,
-                                  (int)P.nsl_bits);
+    build_lut_cta<K, kBSpt<K>()>(samples, P.S, lo, hi, P.nb_max, A.luts + P.lut_off, &s_hdr,
+                                 (int)P.nsl_bits);
     __syncthreads();
     // Speculation: the window's ends as sample ranks, moved outwards by four
     // standard deviations of the number of sampled chunks below them

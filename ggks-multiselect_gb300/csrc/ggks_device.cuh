@@ -5,11 +5,11 @@
 //
 //   (a) keys      order-preserving float/double -> uint key map
 //                 (keyConversion.cu:9-23), applied on load, never stored.
-//   (b) sample    k_sample + k_lut: S pseudo-random keys are gathered; the
-//                 last CTA builds a range-adaptive splitter table (LUT) from them:
-//                 4096 equal-width slices of the sample's key span, each
+//   (b) sample    k_sample, k_bin, k_table (ggks_front.cuh): S pseudo-random
+//                 keys give a range-adaptive splitter table (LUT):
+//                 equal-width slices of the sample's key span, each
 //                 slice cut into 2^b sub-buckets with b chosen from the
-//                 slice's sample count, so that buckets hold about equal
+//                 slice's samples, so that buckets hold about equal
 //                 numbers of elements.  Keys below / above the sample span go
 //                 to open-ended edge buckets, so no min/max pass is needed.
 //                 Replaces the reference's minmax + 1024-sample 17-pivot /
@@ -85,7 +85,7 @@ constexpr int kMaxSubBits = 15;
 //     binade.  A pass over 8-byte keys has half the lookups per byte, so their
 //     extra wavefronts (eight lanes on eight banks per copy) are affordable.
 // The sample is binned in 2^12 fine slices, which place the speculative
-// windows (see build_lut_cta).
+// windows (see k_table).
 template <class K>
 __host__ __device__ constexpr int sv_bits() {
   return sizeof(K) == 4 ? 9 : 12;
@@ -204,15 +204,14 @@ struct Req {
   uint32_t out;
 };
 
-// Device control block (lives in the workspace; k_sample, the call's first
-// kernel, sets every word of it).
+// Device control block (lives in the workspace; the call's first kernel,
+// k_sample, sets every word of it).
 struct Ctrl {
   uint32_t status;
   uint32_t num_slots;
   uint64_t total_surv;
   uint32_t deferred_count;
-  uint32_t sample_done;    // last-CTA ticket of k_lut (reset by that CTA)
-  uint32_t same_key;       // far-apart sample pairs holding one key (k_lut)
+  uint32_t same_key;     // far-apart sample pairs holding one key (k_bin)
   uint32_t nb;             // buckets in use
   uint64_t cap_needed;
   // rank windows of the call's requests, set by the host (0 windows: the
@@ -220,7 +219,7 @@ struct Ctrl {
   uint32_t spec_nwin;
   uint32_t spec_pad;
   uint64_t spec_lo[2], spec_hi[2];  // ascending 0-based ranks, inclusive
-  uint32_t spec_on;    // the table keeps candidate buckets (k_lut)
+  uint32_t spec_on;    // the table keeps candidate buckets (k_table)
   uint32_t spec_ctas;  // compaction CTAs that read candidates
   uint32_t cand_next;  // candidate chunks handed out (k_hist)
   uint32_t fin_done;   // last-CTA ticket of k_finish
@@ -241,14 +240,6 @@ struct LutHeader {
   uint32_t cand_cap;
   uint32_t spec_lo[2];
   uint32_t spec_len[2];
-};
-
-// Inputs of the candidate-window computation (k_lut's last CTA).
-struct SpecArgs {
-  const Ctrl *ctrl;     // spec_nwin, spec_lo, spec_hi
-  uint64_t n;           // elements of the vector
-  uint32_t cand_cap;    // candidate chunks in the pool (0: off)
-  uint32_t G;           // histogram CTAs
 };
 
 template <class K>
@@ -613,325 +604,211 @@ __device__ __forceinline__ V block_reduce(V v, Op op, V *sh /* >= 32 */) {
 }
 
 // ---------------------------------------------------------------------------
-// (b) sample + splitter table
+// (b) splitter table
 // ---------------------------------------------------------------------------
-// Grid: ceil(S / 1024) CTAs of 1024 threads.  Every thread gathers one key;
-// each CTA folds its min / max into Ctrl with one atomic each; the last CTA to
-// finish counts the samples per slice and builds the table.
-//
 // Allocation: a slice with c samples gets 2^b sub-buckets,
 // b = clamp(ceil(log2 c) - t, 0, min(shift, 15, 24 - slice bits)), and empty
-// slices merge into one bucket per run.  The smallest threshold t whose bucket total fits nb_max
-// is found from a histogram of ceil(log2 c) over the slices, so each candidate
-// t costs a 33-term sum on one thread.
-// Builds the splitter table of one problem from its S sampled keys (kmin /
-// kmax: the sample's extremes) with one whole CTA of 4096 / SPT threads; the
-// table goes to lut[0 .. nsl] with nsl = 2^nsl_bits slices (nb_max >= nsl + 2
-// makes every threshold feasible), and thread 0 writes the header.  The
-// samples are in shared memory (SMEM) or in global memory written by other
-// CTAs (read past L1).
-//
-// pre_cnt (global, kLutIdx words): the samples already binned in 2^12 fine
-// slices of the span ((key - kmin) >> fine shift, fine shift = bit length of
-// the span - 12, at least 0); every slice is a run of 2^fold fine slices.
-// With pre_cnt a slice's sub-buckets follow its peak density -- its largest
-// fine count times 2^fold, in place of its count -- so that a slice whose
-// keys crowd into part of its range (the slice holding the sampled maximum,
-// whose keys stop there; a steep stretch of a distribution) gets buckets as
-// narrow as its densest part needs.
-// fine (shared, kLutIdx words, with pre_cnt only): lent by the caller to keep
-// the fine counts, which place the speculative windows (sp) at fine-slice
-// precision; without it no window is computed.
-template <class K, int SPT, bool SMEM>
-__device__ void build_lut_cta(const K *samples, uint32_t S, K kmin, K kmax, uint32_t nb_max,
-                              uint32_t *lut, LutHeader<K> *hdr, int nsl_bits = kLutIdxBits,
-                              uint32_t *pre_cnt = nullptr, int64_t pre_same_key = -1,
-                              const SpecArgs *sp = nullptr, uint32_t dup_cap = 0,
-                              uint32_t *fine = nullptr) {
-  __shared__ uint32_t cnt[kLutIdx];
-  __shared__ uint32_t lch[36];  // [0, 33): slices by ceil(log2 c); [34]: empty-run starts
-  __shared__ uint32_t red32[33];
-  __shared__ int s_t, s_r0;
-  __shared__ uint32_t s_tot[54];
-  __shared__ uint32_t s_cost[34];
-  const uint32_t tid = threadIdx.x;
-  const uint32_t nsl = 1u << nsl_bits;
-  // A caller that tracks single-key buckets (dup_cap) needs at most dup_cap
-  // buckets when keys repeat often; the counted far-apart pairs tell that
-  // before the table exists (with nb_max >= the final bucket count, this test
-  // holds whenever the table's dup flag will).
-  if (dup_cap && pre_same_key >= 0 && S >= 256 &&
-      (uint64_t)pre_same_key * nb_max >= (S / 2 < 4096u ? S / 2 : 4096u) && nb_max > dup_cap)
-    nb_max = dup_cap;
-  const int bl = bitlen<K>(kmax - kmin);
-  const uint32_t shift = bl > nsl_bits ? (uint32_t)(bl - nsl_bits) : 0u;
-  const uint32_t fsh = bl > kLutIdxBits ? (uint32_t)(bl - kLutIdxBits) : 0u;  // fine slices
-  const uint32_t fold = shift - fsh;  // a slice is 2^fold fine slices
-  int bcap = (int)(shift < (uint32_t)kMaxSubBits ? shift : (uint32_t)kMaxSubBits);
-  if (bcap > 24 - nsl_bits) bcap = 24 - nsl_bits;
+// slices merge into one bucket per run.  The smallest threshold t whose bucket
+// total fits nb_max is found from a histogram of ceil(log2 c) over the slices.
+// The rounding to powers of two leaves part of the budget unused: it goes to
+// the slices whose buckets are expected to be the fullest.
 
-  // --- sample counts per slice: counted by the caller in fine slices
-  // (pre_cnt, global, left zero here for the next call), or from the samples
-  if (tid < 36) lch[tid] = 0;
-  if (pre_cnt) {
-    for (uint32_t j = tid; j < nsl; j += blockDim.x) cnt[j] = 0;
-    __syncthreads();
-    for (uint32_t j0 = tid; j0 < kLutIdx; j0 += 4 * blockDim.x) {
-      uint32_t c4[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t j = j0 + u * blockDim.x;
-        c4[u] = j < kLutIdx ? __ldcg(pre_cnt + j) : 0u;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t j = j0 + u * blockDim.x;
-        if (j < kLutIdx) {
-          if (fine) fine[j] = c4[u];
-          if (c4[u] && (j >> fold) < nsl) atomicMax(&cnt[j >> fold], c4[u] << fold);
-          pre_cnt[j] = 0;
-        }
-      }
-    }
-    __syncthreads();
-  } else {
-    for (uint32_t j = tid; j < kLutIdx; j += blockDim.x) cnt[j] = 0;
-    __syncthreads();
-  }
-  // 16 loads per thread in flight before their atomics (loads and shared
-  // atomics interleaved in one loop body complete one at a time)
-  for (uint32_t s0 = tid; s0 < (pre_cnt ? 0u : S); s0 += 16 * blockDim.x) {
-    K kk[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const uint32_t s = s0 + u * blockDim.x;
-      kk[u] = s < S ? (SMEM ? samples[s] : __ldcg(samples + s)) : kmin;
-    }
-#pragma unroll
-    for (int u = 0; u < 16; ++u)
-      if (s0 + u * blockDim.x < S) atomicAdd(&cnt[(uint32_t)((kk[u] - kmin) >> shift)], 1u);
-  }
+// one block barrier per scan: every warp sums the warps before it for itself
+// (buf: 32 shared words, not reused before another barrier)
+__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *buf, uint32_t *total) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t incl = warp_incl_scan(v);
+  if (lane == 31) buf[warp] = incl;
   __syncthreads();
+  const uint32_t w = warp_incl_scan(lane < (blockDim.x >> 5) ? buf[lane] : 0u);
+  *total = __shfl_sync(0xffffffffu, w, 31);
+  const uint32_t before = __shfl_sync(0xffffffffu, w, warp ? warp - 1 : 0);
+  return incl - v + (warp ? before : 0u);
+}
 
-  // Each thread owns SPT consecutive slices [SPT tid, SPT tid + SPT) (those at
-  // or beyond nsl are unused); the top entry (keys above the sampled span) is
-  // written by thread 0 after the scan.
-  int lc[SPT];
+struct TableShared {
+  uint32_t lch[34];   // slices by ceil(log2 c); [33]: empty-run starts
+  uint32_t cost[33];  // buckets that doubling the slices of each fullness costs
+  uint32_t tot[64];   // bucket total of each threshold
+  uint32_t scan[32];
+  int t;
+};
+__device__ __forceinline__ void table_init(TableShared &ts) {  // then a block barrier
+  if (threadIdx.x < 34) ts.lch[threadIdx.x] = 0;
+  if (threadIdx.x < 33) ts.cost[threadIdx.x] = 0;
+  if (threadIdx.x == 0) ts.t = 33;  // total(33) <= 1 + nsl + 1 <= nb_max: always feasible
+}
+
+// Builds the table of nsl <= SPT * blockDim.x slices of width 2^shift from
+// density(j), the samples of slice j (any measure of them), with the whole
+// CTA: the nsl entries go to lut (global or shared memory) and to tab (shared;
+// may be lut), ordered by the caller's next block barrier.  bcap: largest b.
+// Returns the buckets in use; *top: the entry of the keys above the span.
+// A decision that one thread could take alone in a loop is taken by a warp, or
+// by every warp for itself where that saves a block barrier.
+template <class K, int SPT, class D>
+__device__ __forceinline__ uint32_t build_table(D &&density, uint32_t nsl, uint32_t shift, int bcap,
+                                                uint32_t nb_max, uint32_t *lut, uint32_t *tab,
+                                                TableShared &ts, uint32_t *top) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // this thread's slices [SPT tid, SPT tid + SPT)
   uint32_t c[SPT];
   bool prev_nonempty[SPT];
+  int lc[SPT];
 #pragma unroll
-  for (int q = 0; q < SPT; ++q) {
-    const uint32_t j = SPT * tid + q;
-    const bool in = j < nsl;
-    c[q] = in ? cnt[j] : 0u;
-    lc[q] = c[q] ? (c[q] == 1 ? 0 : 32 - __clz(c[q] - 1)) : -1;  // ceil(log2 c)
-    prev_nonempty[q] = in && ((j == 0) ? true : (cnt[j - 1] != 0));
-    if (c[q])
-      atomicAdd(&lch[lc[q]], 1u);
-    else if (prev_nonempty[q])
-      atomicAdd(&lch[34], 1u);
-  }
-  const bool top_run_start = cnt[nsl - 1] != 0;
-  if (tid == 0) s_t = 33;  // total(33) <= 1 + nsl + 1 <= nb_max: always feasible
-  if (tid < 34) s_cost[tid] = 0;
-  __syncthreads();
-  if (tid < 54) {
-    // smallest t with total(t) <= nb_max; one candidate t per thread
-    const int t = -kMaxSubBits - 1 + (int)tid;
-    uint64_t tot = 1u + lch[34] + (top_run_start ? 1u : 0u);
-    for (int l = 0; l < 33; ++l) {
-      int b = l - t;
-      b = b < 0 ? 0 : (b > bcap ? bcap : b);
-      tot += (uint64_t)lch[l] << b;
+  for (int q = 0; q < SPT; ++q) c[q] = SPT * tid + q < nsl ? density(SPT * tid + q) : 0u;
+  {
+    uint32_t before = __shfl_up_sync(0xffffffffu, c[SPT - 1], 1);
+    if (lane == 0) before = tid && SPT * tid < nsl ? density(SPT * tid - 1) : 1u;
+#pragma unroll
+    for (int q = 0; q < SPT; ++q) {
+      prev_nonempty[q] = (q ? c[q - 1] : before) != 0;
+      lc[q] = c[q] ? (c[q] == 1 ? 0 : 32 - __clz(c[q] - 1)) : -1;  // ceil(log2 c)
+      if (SPT * tid + q < nsl) {
+        if (c[q])
+          atomicAdd(&ts.lch[lc[q]], 1u);
+        else if (prev_nonempty[q])
+          atomicAdd(&ts.lch[33], 1u);
+      }
     }
-    s_tot[tid] = (uint32_t)(tot < 0xFFFFFFFFull ? tot : 0xFFFFFFFFull);
-    if (tot <= nb_max) atomicMin(&s_t, t);
+  }
+  const bool top_run_start = density(nsl - 1) != 0;
+  __syncthreads();
+  // smallest threshold t whose bucket total fits (totals stay below 2^12 << 15):
+  // a lane of two warps per candidate, the totals falling with t
+  if (tid < 64) {
+    const int t = -kMaxSubBits - 1 + (int)tid;
+    uint32_t v = 1u + ts.lch[33] + (top_run_start ? 1u : 0u);
+#pragma unroll
+    for (int l = 0; l < 33; ++l) {
+      const int b = l - t;
+      v += ts.lch[l] << (b < 0 ? 0 : (b > bcap ? bcap : b));
+    }
+    ts.tot[tid] = v;
+    const uint32_t fits = __ballot_sync(0xffffffffu, v <= nb_max);
+    if (lane == 0 && fits) atomicMin(&ts.t, t + __ffs(fits) - 1);
   }
   __syncthreads();
-  const int t = s_t;
-  const uint32_t spare = nb_max - s_tot[t + kMaxSubBits + 1];
-
-  // Power-of-two rounding leaves part of the budget unused.  Spend it on the
-  // slices whose buckets are expected to be the fullest: r = 32 * (samples per
-  // bucket) / 2^t in [0, 32]; doubling slice j's buckets costs 2^b_j.  The
-  // largest r first, as long as the whole bin of r fits.
+  const int t = ts.t;
+  const uint32_t spare = nb_max - ts.tot[t + kMaxSubBits + 1];
+  // the fullness of the slice's buckets, r = 32 * (samples per bucket) / 2^t in
+  // [0, 32]; the largest r first, as long as a whole bin of r fits (doubling
+  // slice j's buckets costs 2^b_j)
   int bq[SPT];
   uint32_t rq[SPT];
 #pragma unroll
   for (int q = 0; q < SPT; ++q) {
-    int b = lc[q] - t;
+    const int b = lc[q] - t;
     bq[q] = b < 0 ? 0 : (b > bcap ? bcap : b);
     rq[q] = 0xFFFFFFFFu;  // not a candidate
     if (c[q] && bq[q] < bcap) {
       const int e = bq[q] + t - 5;  // r = c * 32 / 2^(b + t)
-      uint32_t r = e >= 0 ? (e >= 32 ? 0u : c[q] >> e) : (-e >= 32 ? 32u : c[q] << (-e));
+      const uint32_t r = e >= 0 ? (e >= 32 ? 0u : c[q] >> e) : (-e >= 32 ? 32u : c[q] << (-e));
       rq[q] = r > 32u ? 32u : r;
-      atomicAdd(&s_cost[rq[q]], 1u << bq[q]);
+      atomicAdd(&ts.cost[rq[q]], 1u << bq[q]);
     }
   }
   __syncthreads();
-  if (tid == 0) {
-    uint32_t acc = 0;
-    int r0 = 33;
-    for (int r = 32; r >= 0; --r) {
-      if (acc + s_cost[r] > spare) break;
-      acc += s_cost[r];
-      r0 = r;
-    }
-    s_r0 = r0;
+  // r0: the smallest r such that the bins r .. 32 fit (every warp for itself:
+  // lane l sums the bins 31 - l .. 32; the sums grow with l)
+  uint32_t r0;
+  {
+    const uint32_t c32 = ts.cost[32];
+    const uint32_t v = warp_incl_scan(ts.cost[31 - lane]) + c32;
+    const uint32_t ok = __popc(__ballot_sync(0xffffffffu, v <= spare));
+    r0 = c32 > spare ? 33u : 32u - ok;
   }
-  __syncthreads();
-  const uint32_t r0 = (uint32_t)s_r0;
-#pragma unroll
-  for (int q = 0; q < SPT; ++q)
-    if (rq[q] != 0xFFFFFFFFu && rq[q] >= r0) bq[q] += 1;
-
-  auto bits_of = [&](int q) -> int { return bq[q]; };
   uint32_t my[SPT], mysum = 0;
 #pragma unroll
   for (int q = 0; q < SPT; ++q) {
-    my[q] = c[q] ? (1u << bits_of(q)) : (prev_nonempty[q] ? 1u : 0u);
+    if (rq[q] != 0xFFFFFFFFu && rq[q] >= r0) bq[q] += 1;
+    my[q] = SPT * tid + q >= nsl ? 0u : c[q] ? (1u << bq[q]) : (prev_nonempty[q] ? 1u : 0u);
     mysum += my[q];
   }
   uint32_t total;
-  const uint32_t incl = block_incl_scan(mysum, &total, red32);
-  uint32_t run = incl - mysum + 1u;  // bucket 0 is the low edge
-
-  // Candidate windows.  The number of samples below the element of rank r is
-  // about Binomial(S, r / n); each window [lo, hi] of ranks is widened to the
-  // sample ranks E - 6 sd - 4 .. E + 6 sd + 4 of its ends, and the slices
-  // holding those two samples bound its buckets.  A window reaching past the
-  // sample's first or last key takes bucket 0 or the top bucket as well.  The
-  // prediction only decides what the histogram pass keeps: compaction checks
-  // that every segment's bucket was kept before it reads the candidates.
-  __shared__ uint32_t s_sp[8];  // per window: first bucket, last bucket, first / end sample rank
-  const bool spec_on = sp != nullptr && sp->cand_cap != 0 && sp->ctrl->spec_nwin != 0 &&
-                       pre_cnt != nullptr && fine != nullptr;
-  uint32_t wa[2] = {0, 0}, wb[2] = {0, 0}, nwin = 0;
-  bool wlo_open[2] = {false, false}, whi_open[2] = {false, false};
-  if (spec_on) {
-    nwin = sp->ctrl->spec_nwin < 2u ? sp->ctrl->spec_nwin : 2u;
-    // single precision (float64 is slow on this part; sample ranks need
-    // about one unit of 2^16)
-    const float dn = (float)sp->n, dS = (float)S;
-#pragma unroll
-    for (uint32_t w = 0; w < 2; ++w) {
-      if (w >= nwin) break;
-      const float pl = (float)sp->ctrl->spec_lo[w] / dn;
-      const float ph = fminf((float)(sp->ctrl->spec_hi[w] + 1) / dn, 1.0f);
-      const float a = pl * dS - (6.0f * sqrtf(dS * pl * (1.0f - pl)) + 4.0f);
-      const float b = ph * dS + (6.0f * sqrtf(dS * ph * (1.0f - ph)) + 4.0f);
-      wlo_open[w] = a <= 0.0f;
-      whi_open[w] = b >= dS - 1.0f;
-      wa[w] = wlo_open[w] ? 0u : (a >= dS - 1.0f ? S - 1u : (uint32_t)a);
-      wb[w] = whi_open[w] ? S - 1u : (uint32_t)b;
-    }
-    // defaults (replaced below; no fine slice left unmatched): every bucket, every sample
-    if (tid < 8) s_sp[tid] = (tid & 3) == 1 ? 0xFFFFFFFEu : ((tid & 3) == 3 ? S : 0u);
-  }
-  // the table also goes to cnt[] (its counts are no longer read) for the
-  // collision estimate below
+  uint32_t run = block_excl_scan(mysum, ts.scan, &total) + 1u;  // bucket 0 is the low edge
 #pragma unroll
   for (int q = 0; q < SPT; ++q) {
     const uint32_t j = SPT * tid + q;
-    uint32_t e = 0;
-    if (j >= nsl) {
-      continue;  // unused slice
-    } else if (c[q]) {
-      const int b = bits_of(q);
-      e = lut_pack((int32_t)run - (int32_t)(j << b), shift - (uint32_t)b);
-    } else {
-      // one bucket per run of empty slices
-      e = lut_pack((int32_t)(prev_nonempty[q] ? run : run - 1u) - (int32_t)j, shift);
-    }
+    if (j >= nsl) break;
+    // one bucket per run of empty slices
+    const uint32_t e =
+        c[q] ? lut_pack((int32_t)run - (int32_t)(j << bq[q]), shift - (uint32_t)bq[q])
+             : lut_pack((int32_t)(prev_nonempty[q] ? run : run - 1u) - (int32_t)j, shift);
     lut[j] = e;
-    cnt[j] = e;
+    tab[j] = e;
     run += my[q];
   }
-  const uint32_t top = lut_pack((int32_t)(top_run_start ? total + 1u : total),
-                                (uint32_t)KeyMax<K>::bits);
+  *top = lut_pack((int32_t)(top_run_start ? total + 1u : total), (uint32_t)KeyMax<K>::bits);
+  return 1u + total + (top_run_start ? 1u : 0u);
+}
+
+// The splitter table of one problem of a batch, or of a small vector, from its
+// S sampled keys in shared memory (kmin / kmax: the sample's extremes), by one
+// whole CTA; the table goes to lut[0 .. nsl] with nsl = 2^nsl_bits <= SPT *
+// blockDim.x slices (nb_max >= nsl + 2 makes every threshold feasible), and
+// thread 0 writes the header.
+template <class K, int SPT>
+__device__ void build_lut_cta(const K *samples, uint32_t S, K kmin, K kmax, uint32_t nb_max,
+                              uint32_t *lut, LutHeader<K> *hdr, int nsl_bits) {
+  __shared__ uint32_t cnt[kLutIdx];  // samples per slice, then the table
+  __shared__ TableShared ts;
+  __shared__ uint32_t s_same[2];
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const uint32_t nsl = 1u << nsl_bits;
+  const int bl = bitlen<K>(kmax - kmin);
+  const uint32_t shift = bl > nsl_bits ? (uint32_t)(bl - nsl_bits) : 0u;
+  int bcap = (int)(shift < (uint32_t)kMaxSubBits ? shift : (uint32_t)kMaxSubBits);
+  if (bcap > 24 - nsl_bits) bcap = 24 - nsl_bits;
+  table_init(ts);
+  if (tid < 2) s_same[tid] = 0;
+  for (uint32_t j = tid; j < nsl; j += blockDim.x) cnt[j] = 0;
+  __syncthreads();
+  // eight loads per thread ahead of their atomics (a load and a shared atomic
+  // in one loop body complete one at a time)
+  for (uint32_t s0 = tid; s0 < S; s0 += 8 * blockDim.x) {
+    K kk[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) kk[u] = s0 + u * blockDim.x < S ? samples[s0 + u * blockDim.x] : kmin;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (s0 + u * blockDim.x < S) atomicAdd(&cnt[(uint32_t)((kk[u] - kmin) >> shift)], 1u);
+  }
+  __syncthreads();
+  // (a thread reads its own slices' counts and its predecessor's last one
+  // before build_table's barriers, and writes entries after them)
+  uint32_t top;
+  const uint32_t nb = build_table<K, SPT>([&](uint32_t j) { return cnt[j]; }, nsl, shift, bcap,
+                                          nb_max, lut, cnt, ts, &top);
   __syncthreads();
   // Warp-aggregated cursor updates in compaction pay off when lanes of a warp
   // often hit the same bucket (its atomics return positions, which lanes of
   // one address receive one at a time): the chance that two elements share a
   // bucket is estimated from neighbouring samples (2q, 2q + 1), which are
   // neighbouring elements when the samples come in pairs or runs, as the
-  // passes' warps see them.  The
-  // chance that two elements share a key, a property of the whole vector, is
-  // estimated from far-apart samples (q, q + S/2).
+  // passes' warps see them.  The chance that two elements share a key, a
+  // property of the whole vector, is estimated from far-apart samples
+  // (q, q + S/2).
   uint32_t same = 0, same_key = 0;
-  const uint32_t npairs = S / 2 < 4096u ? S / 2 : 4096u;  // enough for a 1/32 estimate
+  const uint32_t npairs = S / 2 < 2048u ? S / 2 : 2048u;  // enough for a 1/32 estimate
   auto bucket = [&](K k) {
     const K d = k - kmin;
     const K idx = d >> shift;
-    const uint32_t j = idx < (K)nsl ? (uint32_t)idx : nsl;
-    const uint32_t e = j == nsl ? top : cnt[j];
+    const uint32_t e = idx < (K)nsl ? cnt[(uint32_t)idx] : top;
     return (uint32_t)((int32_t)e >> 7) + shr_clamp(d, e & 127u);
   };
-  if (spec_on) {
-    // The fine slices split the sample ranks [0, S) in order: the fine slice
-    // holding a window's first (last) sample rank gives the window's first
-    // (last) bucket, that of the fine slice's first (last) key.  Each thread
-    // takes kLutIdx / blockDim.x consecutive fine slices (at most 4).
-    const uint32_t per = kLutIdx / blockDim.x;
-    uint32_t fc[4], fsum = 0;
-#pragma unroll
-    for (uint32_t q = 0; q < 4; ++q) {
-      fc[q] = q < per ? fine[per * tid + q] : 0u;
-      fsum += fc[q];
-    }
-    uint32_t ftot;
-    uint32_t fpre = block_incl_scan(fsum, &ftot, red32) - fsum;
-    const K span = kmax - kmin;
-#pragma unroll
-    for (uint32_t q = 0; q < 4; ++q) {
-      if (q >= per || fc[q] == 0) continue;
-      const uint32_t jf = per * tid + q;
-#pragma unroll
-      for (uint32_t w = 0; w < 2; ++w) {
-        if (w >= nwin) break;
-        if (fpre <= wa[w] && wa[w] < fpre + fc[q]) {
-          s_sp[4 * w + 0] = bucket(kmin + ((K)jf << fsh));
-          s_sp[4 * w + 2] = fpre;
-        }
-        if (fpre <= wb[w] && wb[w] < fpre + fc[q]) {
-          K dend = ((K)(jf + 1u) << fsh) - K(1);
-          dend = dend < span ? dend : span;
-          s_sp[4 * w + 1] = bucket(kmin + dend);
-          s_sp[4 * w + 3] = fpre + fc[q];
-        }
-      }
-      fpre += fc[q];
-    }
-    __syncthreads();
+  for (uint32_t q = tid; q < npairs; q += blockDim.x) {
+    same += bucket(samples[2 * q]) == bucket(samples[2 * q + 1]) ? 1u : 0u;
+    same_key += samples[q] == samples[q + S / 2] ? 1u : 0u;
   }
-  auto ld = [&](uint32_t i) -> K { return SMEM ? samples[i] : __ldcg(samples + i); };
-  // four pairs of each kind per thread and step, all loads issued first (the
-  // far-apart pairs only when the caller has not counted them)
-  const bool far = pre_same_key < 0;
-  for (uint32_t q0 = tid; q0 < npairs; q0 += 4 * blockDim.x) {
-    K a[4], b[4], c[4], d2[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const uint32_t q = q0 + u * blockDim.x;
-      const bool ok = q < npairs;
-      a[u] = ok ? ld(2 * q) : K(0);
-      b[u] = ok ? ld(2 * q + 1) : K(0);
-      c[u] = ok && far ? ld(q) : K(0);
-      d2[u] = ok && far ? ld(q + S / 2) : K(1);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (q0 + u * blockDim.x < npairs) {
-        same += bucket(a[u]) == bucket(b[u]) ? 1u : 0u;
-        same_key += c[u] == d2[u] ? 1u : 0u;
-      }
+  same = __reduce_add_sync(0xffffffffu, same);
+  same_key = __reduce_add_sync(0xffffffffu, same_key);
+  if (lane == 0) {
+    if (same) atomicAdd(&s_same[0], same);
+    if (same_key) atomicAdd(&s_same[1], same_key);
   }
-  same = block_reduce(same, [](uint32_t p, uint32_t q) { return p + q; }, red32);
-  same_key = far ? block_reduce(same_key, [](uint32_t p, uint32_t q) { return p + q; }, red32)
-                 : (uint32_t)pre_same_key;
+  __syncthreads();
   if (tid == 0) {
-    const uint32_t nb = 1u + total + (top_run_start ? 1u : 0u);
     lut[nsl] = top;
     LutHeader<K> h;
     h.base = kmin;
@@ -939,186 +816,15 @@ __device__ void build_lut_cta(const K *samples, uint32_t S, K kmin, K kmax, uint
     h.nb = nb;
     // collision chance >= 1/32: with 32 lanes, about 15 same-bucket pairs per
     // warp access
-    h.heavy = (S >= 256 && 32ull * same >= npairs) ? 1u : 0u;
+    h.heavy = (S >= 256 && 32ull * s_same[0] >= npairs) ? 1u : 0u;
     // two elements share a key with chance >= 1 / nb: buckets holding a single
     // key (many copies of it) are likely
-    h.dup = (S >= 256 && (uint64_t)same_key * nb >= npairs) ? 1u : 0u;
+    h.dup = (S >= 256 && (uint64_t)s_same[1] * nb >= npairs) ? 1u : 0u;
     h.spec = 0;
     h.cand_cap = 0;
     h.spec_lo[0] = h.spec_lo[1] = 0;
     h.spec_len[0] = h.spec_len[1] = 0;
-    if (spec_on) {
-      // bucket intervals and the sample ranks they hold, ordered and merged
-      uint32_t blo[2], bhi[2], clo[2], chi[2];
-#pragma unroll
-      for (uint32_t w = 0; w < 2; ++w) {
-        if (w >= nwin) break;
-        blo[w] = wlo_open[w] ? 0u : s_sp[4 * w + 0];
-        bhi[w] = whi_open[w] ? nb - 1u : s_sp[4 * w + 1];
-        clo[w] = wlo_open[w] ? 0u : s_sp[4 * w + 2];
-        chi[w] = whi_open[w] ? S : s_sp[4 * w + 3];
-      }
-      uint32_t ni = nwin;
-      if (ni == 2) {
-        if (blo[1] < blo[0]) {
-          uint32_t t0 = blo[0]; blo[0] = blo[1]; blo[1] = t0;
-          t0 = bhi[0]; bhi[0] = bhi[1]; bhi[1] = t0;
-          t0 = clo[0]; clo[0] = clo[1]; clo[1] = t0;
-          t0 = chi[0]; chi[0] = chi[1]; chi[1] = t0;
-        }
-        if (blo[1] <= bhi[0] + 1u) {
-          bhi[0] = bhi[1] > bhi[0] ? bhi[1] : bhi[0];
-          chi[0] = chi[1] > chi[0] ? chi[1] : chi[0];
-          ni = 1;
-        }
-      }
-      uint32_t pred = 0;  // samples inside the intervals
-#pragma unroll
-      for (uint32_t i = 0; i < 2; ++i)
-        if (i < ni) pred += chi[i] - clo[i];
-      // the expected candidates with half as much again, plus one partly
-      // filled chunk per histogram warp, must fit the pool
-      const float want = 1.5f * (float)sp->n * (float)pred / (float)S +
-                         (float)sp->G * kCandWarps * kCandChunk;
-      if (want <= (float)sp->cand_cap * kCandChunk) {
-        h.spec = ni;
-        h.cand_cap = sp->cand_cap;
-#pragma unroll
-        for (uint32_t i = 0; i < 2; ++i)
-          if (i < ni) {
-            h.spec_lo[i] = blo[i];
-            h.spec_len[i] = bhi[i] - blo[i] + 1u;
-          }
-      }
-    }
     *hdr = h;
-  }
-}
-
-// Two kernels of ceil(S / 1024) CTAs.  k_sample: each thread gathers one
-// sample (pairs of neighbouring elements at hashed positions), each CTA leaves
-// its samples' smallest and largest key in spans (two keys per CTA), and CTA 0
-// sets the control block to init, which travels in the launch's parameters: no
-// copy or clearing precedes the call's first kernel.
-// k_lut (after it in the stream): each CTA re-reads its 1024 samples, bins
-// them by slice in shared memory against the sample's span, adds its non-zero
-// slice counts to slice_cnt (global, zero on entry) and counts the far-apart
-// pairs (q, q + S/2) that hold one key; the last CTA to finish builds the
-// table from slice_cnt (leaving it zero) and reads back only the neighbouring
-// samples its bucket collision estimate needs.  The kernel boundary takes the
-// place of a grid barrier, so no launch needs every CTA resident at once.
-// The table builder also turns the call's rank windows (Ctrl::spec_*) into
-// the candidate buckets of speculative compaction (n, cand_cap: chunks in the
-// candidate pool, 0 for none; G: histogram CTAs).
-template <class T>
-__global__ void __launch_bounds__(1024) k_sample(const T *__restrict__ x, uint64_t n, uint32_t S,
-                                                 uint32_t seed,
-                                                 typename Traits<T>::K *__restrict__ samples,
-                                                 typename Traits<T>::K *__restrict__ spans,
-                                                 Ctrl *ctrl, const __grid_constant__ Ctrl init) {
-  pdl_start();
-  using K = typename Traits<T>::K;
-  __shared__ K redk[33];
-  if (blockIdx.x == 0 && threadIdx.x < sizeof(Ctrl) / 4)
-    reinterpret_cast<uint32_t *>(ctrl)[threadIdx.x] =
-        reinterpret_cast<const uint32_t *>(&init)[threadIdx.x];
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  K mine_lo = KeyMax<K>::v, mine_hi = 0;
-  if (i < S) {
-    uint64_t pos;
-    if ((uint64_t)S >= n) {
-      pos = i;
-    } else {
-      // pairs of neighbouring elements at hashed positions: samples 2q and
-      // 2q + 1 are neighbours, so the table builder's collision estimate sees
-      // runs of equal buckets (sorted input) as the histogram's warps do
-      pos = (((uint64_t)hash32((i >> 1) * 0x9E3779B9u + seed) * (n - 1)) >> 32) + (i & 1u);
-    }
-    const K k = Traits<T>::key(x[pos]);
-    samples[i] = k;
-    mine_lo = k;
-    mine_hi = k;
-  }
-  mine_lo = block_reduce(mine_lo, [](K p, K q) { return p < q ? p : q; }, redk);
-  mine_hi = block_reduce(mine_hi, [](K p, K q) { return p > q ? p : q; }, redk);
-  if (threadIdx.x == 0) {
-    spans[2 * blockIdx.x] = mine_lo;
-    spans[2 * blockIdx.x + 1] = mine_hi;
-  }
-}
-
-// The sample's smallest and largest key from the parts CTAs' spans (k_sample);
-// every warp reduces them for itself.
-template <class K>
-__device__ __forceinline__ void sample_span(const K *__restrict__ spans, uint32_t parts, K *kmin,
-                                            K *kmax) {
-  K lo = KeyMax<K>::v, hi = 0;
-  for (uint32_t i = threadIdx.x & 31; i < parts; i += 32) {
-    const K a = __ldcg(spans + 2 * i), z = __ldcg(spans + 2 * i + 1);
-    lo = a < lo ? a : lo;
-    hi = z > hi ? z : hi;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const K a = __shfl_xor_sync(0xffffffffu, lo, o), z = __shfl_xor_sync(0xffffffffu, hi, o);
-    lo = a < lo ? a : lo;
-    hi = z > hi ? z : hi;
-  }
-  *kmin = lo;
-  *kmax = hi;
-}
-
-template <class K>
-__global__ void __launch_bounds__(1024) k_lut(const K *__restrict__ samples, uint32_t S,
-                                              const K *__restrict__ spans, Ctrl *ctrl, LutHeader<K> *hdr, uint32_t *lut,
-                                              uint32_t nb_max, uint32_t *slice_cnt, uint64_t n,
-                                              uint32_t cand_cap, uint32_t G) {
-  pdl_start();
-  __shared__ uint32_t red32[33];
-  __shared__ uint32_t s_last;
-  __shared__ uint32_t ccnt[kLutIdx];
-
-  const uint32_t tid = threadIdx.x;
-  const uint32_t i = blockIdx.x * blockDim.x + tid;
-  for (uint32_t j = tid; j < kLutIdx; j += blockDim.x) ccnt[j] = 0;
-  const uint32_t npairs = S / 2 < 4096u ? S / 2 : 4096u;
-  const K k = i < S ? __ldcg(samples + i) : K(0);
-  const K other = i < npairs ? __ldcg(samples + i + S / 2) : K(0);
-  K kmin, kmax;
-  sample_span<K>(spans, gridDim.x, &kmin, &kmax);
-  const int bl = bitlen<K>(kmax - kmin);
-  const uint32_t shift = bl > kLutIdxBits ? (uint32_t)(bl - kLutIdxBits) : 0u;
-  __syncthreads();
-  if (i < S) atomicAdd(&ccnt[(uint32_t)((k - kmin) >> shift)], 1u);
-  // far-apart pairs (q, q + S/2): does the vector hold many copies of a key
-  uint32_t sk = i < npairs && other == k ? 1u : 0u;
-  sk = block_reduce(sk, [](uint32_t p, uint32_t q) { return p + q; }, red32);
-  for (uint32_t j = tid; j < kLutIdx; j += blockDim.x) {
-    const uint32_t c = ccnt[j];
-    if (c) atomicAdd(&slice_cnt[j], c);
-  }
-  // every thread's counts before the CTA reports done (the fence below is
-  // cumulative over what the barrier ordered)
-  __syncthreads();
-  if (tid == 0) {
-    if (sk) atomicAdd(&ctrl->same_key, sk);
-    __threadfence();
-    s_last = (atomicAdd(&ctrl->sample_done, 1u) == gridDim.x - 1) ? 1u : 0u;
-    if (s_last) __threadfence();
-  }
-  __syncthreads();
-  if (!s_last) return;
-
-  // the table has sv_slices<K>() slices; the fine counts (this CTA's ccnt is free
-  // now) place the speculative windows
-  __syncthreads();
-  const SpecArgs sa{ctrl, n, cand_cap, G};
-  build_lut_cta<K, 4, false>(samples, S, kmin, kmax, nb_max, lut, hdr, sv_bits<K>(), slice_cnt,
-                             (int64_t)__ldcg(&ctrl->same_key), &sa, dup_nb_cap<K>(nb_max), ccnt);
-  if (tid == 0) {
-    ctrl->nb = hdr->nb;
-    ctrl->spec_on = hdr->spec != 0 ? 1u : 0u;
-    ctrl->sample_done = 0;  // re-arm for the next call on this workspace
   }
 }
 
@@ -1479,7 +1185,8 @@ __global__ void __launch_bounds__(1024, 1)
 // (d) bucket totals: column sums of the per-CTA rows
 // ---------------------------------------------------------------------------
 // Each CTA sums kScanTile buckets over the rows and writes their exclusive
-// prefix inside the tile and the tile's total; the kernels that search the
+// prefix inside the tile, every eighth of them again to bco (a tile's eight lie
+// in one sector), and the tile's total; the kernels that search the
 // bucket prefix (k_plan, k_reqmap: load_prefix) add the tiles' offsets in
 // shared memory.  A grid-wide scan here would make every tile wait on its
 // predecessors.
@@ -1495,8 +1202,8 @@ constexpr int kScanTile = 64;  // buckets per CTA
 template <class K>
 __global__ void __launch_bounds__(kScanThreads, 4)
     k_colsum(const uint32_t *__restrict__ partials, uint32_t rows, uint32_t nb_max,
-             const LutHeader<K> *hdr, uint32_t *__restrict__ bpre, uint32_t *__restrict__ ttot,
-             const Ctrl *ctrl, const K *__restrict__ reps, uint32_t *__restrict__ bsingle,
+             const LutHeader<K> *hdr, uint32_t *__restrict__ bpre, uint32_t *__restrict__ bco,
+             uint32_t *__restrict__ ttot, const Ctrl *ctrl, const K *__restrict__ reps, uint32_t *__restrict__ bsingle,
              K *__restrict__ bkey) {
   pdl_start();
   constexpr uint32_t kVecs = kScanTile / 4;              // 16-byte vectors per tile row
@@ -1587,7 +1294,9 @@ __global__ void __launch_bounds__(kScanThreads, 4)
   __syncthreads();
   if (col < kScanTile) {
     const uint32_t b = blockIdx.x * kScanTile + col;
-    if (b < nb) bpre[b] = incl - c + (col >= 32 ? s_w2[0] : 0u);
+    const uint32_t pre = incl - c + (col >= 32 ? s_w2[0] : 0u);
+    if (b < nb) bpre[b] = pre;
+    if (col % 8 == 0) bco[b / 8] = b < nb ? pre : 0xFFFFFFFFu;
     if (col == 0) ttot[blockIdx.x] = s_w2[0] + s_w2[1];
     if (track && b < nb) {
       // one key in the whole vector: every row group saw none or the same one
@@ -1824,6 +1533,173 @@ static __global__ void __launch_bounds__(1024)
   }
 }
 
+constexpr uint32_t kPlanFew = 1024;  // requests of k_plan_few, sorted by rank (bring_requests)
+
+// The last of a tile's 64 bucket prefixes (p[0 .. m) are in use, p[0] = 0) that
+// is <= r, found from every eighth of them (q[0 .. 8), the largest value past
+// m) and then eight of p: one 32-byte sector each (eight scattered loads each
+// made the plan of 1001 requests 9 us long, now 6.3).  *lo: its prefix,
+// *hi: the next bucket's (end for the last).
+__device__ __forceinline__ uint32_t tile_bucket(const uint32_t *__restrict__ p,
+                                                const uint32_t *__restrict__ q, uint32_t m,
+                                                uint32_t end, uint32_t r, uint32_t *lo,
+                                                uint32_t *hi) {
+  static_assert(kScanTile == 64, "two rounds of eight");
+  uint32_t a[8];
+  auto load8 = [&](const uint32_t *s) {
+    const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(s));
+    const uint4 y = __ldcg(reinterpret_cast<const uint4 *>(s) + 1);
+    a[0] = x.x; a[1] = x.y; a[2] = x.z; a[3] = x.w;
+    a[4] = y.x; a[5] = y.y; a[6] = y.z; a[7] = y.w;
+  };
+  load8(q);
+  uint32_t g = 0, next = end;
+#pragma unroll
+  for (uint32_t u = 7; u > 0; --u)
+    if (a[u] > r && 8 * u < m) next = a[u];
+#pragma unroll
+  for (uint32_t u = 1; u < 8; ++u)
+    if (a[u] <= r && 8 * u < m) g = u;
+  load8(p + 8 * g);  // may reach past m: masked below
+  uint32_t b = 0, cur = a[0];
+#pragma unroll
+  for (uint32_t u = 7; u > 0; --u)
+    if (a[u] > r && 8 * g + u < m) next = a[u];
+#pragma unroll
+  for (uint32_t u = 1; u < 8; ++u)
+    if (a[u] <= r && 8 * g + u < m) {
+      b = u;
+      cur = a[u];
+    }
+  *lo = cur;
+  *hi = next;
+  return 8 * g + b;
+}
+
+// The plan of at most kPlanFew requests, sorted by rank: one CTA of
+// 1024 threads, a request per thread.  Sorted requests lie in bucket order, so a
+// slot is a run of neighbouring threads with one bucket, its number a scan of
+// the runs' heads, and its request list the run itself; a request finds its
+// bucket by its tile (shared memory) and two rounds of loads in the tile's
+// prefixes.  No flags, counters or prefix over all buckets (k_plan, which
+// serves more requests, takes 11-16 us for these; this 4.6-6.3 us).  Slots as
+// k_plan makes them: seg_size 0 marks a flat slot (one key), answered from
+// seg_lo without survivors.  Bound: latency, four rounds of loads.
+template <class InT>
+__global__ void __launch_bounds__(1024, 1)
+    k_plan_few(const LutHeader<typename Traits<InT>::K> *hdr, const uint32_t *__restrict__ lut_g,
+               const uint32_t *__restrict__ bpre, const uint32_t *__restrict__ bco,
+               const uint32_t *__restrict__ ttot, uint64_t n,
+               const Req *__restrict__ reqs, uint32_t num_req, uint32_t nb_max, Ctrl *ctrl,
+               uint32_t *__restrict__ seg_bucket, uint64_t *__restrict__ seg_off,
+               uint32_t *__restrict__ seg_size, uint32_t *__restrict__ kstart,
+               uint32_t *__restrict__ kcnt, uint32_t *__restrict__ fill,
+               typename Traits<InT>::K *__restrict__ seg_lo,
+               typename Traits<InT>::K *__restrict__ seg_hi, Req *__restrict__ klist,
+               uint64_t surv_cap, const uint32_t *__restrict__ bsingle,
+               const typename Traits<InT>::K *__restrict__ bkey) {
+  using K = typename Traits<InT>::K;
+  constexpr uint32_t kEnt = sv_slices<K>() + 1;
+  constexpr uint32_t kTiles = kMaxNb / kScanTile;
+  static_assert(kTiles < 1024, "a thread per tile and one past the last");
+  __shared__ uint32_t s_lut[kEnt];
+  __shared__ uint32_t s_tile[kTiles + 1];
+  __shared__ uint32_t s_b[kPlanFew], s_head[kPlanFew + 1];
+  __shared__ uint32_t s_scan[3][32];
+  const uint32_t tid = threadIdx.x;
+  pdl_start();
+  const uint32_t status = ctrl->status;
+  const LutHeader<K> h = *hdr;
+  const bool mine = tid < num_req;
+  Req q;
+  q.rank = 0;
+  q.out = 0;
+  if (mine) q = reqs[tid];
+  uint32_t e[(kEnt + 1023) / 1024];
+#pragma unroll
+  for (uint32_t i = 0; i < (kEnt + 1023) / 1024; ++i)
+    e[i] = tid + 1024 * i < kEnt ? __ldcg(lut_g + tid + 1024 * i) : 0u;
+  const uint32_t tt = tid < nb_max / kScanTile ? __ldcg(ttot + tid) : 0u;  // stale past nb
+  if (status & ST_FATAL) return;
+  const uint32_t nb = h.nb;
+  const uint32_t ntile = (nb + kScanTile - 1) / kScanTile;
+#pragma unroll
+  for (uint32_t i = 0; i < (kEnt + 1023) / 1024; ++i)
+    if (tid + 1024 * i < kEnt) s_lut[tid + 1024 * i] = e[i];
+  uint32_t total;
+  const uint32_t tpre = block_excl_scan(tid < ntile ? tt : 0u, s_scan[0], &total);
+  if (tid <= ntile) s_tile[tid] = tpre;
+  // the totals must add up to n (else the input changed under the histogram)
+  if (total != n && tid == 0) atomicOr(&ctrl->status, ST_INTERNAL);
+  __syncthreads();
+  // the request's tile: the last whose prefix is <= the rank (never an empty one)
+  uint32_t t = 0;
+  for (uint32_t step = ntile > 1 ? 1u << (31 - __clz(ntile - 1)) : 0u; step; step >>= 1) {
+    const uint32_t m = t + step;
+    if (m < ntile && s_tile[m] <= q.rank) t = m;
+  }
+  uint32_t b = kNoSlot, pre = 0, next = 0;
+  if (mine) {
+    b = t * kScanTile + tile_bucket(bpre + (uint64_t)t * kScanTile, bco + t * (kScanTile / 8),
+                                    min((uint32_t)kScanTile, nb - t * kScanTile),
+                                    s_tile[t + 1] - s_tile[t], q.rank - s_tile[t], &pre, &next);
+    q.rank -= s_tile[t] + pre;  // now the rank inside the bucket
+  }
+  const uint32_t count = next - pre;
+  s_b[tid] = b;
+  // the bucket's key range, whether it holds one key, and which
+  K klo = 0, khi = 0;
+  bool one = false;
+  if (mine) {
+    klo = bucket_lo<K>(b, h.base, h.shift, s_lut, sv_slices<K>());
+    const K knext =
+        (b + 1 < nb) ? bucket_lo<K>(b + 1, h.base, h.shift, s_lut, sv_slices<K>()) : K(0);
+    // single key iff the next bucket starts one key later; the start of the
+    // top entry's bucket can wrap past the key width, and then bucket b runs
+    // up to the largest key
+    khi = knext > klo ? knext - K(1) : KeyMax<K>::v;
+    one = khi == klo;
+    // a wider bucket that the histogram pass saw holding one key (k_colsum)
+    const uint32_t dcap = dup_nb_cap<K>(nb_max);
+    const bool dtrack = bsingle != nullptr && bkey != nullptr && h.dup && dcap != 0 && nb <= dcap;
+    if (dtrack && !one && __ldcg(bsingle + b) != 0u) {
+      one = true;
+      klo = khi = __ldcg(bkey + b);
+    }
+  }
+  __syncthreads();  // s_b
+  const bool head = mine && (tid == 0 || s_b[tid - 1] != b);
+  uint32_t slots, surv;
+  const uint32_t slot = block_excl_scan(head ? 1u : 0u, s_scan[1], &slots);
+  // (the survivors of all slots are at most n elements)
+  const uint32_t off = block_excl_scan(head && !one ? count : 0u, s_scan[2], &surv);
+  if (head) s_head[slot] = tid;
+  if (tid == 0) s_head[slots] = num_req;
+  __syncthreads();
+  if (mine) klist[tid] = q;
+  if (head) {
+    seg_bucket[slot] = b;
+    seg_off[slot] = off;
+    seg_size[slot] = one ? 0u : count;
+    seg_lo[slot] = klo;
+    seg_hi[slot] = khi;
+    kstart[slot] = tid;
+    kcnt[slot] = s_head[slot + 1] - tid;
+    fill[slot] = 0;
+  }
+  if (tid == 0) {
+    ctrl->deferred_count = 0;
+    ctrl->num_slots = slots;
+    ctrl->total_surv = surv;
+    if (surv > surv_cap) {
+      atomicOr(&ctrl->status, ST_OVERFLOW);
+      ctrl->cap_needed = surv;
+    }
+    // compaction cursors carry the survivor position in 31 bits
+    if (surv >= kInactive) atomicOr(&ctrl->status, ST_INTERNAL);
+  }
+}
+
 // Flag words per lane in k_plan's slot numbering (1024 threads, kMaxNb buckets).
 constexpr uint32_t kPlanRounds = kMaxNb / 4 / 1024;
 static_assert(kPlanRounds * 4 * 1024 == kMaxNb, "k_plan slot numbering covers kMaxNb buckets");
@@ -1865,7 +1741,8 @@ __device__ __forceinline__ void plan_map_requests(const uint32_t *excl, uint32_t
   }
 }
 
-// One CTA of 1024 threads.  Dynamic shared memory: lut[kLutEntries + 1] (u32,
+// More than kPlanFew requests (or requests in any order): one CTA of 1024
+// threads.  Dynamic shared memory: lut[kLutEntries + 1] (u32,
 // padded to 16 bytes), excl[nb_max] (u32), flags[nb_max] (u8).
 //
 // Every bucket that holds a requested rank gets a slot, in bucket order.  A
@@ -1887,16 +1764,7 @@ __global__ void __launch_bounds__(1024, 1)
            uint32_t *__restrict__ req_local, Req *__restrict__ klist, uint64_t surv_cap,
            Premap pm, const uint32_t *__restrict__ bsingle = nullptr,
            const typename Traits<InT>::K *__restrict__ bkey = nullptr) {
-  // At most one request per thread: the requests were complete before the
-  // call's first launch (in host memory, read here in place, or left by an
-  // earlier call), so each thread loads its own ahead of the dependency wait.
-  pdl_trigger();
-  const bool own = num_req <= blockDim.x;
-  Req my_rq;
-  my_rq.rank = 0;
-  my_rq.out = 0;
-  if (own && !pm.bits && threadIdx.x < num_req) my_rq = reqs[threadIdx.x];
-  pdl_wait();
+  pdl_start();
   using K = typename Traits<InT>::K;
   extern __shared__ uint4 smem_raw[];
   uint32_t *lut = reinterpret_cast<uint32_t *>(smem_raw);
@@ -1967,21 +1835,8 @@ __global__ void __launch_bounds__(1024, 1)
   // requests -> bucket (the last b with excl[b] <= rank is never empty) and
   // the rank inside it; with many requests, four per thread and step, so that
   // their loads and searches overlap
-  uint32_t my_b = 0;  // the bucket of the thread's own request
   if (!pm.bits) {
-    if (own) {
-      if (tid < num_req) {
-        const uint32_t top = nb > 1 ? 1u << (31 - __clz(nb - 1)) : 0u;
-        uint32_t lo = 0;
-        for (uint32_t step = top; step; step >>= 1) {
-          const uint32_t m = lo + step;
-          if (m < nb && excl[m] <= my_rq.rank) lo = m;
-        }
-        flag[lo] = 1;
-        my_b = lo;
-        my_rq.rank -= excl[lo];  // now the rank inside the bucket
-      }
-    } else if (num_req >= 4096) {
+    if (num_req >= 4096) {
       plan_map_requests<4>(excl, nb, reqs, num_req, flag, req_bucket, req_local);
     } else {
       plan_map_requests<1>(excl, nb, reqs, num_req, flag, req_bucket, req_local);
@@ -2106,13 +1961,6 @@ __global__ void __launch_bounds__(1024, 1)
   const bool in_smem = !pm.bits && tot_slots <= room;
   if (pm.bits) {
     // counted by k_reqmap; kcnt holds them already
-  } else if (own) {
-    // one request per thread, its bucket in a register
-    if (in_smem) {
-      for (uint32_t q = tid; q < tot_slots; q += nt) s_cnt[q] = 0;
-      __syncthreads();
-    }
-    if (tid < num_req) atomicAdd(in_smem ? &s_cnt[excl[my_b]] : &kcnt[excl[my_b]], 1u);
   } else if (in_smem) {
     for (uint32_t q = tid; q < tot_slots; q += nt) s_cnt[q] = 0;
     __syncthreads();
@@ -2147,11 +1995,6 @@ __global__ void __launch_bounds__(1024, 1)
   __syncthreads();
   if (pm.bits) {
     // k_reqplace writes the lists
-  } else if (own) {
-    if (tid < num_req) {
-      const uint32_t q = excl[my_b];
-      klist[in_smem ? atomicAdd(&s_cur[q], 1u) : kstart[q] + atomicAdd(&kcur[q], 1u)] = my_rq;
-    }
   } else if (in_smem) {
     for (uint32_t i0 = tid; i0 < num_req; i0 += 4 * nt) {
       uint32_t b[4], loc[4], o[4];

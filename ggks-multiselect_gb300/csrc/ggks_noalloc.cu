@@ -41,15 +41,17 @@ constexpr size_t na_align(size_t v) { return (v + 255) / 256 * 256; }
 // scratch layout (byte offsets); the control block and the slice counts are
 // zeroed together at the start of each call
 constexpr size_t kNaCtrl = 0;
-constexpr size_t kNaSliceCnt = na_align(kNaCtrl + sizeof(Ctrl));
-constexpr size_t kNaReqs = na_align(kNaSliceCnt + kSliceCntBytes);
-constexpr size_t kNaHdr = na_align(kNaReqs + kNaMaxK * sizeof(Req));
+constexpr size_t kNaReqs = na_align(kNaCtrl + sizeof(Ctrl));
+constexpr size_t kNaSorted = na_align(kNaReqs + kNaMaxK * sizeof(Req));
+constexpr size_t kNaHdr = na_align(kNaSorted + kPlanFew * sizeof(Req));
 constexpr size_t kNaLut = na_align(kNaHdr + sizeof(LutHeader<uint32_t>));
 constexpr size_t kNaSamples = na_align(kNaLut + kLutPadded * sizeof(uint32_t));
 constexpr size_t kNaSpans = na_align(kNaSamples + kNaS * sizeof(uint32_t));
-constexpr size_t kNaPartials = na_align(kNaSpans + 2 * (kNaS / 1024) * sizeof(uint32_t));
+constexpr size_t kNaFine = na_align(kNaSpans + 2 * (kNaS / 1024) * sizeof(uint32_t));
+constexpr size_t kNaPartials = na_align(kNaFine + kLutIdx * sizeof(uint32_t));
 constexpr size_t kNaCounts = na_align(kNaPartials + (size_t)kNaMaxG * kNaNbMax * 4);
-constexpr size_t kNaTtot = na_align(kNaCounts + kNaNbMax * 4);
+constexpr size_t kNaBco = na_align(kNaCounts + kNaNbMax * 4);
+constexpr size_t kNaTtot = na_align(kNaBco + kNaNbMax / 8 * 4);
 constexpr size_t kNaSegBucket = na_align(kNaTtot + kNaNbMax / kScanTile * 4);
 constexpr size_t kNaSegOff = na_align(kNaSegBucket + kNaNbMax * 4);
 constexpr size_t kNaSegSize = na_align(kNaSegOff + kNaNbMax * 8);
@@ -133,8 +135,10 @@ extern "C" int ggks_multiselect_noalloc_f32(const float *d_vec, uint64_t n, cons
   uint32_t *lut = reinterpret_cast<uint32_t *>(A + kNaLut);
   K *samples = reinterpret_cast<K *>(A + kNaSamples);
   K *spans = reinterpret_cast<K *>(A + kNaSpans);
+  uint32_t *fine = reinterpret_cast<uint32_t *>(A + kNaFine);
   uint32_t *partials = reinterpret_cast<uint32_t *>(A + kNaPartials);
   uint32_t *bpre = reinterpret_cast<uint32_t *>(A + kNaCounts);  // prefix inside 64-bucket tiles
+  uint32_t *bco = reinterpret_cast<uint32_t *>(A + kNaBco);
   uint32_t *ttot = reinterpret_cast<uint32_t *>(A + kNaTtot);
   uint32_t *seg_bucket = reinterpret_cast<uint32_t *>(A + kNaSegBucket);
   uint64_t *seg_off = reinterpret_cast<uint64_t *>(A + kNaSegOff);
@@ -168,25 +172,31 @@ extern "C" int ggks_multiselect_noalloc_f32(const float *d_vec, uint64_t n, cons
   if (e == cudaSuccess) e = set_smem_max<k_finish<K, float>>(finish_smem_bytes<float>());
   if (e != cudaSuccess) return from_cuda(e);
 
-  // the slice counts start at zero; k_sample clears the control block, so the
-  // requests' check of the k's comes after it
-  e = cudaMemsetAsync(A + kNaSliceCnt, 0, kSliceCntBytes, s);
-  if (e != cudaSuccess) return from_cuda(e);
-  k_sample<float><<<(S + 1023) / 1024, 1024, 0, s>>>(d_vec, n, S, 0x5EEDu, samples, spans, ctrl,
-                                                     Ctrl{});
+  // the first kernel sets the control block, so the requests' check of the k's
+  // comes after it
+  const uint32_t fc = front_ctas(S);
+  k_sample<float><<<fc, 1024, 0, s>>>(d_vec, n, S, 0x5EEDu, samples, spans, fine, kLutIdx, ctrl,
+                                      Ctrl{}, ReqCopy{});
+  k_bin<K><<<fc, 1024, 0, s>>>(samples, S, spans, fine, ctrl);
   k_na_reqs<<<(num_k + 255) / 256, 256, 0, s>>>(d_k, num_k, n, reqs, ctrl);
-  k_lut<K><<<(S + 1023) / 1024, 1024, 0, s>>>(samples, S, spans, ctrl, hdr, lut, kNaNbMax,
-                                               reinterpret_cast<uint32_t *>(A + kNaSliceCnt), n,
-                                               0u, G);
+  const bool few = num_k <= kPlanFew;
+  Req *sorted = reinterpret_cast<Req *>(A + kNaSorted);
+  const ReqCopy sort{reqs, sorted, few ? num_k : 0u};
+  k_table<K><<<1 + sort_ctas(sort.num), kTableThreads, 0, s>>>(samples, S, spans, fine, n, RankWindows{},
+                                                          hdr, lut, kNaNbMax, 0u, G, ctrl, sort);
   {
     const int smem = (int)(kRepWords * sizeof(uint32_t) + (size_t)kNaNbMax * 4);
     k_hist<float, UNROLL><<<G, 1024, smem, s>>>(d_vec, n, hdr, lut, partials, kNaNbMax, ctrl,
                                                 nullptr, nullptr, nullptr, nullptr, nullptr,
                                                 nullptr);
   }
-  k_colsum<K><<<col_tiles, kScanThreads, 0, s>>>(partials, G, kNaNbMax, hdr, bpre, ttot, ctrl,
+  k_colsum<K><<<col_tiles, kScanThreads, 0, s>>>(partials, G, kNaNbMax, hdr, bpre, bco, ttot, ctrl,
                                                   nullptr, nullptr, nullptr);
-  {
+  if (few) {
+    k_plan_few<float><<<1, 1024, 0, s>>>(hdr, lut, bpre, bco, ttot, n, sorted, num_k, kNaNbMax, ctrl,
+                                         seg_bucket, seg_off, seg_size, kstart, kcnt, fill, seg_lo,
+                                         seg_hi, klist, n, nullptr, nullptr);
+  } else {
     const int smem = (int)(kLutPadded * sizeof(uint32_t) + (size_t)kNaNbMax * 5);
     k_plan<float, float><<<1, 1024, smem, s>>>(hdr, lut, bpre, ttot, n, reqs, num_k, kNaNbMax,
                                                 ctrl, seg_bucket, seg_off,

@@ -11,6 +11,7 @@
 #include <cstring>
 #include <vector>
 
+#include "ggks_front.cuh"
 #include "ggks_internal.h"
 #include "ggks_small.cuh"
 #include "ggks_tiny.cuh"
@@ -45,7 +46,7 @@ constexpr int kPlanSmemMax = (int)(kLutPadded * sizeof(uint32_t) + (size_t)kMaxN
 struct Plan {
   uint64_t n = 0;
   uint32_t num_req = 0;
-  uint32_t S = 0, sample_grid = 0;
+  uint32_t S = 0;
   uint32_t nb_max = 0;
   uint32_t G = 0;           // hist / compact grid
   bool unroll8 = true;      // tiles of 8 (else 4) vectors per thread in hist / compact
@@ -54,8 +55,8 @@ struct Plan {
   uint32_t fin_grid = 0;
   uint64_t surv_cap = 0;
   // arena offsets
-  size_t out = 0, ctrl = 0, reqs = 0, hdr = 0, lut = 0, samples = 0, spans = 0, partials = 0,
-         bpre = 0, ttot = 0, seg_bucket = 0, seg_off = 0, seg_size = 0, kstart = 0, kcnt = 0, fill = 0,
+  size_t out = 0, ctrl = 0, reqs = 0, hdr = 0, lut = 0, samples = 0, spans = 0, fine = 0, partials = 0, sorted = 0,
+         bpre = 0, bco = 0, ttot = 0, seg_bucket = 0, seg_off = 0, seg_size = 0, kstart = 0, kcnt = 0, fill = 0,
          kcur = 0, seg_lo = 0, seg_hi = 0, deferred = 0, req_bucket = 0, req_local = 0, klist = 0,
          pm_bits = 0, pm_bcount = 0, pm_bslot = 0, cand_cnt = 0, cand_tab = 0, reps = 0,
          bsingle = 0, bkey = 0, total = 0;
@@ -65,16 +66,14 @@ struct Plan {
   uint32_t cand_chunks = 0;
 };
 static_assert(sizeof(Ctrl) <= 256 && sizeof(Ctrl) % 4 == 0, "the control block's 256-byte slot");
-// Host k lists of at most kPinReq requests are read by the kernels from pinned
-// host memory (the plan CTA and the small-vector kernel load one per thread),
-// and at most kPinOut results are written there by the finishing kernels; the
-// control block goes up in k_sample's parameters and comes back by k_finish's
-// last CTA.  Such a call puts no copy on the stream.  More requests go up in a
-// copy (several kernels read them, several times), and more results come back
-// in one (their scattered 4- and 8-byte stores would cross the link one by one).
+// Host k lists are read from pinned host memory (k_sample, the small-vector
+// kernels), and at most kPinOut results are written there by the finishing
+// kernels; the control block goes up in the first kernel's parameters and comes
+// back by k_finish's last CTA.  Such a call puts no copy on the stream.  More
+// results come back in one copy (their scattered 4- and 8-byte stores would
+// cross the link one by one).
 // (2^20 floats, 101 k's: 72 -> 65 us a call; 5003 floats, 11 k's: 47 -> 43 us;
 // 10 M floats, 257 k's: 96 -> 91 us.)
-constexpr uint32_t kPinReq = 1024;
 constexpr uint32_t kPinOut = 4096;
 
 template <class InT, class OutT>
@@ -83,8 +82,7 @@ static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req) {
   Plan p;
   p.n = n;
   p.num_req = num_req;
-  p.S = n <= 65536 ? (uint32_t)n : 65536u;
-  p.sample_grid = (p.S + 1023) / 1024;
+  p.S = n <= kFrontSamples ? (uint32_t)n : kFrontSamples;
   uint64_t want = n / 32;
   uint32_t nb = 8192;
   while (nb < kMaxNb && (uint64_t)nb * 2 <= want) nb *= 2;
@@ -119,9 +117,7 @@ static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req) {
   p.cand_chunks = (uint32_t)(chunks < 0xFFFFFFFFull ? chunks : 0xFFFFFFFFull);
 
   const size_t A = 256;
-  // the arena's head: per-slice sample counts of k_lut, zero between
-  // calls (the arena starts zeroed; every call leaves them zero)
-  size_t o = kSliceCntBytes;
+  size_t o = 0;
   p.out = o;
   o = align_up(o + (size_t)num_req * sizeof(OutT), A);
   p.ctrl = o;
@@ -135,14 +131,18 @@ static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req) {
   p.samples = o;
   o = align_up(o + (size_t)p.S * sizeof(K), A);
   p.spans = o;
-  o = align_up(o + 2 * (size_t)p.sample_grid * sizeof(K), A);
+  o = align_up(o + 2 * (size_t)front_ctas(p.S) * sizeof(K), A);
+  p.fine = o;
+  o = align_up(o + kLutIdx * sizeof(uint32_t) + sizeof(SliceOut<K>), A);
   p.partials = o;
   o = align_up(o + (size_t)p.G * p.nb_max * sizeof(uint32_t), A);
   auto arr = [&](size_t &off, size_t elems, size_t esz) {
     off = o;
     o = align_up(o + elems * esz, A);
   };
+  arr(p.sorted, kPlanFew, sizeof(Req));
   arr(p.bpre, p.nb_max, 4);
+  arr(p.bco, p.nb_max / 8, 4);
   arr(p.ttot, p.scan_tiles, 4);
   arr(p.seg_bucket, p.nb_max, 4);
   arr(p.seg_off, p.nb_max, 8);
@@ -299,8 +299,6 @@ static void collect_pass_times(Context &ctx, const bool *ran) {
   }
 }
 
-__global__ void k_make_topk_reqs(Req *reqs, uint64_t n, uint32_t K);
-
 // Rank windows for speculative compaction: one window over all requested
 // ranks, or, for up to 64 requests, two windows split at the widest gap
 // between neighbouring ranks.  The table builder widens them by the sample's
@@ -344,8 +342,8 @@ static inline void set_windows(Ctrl *ci, const Req *hr, uint32_t num_req, uint64
   if (span > n / 16) ci->spec_nwin = 0;
 }
 
-// Top-k by a sampled threshold (ggks_topk.cuh): k_sample, k_tau, k_filter,
-// k_pick.  *missed: the candidates fell short (or did not fit), nothing is
+// Top-k by a sampled threshold (ggks_topk.cuh): k_sample, k_bin, k_slice,
+// k_filter, k_pick.  *missed: the candidates fell short (or did not fit), nothing is
 // answered, and the caller runs the pipeline; d_in then holds the device copy
 // of an ingested host vector.
 template <class InT>
@@ -364,7 +362,8 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   Kt *tau = reinterpret_cast<Kt *>(A + p.hdr);
   Kt *samples = reinterpret_cast<Kt *>(A + p.samples);
   Kt *spans = reinterpret_cast<Kt *>(A + p.spans);
-  uint32_t *slice_cnt = reinterpret_cast<uint32_t *>(A);
+  uint32_t *fine = reinterpret_cast<uint32_t *>(A + p.fine);
+  SliceOut<Kt> *slice = reinterpret_cast<SliceOut<Kt> *>(fine + kLutIdx);
   Kt *arr = reinterpret_cast<Kt *>(ctx.surv);  // the candidate array
   const uint64_t arr_cap = p.surv_cap;
   InT *d_out = d_out_user;
@@ -386,19 +385,28 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   L(set_smem_max<k_filter<InT, 8>>(filt_smem));
   L(set_smem_max<k_filter<InT, 4>>(filt_smem));
   bool ran[GGKS_NUM_PASSES] = {false, false, false, false, false, false};
+  bool open = false;  // no threshold: every key is a candidate
   {
     PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
-    L(launch(k_sample<InT>, p.sample_grid, 1024, 0, s, ingest ? ingest : d_in, n, p.S, 0x5EEDu,
-             samples, spans, ctrl, Ctrl{}));
-    L(launch(k_tau<Kt>, p.sample_grid, 1024, 0, s, samples, p.S, spans, ctrl, slice_cnt, n, K,
-             tau));
-    ctx.stats.launches++;
+    const uint32_t g = front_ctas(p.S);
+    L(launch(k_sample<InT>, g, 1024, 0, s, ingest ? ingest : d_in, n, p.S, 0x5EEDu, samples, spans,
+             fine, kLutIdx + 4u, ctrl, Ctrl{}, ReqCopy{}));
+    L(launch(k_bin<Kt>, g, 1024, 0, s, samples, p.S, spans, fine, ctrl));
+    // the sample rank below the K-th largest's, with six standard deviations
+    // and four ranks to spare
+    const double pl = (double)(n - K) / (double)n, S = p.S;
+    const double a = pl * S - (6.0 * std::sqrt(S * pl * (1.0 - pl)) + 4.0);
+    open = !(a > 0.0);  // the window reaches the smallest sample
+    SliceWant want{};
+    want.rank[0] = open ? 0u : (a >= S - 1.0 ? p.S - 1u : (uint32_t)a);
+    L(launch(k_slice<Kt, 1>, g, 1024, 0, s, samples, p.S, spans, fine, want, slice));
+    ctx.stats.launches += 2;
     ran[GGKS_PASS_SAMPLE] = true;
   }
   {
     PassTimer t(ctx, s, GGKS_PASS_HIST);
     L(launch(p.unroll8 ? k_filter<InT, 8> : k_filter<InT, 4>, p.G, 1024, filt_smem, s,
-             ingest ? ingest : d_in, n, tau, arr, arr_cap, &ctrl->cand_next,
+             ingest ? ingest : d_in, n, slice, open, tau, arr, arr_cap, &ctrl->cand_next,
              ingest ? const_cast<InT *>(d_in) : nullptr, ctrl));
     ran[GGKS_PASS_HIST] = true;
   }
@@ -433,7 +441,7 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
 // (kSmMaxTopkN for a top-k) elements.
 // *missed: the kernel met a case it leaves to the pipeline (nothing is
 // answered; the caller runs the pipeline, which writes every output again).
-// Arena: [slice counts | phase stamps | cursors' starts]; pinned host memory,
+// Arena: [phase stamps | cursors' starts]; pinned host memory,
 // which the kernel reads and writes in place: [out | status | requests].
 template <class InT, class OutT>
 static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src,
@@ -442,10 +450,10 @@ static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSour
   using K = typename Traits<InT>::K;
   *missed = false;
   const size_t out_span = align_up((size_t)num_req * sizeof(OutT), 256);
-  const size_t o_ctrl = kSliceCntBytes, o_chk = o_ctrl + 256;
+  const size_t o_ctrl = 0, o_chk = o_ctrl + 256;
   cudaError_t e = ensure_pin(ctx, out_span + 256 + (size_t)num_req * sizeof(Req));
   if (e != cudaSuccess) return from_cuda(e);
-  static_assert(kSmMaxReq <= kPinReq && kSmMaxReq <= kPinOut && kSmCtas * 4 <= 256,
+  static_assert(kSmMaxReq <= kPinOut && kSmCtas * 4 <= 256,
                 "requests, results and status in place");
   OutT *d_out = d_out_user ? d_out_user : reinterpret_cast<OutT *>(ctx.pin_dev);
   const volatile uint32_t *h_status = reinterpret_cast<const uint32_t *>(ctx.pin + out_span);
@@ -580,13 +588,15 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   char *A = ctx.arena;
   Ctrl *ctrl = reinterpret_cast<Ctrl *>(A + p.ctrl);
   Req *reqs = reinterpret_cast<Req *>(A + p.reqs);
+  Req *sorted = reinterpret_cast<Req *>(A + p.sorted);
   LutHeader<K> *hdr = reinterpret_cast<LutHeader<K> *>(A + p.hdr);
   uint32_t *lut = reinterpret_cast<uint32_t *>(A + p.lut);
   K *samples = reinterpret_cast<K *>(A + p.samples);
   K *spans = reinterpret_cast<K *>(A + p.spans);
-  uint32_t *slice_cnt = reinterpret_cast<uint32_t *>(A);
+  uint32_t *fine = reinterpret_cast<uint32_t *>(A + p.fine);
   uint32_t *partials = reinterpret_cast<uint32_t *>(A + p.partials);
   uint32_t *bpre = reinterpret_cast<uint32_t *>(A + p.bpre);  // prefix inside 64-bucket tiles
+  uint32_t *bco = reinterpret_cast<uint32_t *>(A + p.bco);    // every eighth of them
   uint32_t *ttot = reinterpret_cast<uint32_t *>(A + p.ttot);  // the tiles' totals
   uint32_t *seg_bucket = reinterpret_cast<uint32_t *>(A + p.seg_bucket);
   uint64_t *seg_off = reinterpret_cast<uint64_t *>(A + p.seg_off);
@@ -610,9 +620,8 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   K *bkey = reinterpret_cast<K *>(A + p.bkey);
   // pinned host memory: [out | control block | requests]
   const bool want_host = host_results != nullptr;
-  const bool host_reqs = src.h_k || (src.topk && num_req <= kPinReq);
   const size_t out_span = p.ctrl - p.out;  // == align_up(num_req * sizeof(OutT), 256)
-  e = ensure_pin(ctx, out_span + 256 + (host_reqs ? (size_t)num_req * sizeof(Req) : 0));
+  e = ensure_pin(ctx, out_span + 256 + (src.h_k ? (size_t)num_req * sizeof(Req) : 0));
   if (e != cudaSuccess) return from_cuda(e);
   Ctrl *h_ctrl = reinterpret_cast<Ctrl *>(ctx.pin + out_span);
   Ctrl *h_ctrl_dev = reinterpret_cast<Ctrl *>(ctx.pin_dev + out_span);
@@ -622,22 +631,17 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
                 : out_in_pin ? reinterpret_cast<OutT *>(ctx.pin_dev)
                              : reinterpret_cast<OutT *>(A + p.out);
   Ctrl ci{};  // the control block's initial words
-  const Req *rq = src.d_reqs ? src.d_reqs : reqs;
-  if (host_reqs) {
+  const Req *rq = src.d_reqs;  // where k_sample finds the requests (null: a top-k)
+  if (src.h_k) {
     // every call ends with a stream synchronisation, so nothing of an earlier
     // one still reads the pinned buffer here
     Req *hr = reinterpret_cast<Req *>(ctx.pin + out_span + 256);
     for (uint32_t i = 0; i < num_req; ++i) {
-      hr[i].rank = src.h_k ? (uint32_t)(n - src.h_k[i]) : (uint32_t)(n - 1 - i);
+      hr[i].rank = (uint32_t)(n - src.h_k[i]);
       hr[i].out = i;
     }
-    if (src.h_k) set_windows(&ci, hr, num_req, n);
-    if (num_req <= kPinReq) {
-      rq = reinterpret_cast<const Req *>(ctx.pin_dev + out_span + 256);
-    } else {
-      e = cudaMemcpyAsync(reqs, hr, (size_t)num_req * sizeof(Req), cudaMemcpyHostToDevice, s);
-      if (e != cudaSuccess) return from_cuda(e);
-    }
+    set_windows(&ci, hr, num_req, n);
+    rq = reinterpret_cast<const Req *>(ctx.pin_dev + out_span + 256);
   }
   if (src.topk && num_req && (uint64_t)num_req <= n / 16) {
     ci.spec_nwin = 1;
@@ -649,19 +653,23 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   auto L = [&le](cudaError_t r) {
     if (le == cudaSuccess) le = r;
   };
-  if (src.topk && !host_reqs) {
-    L(launch(k_make_topk_reqs, (num_req + 255) / 256, 256, 0, s, reqs, n, num_req));
-    ctx.stats.launches++;
-  }
-
-  // ---- (b) sample + splitter table
+  // ---- (b) sample + splitter table; the requests
+  const bool few = num_req <= kPlanFew;
   {
     PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
-    L(launch(k_sample<InT>, p.sample_grid, 1024, 0, s, ingest ? ingest : d_in, n, p.S, 0x5EEDu,
-             samples, spans, ctrl, ci));
-    L(launch(k_lut<K>, p.sample_grid, 1024, 0, s, samples, p.S, spans, ctrl, hdr, lut, p.nb_max,
-             slice_cnt, n, p.cand_chunks, p.G));
-    ctx.stats.launches++;
+    const uint32_t g = front_ctas(p.S);
+    // device requests of a recursive level are read in place
+    const ReqCopy bring{rq, reqs, src.d_reqs ? 0u : num_req};
+    const Req *raw = src.d_reqs ? src.d_reqs : reqs;
+    L(launch(k_sample<InT>, g + (bring.num + 1023) / 1024, 1024, 0, s, ingest ? ingest : d_in, n,
+             p.S, 0x5EEDu, samples, spans, fine, kLutIdx, ctrl, ci, bring));
+    L(launch(k_bin<K>, g, 1024, 0, s, samples, p.S, spans, fine, ctrl));
+    const RankWindows win{ci.spec_nwin, {ci.spec_lo[0], ci.spec_lo[1]}, {ci.spec_hi[0], ci.spec_hi[1]}};
+    const ReqCopy sort{raw, sorted, few ? num_req : 0u};
+    L(launch(k_table<K>, 1 + sort_ctas(sort.num), kTableThreads, 0, s, samples, p.S, spans, fine, n,
+             win, hdr, lut, p.nb_max, p.cand_chunks, p.G, ctrl, sort));
+    rq = few ? sorted : raw;
+    ctx.stats.launches += 2;
     ran[GGKS_PASS_SAMPLE] = true;
   }
   // ---- (c) histogram
@@ -680,7 +688,7 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   {
     PassTimer t(ctx, s, GGKS_PASS_SCAN);
     L(launch(k_colsum<K>, p.scan_tiles, kScanThreads, 0, s, partials, p.G, p.nb_max, hdr, bpre,
-             ttot, ctrl, reps, bsingle, bkey));
+             bco, ttot, ctrl, reps, bsingle, bkey));
     ran[GGKS_PASS_SCAN] = true;
   }
   // ---- (e) plan
@@ -707,9 +715,14 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
       pm.bcount = pm_bcount;
       pm.bslot = pm_bslot;
     }
-    L(launch(k_plan<InT, OutT>, 1, 1024, smem, s, hdr, lut, bpre, ttot, n, rq, num_req, p.nb_max,
-             ctrl, seg_bucket, seg_off, seg_size, kstart, kcnt, kcur, fill, seg_lo, seg_hi,
-             req_bucket, req_local, klist, p.surv_cap, pm, bsingle, bkey));
+    if (few)
+      L(launch(k_plan_few<InT>, 1, 1024, 0, s, hdr, lut, bpre, bco, ttot, n, rq, num_req, p.nb_max, ctrl,
+               seg_bucket, seg_off, seg_size, kstart, kcnt, fill, seg_lo, seg_hi, klist, p.surv_cap,
+               bsingle, bkey));
+    else
+      L(launch(k_plan<InT, OutT>, 1, 1024, smem, s, hdr, lut, bpre, ttot, n, rq, num_req, p.nb_max,
+               ctrl, seg_bucket, seg_off, seg_size, kstart, kcnt, kcur, fill, seg_lo, seg_hi,
+               req_bucket, req_local, klist, p.surv_cap, pm, bsingle, bkey));
     if (premap) {
       L(launch(k_reqplace, (num_req + 1023) / 1024, 1024, 0, s, ctrl, rq, num_req, req_bucket,
                req_local, pm_bslot, kstart, kcur, klist));
@@ -758,9 +771,6 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   for (int round = 0; round < 4; ++round) {
     const Ctrl c = *h_ctrl;
     if (c.status & ST_FATAL) {
-      // a stopped call may leave slice counts behind
-      cudaMemsetAsync(slice_cnt, 0, kSliceCntBytes, s);
-      cudaStreamSynchronize(s);
       return (c.status & ST_TIMEOUT) ? GGKS_TIMEOUT : GGKS_INTERNAL;
     }
     if (c.status & ST_OVERFLOW) {

@@ -259,8 +259,8 @@ __global__ void __launch_bounds__(kSmThreads, 1)
     lo = block_reduce(lo, [](K u, K v) { return u < v ? u : v; }, redk);
     hi = block_reduce(hi, [](K u, K v) { return u > v ? u : v; }, redk);
     GGKS_SMALL_STAMP(1);
-    build_lut_cta<K, (int)(kLutIdx / kSmThreads), true>(samples, S, lo, hi, kSmNb, s_tab, &s_hdr,
-                                                        sv_bits<K>());
+    build_lut_cta<K, (int)((sv_slices<K>() + kSmThreads - 1) / kSmThreads)>(
+        samples, S, lo, hi, kSmNb, s_tab, &s_hdr, sv_bits<K>());
   }
   __syncthreads();
   GGKS_SMALL_STAMP(2);

@@ -7,16 +7,14 @@
 // list and calls the bucket multiselect, bucketMultiselect.cu:837-871), which
 // here is the histogram / plan / compaction / finish pipeline.  For K up to
 // kPickMax the K largest are found with less work:
-//   k_sample  the sample (shared with the pipeline);
-//   k_tau     bins the samples in 4096 fine slices of their span (as k_lut
-//             does); the last CTA finds the sample rank below which the K-th
-//             largest element's sample rank lies with overwhelming
+//   k_sample, k_bin, k_slice (ggks_front.cuh): the sample, and its keys around
+//             the threshold;
+//   k_filter  takes as the threshold tau the sample key of the rank below which
+//             the K-th largest element's sample rank lies with overwhelming
 //             probability (the rank of the K-th largest among S samples is
-//             about Binomial(S, 1 - K / n); six standard deviations plus four
-//             below its mean) and takes the sample key of that rank as the
-//             threshold tau (a radix select among the samples of the
-//             fine slice holding that rank);
-//   k_filter  streams the vector once: each key >= tau is appended to one
+//             about Binomial(S, 1 - K / n): six standard deviations and four
+//             ranks below its mean), and
+//             streams the vector once: each key >= tau is appended to one
 //             contiguous candidate array, nothing else is written;
 //   k_pick    one CTA: a 4096-bin histogram of the candidates over their key
 //             range, the bin holding the K-th largest, a gather of every
@@ -29,148 +27,13 @@
 
 #include <type_traits>
 
-#include "ggks_device.cuh"
+#include "ggks_front.cuh"
 
 namespace ggks {
 
 constexpr uint32_t kPickMax = 4096;     // largest K of the threshold path
 constexpr uint32_t kPickBins = 4096;    // k_pick's histogram
 constexpr uint32_t kPickCap = 8192;     // keys k_pick gathers and sorts at most
-constexpr uint32_t kTauBuf = 2048;      // samples of the threshold's fine slice k_tau sorts
-
-// ---------------------------------------------------------------------------
-// k_tau: the threshold from the sample
-// ---------------------------------------------------------------------------
-// Grid: ceil(S / 1024) CTAs of 1024 threads, after k_sample (spans).
-// slice_cnt (global, kLutIdx words) is zero on entry and left zero.  The last
-// CTA writes tau (0: no useful threshold, which the caller treats as a miss).
-template <class K>
-__global__ void __launch_bounds__(1024) k_tau(const K *__restrict__ samples, uint32_t S,
-                                              const K *__restrict__ spans, Ctrl *ctrl,
-                                              uint32_t *slice_cnt, uint64_t n, uint32_t kk,
-                                              K *tau) {
-  pdl_start();
-  __shared__ uint32_t red32[33];
-  __shared__ uint32_t s_last, s_jf, s_r, s_cnt;
-  __shared__ uint32_t ccnt[kLutIdx];
-  __shared__ K buf[kTauBuf];
-  __shared__ uint32_t s_rcnt[256], s_rsel[2];
-  const uint32_t tid = threadIdx.x;
-  const uint32_t i = blockIdx.x * blockDim.x + tid;
-  for (uint32_t j = tid; j < kLutIdx; j += blockDim.x) ccnt[j] = 0;
-  const K k = i < S ? __ldcg(samples + i) : K(0);
-  K kmin, kmax;
-  sample_span<K>(spans, gridDim.x, &kmin, &kmax);
-  const int bl = bitlen<K>(kmax - kmin);
-  const uint32_t fsh = bl > kLutIdxBits ? (uint32_t)(bl - kLutIdxBits) : 0u;
-  __syncthreads();
-  if (i < S) atomicAdd(&ccnt[(uint32_t)((k - kmin) >> fsh)], 1u);
-  __syncthreads();
-  for (uint32_t j = tid; j < kLutIdx; j += blockDim.x) {
-    const uint32_t c = ccnt[j];
-    if (c) atomicAdd(&slice_cnt[j], c);
-  }
-  // every thread's counts before the CTA reports done (the fence below is
-  // cumulative over what the barrier ordered)
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    s_last = (atomicAdd(&ctrl->sample_done, 1u) == gridDim.x - 1) ? 1u : 0u;
-    if (s_last) __threadfence();
-  }
-  __syncthreads();
-  if (!s_last) return;
-
-  // the sample rank below the K-th largest's, with six standard deviations and
-  // four ranks to spare (single precision: ranks need about one unit of 2^16)
-  const float dS = (float)S;
-  const float pl = (float)(n - kk) / (float)n;
-  const float a = pl * dS - (6.0f * sqrtf(dS * pl * (1.0f - pl)) + 4.0f);
-  const bool open = !(a > 0.0f);  // the window reaches the smallest sample
-  const uint32_t wa = open ? 0u : (a >= dS - 1.0f ? S - 1u : (uint32_t)a);
-  // fine slice holding sample rank wa (4 fine slices per thread, in order)
-  const uint32_t per = kLutIdx / blockDim.x;
-  uint32_t fc[4], fsum = 0;
-#pragma unroll
-  for (uint32_t q = 0; q < 4; ++q) {
-    const uint32_t j = per * tid + q;
-    fc[q] = q < per ? __ldcg(slice_cnt + j) : 0u;
-    if (q < per) slice_cnt[j] = 0;  // zero for the next call
-    fsum += fc[q];
-  }
-  if (tid == 0) {
-    s_jf = 0;
-    s_r = 0;
-    s_cnt = 0;
-  }
-  uint32_t ftot;
-  uint32_t fpre = block_incl_scan(fsum, &ftot, red32) - fsum;
-#pragma unroll
-  for (uint32_t q = 0; q < 4; ++q) {
-    if (q < per && fc[q] && fpre <= wa && wa < fpre + fc[q]) {
-      s_jf = per * tid + q;
-      s_r = wa - fpre;
-    }
-    fpre += fc[q];
-  }
-  __syncthreads();
-  const uint32_t jf = s_jf, r = s_r;
-  // the samples of that fine slice; their r-th smallest is tau.  Eight
-  // 128-bit loads per thread in flight before their compares (a load and a
-  // shared atomic in one loop body would complete one at a time): 65 536
-  // four-byte samples take two rounds.  The sample array starts 256-byte aligned; keys
-  // past its last whole vector are read one by one.
-  using SV = typename std::conditional<sizeof(K) == 4, uint4, ulonglong2>::type;
-  constexpr uint32_t PV = 16 / sizeof(K);
-  const uint32_t nv = S / PV;
-  const SV *sv = reinterpret_cast<const SV *>(samples);
-  // the slice holds a few dozen samples: a lane that finds one takes its
-  // place with its own shared atomic (no vote per key)
-  auto take = [&](K key, bool valid) {
-    if (valid && (uint32_t)((key - kmin) >> fsh) == jf) {
-      const uint32_t at = atomicAdd(&s_cnt, 1u);
-      if (at < kTauBuf) buf[at] = key;
-    }
-  };
-  for (uint32_t v0 = tid; v0 < nv; v0 += 8 * blockDim.x) {
-    SV xs[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const uint32_t q = v0 + u * blockDim.x;
-      if (q < nv) xs[u] = __ldcg(sv + q);
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const bool ok = v0 + u * blockDim.x < nv;
-      if constexpr (sizeof(K) == 4) {
-        take(ok ? (K)xs[u].x : kmin, ok);
-        take(ok ? (K)xs[u].y : kmin, ok);
-        take(ok ? (K)xs[u].z : kmin, ok);
-        take(ok ? (K)xs[u].w : kmin, ok);
-      } else {
-        take(ok ? (K)xs[u].x : kmin, ok);
-        take(ok ? (K)xs[u].y : kmin, ok);
-      }
-    }
-  }
-  for (uint32_t q = nv * PV + tid; q < S; q += blockDim.x) take(__ldcg(samples + q), true);
-  __syncthreads();
-  const uint32_t cnt = s_cnt;
-  K t;
-  if (open) {
-    t = K(0);
-  } else if (cnt > kTauBuf || r >= cnt) {
-    t = kmin + ((K)jf << fsh);  // the fine slice's first key: a lower threshold
-  } else {
-    // the r-th smallest of the slice's samples by radix select (16 block
-    // barriers for 4-byte keys; a bitonic sort of up to 2048 keys took 66)
-    t = cta_select_rank<K>(buf, cnt, r, s_rcnt, s_rsel);
-  }
-  if (tid == 0) {
-    *tau = t;
-    ctrl->sample_done = 0;  // re-arm for the next call on this workspace
-  }
-}
 
 // ---------------------------------------------------------------------------
 // k_filter: one pass, keys >= tau appended to one contiguous array
@@ -287,21 +150,26 @@ __device__ __forceinline__ void filter_body(const T *__restrict__ x, uint64_t n,
   }
 }
 
-// Grid and tiles as k_hist; 1024 threads; dynamic shared memory
+// The threshold is the key of slice's list 0, or 0 (open: the rank reaches the
+// smallest sample, every key is a candidate).  Grid and tiles as k_hist; 1024
+// threads; dynamic shared memory
 // kCandWarps * kFiltBuf keys.  arr[0 .. cap) receives the candidates and
 // *len (zero on entry) their count.
 template <class T, int UNROLL>
 __global__ void __launch_bounds__(1024, 1)
-    k_filter(const T *__restrict__ x, uint64_t n, const typename Traits<T>::K *tau,
-             typename Traits<T>::K *__restrict__ arr, uint64_t cap, uint32_t *len,
-             T *__restrict__ copy_to, const Ctrl *ctrl) {
+    k_filter(const T *__restrict__ x, uint64_t n, const SliceOut<typename Traits<T>::K> *slice,
+             bool open, typename Traits<T>::K *tau, typename Traits<T>::K *__restrict__ arr,
+             uint64_t cap, uint32_t *len, T *__restrict__ copy_to, const Ctrl *ctrl) {
   pdl_start();
   using K = typename Traits<T>::K;
   extern __shared__ uint4 smem_raw[];
   __shared__ uint32_t s_wcnt[kCandWarps];
   __shared__ uint32_t s_base;
-  if (ctrl->status & ST_FATAL) return;
-  const K t = *tau;
+  __shared__ RankShared<K> s_rank;
+  const uint32_t status = ctrl->status;
+  const K t = open ? K(0) : rank_key<K>(slice, 0, s_rank);
+  if (status & ST_FATAL) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *tau = t;  // for k_pick
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   FiltWarp<K> fw;
   fw.buf = reinterpret_cast<K *>(smem_raw) + warp * kFiltBuf;
