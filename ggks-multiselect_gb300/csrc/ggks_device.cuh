@@ -2805,7 +2805,7 @@ __global__ void __launch_bounds__(kFinThreads)
   pdl_start();
   extern __shared__ uint4 smem_raw[];
   const uint32_t num_slots =
-      (ctrl->status & (ST_FATAL | ST_OVERFLOW)) ? 0u : ctrl->num_slots;
+      (ctrl->status & (ST_FATAL | ST_OVERFLOW | ST_TOPK_MISS)) ? 0u : ctrl->num_slots;
   for (uint32_t slot = blockIdx.x; slot < num_slots; slot += gridDim.x) {
     const bool done = finish_slot<K, OutT>(surv + seg_off[slot], seg_size[slot], seg_lo[slot],
                                            seg_hi[slot], klist + kstart[slot], kcnt[slot], bcap,

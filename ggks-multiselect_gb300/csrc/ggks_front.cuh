@@ -7,7 +7,7 @@
 //   k_slice   the samples of the fine slices that hold given sample ranks
 //             (thresholds of a top-k, ggks_topk.cuh)
 //
-// Workspace: [fine counts kLutIdx words][SliceOut].
+// Workspace: [fine counts kLutIdx words][window path's bins and counters][SliceOut].
 //
 // Bound: latency.  A kernel boundary under programmatic dependent launch costs
 // about 0.9 us here, less than any other way for CTAs to wait for one another:
@@ -454,14 +454,20 @@ __global__ void __launch_bounds__(kTableThreads, 1)
 struct SliceWant {
   uint32_t rank[2];  // 0-based among the S samples
 };
-constexpr uint32_t kSliceBuf = 1024;  // samples of one list that are ranked
+// samples of one list that are ranked (values of 8 bits put 2048 samples into a
+// fine slice; an unranked slice widens the window by its other values)
+constexpr uint32_t kSliceBuf = 4096;
 template <class K>
 struct SliceOut {
-  uint32_t cnt[2];   // samples in the slice (zero on entry)
-  uint32_t rank[2];  // the wanted rank inside the slice
-  K first[2];        // the slice's first key
+  uint32_t at[2];                // list lengths so far (zero on entry)
+  uint32_t pad[2];
+  unsigned long long lo_inv[2];  // slices of more than kSliceBuf samples: the
+  unsigned long long hi[2];      // complement of the smallest and the largest (zero on entry)
+  uint32_t cnt[2];               // samples in the slice
+  uint32_t rank[2];              // the wanted rank inside the slice
   K buf[2][kSliceBuf];
 };
+constexpr uint32_t kSliceZeroWords = 12;  // words that are zero on entry
 
 template <class K, int W>
 __global__ void __launch_bounds__(1024)
@@ -470,12 +476,12 @@ __global__ void __launch_bounds__(1024)
             SliceOut<K> *out) {
   pdl_start();
   __shared__ uint32_t s_scan[32];
-  __shared__ uint32_t s_slice[W], s_rank[W];
+  __shared__ uint32_t s_slice[W], s_rank[W], s_cnt[W];
   const uint32_t tid = threadIdx.x, i = blockIdx.x * 1024 + tid;
   const uint4 c4 = __ldcg(reinterpret_cast<const uint4 *>(fine_g) + tid);
   const K k = i < S ? __ldcg(samples + i) : K(0);
   const SampleSpan<K> sp = sample_span<K>(spans, gridDim.x);
-  if (tid < W) s_slice[tid] = s_rank[tid] = 0;
+  if (tid < W) s_slice[tid] = s_rank[tid] = s_cnt[tid] = 0;
   const uint32_t fc[4] = {c4.x, c4.y, c4.z, c4.w};
   uint32_t all;
   uint32_t pre = block_excl_scan(fc[0] + fc[1] + fc[2] + fc[3], s_scan, &all);
@@ -486,6 +492,7 @@ __global__ void __launch_bounds__(1024)
       if (fc[q] && pre <= want.rank[w] && want.rank[w] < pre + fc[q]) {
         s_slice[w] = 4 * tid + q;
         s_rank[w] = want.rank[w] - pre;
+        s_cnt[w] = fc[q];
       }
     pre += fc[q];
   }
@@ -493,22 +500,38 @@ __global__ void __launch_bounds__(1024)
   const uint32_t j = (uint32_t)((k - sp.kmin) >> sp.shift);
 #pragma unroll
   for (int w = 0; w < W; ++w) {
-    if (i < S && j == s_slice[w]) {
-      const uint32_t at = atomicAdd(&out->cnt[w], 1u);
-      if (at < kSliceBuf) out->buf[w][at] = k;
+    const bool in = i < S && j == s_slice[w];
+    if (s_cnt[w] <= kSliceBuf) {
+      if (in) {
+        const uint32_t at = atomicAdd(&out->at[w], 1u);
+        if (at < kSliceBuf) out->buf[w][at] = k;
+      }
+    } else if (__any_sync(0xffffffffu, in)) {
+      K lo = in ? k : KeyMax<K>::v, hi = in ? k : K(0);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const K a = __shfl_xor_sync(0xffffffffu, lo, o), z = __shfl_xor_sync(0xffffffffu, hi, o);
+        lo = a < lo ? a : lo;
+        hi = z > hi ? z : hi;
+      }
+      if ((tid & 31) == 0) {
+        atomicMax(&out->lo_inv[w], (unsigned long long)~(uint64_t)lo);
+        atomicMax(&out->hi[w], (unsigned long long)hi);
+      }
     }
     if (i == 0) {
       out->rank[w] = s_rank[w];
-      out->first[w] = sp.kmin + ((K)s_slice[w] << sp.shift);
+      out->cnt[w] = s_cnt[w];
     }
   }
 }
 
 // The key of the wanted rank of list w, by the whole CTA (1024 threads): up to
 // 256 samples are ranked by counting the samples before each (four threads per
-// sample), more by a radix select.  A list of more than kSliceBuf samples gives
-// the slice's first key (a smaller one).  Everything is loaded in one round
-// (the list's unused end too), through L1; ends with a barrier.
+// sample), more by a radix select.  A slice of more than kSliceBuf samples gives
+// its smallest sample (list 0) or its largest (list 1): a wider window.  A list
+// of up to 1024 samples comes in one round of loads (with its unused end),
+// through L1; ends with a barrier.
 template <class K>
 struct RankShared {
   K keys[kSliceBuf];
@@ -519,10 +542,10 @@ template <class K>
 __device__ __forceinline__ K rank_key(const SliceOut<K> *out, int w, RankShared<K> &sh) {
   const uint32_t tid = threadIdx.x;
   const uint32_t cnt = out->cnt[w], r = out->rank[w];
-  const K first = out->first[w];
-  static_assert(kSliceBuf == 1024, "a sample per thread");
   sh.keys[tid] = out->buf[w][tid];
-  if (tid == 0) sh.found = first;
+  if (tid == 0) sh.found = (K)(w == 0 ? ~out->lo_inv[w] : out->hi[w]);
+  if (cnt <= kSliceBuf)
+    for (uint32_t i = 1024 + tid; i < cnt; i += 1024) sh.keys[i] = out->buf[w][i];
   __syncthreads();
   if (cnt <= kSliceBuf && r < cnt) {
     if (cnt <= 256) {

@@ -16,6 +16,7 @@
 #include "ggks_small.cuh"
 #include "ggks_tiny.cuh"
 #include "ggks_topk.cuh"
+#include "ggks_window.cuh"
 
 namespace ggks {
 
@@ -43,6 +44,16 @@ constexpr size_t kPlanSlotBytes = 6144 * 8;
 constexpr int kPlanSmemMax = (int)(kLutPadded * sizeof(uint32_t) + (size_t)kMaxNb * 5 + 16 +
                                    kPlanSlotBytes);
 
+// The words after the fine counts, cleared by k_sample with them where a path
+// uses them: the window path's bins, cursors, large bins' extreme keys (64-bit)
+// and counters, then the sample keys around thresholds (SliceOut, whose first
+// words are cleared too).
+constexpr uint32_t kWinBinsAt = kLutIdx, kWinCurAt = kWinBinsAt + kWinBins,
+                   kWinLoAt = kWinCurAt + kWinBins, kWinHiAt = kWinLoAt + 2 * kWinBins,
+                   kWinCtlAt = kWinHiAt + 2 * kWinBins, kFineWords = kWinCtlAt + 16;
+static_assert(sizeof(WinCtl<uint64_t>) <= 64 && kWinLoAt % 2 == 0 && kFineWords % 4 == 0,
+              "the counters' place and alignment");
+
 struct Plan {
   uint64_t n = 0;
   uint32_t num_req = 0;
@@ -55,7 +66,7 @@ struct Plan {
   uint32_t fin_grid = 0;
   uint64_t surv_cap = 0;
   // arena offsets
-  size_t out = 0, ctrl = 0, reqs = 0, hdr = 0, lut = 0, samples = 0, spans = 0, fine = 0, partials = 0, sorted = 0,
+  size_t out = 0, ctrl = 0, reqs = 0, hdr = 0, lut = 0, samples = 0, spans = 0, fine = 0, wpre = 0, partials = 0, sorted = 0,
          bpre = 0, bco = 0, ttot = 0, seg_bucket = 0, seg_off = 0, seg_size = 0, kstart = 0, kcnt = 0, fill = 0,
          kcur = 0, seg_lo = 0, seg_hi = 0, deferred = 0, req_bucket = 0, req_local = 0, klist = 0,
          pm_bits = 0, pm_bcount = 0, pm_bslot = 0, cand_cnt = 0, cand_tab = 0, reps = 0,
@@ -133,7 +144,9 @@ static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req) {
   p.spans = o;
   o = align_up(o + 2 * (size_t)front_ctas(p.S) * sizeof(K), A);
   p.fine = o;
-  o = align_up(o + kLutIdx * sizeof(uint32_t) + sizeof(SliceOut<K>), A);
+  o = align_up(o + kFineWords * sizeof(uint32_t) + sizeof(SliceOut<K>), A);
+  p.wpre = o;
+  o = align_up(o + kWinBins * sizeof(uint32_t), A);
   p.partials = o;
   o = align_up(o + (size_t)p.G * p.nb_max * sizeof(uint32_t), A);
   auto arr = [&](size_t &off, size_t elems, size_t esz) {
@@ -363,7 +376,7 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   Kt *samples = reinterpret_cast<Kt *>(A + p.samples);
   Kt *spans = reinterpret_cast<Kt *>(A + p.spans);
   uint32_t *fine = reinterpret_cast<uint32_t *>(A + p.fine);
-  SliceOut<Kt> *slice = reinterpret_cast<SliceOut<Kt> *>(fine + kLutIdx);
+  SliceOut<Kt> *slice = reinterpret_cast<SliceOut<Kt> *>(fine + kFineWords);
   Kt *arr = reinterpret_cast<Kt *>(ctx.surv);  // the candidate array
   const uint64_t arr_cap = p.surv_cap;
   InT *d_out = d_out_user;
@@ -390,7 +403,7 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
     PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
     const uint32_t g = front_ctas(p.S);
     L(launch(k_sample<InT>, g, 1024, 0, s, ingest ? ingest : d_in, n, p.S, 0x5EEDu, samples, spans,
-             fine, kLutIdx + 4u, ctrl, Ctrl{}, ReqCopy{}));
+             fine, kFineWords + kSliceZeroWords, ctrl, Ctrl{}, ReqCopy{}));
     L(launch(k_bin<Kt>, g, 1024, 0, s, samples, p.S, spans, fine, ctrl));
     // the sample rank below the K-th largest's, with six standard deviations
     // and four ranks to spare
@@ -431,6 +444,159 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
     return GGKS_OK;
   }
   ctx.stats.topk_threshold_calls++;
+  if (want_host) *host_results = reinterpret_cast<const InT *>(ctx.pin);
+  return GGKS_OK;
+}
+
+// The window path's choice (ggks_window.cuh): the sample ranks around the
+// requested ascending ranks [rlo, rhi] -- six standard deviations and four ranks
+// outside them, or an open end -- and the candidates to expect.
+struct WindowPlan {
+  bool ok = false, lo_open = false, hi_open = false;
+  SliceWant want{};
+  double expect = 0.0;
+};
+// Taken for ranks that span at most n / 32 of a vector of more than 2^18
+// elements (the pipeline's speculating pass and its further kernels cost more:
+// 2^26 uint32, top-65536: 167 us a call, here 94; the median of 50 M floats 132,
+// here 77; of a smaller vector the sample is a good part, and most calls on one
+// take the one-launch path), when the window is closed on one side at least and the
+// candidates, with half again to spare, fit the survivor buffer's lower half.
+// A top-k also needs bins that a warp can sort: at most 32 keys on average.
+static inline WindowPlan plan_window(const Plan &p, uint64_t rlo, uint64_t rhi, bool topk) {
+  WindowPlan w;
+  const double n = (double)p.n, S = p.S;
+  if (p.n <= (1u << 18) || (rhi - rlo + 1) * 32 > p.n) return w;
+  const double pl = rlo / n, ph = (rhi + 1) / n;
+  const double a = pl * S - (6.0 * std::sqrt(S * pl * (1.0 - pl)) + 4.0);
+  const double b = ph * S + (6.0 * std::sqrt(S * ph * (1.0 - ph)) + 4.0);
+  w.lo_open = a <= 0.0;
+  w.hi_open = b >= S - 1.0;
+  if (w.lo_open && w.hi_open) return w;
+  w.want.rank[0] = w.lo_open ? 0u : (uint32_t)a;
+  w.want.rank[1] = w.hi_open ? p.S - 1u : (uint32_t)b;
+  w.expect = ((w.hi_open ? S : b) - (w.lo_open ? 0.0 : a)) / S * n;
+  w.ok = w.expect * 1.5 <= (double)p.surv_half && (!topk || w.expect <= 32.0 * kWinBins);
+  return w;
+}
+
+// *missed: as in topk_threshold.
+template <class InT>
+static int select_window(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src,
+                         uint32_t num_req, uint64_t rlo, uint64_t rhi, InT *d_out_user,
+                         const InT **host_results, cudaStream_t s, const InT *ingest,
+                         bool *missed) {
+  using K = typename Traits<InT>::K;
+  *missed = true;
+  const Plan p = make_plan<InT, InT>(ctx, n, num_req);
+  const WindowPlan w = plan_window(p, rlo, rhi, src.topk);
+  if (!w.ok) return GGKS_OK;
+  cudaError_t e = ensure_arena(ctx, p.total);
+  if (e != cudaSuccess) return from_cuda(e);
+  e = ensure_surv(ctx, (size_t)p.surv_cap * sizeof(K));
+  if (e != cudaSuccess) return from_cuda(e);
+  char *A = ctx.arena;
+  Ctrl *ctrl = reinterpret_cast<Ctrl *>(A + p.ctrl);
+  Req *reqs = reinterpret_cast<Req *>(A + p.reqs);
+  K *samples = reinterpret_cast<K *>(A + p.samples);
+  K *spans = reinterpret_cast<K *>(A + p.spans);
+  uint32_t *fine = reinterpret_cast<uint32_t *>(A + p.fine);
+  uint32_t *bins = fine + kWinBinsAt, *cur = fine + kWinCurAt;
+  auto *big_lo = reinterpret_cast<unsigned long long *>(fine + kWinLoAt);
+  auto *big_hi = reinterpret_cast<unsigned long long *>(fine + kWinHiAt);
+  WinCtl<K> *wc = reinterpret_cast<WinCtl<K> *>(fine + kWinCtlAt);
+  SliceOut<K> *slice = reinterpret_cast<SliceOut<K> *>(fine + kFineWords);
+  uint32_t *wpre = reinterpret_cast<uint32_t *>(A + p.wpre);
+  K *arr = reinterpret_cast<K *>(ctx.surv), *placed = arr + p.surv_half;
+  // pinned: [out | control block | requests]
+  const bool want_host = host_results != nullptr;
+  const size_t out_span = p.ctrl - p.out;
+  e = ensure_pin(ctx, out_span + 256 + (src.h_k ? (size_t)num_req * sizeof(Req) : 0));
+  if (e != cudaSuccess) return from_cuda(e);
+  Ctrl *h_ctrl = reinterpret_cast<Ctrl *>(ctx.pin + out_span);
+  // results in place: at most kPlanFew of a k list, and a top-k's warps write
+  // neighbouring ones (65536 uint32: 4 us a call less than by a copy)
+  static_assert(kPlanFew <= kPinOut, "results of a k list");
+  InT *d_out = d_out_user ? d_out_user : reinterpret_cast<InT *>(ctx.pin_dev);
+  if (src.h_k) {
+    Req *hr = reinterpret_cast<Req *>(ctx.pin + out_span + 256);
+    for (uint32_t i = 0; i < num_req; ++i) {
+      hr[i].rank = (uint32_t)(n - src.h_k[i]);
+      hr[i].out = i;
+    }
+  }
+  cudaError_t le = cudaSuccess;
+  auto L = [&le](cudaError_t r) {
+    if (le == cudaSuccess) le = r;
+  };
+  bool ran[GGKS_NUM_PASSES] = {false, false, false, false, false, false};
+  const uint32_t g = front_ctas(p.S);
+  {
+    PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
+    const ReqCopy bring{src.h_k ? reinterpret_cast<const Req *>(ctx.pin_dev + out_span + 256) : nullptr,
+                        reqs, src.h_k ? num_req : 0u};
+    L(launch(k_sample<InT>, g + (bring.num + 1023) / 1024, 1024, 0, s, ingest ? ingest : d_in, n,
+             p.S, 0x5EEDu, samples, spans, fine, kFineWords + kSliceZeroWords, ctrl, Ctrl{}, bring));
+    L(launch(k_bin<K>, g, 1024, 0, s, samples, p.S, spans, fine, ctrl));
+    L(launch(k_slice<K, 2>, g, 1024, 0, s, samples, p.S, spans, fine, w.want, slice));
+    ctx.stats.launches += 2;
+    ran[GGKS_PASS_SAMPLE] = true;
+  }
+  {
+    const int smem = (int)wfilter_smem_bytes<K>();
+    L(set_smem_max<k_wfilter<InT>>(smem));
+    PassTimer t(ctx, s, GGKS_PASS_HIST);
+    L(launch(k_wfilter<InT>, p.G, 1024, smem, s, ingest ? ingest : d_in, n, slice, spans, g,
+             w.lo_open, w.hi_open, wc, arr, p.surv_half, bins,
+             ingest ? const_cast<InT *>(d_in) : nullptr));
+    ran[GGKS_PASS_HIST] = true;
+  }
+  WinSlots<K> sl;
+  sl.seg_off = reinterpret_cast<uint64_t *>(A + p.seg_off);
+  sl.seg_size = reinterpret_cast<uint32_t *>(A + p.seg_size);
+  sl.kstart = reinterpret_cast<uint32_t *>(A + p.kstart);
+  sl.kcnt = reinterpret_cast<uint32_t *>(A + p.kcnt);
+  sl.seg_lo = reinterpret_cast<K *>(A + p.seg_lo);
+  sl.seg_hi = reinterpret_cast<K *>(A + p.seg_hi);
+  sl.klist = reinterpret_cast<Req *>(A + p.klist);
+  {
+    PassTimer t(ctx, s, GGKS_PASS_COMPACT);
+    const uint32_t grid = (uint32_t)std::min<double>(ctx.sm_count, 1.0 + w.expect / 4096.0);
+    L(launch(k_wplace<K>, grid, 1024, 0, s, arr, p.surv_half, n, src.topk ? num_req : 0u, w.lo_open,
+             w.hi_open, reqs, num_req, wc, bins, cur, wpre, placed, p.surv_cap - p.surv_half, big_lo,
+             big_hi, sl, ctrl));
+    ran[GGKS_PASS_COMPACT] = true;
+  }
+  Ctrl *h_ctrl_dev = reinterpret_cast<Ctrl *>(ctx.pin_dev + out_span);
+  {
+    PassTimer t(ctx, s, GGKS_PASS_FINISH);
+    if (src.topk) {
+      L(launch(k_wsort<K, InT>, 2u * (uint32_t)ctx.sm_count, kWinSortThreads, 0, s, placed, wc, bins,
+               wpre, big_lo, big_hi, num_req, d_out, ctrl, &h_ctrl_dev->status));
+    } else {
+      const int smem = finish_smem_bytes<InT>();
+      L(set_smem_max<k_finish<K, InT>>(smem));
+      L(launch(k_finish<K, InT>, num_req, kFinThreads, smem, s, placed, ctrl, sl.seg_off,
+               sl.seg_size, sl.seg_lo, sl.seg_hi, sl.kstart, sl.kcnt, sl.klist,
+               reinterpret_cast<uint32_t *>(A + p.deferred), p.cap_keys, d_out, h_ctrl_dev));
+    }
+    ran[GGKS_PASS_FINISH] = true;
+  }
+  e = le != cudaSuccess ? le : cudaGetLastError();
+  if (e != cudaSuccess) return from_cuda(e);
+  if (want_host && d_out_user)
+    e = cudaMemcpyAsync(ctx.pin, d_out, (size_t)num_req * sizeof(InT), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return from_cuda(e);
+  collect_pass_times(ctx, ran);
+  const uint32_t status = *reinterpret_cast<const volatile uint32_t *>(&h_ctrl->status);
+  if (status & ST_FATAL) return (status & ST_TIMEOUT) ? GGKS_TIMEOUT : GGKS_INTERNAL;
+  // a miss, or a slot that needs a recursive level: the pipeline answers (the
+  // streaming pass has written the device copy of an ingested vector)
+  *missed = (status & (ST_TOPK_MISS | ST_DEFERRED)) != 0;
+  if (*missed) return GGKS_OK;
+  ctx.stats.spec_calls++;
+  ctx.stats.spec_ctas += p.G;
   if (want_host) *host_results = reinterpret_cast<const InT *>(ctx.pin);
   return GGKS_OK;
 }
@@ -578,6 +744,21 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
                                          ingest, &missed);
       if (st != GGKS_OK || !missed) return st;
       ingest = nullptr;  // the filter pass wrote the device copy
+    } else if (ctx.depth == 0 && num_req >= 1 &&
+               (src.topk ? !src.topk_pipeline : src.h_k && num_req <= kPlanFew)) {
+      // clustered ranks: the window path, unless its candidates fall short
+      uint64_t rlo = n - num_req, rhi = n - 1;
+      if (src.h_k) {
+        const auto mm = std::minmax_element(src.h_k, src.h_k + num_req);
+        rlo = n - *mm.second;
+        rhi = n - *mm.first;
+      }
+      bool missed = false;
+      const uint64_t done = ctx.stats.launches;
+      const int st = select_window<InT>(ctx, d_in, n, src, num_req, rlo, rhi, d_out_user,
+                                        host_results, s, ingest, &missed);
+      if (st != GGKS_OK || !missed) return st;
+      if (ctx.stats.launches != done) ingest = nullptr;  // the pass wrote the device copy
     }
   }
   const Plan p = make_plan<InT, OutT>(ctx, n, num_req);

@@ -1,0 +1,511 @@
+// ggks_window.cuh -- clustered ranks (one k, k's close together, a long top-k) by a
+// sampled window: one streaming pass keeps the keys that can hold the requested
+// ranks and counts the keys below them, and the requests are answered from those.
+//
+// The reference computes every selection over the whole vector twice
+// (bucketMultiselect.cu:571-574, :780-797).  Here, when the requests' ranks lie
+// within a small part of the order:
+//   k_sample, k_bin, k_slice (ggks_front.cuh): the sample, and its keys around
+//             the window's two ends;
+//   k_wfilter takes as the window [tlo, thi] the sample keys six standard
+//             deviations and four ranks outside the requests' extreme ranks (an
+//             end past the sample is open) and streams the vector once: keys
+//             inside go to one contiguous candidate array and are counted in
+//             kWinBins equal-width bins, keys below are counted;
+//   k_wplace  every CTA takes the bins' prefix, finds the bins that hold the
+//             requested ranks, and the candidates of those bins go to the
+//             places of their ranks (bin by bin, unordered inside a bin);
+//   k_wsort   (top-k) a warp per bin sorts and writes its values, descending; or
+//   k_finish  (requests) a CTA per request selects inside its bin.
+// No second read of the vector, no splitter table, no bucket atomics per key:
+// the pass does two or three compares per key and is bound by HBM, where the
+// speculating histogram pass (ggks_device.cuh) did a table lookup, a shared
+// atomic and a vote: 50 M floats, their median: 81 us, now 43; the call 132 ->
+// 77 us.
+// Correctness never rests on the prediction: k_wplace checks that the candidates
+// were all kept and hold every requested rank, and k_wsort that a bin too large
+// to sort holds copies of one key; else the call reports ST_TOPK_MISS (or a slot
+// that k_finish would leave to a recursive level) and the caller runs the
+// pipeline.
+#pragma once
+
+#include "ggks_front.cuh"
+#include "ggks_tiny.cuh"
+
+namespace ggks {
+
+constexpr int kWinBinBits = 13;
+constexpr uint32_t kWinBins = 1u << kWinBinBits;
+constexpr uint32_t kWinCol = 16;    // keys of one lane's column (k_wfilter)
+constexpr uint32_t kWinSort = 256;  // keys of a bin that a warp sorts (k_wsort)
+
+// The window, its bins and what k_wfilter counted (device; len and below are
+// zero on entry).
+template <class K>
+struct WinCtl {
+  uint32_t len;    // candidates
+  uint32_t below;  // keys below the window
+  uint32_t first;  // first bin that a top-k needs (k_wplace)
+  uint32_t big;    // needed bins of more than kWinSort keys exist (k_wplace)
+  K lo;            // smallest key of bin 1's left end: bin(k) = (k - lo) >> shift, clamped
+  uint32_t shift, nbins;
+};
+
+// bin of a candidate; keys outside [lo, ...] (beyond the sampled extremes, at an
+// open end) go to the end bins
+template <class K>
+__device__ __forceinline__ uint32_t win_bin(K k, K lo, uint32_t shift, uint32_t nbins) {
+  const K j = (k - lo) >> shift;
+  return k < lo ? 0u : j < (K)nbins ? (uint32_t)j : nbins - 1u;
+}
+
+// bins one key wide hold copies of lo + b; an end bin at an open end also holds
+// the keys beyond the sampled extremes
+__device__ __forceinline__ bool win_one_key(uint32_t b, uint32_t shift, uint32_t nbins, bool lo_open,
+                                            bool hi_open) {
+  return shift == 0 && !(lo_open && b == 0) && !(hi_open && b + 1 == nbins);
+}
+
+// One warp's candidates: each lane keeps its own in a column of shared memory --
+// a predicated store and increment per key, no votes -- and when a column could
+// fill up the warp moves all of them to the array with one atomic on its length,
+// counting them in the CTA's bins on the way.  (With a vote and a position per
+// kept key, as k_filter does, a window of 2.4 % of the keys took the pass from
+// 36 to 52 us at 50 M floats: nearly every vector holds some.)
+template <class K>
+struct WinWarp {
+  K *col;            // this lane's column: entry c at col[32 c]
+  uint32_t cnt = 0;  // keys in it
+  K *arr;
+  uint64_t cap;
+  uint32_t *len;
+  uint32_t *bins;  // the CTA's
+  K lo;
+  uint32_t shift, nbins;
+  __device__ __forceinline__ void put(K k, bool keep) {
+    if (keep) col[32 * cnt++] = k;
+  }
+  // every lane calls this after at most four puts
+  __device__ __forceinline__ void check() {
+    if (__any_sync(0xffffffffu, cnt > kWinCol - 4)) flush();
+  }
+  __device__ __forceinline__ void flush() {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t total = __reduce_add_sync(0xffffffffu, cnt);
+    const uint32_t most = __reduce_max_sync(0xffffffffu, cnt);
+    uint32_t base = 0;
+    if (lane == 0 && total) base = atomicAdd(len, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (uint32_t c = 0; c < most; ++c) {
+      const bool have = cnt > c;
+      const uint32_t m = __ballot_sync(0xffffffffu, have);
+      if (have) {
+        const K k = col[32 * c];
+        atomicAdd(&bins[win_bin(k, lo, shift, nbins)], 1u);
+        const uint64_t at = (uint64_t)base + __popc(m & ((1u << lane) - 1u));
+        if (at < cap) arr[at] = k;
+      }
+      base += __popc(m);
+    }
+    cnt = 0;
+  }
+};
+
+template <class K>
+__host__ __device__ constexpr size_t wfilter_smem_bytes() {
+  return kWinBins * 4 + (size_t)1024 * kWinCol * sizeof(K);
+}
+
+// Grid and tiles as k_hist; 1024 threads.  COUNT: the keys below the window are
+// counted (neither end open: a window that is open below has none, one that is
+// open above has all keys that are not candidates).  A window of one key (a
+// value that a good part of the vector holds) keeps nothing: *same counts its
+// copies.  copy_to: as in k_filter.
+template <class T, bool COUNT, bool INGEST>
+__device__ __forceinline__ uint32_t wfilter_body(const T *__restrict__ x, uint64_t n,
+                                                 typename Traits<T>::K tlo,
+                                                 typename Traits<T>::K width,
+                                                 T *__restrict__ copy_to,
+                                                 WinWarp<typename Traits<T>::K> &ww,
+                                                 uint32_t *same) {
+  using K = typename Traits<T>::K;
+  using V = typename Traits<T>::Vec;
+  constexpr int PV = Traits<T>::kPerVec;
+  constexpr int UNROLL = 4;
+  const Span<T> sp = split_span(x, n);
+  const V *xv = reinterpret_cast<const V *>(x + sp.head);
+  V *cv = reinterpret_cast<V *>(copy_to + sp.head);
+  const uint64_t tile_v = (uint64_t)blockDim.x * UNROLL;
+  const uint64_t ntiles = sp.nvec / tile_v;
+  uint32_t below = 0, equal = 0;
+  const bool single = width == 0;  // one key: its copies are only counted
+  for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const uint64_t off = tile * tile_v + threadIdx.x;
+    V v[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u)
+      v[u] = INGEST ? xv[off + (uint64_t)u * blockDim.x] : ldg_stream(xv + off + (uint64_t)u * blockDim.x);
+    if (INGEST) {
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) cv[off + (uint64_t)u * blockDim.x] = v[u];
+    }
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      K k[PV];
+      vec_keys<T>(v[u], k);
+      if (COUNT && single) {
+#pragma unroll
+        for (int e = 0; e < PV; ++e) {
+          below += k[e] < tlo ? 1u : 0u;
+          equal += k[e] == tlo ? 1u : 0u;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < PV; ++e) {
+          if (COUNT) below += k[e] < tlo ? 1u : 0u;
+          ww.put(k[e], (K)(k[e] - tlo) <= width);
+        }
+        ww.check();
+      }
+    }
+  }
+  // leftover vectors and the scalar head / tail: every lane runs every round
+  if (blockIdx.x == (uint32_t)(ntiles % gridDim.x)) {
+    auto one = [&](K k, bool valid) {
+      if (COUNT) below += valid && k < tlo ? 1u : 0u;
+      if (COUNT && single)
+        equal += valid && k == tlo ? 1u : 0u;
+      else
+        ww.put(k, valid && (K)(k - tlo) <= width);
+    };
+    for (uint64_t vb = ntiles * tile_v; vb < sp.nvec; vb += blockDim.x) {
+      const uint64_t vi = vb + threadIdx.x;
+      const bool valid = vi < sp.nvec;
+      V vv{};
+      if (valid) {
+        vv = INGEST ? xv[vi] : ldg_stream(xv + vi);
+        if (INGEST) cv[vi] = vv;
+      }
+      K k[PV];
+      vec_keys<T>(vv, k);
+#pragma unroll
+      for (int e = 0; e < PV; ++e) one(k[e], valid);
+      ww.check();
+    }
+    auto scalar = [&](uint64_t e0, uint64_t e1) {
+      for (uint64_t eb = e0; eb < e1; eb += blockDim.x) {
+        const uint64_t e = eb + threadIdx.x;
+        const bool valid = e < e1;
+        K k = 0;
+        if (valid) {
+          const T v = x[e];
+          if (INGEST) copy_to[e] = v;
+          k = Traits<T>::key(v);
+        }
+        one(k, valid);
+        ww.check();
+      }
+    };
+    scalar(0, sp.head);
+    scalar(sp.tail0, n);
+  }
+  *same = equal;
+  return below;
+}
+
+// bins: kWinBins words, zero on entry.
+template <class T>
+__global__ void __launch_bounds__(1024, 1)
+    k_wfilter(const T *__restrict__ x, uint64_t n, const SliceOut<typename Traits<T>::K> *slice,
+              const typename Traits<T>::K *__restrict__ spans, uint32_t parts, bool lo_open,
+              bool hi_open, WinCtl<typename Traits<T>::K> *wc,
+              typename Traits<T>::K *__restrict__ arr, uint64_t cap, uint32_t *__restrict__ bins_g,
+              T *__restrict__ copy_to) {
+  pdl_trigger();
+  using K = typename Traits<T>::K;
+  extern __shared__ uint4 smem_raw[];
+  uint32_t *bins = reinterpret_cast<uint32_t *>(smem_raw);
+  __shared__ RankShared<K> s_rank;
+  __shared__ uint32_t s_below[32];
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  fill_words(bins, kWinBins, 0u);
+  pdl_wait();
+  const SampleSpan<K> sp = sample_span<K>(spans, parts);
+  const K tlo = lo_open ? K(0) : rank_key<K>(slice, 0, s_rank);
+  const K thi = hi_open ? KeyMax<K>::v : rank_key<K>(slice, 1, s_rank);
+  __syncthreads();  // the cleared bins
+  WinWarp<K> ww;
+  // at an open end the bins reach a quarter of the range and 64 keys past the
+  // sampled extreme, for the keys the sample missed (of 65536 values, 1024 copies
+  // each, it misses the largest in one vector of three)
+  K lo = lo_open ? sp.kmin : tlo, hi = hi_open ? sp.kmax : thi;
+  const K more = (hi > lo ? hi - lo : K(0)) / 4 + 64;
+  if (lo_open) lo = lo > more ? lo - more : K(0);
+  if (hi_open) hi = hi < KeyMax<K>::v - more ? hi + more : KeyMax<K>::v;
+  ww.lo = lo;
+  const K range = hi > lo ? hi - lo : K(0);
+  const int bl = bitlen<K>(range);
+  ww.shift = bl > kWinBinBits ? (uint32_t)(bl - kWinBinBits) : 0u;
+  ww.nbins = (uint32_t)(range >> ww.shift) + 1u;
+  ww.col = reinterpret_cast<K *>(bins + kWinBins) + warp * (32 * kWinCol) + lane;
+  ww.arr = arr;
+  ww.cap = cap;
+  ww.len = &wc->len;
+  ww.bins = bins;
+  if (blockIdx.x == 0 && tid == 0) {
+    wc->lo = ww.lo;
+    wc->shift = ww.shift;
+    wc->nbins = ww.nbins;
+  }
+  const K width = thi - tlo;
+  uint32_t below = 0, same = 0;
+  if (copy_to) {
+    if (lo_open || hi_open)
+      wfilter_body<T, false, true>(x, n, tlo, width, copy_to, ww, &same);
+    else
+      below = wfilter_body<T, true, true>(x, n, tlo, width, copy_to, ww, &same);
+  } else if (lo_open || hi_open) {
+    wfilter_body<T, false, false>(x, n, tlo, width, nullptr, ww, &same);
+  } else {
+    below = wfilter_body<T, true, false>(x, n, tlo, width, nullptr, ww, &same);
+  }
+  ww.flush();
+  below = __reduce_add_sync(0xffffffffu, below);
+  same = __reduce_add_sync(0xffffffffu, same);
+  if (lane == 0) {
+    s_below[warp] = below;
+    if (same) {
+      atomicAdd(&bins[0], same);
+      atomicAdd(&wc->len, same);
+    }
+  }
+  __syncthreads();
+  for (uint32_t b = tid; b < ww.nbins; b += blockDim.x)
+    if (bins[b]) atomicAdd(&bins_g[b], bins[b]);
+  if (warp == 0) {
+    below = __reduce_add_sync(0xffffffffu, s_below[lane]);
+    if (lane == 0 && below) atomicAdd(&wc->below, below);
+  }
+}
+
+// The slots that k_finish reads, one per request (k_wplace).
+template <class K>
+struct WinSlots {
+  uint64_t *seg_off;
+  uint32_t *seg_size, *kstart, *kcnt;
+  K *seg_lo, *seg_hi;
+  Req *klist;
+};
+
+// Bins that hold requested ranks: their candidates go to placed[prefix of the bin
+// ...), which holds the keys of local ranks (rank - below) prefix ... .  kk > 0:
+// a top-k (every bin from the one of the kk-th largest up; bins of more than
+// kWinSort keys are not placed, the complement of their smallest key and their
+// largest key go to big_lo_inv / big_hi); else num_req requests, whose slots CTA
+// 0 writes.  cur, big_lo_inv, big_hi: kWinBins entries, zero on entry; pre_g: the
+// bins' prefix, written by CTA 0 for a top-k.
+template <class K>
+__global__ void __launch_bounds__(1024, 1)
+    k_wplace(const K *__restrict__ arr, uint64_t cap, uint64_t n, uint32_t kk, bool lo_open,
+             bool hi_open, const Req *__restrict__ reqs, uint32_t num_req, WinCtl<K> *wc,
+             const uint32_t *__restrict__ bins_g, uint32_t *cur, uint32_t *__restrict__ pre_g,
+             K *__restrict__ placed, uint64_t placed_cap, unsigned long long *big_lo_inv,
+             unsigned long long *big_hi, WinSlots<K> sl, Ctrl *ctrl) {
+  pdl_start();
+  __shared__ __align__(16) uint32_t pre[kWinBins];
+  __shared__ uint32_t need[kWinBins / 32];
+  __shared__ uint32_t s_scan[32];
+  __shared__ bool s_miss;
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const uint32_t C = wc->len, nbins = wc->nbins, shift = wc->shift;
+  const K lo = wc->lo;
+  // keys below the window: none below an open low end, all that are no
+  // candidates below an open high end, else counted
+  const uint64_t below = lo_open ? 0u : hi_open ? n - C : wc->below;
+  constexpr uint32_t kPer = kWinBins / 1024;
+  uint32_t c[kPer], sum = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kPer / 4; ++q) {
+    const uint4 v = reinterpret_cast<const uint4 *>(bins_g)[tid * (kPer / 4) + q];
+    c[4 * q] = v.x; c[4 * q + 1] = v.y; c[4 * q + 2] = v.z; c[4 * q + 3] = v.w;
+    sum += v.x + v.y + v.z + v.w;
+  }
+  if (tid < kWinBins / 32) need[tid] = 0;
+  // a window of one key: its copies were counted, not kept
+  const bool single = nbins == 1 && shift == 0 && !lo_open && !hi_open;
+  if (tid == 0) s_miss = ((uint64_t)C > cap && !single) || (kk && (C < kk || !hi_open));
+  uint32_t total;
+  uint32_t run = block_excl_scan(sum, s_scan, &total);
+  bool big = false;
+#pragma unroll
+  for (uint32_t q = 0; q < kPer; ++q) {
+    pre[tid * kPer + q] = run;
+    run += c[q];
+  }
+  __syncthreads();
+  // the last bin whose prefix is <= r, for r < C (never an empty one)
+  auto bin_at = [&](uint32_t r) -> uint32_t {
+    uint32_t b = 0;
+#pragma unroll
+    for (uint32_t step = kWinBins / 2; step; step >>= 1)
+      if (pre[b + step] <= r && b + step < nbins) b += step;
+    return b;
+  };
+  auto count_of = [&](uint32_t b) -> uint32_t {
+    return (b + 1 < kWinBins ? pre[b + 1] : total) - pre[b];
+  };
+  // bins one key wide (but the end bins at open ends): their key is known
+  auto one_key = [&](uint32_t b) -> bool { return win_one_key(b, shift, nbins, lo_open, hi_open); };
+  uint32_t first = 0;
+  if (!s_miss && kk) {
+    first = bin_at(C - kk);
+#pragma unroll
+    for (uint32_t q = 0; q < kPer; ++q) big |= tid * kPer + q >= first && c[q] > kWinSort;
+  }
+  big = __syncthreads_or(big);
+  if (!s_miss && !kk && tid < num_req) {
+    const Req q = reqs[tid];
+    if (q.rank < below || q.rank - below >= C) {
+      s_miss = true;
+    } else {
+      const uint32_t r = (uint32_t)(q.rank - below), b = bin_at(r);
+      if (!one_key(b)) atomicOr(&need[b >> 5], 1u << (b & 31));
+      if (blockIdx.x == 0) {
+        sl.seg_off[tid] = pre[b];
+        sl.seg_size[tid] = one_key(b) ? 0u : count_of(b);  // 0: a flat slot, answered from seg_lo
+        // an end bin also holds the keys beyond the sampled extremes
+        sl.seg_lo[tid] = b == 0 && lo_open ? K(0) : lo + ((K)b << shift);
+        sl.seg_hi[tid] = b + 1 >= nbins ? KeyMax<K>::v : lo + (((K)b + 1) << shift) - K(1);
+        sl.kstart[tid] = tid;
+        sl.kcnt[tid] = 1;
+        Req e;
+        e.rank = r - pre[b];
+        e.out = q.out;
+        sl.klist[tid] = e;
+      }
+    }
+  }
+  __syncthreads();
+  const bool miss = s_miss || ((uint64_t)total > placed_cap && !single);
+  if (blockIdx.x == 0) {
+    if (tid == 0) {
+      if (miss) atomicOr(&ctrl->status, ST_TOPK_MISS);
+      ctrl->num_slots = num_req;
+      ctrl->total_surv = C;
+      wc->first = first;
+      wc->big = big ? 1u : 0u;
+    }
+    if (kk)
+      for (uint32_t b = tid; b < kWinBins; b += blockDim.x) pre_g[b] = pre[b];
+  }
+  if (miss || single) return;
+  // whole warps over the candidates, four loads in flight per lane
+  constexpr uint32_t U = 4;
+  const uint32_t step = gridDim.x * 1024 * U;
+  for (uint32_t i0 = blockIdx.x * 1024 * U + (tid >> 5) * 32 * U; i0 < C; i0 += step) {
+    K k[U];
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      const uint32_t i = i0 + 32 * u + lane;
+      k[u] = i < C ? __ldcg(arr + i) : K(0);
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      const bool valid = i0 + 32 * u + lane < C;
+      const uint32_t b = win_bin(k[u], lo, shift, nbins);
+      const bool want =
+          valid && (kk ? b >= first && !one_key(b) : ((need[b >> 5] >> (b & 31)) & 1u) != 0u);
+      const uint32_t m = __ballot_sync(0xffffffffu, want);
+      if (!m) continue;
+      // lanes of one bin take one atomic
+      const uint32_t peers = __match_any_sync(0xffffffffu, want ? b : 0xFFFFFFFFu);
+      const int leader = __ffs(peers) - 1;
+      const bool place = want && !(kk && count_of(b) > kWinSort);
+      uint32_t base = 0;
+      if (place && (int)lane == leader) base = atomicAdd(&cur[b], (uint32_t)__popc(peers));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (place) {
+        placed[pre[b] + base + __popc(peers & ((1u << lane) - 1u))] = k[u];
+      } else if (want) {
+        // a large bin: does it hold one key?  (the complement of the smallest)
+        if ((unsigned long long)~(uint64_t)k[u] > __ldcg(big_lo_inv + b))
+          atomicMax(big_lo_inv + b, (unsigned long long)~(uint64_t)k[u]);
+        if ((unsigned long long)k[u] > __ldcg(big_hi + b))
+          atomicMax(big_hi + b, (unsigned long long)k[u]);
+      }
+    }
+  }
+}
+
+// A top-k's values from the placed bins: a warp per bin from wc->first up, the
+// values in descending order to out[0 .. kk).  The last CTA leaves the call's
+// status in *host_status.
+constexpr uint32_t kWinSortThreads = 256;
+template <class K, class OutT>
+__global__ void __launch_bounds__(kWinSortThreads)
+    k_wsort(const K *__restrict__ placed, const WinCtl<K> *wc, const uint32_t *__restrict__ bins_g,
+            const uint32_t *__restrict__ pre_g, const unsigned long long *__restrict__ big_lo_inv,
+            const unsigned long long *__restrict__ big_hi, uint32_t kk, OutT *__restrict__ out,
+            Ctrl *ctrl, uint32_t *host_status) {
+  pdl_start();
+  __shared__ uint32_t s_last;
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const uint32_t status = ctrl->status;
+  if (!(status & (ST_FATAL | ST_TOPK_MISS))) {
+    const uint32_t C = wc->len, nbins = wc->nbins, first = wc->first;
+    const uint32_t warps = gridDim.x * (kWinSortThreads / 32);
+    // position p of the candidates' order is the (C - p)-th largest
+    auto put = [&](uint32_t p, K k) {
+      const uint32_t i = C - 1 - p;
+      if (i < kk) out[i] = Traits<OutT>::value(k);
+    };
+    auto sorted = [&](auto regs, uint32_t p0, uint32_t c) {
+      constexpr int R = decltype(regs)::value;
+      K v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        v[r] = r * 32 + lane < c ? __ldcg(placed + p0 + r * 32 + lane) : KeyMax<K>::v;
+      warp_bitonic_regs<K, R>(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (r * 32 + lane < c) put(p0 + r * 32 + lane, v[r]);
+    };
+    const K lo = wc->lo;
+    const uint32_t shift = wc->shift;
+    auto one_key = [&](uint32_t b) -> bool { return win_one_key(b, shift, nbins, false, true); };
+    for (uint32_t b = first + blockIdx.x * (kWinSortThreads / 32) + (tid >> 5); b < nbins; b += warps) {
+      const uint32_t c = bins_g[b], p0 = pre_g[b];
+      if (c == 0) continue;
+      if (one_key(b)) {
+        for (uint32_t j = lane; c <= kWinSort && j < c; j += 32) put(p0 + j, lo + (K)b);
+      } else if (c <= 32)
+        sorted(std::integral_constant<int, 1>{}, p0, c);
+      else if (c <= 64)
+        sorted(std::integral_constant<int, 2>{}, p0, c);
+      else if (c <= kWinSort)
+        sorted(std::integral_constant<int, (int)(kWinSort / 32)>{}, p0, c);
+      else if (lane == 0 && ~big_lo_inv[b] != big_hi[b])
+        atomicOr(&ctrl->status, ST_TOPK_MISS);  // too many distinct keys: the pipeline
+    }
+    // copies of one key: every thread writes its share of the outputs in large bins
+    if (wc->big) {
+      for (uint32_t i = blockIdx.x * kWinSortThreads + tid; i < kk; i += gridDim.x * kWinSortThreads) {
+        const uint32_t p = C - 1 - i;
+        uint32_t b = 0;
+        for (uint32_t step = kWinBins / 2; step; step >>= 1)
+          if (b + step < nbins && pre_g[b + step] <= p) b += step;
+        if (bins_g[b] > kWinSort)
+          out[i] = Traits<OutT>::value(one_key(b) ? lo + (K)b : (K)big_hi[b]);
+      }
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(&ctrl->fin_done, 1u) == gridDim.x - 1 ? 1u : 0u;
+    __threadfence();
+    if (s_last) *host_status = __ldcg(&ctrl->status);
+  }
+}
+
+}  // namespace ggks
