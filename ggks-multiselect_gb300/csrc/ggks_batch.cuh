@@ -53,6 +53,7 @@
 // ld.global.cg (L2), never through a possibly stale L1 line.
 #pragma once
 
+#include <cstddef>
 #include <type_traits>
 
 #include "ggks_device.cuh"
@@ -72,9 +73,9 @@ template <class K>
 __host__ __device__ constexpr uint32_t b_slice_bits() {
   return sizeof(K) == 4 ? 7u : 10u;
 }
-constexpr uint32_t kBRepLut = ((1u << 7) + 1) * 32;  // words of the copies: 32 of 2^7 + 1 entries
-static_assert(((1u << b_slice_bits<uint64_t>()) + 1) * sv_copies<uint64_t>() <= kBRepLut &&
-                  ((1u << b_slice_bits<uint32_t>()) + 1) * sv_copies<uint32_t>() <= kBRepLut,
+constexpr uint32_t kBRepLut = ((1u << 7) + 2) * 32;  // words of the copies: 32 of 2^7 + 2 entries
+static_assert(((1u << b_slice_bits<uint64_t>()) + 2) * sv_copies<uint64_t>() <= kBRepLut &&
+                  ((1u << b_slice_bits<uint32_t>()) + 2) * sv_copies<uint32_t>() <= kBRepLut,
               "the table's copies fit their shared memory");
 // shared-memory words in front of the tile phases' histogram / cursors
 constexpr uint32_t kBTileLut = kBRepLut > kLutPadded ? kBRepLut : kLutPadded;
@@ -107,7 +108,7 @@ __host__ __device__ constexpr uint32_t warp_cap() {
 struct BProb {
   const void *x;
   uint64_t n;
-  uint64_t lut_off;  // u32 index of the splitter table (nsl + 1 entries, 16-byte aligned)
+  uint64_t lut_off;  // u32 index of the splitter table (nsl + 2 entries, 16-byte aligned)
   uint64_t cnt_off;  // u32 index of the bucket counts (nb_max entries)
   uint64_t row0;     // u32 index of the first tile's row (tile r: row0 + r * nb_max)
   uint32_t req_off, num_req;  // requests [req_off, req_off + num_req); slots use the same range
@@ -119,15 +120,16 @@ struct BProb {
 };
 
 // splitter-table header and plan results of one problem (device-written)
-struct BHdr {
+struct alignas(16) BHdr {  // (load_hdr reads it in 16-byte vectors)
   uint64_t base;
   uint64_t surv_off;
   uint32_t shift, nb, heavy, num_slots;
   uint32_t dup;      // tiles track whether each bucket holds a single key
   uint32_t spec_on;  // phase 1 set the candidate window [tau_lo, tau_hi]
   uint32_t spec_ok;  // phase 3: every slot's bucket lies strictly inside it
-  uint32_t pad;
+  uint32_t low;      // 1: the table has a low entry
   uint64_t tau_lo, tau_hi;  // keys; tau_lo 0 / tau_hi the largest key: open end
+  uint64_t top;      // position of the table's top entry
 };
 
 // one (problem, tile) work item (host-written)
@@ -254,31 +256,23 @@ __device__ __forceinline__ uint32_t queue_pop(uint32_t *q, uint32_t *s_item) {
   return *s_item;
 }
 
-// Shared-memory position of bucket / slice x in the tile phases: x with its
-// low five bits XORed by the next five.  Inputs with few distinct values
-// (integer-valued floats, say) put their buckets and slices at regular
-// power-of-two strides, which without the swizzle fall into one bank.  A
+// Shared-memory position of bucket x in the tile phases of a problem whose keys
+// repeat often (dup): x with its low five bits XORed by the next five.  Inputs
+// with few distinct values (integer-valued floats, say) put their buckets at
+// regular power-of-two strides, which without the swizzle fall into one bank; on
+// other inputs it costs two instructions per key (a batch of 2 GB of uniform
+// floats: compaction 508 -> 464 us without it, counting 454 -> 439).  A
 // permutation inside every group of 32 entries.
 __device__ __forceinline__ uint32_t swz(uint32_t x) { return x ^ ((x >> 5) & 31u); }
-
-// bucket_of with the splitter table's copies (as bucket_of_rep, with a slice
-// count of the problem's own): entry j at lane_lut[j * copies]
-template <class K>
-__device__ __forceinline__ uint32_t bucket_of_lane(K key, K base, uint32_t shift,
-                                                   const uint32_t *lane_lut, uint32_t nsl) {
-  const K d = key - base;  // wraps for key < base; that result is discarded
-  const K idx = d >> shift;
-  const uint32_t j = idx < (K)nsl ? (uint32_t)idx : nsl;
-  const uint32_t e = lane_lut[j << sv_copy_bits<K>()];
-  const uint32_t b = (uint32_t)((int32_t)e >> 7) + shr_clamp(d, e & 127u);
-  return key < base ? 0u : b;
-}
 
 __device__ __forceinline__ uint32_t ldcg_u(const uint32_t *p) { return __ldcg(p); }
 __device__ __forceinline__ uint64_t ldcg_u(const uint64_t *p) {
   return __ldcg(reinterpret_cast<const unsigned long long *>(p));
 }
 
+static_assert(sizeof(BHdr) % 16 == 0 && offsetof(BHdr, shift) % 16 == 0 &&
+                  offsetof(BHdr, dup) % 16 == 0,
+              "16-byte vectors of every problem's header");
 __device__ __forceinline__ BHdr load_hdr(const BHdr *h) {
   BHdr r;
   r.base = ldcg_u(&h->base);
@@ -292,6 +286,8 @@ __device__ __forceinline__ BHdr load_hdr(const BHdr *h) {
   r.dup = w2.x;
   r.spec_on = w2.y;
   r.spec_ok = w2.z;
+  r.low = w2.w;
+  r.top = ldcg_u(&h->top);
   r.tau_lo = ldcg_u(&h->tau_lo);
   r.tau_hi = ldcg_u(&h->tau_hi);
   return r;
@@ -624,6 +620,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
   __shared__ uint64_t s_base;
   __shared__ uint32_t s_lb[3];
   __shared__ LutHeader<K> s_hdr;
+  __shared__ uint32_t s_tab[(1u << b_slice_bits<K>()) + 2];
   __shared__ bool s_bad;
   __shared__ uint32_t s_rcnt[256], s_rsel[2], s_ccnt;
   BCtrl *ctrl = A.ctrl;
@@ -678,10 +675,10 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
 #ifdef GGKS_BATCH_TIMING
     const long long c1 = clock64();
 #endif
-    if (!BCHECK(P.lut_off + (1u << P.nsl_bits) < A.lut_words && P.S <= kBMaxS, 1, p, P.lut_off))
+    if (!BCHECK(P.lut_off + (1u << P.nsl_bits) + 2 <= A.lut_words && P.S <= kBMaxS, 1, p, P.lut_off))
       continue;
-    build_lut_cta<K, kBSpt<K>()>(samples, P.S, lo, hi, P.nb_max, A.luts + P.lut_off, &s_hdr,
-                                 (int)P.nsl_bits);
+    build_lut_cta<K, kBSpt<K>()>(samples, P.S, lo, hi, P.nb_max, A.luts + P.lut_off, s_tab,
+                                 &s_hdr, (int)P.nsl_bits);
     __syncthreads();
     // Speculation: the window's ends as sample ranks, moved outwards by four
     // standard deviations of the number of sampled chunks below them
@@ -710,6 +707,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
     if (tid == 0) {
       BHdr h;
       h.base = s_hdr.base;
+      h.top = s_hdr.top;
       h.surv_off = 0;
       h.shift = s_hdr.shift;
       h.nb = s_hdr.nb;
@@ -718,7 +716,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       h.dup = (s_hdr.dup && P.nb_max * sizeof(K) <= kBRepBytes) ? 1u : 0u;
       h.spec_on = spec_on ? 1u : 0u;
       h.spec_ok = 0;
-      h.pad = 0;
+      h.low = s_hdr.low;
       h.tau_lo = (uint64_t)tau_lo;
       h.tau_hi = (uint64_t)tau_hi;
       A.hdrs[p] = h;
@@ -743,7 +741,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       const BHdr H = load_hdr(A.hdrs + tl.prob);
       const uint32_t nsl = 1u << P.nsl_bits;
       if (s_cur != tl.prob)
-        for (uint32_t w = tid; w < (nsl + 1) * sv_copies<K>(); w += nt)
+        for (uint32_t w = tid; w < (nsl + 2) * sv_copies<K>(); w += nt)
           sm[w] = __ldcg(A.luts + P.lut_off + (w >> sv_copy_bits<K>()));
       for (uint32_t b = tid; b < ((H.nb + 31) & ~31u); b += nt) {
         hist[b] = 0;
@@ -752,13 +750,12 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       if (tid == 0) s_ccnt = 0;
       __syncthreads();
       if (tid == 0) s_cur = tl.prob;
-      const K base = (K)H.base;
-      const uint32_t shift = H.shift;
+      const KeyTable<K> kt((K)H.base, (K)H.top, H.shift);
       if (H.dup) {
         // count, and keep the bucket's first key; a second distinct key (or
         // the largest key, which marks an empty entry) sets the mixed bit
         for_range_p<T>(P.x, P.flt, tl.begin, tl.end, [&](K k, bool) {
-          const uint32_t ub = bucket_of_lane<K>(k, base, shift, lane_lut, nsl);
+          const uint32_t ub = bucket_byte_of<K>(k, kt, lane_lut) >> 2;
           if (!BCHECK(ub < H.nb, 2, ub, H.nb)) return;
           const uint32_t b = swz(ub);
           atomicAdd(&hist[b], 1u);
@@ -782,8 +779,8 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
         K *cand = reinterpret_cast<K *>(A.cand) + tl.cand_off;
         const uint32_t ccap = tl.cand_cap;
         for_range_p<T>(P.x, P.flt, tl.begin, tl.end, [&](K k, bool) {
-          const uint32_t ub = bucket_of_lane<K>(k, base, shift, lane_lut, nsl);
-          if (BCHECK(ub < H.nb, 4, ub, H.nb)) atomicAdd(&hist[swz(ub)], 1u);
+          const uint32_t byte = bucket_byte_of<K>(k, kt, lane_lut);
+          if (BCHECK(byte / 4 < H.nb, 4, byte, H.nb)) atomicAdd(&word_at(hist, byte), 1u);
           if ((K)(k - tlo) <= span) {
             const uint32_t pos = atomicAdd(&s_ccnt, 1u);
             if (pos < ccap) cand[pos] = k;
@@ -795,9 +792,9 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
         // different ones, so warp aggregation (compaction's) would only slow
         // this phase down.  Eight vectors in flight per thread.
         for_range_p<T, kBTileVecs>(P.x, P.flt, tl.begin, tl.end, [&](K k, bool) {
-          const uint32_t ub = bucket_of_lane<K>(k, base, shift, lane_lut, nsl);
-          if (!BCHECK(ub < H.nb, 4, ub, H.nb)) return;
-          atomicAdd(&hist[swz(ub)], 1u);
+          const uint32_t byte = bucket_byte_of<K>(k, kt, lane_lut);
+          if (!BCHECK(byte / 4 < H.nb, 4, byte, H.nb)) return;
+          atomicAdd(&word_at(hist, byte), 1u);
         });
       }
       __syncthreads();
@@ -807,7 +804,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       // the tile's row, and its counts added to the problem's bucket totals
       uint32_t *tot = A.counts + P.cnt_off;
       for (uint32_t b = tid; b < H.nb; b += nt) {
-        const uint32_t c = hist[swz(b)];
+        const uint32_t c = hist[H.dup ? swz(b) : b];
         A.rows[ro + b] = c;
         if (c & ~kMixed) atomicAdd(tot + b, c & ~kMixed);
         if (H.dup) reps[ro + b] = rep[swz(b)];
@@ -830,7 +827,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
                       P.cnt_off + P.nb_max <= A.cnt_words && P.req_off + P.num_req <= A.num_req,
                   6, p, nb))
         continue;
-      for (uint32_t j = tid; j <= nsl; j += nt) lut[j] = __ldcg(A.luts + P.lut_off + j);
+      for (uint32_t j = tid; j < nsl + 2; j += nt) lut[j] = __ldcg(A.luts + P.lut_off + j);
       // bucket totals (added by the tiles of phase 2) -> exclusive prefix in
       // shared memory; the flags start clear
       load_totals(cnt, nb, excl);
@@ -931,14 +928,16 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       // speculation holds when every slot with survivors lies strictly between
       // the buckets of the window's ends (an open end bounds nothing)
       const bool lo_open = H.tau_lo == 0, hi_open = (K)H.tau_hi == KeyMax<K>::v;
-      const uint32_t b_tlo = lo_open ? 0u : bucket_of<K>((K)H.tau_lo, (K)H.base, H.shift, lut, nsl);
-      const uint32_t b_thi = hi_open ? 0u : bucket_of<K>((K)H.tau_hi, (K)H.base, H.shift, lut, nsl);
+      const KeyTable<K> kt((K)H.base, (K)H.top, H.shift);
+      const uint32_t ents = nsl + 1 + H.low;
+      const uint32_t b_tlo = lo_open ? 0u : bucket_of<K>((K)H.tau_lo, kt, lut);
+      const uint32_t b_thi = hi_open ? 0u : bucket_of<K>((K)H.tau_hi, kt, lut);
       bool outside = false;
       for (uint32_t q = s0; q < s1; ++q) {
         const uint32_t g = P.req_off + q;
         const uint32_t b = __ldcg(A.seg_bucket + g);
-        K klo = bucket_lo<K>(b, (K)H.base, H.shift, lut, nsl);
-        const K knext = (b + 1 < nb) ? bucket_lo<K>(b + 1, (K)H.base, H.shift, lut, nsl) : K(0);
+        K klo = bucket_lo<K>(b, (K)H.base, H.shift, lut, ents);
+        const K knext = (b + 1 < nb) ? bucket_lo<K>(b + 1, (K)H.base, H.shift, lut, ents) : K(0);
         // single key iff the next bucket starts one key later (see k_plan), or
         // every tile saw one and the same key in the bucket
         bool single = (knext > klo) ? (knext - klo == K(1)) : (klo == KeyMax<K>::v);
@@ -1079,7 +1078,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       const BHdr H = load_hdr(A.hdrs + tl.prob);
       const uint32_t nsl = 1u << P.nsl_bits;
       if (s_cur != tl.prob)
-        for (uint32_t w = tid; w < (nsl + 1) * sv_copies<K>(); w += nt)
+        for (uint32_t w = tid; w < (nsl + 2) * sv_copies<K>(); w += nt)
           sm[w] = __ldcg(A.luts + P.lut_off + (w >> sv_copy_bits<K>()));
       for (uint32_t b = tid; b < ((H.nb + 31) & ~31u); b += nt) cursor[b] = kInactive;
       __syncthreads();
@@ -1098,7 +1097,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
         const uint32_t c = __ldcg(row + b) & ~kMixed;
         const uint32_t pre = c ? atomicAdd(A.fill + g, c) : 0u;
         const uint32_t at = (uint32_t)(ldcg_u(A.seg_off + g) - H.surv_off + pre);
-        cursor[swz(b)] = at;
+        cursor[H.dup ? swz(b) : b] = at;
         row[b] = at + c;
       }
       __syncthreads();
@@ -1107,8 +1106,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       // and every store inside the buffer (see compact_one)
       const uint64_t room = A.surv_cap - H.surv_off;
       const uint32_t cap = (uint32_t)(room < (uint64_t)kInactive ? room : kInactive);
-      const K base = (K)H.base;
-      const uint32_t shift = H.shift;
+      const KeyTable<K> kt((K)H.base, (K)H.top, H.shift);
       const uint32_t ncand = H.spec_ok ? __ldcg(A.cand_cnt + t) : 0xFFFFFFFFu;
       if (H.spec_ok && ncand <= tl.cand_cap) {
         // the tile's complete candidate list holds every key of its slots'
@@ -1116,9 +1114,9 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
         const K *cand = reinterpret_cast<const K *>(A.cand) + tl.cand_off;
         for (uint32_t i = tid; i < ncand; i += nt) {
           const K k = ldcg_u(cand + i);
-          const uint32_t ub = bucket_of_lane<K>(k, base, shift, lane_lut, nsl);
-          if (!BCHECK(ub < H.nb, 9, ub, H.nb)) continue;
-          const uint32_t pos = atomicAdd(&cursor[swz(ub)], 1u);
+          const uint32_t byte = bucket_byte_of<K>(k, kt, lane_lut);  // (no dup problem speculates)
+          if (!BCHECK(byte / 4 < H.nb, 9, byte, H.nb)) continue;
+          const uint32_t pos = atomicAdd(&word_at(cursor, byte), 1u);
           st_global_if(sp + pos, k, pos < cap);
         }
         if (tid == 0) atomicAdd(&ctrl->spec_tiles, 1u);
@@ -1129,20 +1127,21 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
         // consecutive positions.  A key whose bucket fails the check (the call
         // is then failed) stays in the vote under bucket 0 but is not stored.
         for_range_p<T>(P.x, P.flt, tl.begin, tl.end, [&](K k, bool full) {
-          uint32_t ub = bucket_of_lane<K>(k, base, shift, lane_lut, nsl);
+          uint32_t ub = bucket_byte_of<K>(k, kt, lane_lut) >> 2;
           const bool ok = BCHECK(ub < H.nb, 9, ub, H.nb);
           if (!ok) ub = 0;
+          if (H.dup) ub = swz(ub);
           uint32_t pos;
           if (full) {
             const uint32_t peers = __match_any_sync(0xffffffffu, ub);
             const uint32_t lane = threadIdx.x & 31;
             const int leader = __ffs(peers) - 1;
             uint32_t p0 = 0;
-            if ((int)lane == leader) p0 = atomicAdd(&cursor[swz(ub)], (uint32_t)__popc(peers));
+            if ((int)lane == leader) p0 = atomicAdd(&cursor[ub], (uint32_t)__popc(peers));
             p0 = __shfl_sync(peers, p0, leader);
             pos = p0 + __popc(peers & ((1u << lane) - 1u));
           } else {
-            pos = atomicAdd(&cursor[swz(ub)], 1u);
+            pos = atomicAdd(&cursor[ub], 1u);
           }
           st_global_if(sp + pos, k, ok && pos < cap);
         });
@@ -1150,12 +1149,20 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
         // eight vectors in flight, four for float batches (whose kernel
         // spills 256 bytes of loads with eight)
         constexpr int CV = std::is_same<T, float>::value ? 4 : kBTileVecs;
-        for_range_p<T, CV>(P.x, P.flt, tl.begin, tl.end, [&](K k, bool) {
-          uint32_t ub = bucket_of_lane<K>(k, base, shift, lane_lut, nsl);
-          if (!BCHECK(ub < H.nb, 9, ub, H.nb)) return;
-          const uint32_t pos = atomicAdd(&cursor[swz(ub)], 1u);
-          st_global_if(sp + pos, k, pos < cap);
-        });
+        if (H.dup)
+          for_range_p<T, 4>(P.x, P.flt, tl.begin, tl.end, [&](K k, bool) {
+            const uint32_t ub = bucket_byte_of<K>(k, kt, lane_lut) >> 2;
+            if (!BCHECK(ub < H.nb, 9, ub, H.nb)) return;
+            const uint32_t pos = atomicAdd(&cursor[swz(ub)], 1u);
+            st_global_if(sp + pos, k, pos < cap);
+          });
+        else
+          for_range_p<T, CV>(P.x, P.flt, tl.begin, tl.end, [&](K k, bool) {
+            const uint32_t byte = bucket_byte_of<K>(k, kt, lane_lut);
+            if (!BCHECK(byte / 4 < H.nb, 9, byte, H.nb)) return;
+            const uint32_t pos = atomicAdd(&word_at(cursor, byte), 1u);
+            st_global_if(sp + pos, k, pos < cap);
+          });
       }
       __syncthreads();
       // each cursor must end where the tile's share of the segment ends
@@ -1163,7 +1170,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
         const uint32_t g = P.req_off + s;
         if (__ldcg(A.seg_size + g) == 0) continue;
         const uint32_t b = __ldcg(A.seg_bucket + g);
-        if (cursor[swz(b)] != __ldcg(row + b)) s_bad = true;
+        if (cursor[H.dup ? swz(b) : b] != __ldcg(row + b)) s_bad = true;
       }
     }
     __syncthreads();

@@ -121,7 +121,7 @@ int select_batch(Context &ctx, const BatchInput &in, T *d_out_user, T *h_out, cu
       }
     }
     b.lut_off = lut_words;
-    lut_words += ((1u << nsl_bits) + 1 + 3) & ~3u;
+    lut_words += ((1u << nsl_bits) + 2 + 3) & ~3u;
     b.cnt_off = cnt_words;
     cnt_words += nbm;
     b.row0 = row_words;

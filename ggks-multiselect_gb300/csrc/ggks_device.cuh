@@ -63,7 +63,7 @@ namespace ggks {
 // ---------------------------------------------------------------------------
 constexpr int kLutIdxBits = 12;
 constexpr uint32_t kLutIdx = 1u << kLutIdxBits;  // slices over the sample span
-constexpr uint32_t kLutEntries = kLutIdx + 1;    // + one for keys above the span
+constexpr uint32_t kLutEntries = kLutIdx + 2;    // + keys below and above the span
 constexpr uint32_t kLutPadded = (kLutEntries + 3) & ~3u;  // 16-byte multiple
 // at most 2^15 buckets per slice, and 2^(24 - slice bits) so that a packed
 // table entry's first-bucket offset fits its signed 25-bit field
@@ -102,9 +102,13 @@ template <class K>
 __host__ __device__ constexpr uint32_t sv_copies() {
   return 1u << sv_copy_bits<K>();
 }
-constexpr uint32_t kRepWords = ((1u << 9) + 1) * 32;  // words of the copies: 32 of 2^9 + 1 entries
-static_assert((sv_slices<uint64_t>() + 1) * sv_copies<uint64_t>() <= kRepWords &&
-                  (sv_slices<uint32_t>() + 1) * sv_copies<uint32_t>() <= kRepWords,
+template <class K>
+__host__ __device__ constexpr uint32_t sv_entries() {
+  return sv_slices<K>() + 2;
+}
+constexpr uint32_t kRepWords = ((1u << 9) + 2) * 32;  // words of the copies: 32 of 2^9 + 2 entries
+static_assert(sv_entries<uint64_t>() * sv_copies<uint64_t>() <= kRepWords &&
+                  sv_entries<uint32_t>() * sv_copies<uint32_t>() <= kRepWords,
               "the table's copies fit their shared memory");
 constexpr uint32_t kMaxNb = 32768;  // buckets of one vector: shared-memory histogram limit (u32)
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
@@ -228,8 +232,11 @@ struct Ctrl {
 
 template <class K>
 struct LutHeader {
-  K base;          // smallest sampled key
-  uint32_t shift;  // slice index = (key - base) >> shift
+  K base;          // the table's first key: one slice below the smallest sampled key
+                   // (low == 1), or that key itself where no slice fits below it
+  K top;           // position of the top entry: one slice past the sampled span
+  uint32_t shift;  // entry of a key: its position (table_pos) >> shift
+  uint32_t low;    // 1: entry 0 is the keys below the smallest sampled one
   uint32_t nb;     // number of buckets
   uint32_t heavy;  // 1: warp-aggregate compaction's cursor updates
   uint32_t dup;    // 1: sampled keys repeat often (at least once per nb pairs)
@@ -385,16 +392,6 @@ __device__ __forceinline__ void st_global_if(uint64_t *p, uint64_t v, bool pred)
       : "memory");
 }
 
-// right shift that yields 0 for shift >= width (the splitter table's top
-// entry shifts by the key width).  __funnelshift_rc clamps the shift to 32;
-// __funnelshift_r would wrap it to shift & 31.
-__device__ __forceinline__ uint32_t shr_clamp(uint32_t d, uint32_t s) {
-  return __funnelshift_rc(d, 0u, s);
-}
-__device__ __forceinline__ uint32_t shr_clamp(uint64_t d, uint32_t s) {
-  return s >= 64 ? 0u : (uint32_t)(d >> s);
-}
-
 template <class K>
 __device__ __forceinline__ int bitlen(K v);
 template <>
@@ -419,45 +416,64 @@ __device__ __forceinline__ uint32_t hash32(uint32_t a) {
 // ---------------------------------------------------------------------------
 // bucket function: slice lookup + sub-bucket by the next bits of the key
 // ---------------------------------------------------------------------------
-// lut[j] = (C_j << 7) | rs_j.  For slice j with first bucket B_j cut into 2^b_j
-// sub-buckets: rs_j = shift - b_j and C_j = B_j - (j << b_j), a signed 25-bit
-// value (|j << b_j| < 2^24 because a table of 2^s slices has j < 2^s and
-// b_j <= 24 - s).  Then
-//   bucket = C_j + ((key - base) >> rs_j),
-// since (key - base) >> rs_j = (j << b_j) + sub-bucket on slice j.  Empty
-// slices of one run share a bucket (b = 0); the top entry (keys above the
-// sampled span) has rs = key width, i.e. the constant bucket C.  Bucket 0
-// holds the keys below `base` (the sampled minimum), so the first slice's
-// buckets start at 1 and its first bucket starts exactly at `base`.  One 4-byte
-// entry per slice keeps the shared-memory lookup to a single wavefront for
-// runs of neighbouring slices; the bucket costs two ALU operations.
+// A key's position is the key clamped to the table's range, less its first key:
+//   d = min(max(key, base) - base, top),
+// and its entry is d >> shift: [low] slices 0 .. nsl - 1, [top].  lut[j] =
+// (C_j << 7) | rs_j; for an entry with first bucket B_j cut into 2^b_j
+// sub-buckets rs_j = shift - b_j and C_j = B_j - (j << b_j) modulo 2^25.  Then
+//   bucket = C_j + (d >> rs_j),
+// since d >> rs_j = (j << b_j) + sub-bucket.  Empty slices of one run share a
+// bucket (b = 0); the low and top entries are buckets too (b = 0): keys below the
+// smallest sampled one reach the low entry, those further below by the clamp,
+// and keys above the sampled span the top one.  Without a low entry (fewer than
+// 2^shift keys below) they share the first slice's first bucket.
 //
-// nsl (a power of two <= kLutIdx) is the number of slices; the top entry sits
-// at lut[nsl].  The single-vector path always uses kLutIdx slices; small
-// problems of a batch use fewer.
+// For 4-byte keys the bucket's byte offset in an array of words takes three
+// operations after the lookup: x = d >> rs (a shift by the entry's low five
+// bits), (x << 7) + entry = (bucket << 7) | rs, >> 5.  With the clamps that is
+// three instructions per key fewer than a table of the same shape that
+// compared key and base, clamped the slice index and unpacked the entry
+// (2^28 floats, 1001 ks: histogram 192 -> 187 us; 2^20 floats in one launch,
+// 101 ks: 56 -> 53 us a call).
 template <class K>
-__device__ __forceinline__ uint32_t bucket_of(K key, K base, uint32_t shift, const uint32_t *lut,
-                                              uint32_t nsl = kLutIdx) {
-  const K d = key - base;  // wraps for key < base; that result is discarded
-  const K idx = d >> shift;
-  const uint32_t j = idx < (K)nsl ? (uint32_t)idx : nsl;
-  const uint32_t e = lut[j];
-  const uint32_t b = (uint32_t)((int32_t)e >> 7) + shr_clamp(d, e & 127u);
-  return key < base ? 0u : b;
+struct KeyTable {
+  K base, top;
+  uint32_t shift;
+  __device__ __forceinline__ KeyTable(K b, K t, uint32_t s) : base(b), top(t), shift(s) {}
+  __device__ __forceinline__ explicit KeyTable(const LutHeader<K> &h)
+      : base(h.base), top(h.top), shift(h.shift) {}
+  __device__ __forceinline__ K pos(K key) const {
+    const K c = key > base ? key : base;
+    const K d = c - base;
+    return d < top ? d : top;
+  }
+};
+
+// byte offset of the word of d's bucket, e = d's entry
+__device__ __forceinline__ uint32_t bucket_byte(uint32_t d, uint32_t e) {
+  return ((__funnelshift_r(d, 0u, e) << 7) + e) >> 5;
+}
+__device__ __forceinline__ uint32_t bucket_byte(uint64_t d, uint32_t e) {
+  return ((uint32_t)((int32_t)e >> 7) + (uint32_t)(d >> (e & 127u))) << 2;
+}
+__device__ __forceinline__ uint32_t &word_at(uint32_t *a, uint32_t byte) {
+  return *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(a) + byte);
 }
 
-// bucket_of on the single-vector table (sv_slices<K>() slices) held in copies in
-// shared memory: lane_lut = sv_lane_table(table), entry j at
-// lane_lut[j * copies].
+// The byte offset of a key's bucket word, from a table held in interleaved copies
+// in shared memory (lane_lut = sv_lane_table(table)).
 template <class K>
-__device__ __forceinline__ uint32_t bucket_of_rep(K key, K base, uint32_t shift,
-                                                  const uint32_t *lane_lut) {
-  const K d = key - base;  // wraps for key < base; that result is discarded
-  const K idx = d >> shift;
-  const uint32_t j = idx < (K)sv_slices<K>() ? (uint32_t)idx : sv_slices<K>();
-  const uint32_t e = lane_lut[j << sv_copy_bits<K>()];
-  const uint32_t b = (uint32_t)((int32_t)e >> 7) + shr_clamp(d, e & 127u);
-  return key < base ? 0u : b;
+__device__ __forceinline__ uint32_t bucket_byte_of(K key, const KeyTable<K> &t,
+                                                   const uint32_t *lane_lut) {
+  const K d = t.pos(key);
+  return bucket_byte(d, lane_lut[(uint32_t)(d >> t.shift) << sv_copy_bits<K>()]);
+}
+
+// A key's bucket, from a single copy of the table.
+template <class K>
+__device__ __forceinline__ uint32_t bucket_of(K key, const KeyTable<K> &t, const uint32_t *lut) {
+  const K d = t.pos(key);
+  return bucket_byte(d, lut[(uint32_t)(d >> t.shift)]) >> 2;
 }
 
 // this lane's copy of the table
@@ -466,17 +482,17 @@ __device__ __forceinline__ const uint32_t *sv_lane_table(const uint32_t *rep) {
   return rep + (threadIdx.x & (sv_copies<K>() - 1u));
 }
 
-// Copies the single-vector table (sv_slices<K>() + 1 entries, global) into its
+// Copies the single-vector table (sv_entries<K>() entries, global) into its
 // copies in shared memory, by a CTA of 1024 threads: each entry is read once
 // per CTA, coalesced, in one round of loads (every CTA reads the same few
 // kilobytes at the same time: a gather that asked L2 for each warp's own
 // sectors cost 2-4 us), and the copies are written with 16-byte stores.  tab:
-// sv_slices<K>() + 1 shared words (sv_copies 32; else unused).  Ends with a
+// sv_entries<K>() shared words (sv_copies 32; else unused).  Ends with a
 // barrier for the caller's shared memory.
 template <class K>
 __device__ __forceinline__ void load_rep_table(uint32_t *rep, const uint32_t *__restrict__ lut_g,
                                                uint32_t *tab) {
-  constexpr uint32_t kEnt = sv_slices<K>() + 1;
+  constexpr uint32_t kEnt = sv_entries<K>();
   constexpr uint32_t kPer = (kEnt + 1023) / 1024;
   uint32_t e[kPer];
 #pragma unroll
@@ -520,36 +536,31 @@ __device__ __forceinline__ uint32_t lut_pack(int32_t C, uint32_t rs) {
 
 // first bucket and sub-bucket bits of entry j
 __device__ __forceinline__ void lut_entry(uint32_t e, uint32_t j, uint32_t shift, uint32_t *B,
-                                          uint32_t *bb, uint32_t nsl = kLutIdx) {
-  const int32_t C = (int32_t)e >> 7;
-  if (j == nsl) {
-    *B = (uint32_t)C;
-    *bb = 0;
-  } else {
-    *bb = shift - (e & 127u);
-    *B = (uint32_t)(C + (int32_t)(j << *bb));
-  }
+                                          uint32_t *bb) {
+  *bb = shift - (e & 127u);
+  *B = (uint32_t)(((int32_t)e >> 7) + (int32_t)(j << *bb));
 }
 
-// smallest key that maps to bucket b (b < nb); bucket 0 starts at key 0.
+// smallest key that maps to bucket b (b < nb), from a table of ents entries;
+// bucket 0 starts at key 0.
 template <class K>
 __device__ __forceinline__ K bucket_lo(uint32_t b, K base, uint32_t shift, const uint32_t *lut,
-                                       uint32_t nsl = kLutIdx) {
+                                       uint32_t ents) {
   if (b == 0) return K(0);
   // first entry whose last bucket >= b (bucket ranges are non-decreasing in j)
-  uint32_t lo = 0, hi = nsl;
+  uint32_t lo = 0, hi = ents - 1;
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
     uint32_t B, bb;
-    lut_entry(lut[mid], mid, shift, &B, &bb, nsl);
+    lut_entry(lut[mid], mid, shift, &B, &bb);
     if (B + (1u << bb) - 1u >= b)
       hi = mid;
     else
       lo = mid + 1;
   }
   uint32_t B, bb;
-  lut_entry(lut[lo], lo, shift, &B, &bb, nsl);
-  const K dstart = ((K)lo) << shift;  // for lo == nsl this may wrap: see the caller
+  lut_entry(lut[lo], lo, shift, &B, &bb);
+  const K dstart = ((K)lo) << shift;  // for the top entry this may wrap: see the caller
   if (B >= b) return base + dstart;
   return base + dstart + (((K)(b - B)) << (shift - bb));
 }
@@ -641,15 +652,16 @@ __device__ __forceinline__ void table_init(TableShared &ts) {  // then a block b
 
 // Builds the table of nsl <= SPT * blockDim.x slices of width 2^shift from
 // density(j), the samples of slice j (any measure of them), with the whole
-// CTA: the nsl entries go to lut (global or shared memory) and to tab (shared;
-// may be lut), ordered by the caller's next block barrier.  bcap: largest b.
-// Returns the buckets in use; *top: the entry of the keys above the span.
+// CTA: the low + nsl + 1 entries go to lut (global or shared memory) and to tab
+// (shared; may be lut), ordered by the caller's next block barrier.  low: 1 for
+// an entry of the keys below the smallest sampled one.  bcap: largest b.
+// Returns the buckets in use.
 // A decision that one thread could take alone in a loop is taken by a warp, or
 // by every warp for itself where that saves a block barrier.
 template <class K, int SPT, class D>
-__device__ __forceinline__ uint32_t build_table(D &&density, uint32_t nsl, uint32_t shift, int bcap,
-                                                uint32_t nb_max, uint32_t *lut, uint32_t *tab,
-                                                TableShared &ts, uint32_t *top) {
+__device__ __forceinline__ uint32_t build_table(D &&density, uint32_t nsl, uint32_t low,
+                                                uint32_t shift, int bcap, uint32_t nb_max,
+                                                uint32_t *lut, uint32_t *tab, TableShared &ts) {
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // this thread's slices [SPT tid, SPT tid + SPT)
   uint32_t c[SPT];
@@ -726,32 +738,49 @@ __device__ __forceinline__ uint32_t build_table(D &&density, uint32_t nsl, uint3
     mysum += my[q];
   }
   uint32_t total;
-  uint32_t run = block_excl_scan(mysum, ts.scan, &total) + 1u;  // bucket 0 is the low edge
+  uint32_t run = block_excl_scan(mysum, ts.scan, &total) + low;  // bucket 0: the low entry
+  auto put = [&](uint32_t j, uint32_t e) {
+    tab[j] = e;
+    if (tab != lut) lut[j] = e;
+  };
 #pragma unroll
   for (int q = 0; q < SPT; ++q) {
-    const uint32_t j = SPT * tid + q;
-    if (j >= nsl) break;
+    if (SPT * tid + q >= nsl) break;
+    const uint32_t j = low + SPT * tid + q;
     // one bucket per run of empty slices
-    const uint32_t e =
-        c[q] ? lut_pack((int32_t)run - (int32_t)(j << bq[q]), shift - (uint32_t)bq[q])
-             : lut_pack((int32_t)(prev_nonempty[q] ? run : run - 1u) - (int32_t)j, shift);
-    lut[j] = e;
-    tab[j] = e;
+    put(j, c[q] ? lut_pack((int32_t)run - (int32_t)(j << bq[q]), shift - (uint32_t)bq[q])
+                : lut_pack((int32_t)(prev_nonempty[q] ? run : run - 1u) - (int32_t)j, shift));
     run += my[q];
   }
-  *top = lut_pack((int32_t)(top_run_start ? total + 1u : total), (uint32_t)KeyMax<K>::bits);
-  return 1u + total + (top_run_start ? 1u : 0u);
+  if (tid == 0) {
+    if (low) put(0, lut_pack(0, shift));
+    put(low + nsl, lut_pack((int32_t)(low + total - (top_run_start ? 0u : 1u)) - (int32_t)(low + nsl),
+                            shift));
+  }
+  return low + total + (top_run_start ? 1u : 0u);
+}
+
+// The table's place around a sampled span: its first key and the position of its
+// top entry (see bucket_of).
+template <class K>
+__device__ __forceinline__ void table_place(LutHeader<K> &h, K kmin, uint32_t shift, uint32_t nsl) {
+  h.low = kmin >= ((K)1 << shift) ? 1u : 0u;
+  h.base = h.low ? kmin - ((K)1 << shift) : kmin;
+  const K ents = (K)(nsl + h.low);
+  h.top = ents > (KeyMax<K>::v >> shift) ? KeyMax<K>::v : ents << shift;
+  h.shift = shift;
 }
 
 // The splitter table of one problem of a batch, or of a small vector, from its
 // S sampled keys in shared memory (kmin / kmax: the sample's extremes), by one
-// whole CTA; the table goes to lut[0 .. nsl] with nsl = 2^nsl_bits <= SPT *
+// whole CTA; the table goes to lut[0 .. nsl + 2) with nsl = 2^nsl_bits <= SPT *
 // blockDim.x slices (nb_max >= nsl + 2 makes every threshold feasible), and
-// thread 0 writes the header.
+// thread 0 writes the header.  tab: nsl + 2 shared words (may be lut; a second
+// copy of 16 KB cost k_small 2-3 us a call on doubles).  At most 1024 threads.
 template <class K, int SPT>
 __device__ void build_lut_cta(const K *samples, uint32_t S, K kmin, K kmax, uint32_t nb_max,
-                              uint32_t *lut, LutHeader<K> *hdr, int nsl_bits) {
-  __shared__ uint32_t cnt[kLutIdx];  // samples per slice, then the table
+                              uint32_t *lut, uint32_t *tab, LutHeader<K> *hdr, int nsl_bits) {
+  __shared__ uint32_t cnt[SPT * 1024];  // samples per slice
   __shared__ TableShared ts;
   __shared__ uint32_t s_same[2];
   const uint32_t tid = threadIdx.x, lane = tid & 31;
@@ -775,11 +804,10 @@ __device__ void build_lut_cta(const K *samples, uint32_t S, K kmin, K kmax, uint
       if (s0 + u * blockDim.x < S) atomicAdd(&cnt[(uint32_t)((kk[u] - kmin) >> shift)], 1u);
   }
   __syncthreads();
-  // (a thread reads its own slices' counts and its predecessor's last one
-  // before build_table's barriers, and writes entries after them)
-  uint32_t top;
-  const uint32_t nb = build_table<K, SPT>([&](uint32_t j) { return cnt[j]; }, nsl, shift, bcap,
-                                          nb_max, lut, cnt, ts, &top);
+  LutHeader<K> h;
+  table_place<K>(h, kmin, shift, nsl);
+  const uint32_t nb = build_table<K, SPT>([&](uint32_t j) { return cnt[j]; }, nsl, h.low, shift, bcap,
+                                          nb_max, lut, tab, ts);
   __syncthreads();
   // Warp-aggregated cursor updates in compaction pay off when lanes of a warp
   // often hit the same bucket (its atomics return positions, which lanes of
@@ -791,12 +819,8 @@ __device__ void build_lut_cta(const K *samples, uint32_t S, K kmin, K kmax, uint
   // (q, q + S/2).
   uint32_t same = 0, same_key = 0;
   const uint32_t npairs = S / 2 < 2048u ? S / 2 : 2048u;  // enough for a 1/32 estimate
-  auto bucket = [&](K k) {
-    const K d = k - kmin;
-    const K idx = d >> shift;
-    const uint32_t e = idx < (K)nsl ? cnt[(uint32_t)idx] : top;
-    return (uint32_t)((int32_t)e >> 7) + shr_clamp(d, e & 127u);
-  };
+  const KeyTable<K> kt(h);
+  auto bucket = [&](K k) { return bucket_of<K>(k, kt, tab); };
   for (uint32_t q = tid; q < npairs; q += blockDim.x) {
     same += bucket(samples[2 * q]) == bucket(samples[2 * q + 1]) ? 1u : 0u;
     same_key += samples[q] == samples[q + S / 2] ? 1u : 0u;
@@ -809,10 +833,6 @@ __device__ void build_lut_cta(const K *samples, uint32_t S, K kmin, K kmax, uint
   }
   __syncthreads();
   if (tid == 0) {
-    lut[nsl] = top;
-    LutHeader<K> h;
-    h.base = kmin;
-    h.shift = shift;
     h.nb = nb;
     // collision chance >= 1/32: with 32 lanes, about 15 same-bucket pairs per
     // warp access
@@ -972,8 +992,8 @@ __device__ __forceinline__ void cand_put_warp(const CandPool<K> &cp, K k, bool k
 template <class T, int UNROLL, bool INGEST, bool SPEC, bool SWZ>
 __device__ __forceinline__ void hist_body(const T *__restrict__ x, uint64_t n, uint32_t *hist,
                                           const uint32_t *lut /* lane's table */,
-                                          typename Traits<T>::K base,
-                                          uint32_t shift, T *__restrict__ copy_to,
+                                          const KeyTable<typename Traits<T>::K> &kt,
+                                          T *__restrict__ copy_to,
                                           const CandPool<typename Traits<T>::K> &cr,
                                           uint32_t *wcount, uint32_t *wtab,
                                           typename Traits<T>::K *rep) {
@@ -986,6 +1006,18 @@ __device__ __forceinline__ void hist_body(const T *__restrict__ x, uint64_t n, u
   const uint64_t tile_v = (uint64_t)blockDim.x * UNROLL;
   const uint64_t ntiles = sp.nvec / tile_v;
   CandList cl;  // this warp's candidates (SPEC)
+  // counts the key and returns its bucket
+  auto count = [&](K k) -> uint32_t {
+    const uint32_t byte = bucket_byte_of<K>(k, kt, lut);
+    if (SWZ) {
+      const uint32_t i = bank_swz(byte >> 2);
+      atomicAdd(&hist[i], 1u);
+      track_key<K>(hist, rep, i, k);
+    } else {
+      atomicAdd(&word_at(hist, byte), 1u);
+    }
+    return byte >> 2;
+  };
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const uint64_t off = tile * tile_v + threadIdx.x;
     V v[UNROLL];
@@ -1008,10 +1040,7 @@ __device__ __forceinline__ void hist_body(const T *__restrict__ x, uint64_t n, u
       bool any = false;
 #pragma unroll
       for (int e = 0; e < PV; ++e) {
-        b[e] = bucket_of_rep<K>(k[e], base, shift, lut);
-        const uint32_t i = SWZ ? bank_swz(b[e]) : b[e];
-        atomicAdd(&hist[i], 1u);
-        if (SWZ) track_key<K>(hist, rep, i, k[e]);
+        b[e] = count(k[e]);
         if (SPEC) any |= cr.keep(b[e]);
       }
       // one vote per vector; the per-key votes only when a lane keeps one
@@ -1037,12 +1066,7 @@ __device__ __forceinline__ void hist_body(const T *__restrict__ x, uint64_t n, u
       vec_keys<T>(vv, k);
 #pragma unroll
       for (int e = 0; e < PV; ++e) {
-        const uint32_t b = valid ? bucket_of_rep<K>(k[e], base, shift, lut) : 0u;
-        if (valid) {
-          const uint32_t i = SWZ ? bank_swz(b) : b;
-          atomicAdd(&hist[i], 1u);
-          if (SWZ) track_key<K>(hist, rep, i, k[e]);
-        }
+        const uint32_t b = valid ? count(k[e]) : 0u;
         if (SPEC) cand_put_warp<K>(cr, k[e], valid && cr.keep(b), cl, wtab);
       }
     }
@@ -1056,10 +1080,7 @@ __device__ __forceinline__ void hist_body(const T *__restrict__ x, uint64_t n, u
           const T v = x[e];
           if (INGEST) copy_to[e] = v;
           k = Traits<T>::key(v);
-          b = bucket_of_rep<K>(k, base, shift, lut);
-          const uint32_t i = SWZ ? bank_swz(b) : b;
-          atomicAdd(&hist[i], 1u);
-          if (SWZ) track_key<K>(hist, rep, i, k);
+          b = count(k);
         }
         if (SPEC) cand_put_warp<K>(cr, k, valid && cr.keep(b), cl, wtab);
       }
@@ -1084,10 +1105,10 @@ __device__ __forceinline__ void hist_dispatch(const T *__restrict__ x, uint64_t 
   // (measured at 2^26: two-valued, constant and sorted inputs 74 -> 55 us).
   // rep: single-key tracking (and swizzled positions), see k_hist.
   if (rep)
-    hist_body<T, UNROLL, INGEST, SPEC, true>(x, n, hist, lut, h.base, h.shift, copy_to, cr,
+    hist_body<T, UNROLL, INGEST, SPEC, true>(x, n, hist, lut, KeyTable<typename Traits<T>::K>(h), copy_to, cr,
                                              wcount, wtab, rep);
   else
-    hist_body<T, UNROLL, INGEST, SPEC, false>(x, n, hist, lut, h.base, h.shift, copy_to, cr,
+    hist_body<T, UNROLL, INGEST, SPEC, false>(x, n, hist, lut, KeyTable<typename Traits<T>::K>(h), copy_to, cr,
                                               wcount, wtab, nullptr);
 }
 
@@ -1123,7 +1144,7 @@ __global__ void __launch_bounds__(1024, 1)
   const uint32_t *lut = sv_lane_table<K>(rep_lut);  // this lane's copy
   __shared__ uint32_t s_wcnt[kCandWarps];
   __shared__ uint32_t s_tab[kCandWarps * kCandChunksPerWarp];
-  static_assert(sv_slices<uint32_t>() + 1 <= kCandWarps * kCandChunksPerWarp, "s_tab lends its space");
+  static_assert(sv_entries<uint32_t>() <= kCandWarps * kCandChunksPerWarp, "s_tab lends its space");
   fill_words(hist, nb_max, 0u);
   pdl_wait();
   const uint32_t status = ctrl->status;
@@ -1599,7 +1620,7 @@ __global__ void __launch_bounds__(1024, 1)
                uint64_t surv_cap, const uint32_t *__restrict__ bsingle,
                const typename Traits<InT>::K *__restrict__ bkey) {
   using K = typename Traits<InT>::K;
-  constexpr uint32_t kEnt = sv_slices<K>() + 1;
+  constexpr uint32_t kEnt = sv_entries<K>();
   constexpr uint32_t kTiles = kMaxNb / kScanTile;
   static_assert(kTiles < 1024, "a thread per tile and one past the last");
   __shared__ uint32_t s_lut[kEnt];
@@ -1651,9 +1672,9 @@ __global__ void __launch_bounds__(1024, 1)
   K klo = 0, khi = 0;
   bool one = false;
   if (mine) {
-    klo = bucket_lo<K>(b, h.base, h.shift, s_lut, sv_slices<K>());
-    const K knext =
-        (b + 1 < nb) ? bucket_lo<K>(b + 1, h.base, h.shift, s_lut, sv_slices<K>()) : K(0);
+    const uint32_t ents = sv_slices<K>() + 1 + h.low;
+    klo = bucket_lo<K>(b, h.base, h.shift, s_lut, ents);
+    const K knext = (b + 1 < nb) ? bucket_lo<K>(b + 1, h.base, h.shift, s_lut, ents) : K(0);
     // single key iff the next bucket starts one key later; the start of the
     // top entry's bucket can wrap past the key width, and then bucket b runs
     // up to the largest key
@@ -1904,8 +1925,9 @@ __global__ void __launch_bounds__(1024, 1)
   const bool dtrack = bsingle != nullptr && bkey != nullptr && h.dup && dcap != 0 && nb <= dcap;
   for (uint32_t q = s0; q < s1; ++q) {
     const uint32_t b = segb_smem ? s_segb[q] : __ldcg(seg_bucket + q);
-    const K klo = bucket_lo<K>(b, h.base, h.shift, lut, sv_slices<K>());
-    const K knext = (b + 1 < nb) ? bucket_lo<K>(b + 1, h.base, h.shift, lut, sv_slices<K>()) : K(0);
+    const uint32_t ents = sv_slices<K>() + 1 + h.low;
+    const K klo = bucket_lo<K>(b, h.base, h.shift, lut, ents);
+    const K knext = (b + 1 < nb) ? bucket_lo<K>(b + 1, h.base, h.shift, lut, ents) : K(0);
     // single key iff the next bucket starts one key later; the start of the
     // top entry's bucket can wrap past the key width, and then bucket b runs
     // up to the largest key
@@ -2041,22 +2063,23 @@ __global__ void __launch_bounds__(1024, 1)
 // In heavy mode lanes of a warp that hit the same bucket share one atomic
 // (match.any) and take consecutive positions.
 template <class T, bool HEAVY>
-__device__ __forceinline__ void compact_one(typename Traits<T>::K k, typename Traits<T>::K base,
-                                            uint32_t shift, const uint32_t *lut /* lane's table */,
+__device__ __forceinline__ void compact_one(typename Traits<T>::K k,
+                                            const KeyTable<typename Traits<T>::K> &kt,
+                                            const uint32_t *lut /* lane's table */,
                                             uint32_t *cursor,
                                             typename Traits<T>::K *__restrict__ surv, uint32_t cap) {
-  const uint32_t b = bucket_of_rep(k, base, shift, lut);
+  const uint32_t b = bucket_byte_of(k, kt, lut);
   uint32_t pos;
   if (HEAVY) {
     const uint32_t peers = __match_any_sync(0xffffffffu, b);
     const int lane = threadIdx.x & 31;
     const int leader = __ffs(peers) - 1;
     uint32_t p0 = 0;
-    if (lane == leader) p0 = atomicAdd(&cursor[b], (uint32_t)__popc(peers));
+    if (lane == leader) p0 = atomicAdd(&word_at(cursor, b), (uint32_t)__popc(peers));
     p0 = __shfl_sync(peers, p0, leader);
     pos = p0 + __popc(peers & ((1u << lane) - 1u));
   } else {
-    pos = atomicAdd(&cursor[b], 1u);
+    pos = atomicAdd(&word_at(cursor, b), 1u);
   }
   // store without a branch: a predicated st.global
   st_global_if(surv + pos, k, pos < cap);
@@ -2164,7 +2187,7 @@ __global__ void __launch_bounds__(1024, 1)
   __shared__ bool s_spec_miss;
   __shared__ uint32_t s_wcnt[kCandWarps];
   __shared__ uint32_t s_tab[kCandWarps * kCandChunksPerWarp];
-  static_assert(sv_slices<uint32_t>() + 1 <= kCandWarps * kCandChunksPerWarp, "s_tab lends its space");
+  static_assert(sv_entries<uint32_t>() <= kCandWarps * kCandChunksPerWarp, "s_tab lends its space");
   fill_words(cursor, nb_max, kInactive);
   if (threadIdx.x == 0) {
     s_bad = false;
@@ -2230,6 +2253,7 @@ __global__ void __launch_bounds__(1024, 1)
   }
   __syncthreads();
   const uint32_t cap = (uint32_t)(surv_cap < (uint64_t)kInactive ? surv_cap : kInactive);
+  const KeyTable<K> kt(h);
   if (spec && !s_spec_miss && total_surv <= surv_half) {
     // warp w reads the candidates of the histogram pass's warp w
     const uint32_t w = threadIdx.x >> 5;
@@ -2238,7 +2262,7 @@ __global__ void __launch_bounds__(1024, 1)
     const uint32_t cap_lo = (uint32_t)(surv_half < (uint64_t)cap ? surv_half : cap);
     for (uint32_t i = lane; i < cw; i += 32)
       compact_one<T, false>(cand[(uint64_t)wt[i / kCandChunk] * kCandChunk + i % kCandChunk],
-                            h.base, h.shift, lut, cursor, surv, cap_lo);
+                            kt, lut, cursor, surv, cap_lo);
     if (threadIdx.x == 0) atomicAdd(&ctrl->spec_ctas, 1u);
   } else if (h.heavy) {
     constexpr int PV = Traits<T>::kPerVec;
@@ -2248,12 +2272,12 @@ __global__ void __launch_bounds__(1024, 1)
 #pragma unroll
           for (int e = 0; e < PV; ++e) {
             if (in_tiles)
-              compact_one<T, true>(kk[e], h.base, h.shift, lut, cursor, surv, cap);
+              compact_one<T, true>(kk[e], kt, lut, cursor, surv, cap);
             else
-              compact_one<T, false>(kk[e], h.base, h.shift, lut, cursor, surv, cap);
+              compact_one<T, false>(kk[e], kt, lut, cursor, surv, cap);
           }
         },
-        [&](K k) { compact_one<T, false>(k, h.base, h.shift, lut, cursor, surv, cap); });
+        [&](K k) { compact_one<T, false>(k, kt, lut, cursor, surv, cap); });
   } else {
     constexpr int PV = Traits<T>::kPerVec;
     compact_body<T, UNROLL>(
@@ -2261,9 +2285,9 @@ __global__ void __launch_bounds__(1024, 1)
         [&](const K(&kk)[PV], bool) {
 #pragma unroll
           for (int e = 0; e < PV; ++e)
-            compact_one<T, false>(kk[e], h.base, h.shift, lut, cursor, surv, cap);
+            compact_one<T, false>(kk[e], kt, lut, cursor, surv, cap);
         },
-        [&](K k) { compact_one<T, false>(k, h.base, h.shift, lut, cursor, surv, cap); });
+        [&](K k) { compact_one<T, false>(k, kt, lut, cursor, surv, cap); });
   }
   __syncthreads();
   // every cursor must have reached the end of the CTA's share; anything else

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kTableThreads, 1)
   constexpr int SPT = (int)(nsl / kTableThreads);  // slices per thread
   static_assert(nsl % kTableThreads == 0 && kLutIdx == 8 * kTableThreads, "shares of the slices");
   __shared__ __align__(16) uint32_t fine[kLutIdx];
-  __shared__ uint32_t tab[nsl];
+  __shared__ uint32_t tab[sv_entries<K>()];
   __shared__ TableShared ts;
   __shared__ uint32_t s_scan[32];
   __shared__ uint32_t s_same;
@@ -295,9 +295,9 @@ __global__ void __launch_bounds__(kTableThreads, 1)
     for (uint32_t i = j << fold; i < (j + 1) << fold; ++i) m = max(m, fine[i]);
     return m << fold;
   };
-  uint32_t top;
-  const uint32_t nb = build_table<K, SPT>(density, nsl, shift, bcap, nb_max, lut, tab, ts, &top);
-  if (tid == 0) lut[nsl] = top;
+  LutHeader<K> h;
+  table_place<K>(h, kmin, shift, nsl);
+  const uint32_t nb = build_table<K, SPT>(density, nsl, h.low, shift, bcap, nb_max, lut, tab, ts);
 
   // Candidate windows.  The number of samples below the element of rank r is
   // about Binomial(S, r / n); each window [lo, hi] of ranks is widened to the
@@ -329,12 +329,8 @@ __global__ void __launch_bounds__(kTableThreads, 1)
     if (tid < 8) s_sp[tid] = (tid & 3) == 1 ? 0xFFFFFFFEu : ((tid & 3) == 3 ? S : 0u);
   }
   __syncthreads();  // the table
-  auto bucket = [&](K k) {
-    const K d = k - kmin;
-    const K idx = d >> shift;
-    const uint32_t e = idx < (K)nsl ? tab[(uint32_t)idx] : top;
-    return (uint32_t)((int32_t)e >> 7) + shr_clamp(d, e & 127u);
-  };
+  const KeyTable<K> kt(h);
+  auto bucket = [&](K k) { return bucket_of<K>(k, kt, tab); };
   if (nwin) {
     // the fine slices split the sample ranks [0, S) in order: eight per thread
     uint32_t fc[8], sum = 0;
@@ -380,9 +376,6 @@ __global__ void __launch_bounds__(kTableThreads, 1)
   if (lane == 0 && near_same) atomicAdd(&s_same, near_same);
   __syncthreads();
   if (tid == 0) {
-    LutHeader<K> h;
-    h.base = kmin;
-    h.shift = shift;
     h.nb = nb;
     // collision chance >= 1/32: with 32 lanes, about 15 same-bucket pairs per
     // warp access

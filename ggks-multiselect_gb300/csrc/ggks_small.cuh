@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   extern __shared__ uint4 smem_raw[];
   uint32_t *rep = reinterpret_cast<uint32_t *>(smem_raw);
   uint32_t *hc = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(smem_raw) + kSmHcOff);
-  __shared__ uint32_t s_tab[sv_slices<K>() + 1];  // the splitter table
+  __shared__ uint32_t s_tab[sv_entries<K>()];  // the splitter table
   __shared__ LutHeader<K> s_hdr;
   __shared__ K redk[33];
   __shared__ uint32_t red32[33];
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
     hi = block_reduce(hi, [](K u, K v) { return u > v ? u : v; }, redk);
     GGKS_SMALL_STAMP(1);
     build_lut_cta<K, (int)((sv_slices<K>() + kSmThreads - 1) / kSmThreads)>(
-        samples, S, lo, hi, kSmNb, s_tab, &s_hdr, sv_bits<K>());
+        samples, S, lo, hi, kSmNb, s_tab, s_tab, &s_hdr, sv_bits<K>());
   }
   __syncthreads();
   GGKS_SMALL_STAMP(2);
@@ -268,14 +268,15 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   // ---------------- B: histogram of this CTA's share
   for (uint32_t b = tid; b < kSmNb; b += kSmThreads) hc[b] = 0;
   __syncthreads();
-  for (uint32_t i = tid; i < (sv_slices<K>() + 1) * sv_copies<K>(); i += kSmThreads)
+  for (uint32_t i = tid; i < sv_entries<K>() * sv_copies<K>(); i += kSmThreads)
     rep[i] = s_tab[i >> sv_copy_bits<K>()];
   const LutHeader<K> h = s_hdr;
+  const KeyTable<K> kt(h);
   const uint64_t a0 = n * r / kSmCtas, a1 = n * (r + 1) / kSmCtas;
   const uint32_t *lut = sv_lane_table<K>(rep);
   __syncthreads();
   for_range<T>(x, a0, a1, [&](K k, bool) {
-    atomicAdd(&hc[bucket_of_rep<K>(k, h.base, h.shift, lut)], 1u);
+    atomicAdd(&word_at(hc, bucket_byte_of<K>(k, kt, lut)), 1u);
   });
   cl.sync();  // 1: every histogram is complete (and every CTA has started)
   GGKS_SMALL_STAMP(3);
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   {
     const uint32_t cap = (uint32_t)(surv_cap < (uint64_t)kInactive ? surv_cap : kInactive);
     for_range<T>(x, a0, a1, [&](K k, bool) {
-      const uint32_t pos = atomicAdd(&hc[bucket_of_rep<K>(k, h.base, h.shift, lut)], 1u);
+      const uint32_t pos = atomicAdd(&word_at(hc, bucket_byte_of<K>(k, kt, lut)), 1u);
       st_global_if(surv + pos, k, pos < cap);
     });
   }
@@ -391,8 +392,9 @@ __global__ void __launch_bounds__(kSmThreads, 1)
     const uint32_t nsmall = s_nsmall, nlarge = s_nlarge;
     // key range of bucket gb: from its first key to the next bucket's
     auto range = [&](uint32_t gb, K *klo, K *khi) {
-      const K lo = bucket_lo<K>(gb, h.base, h.shift, s_tab, sv_slices<K>());
-      const K nx = gb + 1 < h.nb ? bucket_lo<K>(gb + 1, h.base, h.shift, s_tab, sv_slices<K>()) : K(0);
+      const uint32_t ents = sv_slices<K>() + 1 + h.low;
+      const K lo = bucket_lo<K>(gb, h.base, h.shift, s_tab, ents);
+      const K nx = gb + 1 < h.nb ? bucket_lo<K>(gb + 1, h.base, h.shift, s_tab, ents) : K(0);
       *klo = lo;
       *khi = nx > lo ? nx - K(1) : KeyMax<K>::v;
     };
