@@ -369,8 +369,11 @@ static int api_batch(const T *const *vecs, const uint64_t *n, uint32_t P, const 
     if (K) {
       if ((uint64_t)K[p] > n[p]) return GGKS_INVALID_ARG;
     } else {
-      for (uint32_t j = k_off[p]; j < k_off[p + 1]; ++j)
-        if (h_k[j] < 1 || (uint64_t)h_k[j] > n[p]) return GGKS_INVALID_ARG;
+      // 1 <= k <= n < 2^32, without an exit from the loop (it vectorises)
+      const uint32_t *ks = h_k + k_off[p], n32 = (uint32_t)n[p];
+      uint32_t bad = 0;
+      for (uint32_t j = 0; j < nr; ++j) bad |= ks[j] - 1u >= n32 ? 1u : 0u;
+      if (bad) return GGKS_INVALID_ARG;
     }
     bytes += n[p] * sizeof(T);
     elems += n[p];
