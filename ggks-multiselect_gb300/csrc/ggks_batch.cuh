@@ -137,7 +137,9 @@ struct BTile {
   uint64_t begin, end;  // elements [begin, end) of problem prob
   uint32_t prob, rank;  // rank of the tile among its problem's tiles
   uint64_t cand_off;    // key index of the tile's candidate area (speculating problems)
-  uint32_t cand_cap, pad;
+  uint32_t cand_cap;
+  uint32_t nsl_bits;    // its problem's, and lut_off: the table is loaded with the header
+  uint64_t lut_off;
 };
 
 struct BCtrl {
@@ -247,6 +249,13 @@ __device__ __forceinline__ uint32_t grid_barrier(BCtrl *c, uint32_t *s_status, i
   __syncthreads();
   return *s_status;
 }
+
+// Problems of at most this many tiles have their bucket totals summed from the
+// tiles' rows in the plan phase; the tiles of longer ones add to the totals (one
+// global atomic per bucket and tile).  (Sums for all short problems: counting 1600 ->
+// 1554 us, plan 168 -> 187 us with 2^20-element tiles (4096 vectors of 2^10 to
+// 2^22 floats).)
+constexpr uint32_t kBSumRows = 8;
 
 // next item of a work queue, shared with the whole CTA
 __device__ __forceinline__ uint32_t queue_pop(uint32_t *q, uint32_t *s_item) {
@@ -722,7 +731,8 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       A.hdrs[p] = h;
     }
     // the bucket totals start at zero: the tiles of phase 2 add to them
-    for (uint32_t b = tid; b < P.nb_max; b += nt) A.counts[P.cnt_off + b] = 0;
+    if (P.ntiles > kBSumRows)
+      for (uint32_t b = tid; b < P.nb_max; b += nt) A.counts[P.cnt_off + b] = 0;
   }
   uint32_t st = grid_barrier(ctrl, &s_status, 1);
 
@@ -733,16 +743,20 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
   uint32_t *hist = sm + kBTileLut;
   K *rep = reinterpret_cast<K *>(hist + kBMaxNb);
   K *reps = reinterpret_cast<K *>(A.reps);
+  // the copies of a tile's splitter table, unless its problem's is there already
+  auto load_table = [&](const BTile &tl) {
+    if (s_cur != tl.prob)
+      for (uint32_t w = tid; w < ((1u << tl.nsl_bits) + 2) * sv_copies<K>(); w += nt)
+        sm[w] = __ldcg(A.luts + tl.lut_off + (w >> sv_copy_bits<K>()));
+  };
   if (!(st & ST_FATAL)) {
-    for (uint32_t t = queue_pop(&ctrl->queue[1], &s_item); t < A.num_tiles;
-         t = queue_pop(&ctrl->queue[1], &s_item)) {
-      const BTile tl = A.tiles[t];
+    uint32_t t = queue_pop(&ctrl->queue[1], &s_item);
+    BTile tl{};
+    if (t < A.num_tiles) tl = A.tiles[t];
+    while (t < A.num_tiles) {
+      load_table(tl);
       const BProb P = A.probs[tl.prob];
       const BHdr H = load_hdr(A.hdrs + tl.prob);
-      const uint32_t nsl = 1u << P.nsl_bits;
-      if (s_cur != tl.prob)
-        for (uint32_t w = tid; w < (nsl + 2) * sv_copies<K>(); w += nt)
-          sm[w] = __ldcg(A.luts + P.lut_off + (w >> sv_copy_bits<K>()));
       for (uint32_t b = tid; b < ((H.nb + 31) & ~31u); b += nt) {
         hist[b] = 0;
         if (H.dup) rep[b] = KeyMax<K>::v;
@@ -797,18 +811,28 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
           atomicAdd(&word_at(hist, byte), 1u);
         });
       }
+      if (tid == 0) s_item = atomicAdd(&ctrl->queue[1], 1u);
       __syncthreads();
       if (H.spec_on && tid == 0) A.cand_cnt[t] = s_ccnt;
       const uint64_t ro = P.row0 + (uint64_t)tl.rank * P.nb_max;
-      if (!BCHECK(ro + H.nb <= A.row_words && H.nb <= P.nb_max, 5, ro, H.nb)) continue;
-      // the tile's row, and its counts added to the problem's bucket totals
-      uint32_t *tot = A.counts + P.cnt_off;
-      for (uint32_t b = tid; b < H.nb; b += nt) {
-        const uint32_t c = hist[H.dup ? swz(b) : b];
-        A.rows[ro + b] = c;
-        if (c & ~kMixed) atomicAdd(tot + b, c & ~kMixed);
-        if (H.dup) reps[ro + b] = rep[swz(b)];
+      const bool ok = BCHECK(ro + H.nb <= A.row_words && H.nb <= P.nb_max, 5, ro, H.nb);
+      t = s_item;
+      if (t < A.num_tiles) tl = A.tiles[t];
+      // the tile's row (and its counts added to a long problem's bucket totals)
+      if (!ok) {
+      } else if (H.dup || P.ntiles > kBSumRows) {
+        uint32_t *tot = A.counts + P.cnt_off;
+        for (uint32_t b = tid; b < H.nb; b += nt) {
+          const uint32_t c = hist[H.dup ? swz(b) : b];
+          A.rows[ro + b] = c;
+          if (P.ntiles > kBSumRows && (c & ~kMixed)) atomicAdd(tot + b, c & ~kMixed);
+          if (H.dup) reps[ro + b] = rep[swz(b)];
+        }
+      } else {
+        for (uint32_t v = tid; v < (H.nb + 3) / 4; v += nt)
+          reinterpret_cast<uint4 *>(A.rows + ro)[v] = reinterpret_cast<const uint4 *>(hist)[v];
       }
+      __syncthreads();
     }
   }
   st = grid_barrier(ctrl, &s_status, 2);
@@ -828,9 +852,30 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
                   6, p, nb))
         continue;
       for (uint32_t j = tid; j < nsl + 2; j += nt) lut[j] = __ldcg(A.luts + P.lut_off + j);
-      // bucket totals (added by the tiles of phase 2) -> exclusive prefix in
-      // shared memory; the flags start clear
-      load_totals(cnt, nb, excl);
+      // bucket totals -> exclusive prefix in shared memory; the flags start clear
+      if (nr > kBSumRows) {
+        load_totals(cnt, nb, excl);
+      } else {
+        // the sums of the tiles' rows, four buckets per thread; zero past nb
+        const uint4 *rv = reinterpret_cast<const uint4 *>(A.rows + P.row0);
+        for (uint32_t v = tid; v < (nb + 3) / 4; v += nt) {
+          uint4 s = make_uint4(0, 0, 0, 0);
+#pragma unroll
+          for (uint32_t r = 0; r < kBSumRows; ++r) {
+            if (r >= nr) break;
+            const uint4 e = __ldcg(rv + (uint64_t)r * (P.nb_max / 4) + v);
+            s.x += e.x & ~kMixed;
+            s.y += e.y & ~kMixed;
+            s.z += e.z & ~kMixed;
+            s.w += e.w & ~kMixed;
+          }
+          if (4 * v + 1 >= nb) s.y = 0;
+          if (4 * v + 2 >= nb) s.z = 0;
+          if (4 * v + 3 >= nb) s.w = 0;
+          reinterpret_cast<uint4 *>(excl)[v] = s;
+          reinterpret_cast<uint4 *>(cnt)[v] = s;
+        }
+      }
       for (uint32_t v = tid; v < ((nb + 3) >> 2); v += nt) reinterpret_cast<uint32_t *>(flag)[v] = 0;
       __syncthreads();
       if (smem_excl_scan(excl, nb, red32) != P.n && tid == 0) atomicOr(&ctrl->status, ST_INTERNAL);
@@ -1071,15 +1116,18 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       s_bad = false;
     }
     uint32_t *cursor = sm + kBTileLut;
-    for (uint32_t t = queue_pop(&ctrl->queue[3], &s_item); t < A.num_tiles;
-         t = queue_pop(&ctrl->queue[3], &s_item)) {
-      const BTile tl = A.tiles[t];
+    uint32_t t = queue_pop(&ctrl->queue[3], &s_item);
+    BTile tl{};
+    if (t < A.num_tiles) tl = A.tiles[t];
+    while (t < A.num_tiles) {
+      load_table(tl);
       const BProb P = A.probs[tl.prob];
       const BHdr H = load_hdr(A.hdrs + tl.prob);
-      const uint32_t nsl = 1u << P.nsl_bits;
-      if (s_cur != tl.prob)
-        for (uint32_t w = tid; w < (nsl + 2) * sv_copies<K>(); w += nt)
-          sm[w] = __ldcg(A.luts + P.lut_off + (w >> sv_copy_bits<K>()));
+      // this thread's first slot: its size, bucket and place in one round of loads
+      const bool has0 = tid < P.num_req;
+      const uint32_t sz0 = has0 ? __ldcg(A.seg_size + P.req_off + tid) : 0u;
+      const uint32_t b0 = has0 ? __ldcg(A.seg_bucket + P.req_off + tid) : 0u;
+      const uint64_t off0 = has0 ? ldcg_u(A.seg_off + P.req_off + tid) : 0u;
       for (uint32_t b = tid; b < ((H.nb + 31) & ~31u); b += nt) cursor[b] = kInactive;
       __syncthreads();
       if (tid == 0) s_cur = tl.prob;
@@ -1087,18 +1135,33 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       // Positions relative to the problem's survivor range (flat slots have
       // none): the tile takes its share of each slot's segment with one
       // atomic on the slot's fill counter (tiles take their shares in any
-      // order; the order of a segment's keys does not matter), and leaves the
-      // end of its share in its row for the check below.
-      for (uint32_t s = tid; s < H.num_slots; s += nt) {
+      // order; the order of a segment's keys does not matter).  The end of its
+      // share is kept for the check below: a thread's first slot's in a
+      // register, further ones' in the tile's row.  A problem's only tile takes
+      // the whole segments.
+      auto share = [&](uint32_t g, uint32_t sz, uint32_t b, uint64_t off, uint32_t *end) {
+        uint32_t c = sz, pre = 0;
+        if (P.ntiles > 1) {
+          c = __ldcg(row + b) & ~kMixed;
+          pre = c ? atomicAdd(A.fill + g, c) : 0u;
+        }
+        const uint32_t at = (uint32_t)(off - H.surv_off + pre);
+        cursor[H.dup ? swz(b) : b] = at;
+        *end = at + c;
+      };
+      bool live0 = tid < H.num_slots && sz0 != 0;
+      uint32_t end0 = 0;
+      if (live0) {
+        live0 = BCHECK(b0 < H.nb && tid < P.num_req, 10, b0, tid);
+        if (live0) share(P.req_off + tid, sz0, b0, off0, &end0);
+      }
+      for (uint32_t s = tid + nt; s < H.num_slots; s += nt) {
         const uint32_t g = P.req_off + s;
-        if (__ldcg(A.seg_size + g) == 0) continue;
+        const uint32_t sz = __ldcg(A.seg_size + g);
+        if (sz == 0) continue;
         const uint32_t b = __ldcg(A.seg_bucket + g);
         if (!BCHECK(b < H.nb && s < P.num_req, 10, b, s)) continue;
-        const uint32_t c = __ldcg(row + b) & ~kMixed;
-        const uint32_t pre = c ? atomicAdd(A.fill + g, c) : 0u;
-        const uint32_t at = (uint32_t)(ldcg_u(A.seg_off + g) - H.surv_off + pre);
-        cursor[H.dup ? swz(b) : b] = at;
-        row[b] = at + c;
+        share(g, sz, b, ldcg_u(A.seg_off + g), row + b);
       }
       __syncthreads();
       K *sp = surv + H.surv_off;
@@ -1164,16 +1227,21 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
             st_global_if(sp + pos, k, pos < cap);
           });
       }
+      if (tid == 0) s_item = atomicAdd(&ctrl->queue[3], 1u);
       __syncthreads();
+      t = s_item;
+      const uint32_t num_slots = H.num_slots, req_off = P.req_off;
+      if (t < A.num_tiles) tl = A.tiles[t];
       // each cursor must end where the tile's share of the segment ends
-      for (uint32_t s = tid; s < H.num_slots; s += nt) {
-        const uint32_t g = P.req_off + s;
+      if (live0 && cursor[H.dup ? swz(b0) : b0] != end0) s_bad = true;
+      for (uint32_t s = tid + nt; s < num_slots; s += nt) {
+        const uint32_t g = req_off + s;
         if (__ldcg(A.seg_size + g) == 0) continue;
         const uint32_t b = __ldcg(A.seg_bucket + g);
         if (cursor[H.dup ? swz(b) : b] != __ldcg(row + b)) s_bad = true;
       }
+      __syncthreads();
     }
-    __syncthreads();
     if (tid == 0 && s_bad) atomicOr(&ctrl->status, ST_INTERNAL);
   }
   st = grid_barrier(ctrl, &s_status, 4);

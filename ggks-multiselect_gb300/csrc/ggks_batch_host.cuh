@@ -198,6 +198,8 @@ int select_batch(Context &ctx, const BatchInput &in, T *d_out_user, T *h_out, cu
       t.prob = np;
       t.rank = r;
       t.cand_off = cand_words;
+      t.nsl_bits = nsl_bits;
+      t.lut_off = b.lut_off;
       const uint64_t len = t.end - t.begin;
       if (b.spec) {
         const uint64_t cap = std::min<uint64_t>(len, (uint64_t)(cand_per * (double)len) + 256);

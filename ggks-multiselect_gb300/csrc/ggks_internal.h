@@ -22,10 +22,15 @@ namespace ggks {
 constexpr int kMaxDevices = 64;
 
 // Tunables of the batched path: bucket budget of a problem is about n / div
-// buckets; tiles of the (problem, tile) queue hold `tile` elements.
+// buckets; tiles of the (problem, tile) queue hold `tile` elements, or fewer when
+// that would leave less than two tiles per resident CTA.  Large tiles because each
+// one clears and writes its counts (4096 vectors of 2^10 to 2^22 floats, counting /
+// compaction: 2^18 elements 1790 / 1782 us, 2^20 1600 / 1677, 2^21
+// 1577 / 1670; tile sizes that shrink as the work runs out were slower, 4335-4370
+// us a call against 4200, and so was taking the next tile early).
 struct BatchTune {
   uint32_t div = 256;
-  uint32_t tile = 1u << 18;
+  uint32_t tile = 1u << 21;
 };
 
 // Orders the batched launches of several contexts (a server's lanes) on the

@@ -54,3 +54,27 @@ def test_batch_k_out_of_range(g, bad):
     ks[17] = bad
     with pytest.raises(Exception):
         g.multiselect_batch_ptr([d.ptr, d.ptr], [5000, 5000], np.float32, [ks[:3], ks])
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.uint32, np.float64])
+@pytest.mark.parametrize("values", ["many", "few", "sorted"])
+def test_batch_totals(g, dtype, values):
+    """Problems of 1, 2, 8, 9 and 17 tiles: bucket totals come from the rows of up
+    to eight tiles and by atomics beyond, a problem's only tile takes whole
+    segments, and more than 512 slots leave a thread more than one."""
+    tile = 65536
+    r = np.random.default_rng(5)
+    lens = [100, tile - 3, tile, tile + 1, 8 * tile, 8 * tile + 1, 17 * tile - 9]
+    x = r.integers(0, 50 if values == "few" else 1 << 32, max(lens), dtype=np.uint32)
+    x = x.astype(dtype) if dtype == np.uint32 or values == "few" else \
+        r.standard_normal(max(lens)).astype(dtype)
+    if values == "sorted":
+        x = np.sort(x)
+    d = DeviceArray(x)
+    ctx = g.Context(0)
+    g.batch_set_tuning(ctx, 16, tile)
+    ks = [np.unique(r.integers(1, n + 1, 1500)).astype(np.uint32) for n in lens]
+    got = g.multiselect_batch_ptr([d.ptr] * len(lens), lens, x.dtype, ks, ctx=ctx)
+    for n, k, o in zip(lens, ks, got):
+        assert_same(o, np.sort(x[:n])[::-1][k.astype(np.int64) - 1], f"n={n}")
+    ctx.close()
