@@ -25,9 +25,10 @@ constexpr int kMaxDevices = 64;
 // buckets; tiles of the (problem, tile) queue hold `tile` elements, or fewer when
 // that would leave less than two tiles per resident CTA.  Large tiles because each
 // one clears and writes its counts (4096 vectors of 2^10 to 2^22 floats, counting /
-// compaction: 2^18 elements 1790 / 1782 us, 2^20 1600 / 1677, 2^21
-// 1577 / 1670; tile sizes that shrink as the work runs out were slower, 4335-4370
-// us a call against 4200, and so was taking the next tile early).
+// compaction: 2^18 elements 1790 / 1782 us, 2^20 1600 / 1677; with the row sums of
+// kBSumRows 2^20 1554 / 1697, 2^21 1532 / 1688; tile sizes that shrink as the work
+// runs out were slower, 4335-4370 us a call against 4200, and taking the next tile
+// early cost the batches of few vectors 4 %).
 struct BatchTune {
   uint32_t div = 256;
   uint32_t tile = 1u << 21;
