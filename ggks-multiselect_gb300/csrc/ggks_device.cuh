@@ -221,12 +221,14 @@ struct Ctrl {
   // rank windows of the call's requests, set by the host (0 windows: the
   // requests are spread out or unknown)
   uint32_t spec_nwin;
-  uint32_t spec_pad;
+  uint32_t dense_lo;  // keys below a dense table's range (k_hist)
   uint64_t spec_lo[2], spec_hi[2];  // ascending 0-based ranks, inclusive
   uint32_t spec_on;    // the table keeps candidate buckets (k_table)
   uint32_t spec_ctas;  // compaction CTAs that read candidates
   uint32_t cand_next;  // candidate chunks handed out (k_hist)
   uint32_t fin_done;   // last-CTA ticket of k_finish
+  uint32_t dense_hi;   // keys above a dense table's range (k_hist)
+  uint32_t pad;
   uint64_t t_ns[16];   // phase stamps of the small-vector kernel (GGKS_SMALL_TIMING builds)
 };
 
@@ -247,7 +249,24 @@ struct LutHeader {
   uint32_t cand_cap;
   uint32_t spec_lo[2];
   uint32_t spec_len[2];
+  uint32_t dense;  // 1: bucket b is the key base + b, counted in 16 bits (kDenseKeys buckets)
 };
+// A dense table: integer keys whose sampled span lies between 2^15 and 2^16 (16-bit
+// pixels, codes, counts; a narrower span's ordinary table already has a bucket
+// per key).  Every key of a range of kDenseKeys around the sample is a bucket, two
+// 16-bit counts to a word of the histogram's rows, so the plan answers the
+// requests from the counts: no compaction, no segments.  The histogram pass needs no
+// table; it counts the keys outside the range in the end buckets and lists them
+// (the sample missed them, so they are few), and a request that falls on one is
+// answered from its side's list, a segment like any other.  A list that overflows,
+// or a count past 16 bits, which shows in the total, has the host run the call again
+// without (ST_TOPK_MISS); k_table takes a dense table only where no sampled slice
+// of keys could fill a count.  Bound: the counts' shared-memory atomics.  2^26
+// values of 2^16, 1001 k's: 174 -> 96 us a call (histogram 57 -> 54 us, compaction
+// 64 -> 6, finisher 21 -> 10).
+constexpr uint32_t kDenseKeys = 1u << 16;
+constexpr uint32_t kDenseList = 32768;  // keys outside the range that a side's list holds
+constexpr float kDenseFill = 29000.0f;  // expected keys of a CTA in one slice, at most
 
 template <class K>
 __device__ __forceinline__ bool in_spec(const LutHeader<K> &h, uint32_t b) {
@@ -769,6 +788,7 @@ __device__ __forceinline__ void table_place(LutHeader<K> &h, K kmin, uint32_t sh
   const K ents = (K)(nsl + h.low);
   h.top = ents > (KeyMax<K>::v >> shift) ? KeyMax<K>::v : ents << shift;
   h.shift = shift;
+  h.dense = 0;
 }
 
 // The splitter table of one problem of a batch, or of a small vector, from its
@@ -1112,6 +1132,59 @@ __device__ __forceinline__ void hist_dispatch(const T *__restrict__ x, uint64_t 
                                               wcount, wtab, nullptr);
 }
 
+// Counts of a dense table: the halves of hist[0 .. kDenseKeys / 2).  Keys outside
+// [base, base + kDenseKeys) also go to list (those below) or list + kDenseList.
+template <int UNROLL>
+__device__ __forceinline__ void dense_body(const uint32_t *__restrict__ x, uint64_t n,
+                                           uint32_t *hist, const KeyTable<uint32_t> &kt,
+                                           uint32_t *__restrict__ list, Ctrl *ctrl) {
+  auto count = [&](uint32_t k) {
+    const uint32_t d = kt.pos(k);
+    atomicAdd(hist + (d >> 1), (d & 1u) * 65535u + 1u);
+  };
+  auto outside = [&](uint32_t k) {
+    if (k - kt.base < kDenseKeys) return;
+    const bool below = k < kt.base;
+    const uint32_t at = atomicAdd(below ? &ctrl->dense_lo : &ctrl->dense_hi, 1u);
+    if (at < kDenseList) list[(below ? 0u : kDenseList) + at] = k;
+  };
+  const Span<uint32_t> sp = split_span(x, n);
+  const uint4 *xv = reinterpret_cast<const uint4 *>(x + sp.head);
+  const uint64_t tile_v = (uint64_t)blockDim.x * UNROLL;
+  const uint64_t ntiles = sp.nvec / tile_v;
+  auto count4 = [&](const uint4 &v) {
+    count(v.x);
+    count(v.y);
+    count(v.z);
+    count(v.w);
+    // (one test for the four keys)
+    if (((v.x - kt.base) | (v.y - kt.base) | (v.z - kt.base) | (v.w - kt.base)) >= kDenseKeys) {
+      outside(v.x);
+      outside(v.y);
+      outside(v.z);
+      outside(v.w);
+    }
+  };
+  auto one = [&](uint32_t k) {
+    count(k);
+    outside(k);
+  };
+  for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const uint4 *p = xv + tile * tile_v + threadIdx.x;
+    uint4 v[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) v[u] = ldg_stream(p + (uint64_t)u * blockDim.x);
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) count4(v[u]);
+  }
+  if (blockIdx.x == (uint32_t)(ntiles % gridDim.x)) {
+    for (uint64_t vi = ntiles * tile_v + threadIdx.x; vi < sp.nvec; vi += blockDim.x)
+      count4(ldg_stream(xv + vi));
+    for (uint64_t e = threadIdx.x; e < sp.head; e += blockDim.x) one(x[e]);
+    for (uint64_t e = sp.tail0 + threadIdx.x; e < n; e += blockDim.x) one(x[e]);
+  }
+}
+
 // copy_to == nullptr: x is the device vector.  Otherwise x is a mapped host
 // vector and this pass also writes the device copy (see hist_body).  cand:
 // the candidate pool (nullptr: no speculation); when the table keeps
@@ -1128,7 +1201,7 @@ template <class T, int UNROLL>
 __global__ void __launch_bounds__(1024, 1)
     k_hist(const T *__restrict__ x, uint64_t n, const LutHeader<typename Traits<T>::K> *hdr,
            const uint32_t *__restrict__ lut_g, uint32_t *__restrict__ partials, uint32_t nb_max,
-           const Ctrl *ctrl, T *__restrict__ copy_to, typename Traits<T>::K *__restrict__ cand,
+           Ctrl *ctrl, T *__restrict__ copy_to, typename Traits<T>::K *__restrict__ cand,
            uint32_t *__restrict__ cand_cnt, uint32_t *__restrict__ cand_tab,
            uint32_t *cand_next, typename Traits<T>::K *__restrict__ reps) {
   // Clearing the counts needs nothing of the kernels before: it runs ahead of
@@ -1151,6 +1224,16 @@ __global__ void __launch_bounds__(1024, 1)
   const LutHeader<K> h = *hdr;
   load_rep_table<K>(rep_lut, lut_g, s_tab);
   if (status & ST_FATAL) return;
+  if constexpr (std::is_same<T, uint32_t>::value) {
+    if (h.dense) {
+      dense_body<UNROLL>(x, n, hist, KeyTable<K>(h), cand, ctrl);
+      __syncthreads();
+      uint4 *row = reinterpret_cast<uint4 *>(partials + (uint64_t)blockIdx.x * nb_max);
+      for (uint32_t v = threadIdx.x; v < kDenseKeys / 8; v += blockDim.x)
+        row[v] = reinterpret_cast<const uint4 *>(hist)[v];
+      return;
+    }
+  }
   const uint32_t dcap = dup_nb_cap<K>(nb_max);
   const bool track = reps != nullptr && h.dup && dcap != 0 && h.nb <= dcap;
   K *rep = track ? reinterpret_cast<K *>(hist + dcap) : nullptr;
@@ -1230,15 +1313,17 @@ __global__ void __launch_bounds__(kScanThreads, 4)
   constexpr uint32_t kVecs = kScanTile / 4;              // 16-byte vectors per tile row
   constexpr uint32_t kGroups = kScanThreads / kVecs;     // row groups
   constexpr uint32_t kBatch = 8;                         // loads in flight per thread
-  __shared__ uint32_t gsum[kGroups][kScanTile];
+  __shared__ __align__(16) uint32_t gsum[kGroups][kScanTile], ghigh[kGroups][kScanTile];
   __shared__ uint32_t s_w2[2];
   __shared__ uint8_t gstate[kGroups][kScanTile];  // single-key tracking: 0 none, 1 one key, 2 more
   __shared__ K gkey[kGroups][kScanTile];
   if (ctrl->status & ST_FATAL) return;
-  const uint32_t nb = hdr->nb;
+  const bool dense = hdr->dense != 0;
+  // a dense table: the 64 columns of words are 128 buckets, two tiles
+  const uint32_t nb = dense ? kDenseKeys / 2 : hdr->nb;
   if ((uint64_t)blockIdx.x * kScanTile >= nb) return;
   const uint32_t dcap = dup_nb_cap<K>(nb_max);
-  const bool track = reps != nullptr && hdr->dup && dcap != 0 && nb <= dcap;
+  const bool track = reps != nullptr && hdr->dup && dcap != 0 && nb <= dcap;  // (a dense table: not)
   // thread t sums buckets 4 (t % kVecs) .. + 3 of the tile over row group
   // t / kVecs: a row's 64 buckets are one 256-byte span read by 16 lanes
   const uint32_t v = threadIdx.x % kVecs, grp = threadIdx.x / kVecs;
@@ -1248,6 +1333,44 @@ __global__ void __launch_bounds__(kScanThreads, 4)
   const uint4 *p = reinterpret_cast<const uint4 *>(partials + b0);
   const uint32_t row4 = nb_max / 4;  // nb_max is a multiple of 4
   uint4 gs = make_uint4(0, 0, 0, 0);
+  if (dense) {
+    uint4 gh = make_uint4(0, 0, 0, 0);  // the high halves
+    for (uint32_t r = r0; r < r1; r += kBatch) {
+      uint4 e[kBatch];
+#pragma unroll
+      for (uint32_t q = 0; q < kBatch; ++q)
+        e[q] = r + q < r1 ? __ldcg(p + (uint64_t)(r + q) * row4) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (uint32_t q = 0; q < kBatch; ++q) {
+        gs.x += e[q].x & 0xFFFFu;
+        gs.y += e[q].y & 0xFFFFu;
+        gs.z += e[q].z & 0xFFFFu;
+        gs.w += e[q].w & 0xFFFFu;
+        gh.x += e[q].x >> 16;
+        gh.y += e[q].y >> 16;
+        gh.z += e[q].z >> 16;
+        gh.w += e[q].w >> 16;
+      }
+    }
+    reinterpret_cast<uint4 *>(gsum[grp])[v] = gs;
+    reinterpret_cast<uint4 *>(ghigh[grp])[v] = gh;
+    __syncthreads();
+    const uint32_t col = threadIdx.x;  // a word; the first warp's are one tile, the second's the next
+    if (col < kScanTile) {
+      uint32_t lo = 0, hi = 0;
+#pragma unroll
+      for (uint32_t g = 0; g < kGroups; ++g) {
+        lo += gsum[g][col];
+        hi += ghigh[g][col];
+      }
+      const uint32_t incl = warp_incl_scan(lo + hi), pre = incl - lo - hi;
+      const uint32_t b = 2 * (blockIdx.x * kScanTile + col);
+      *reinterpret_cast<uint2 *>(bpre + b) = make_uint2(pre, pre + lo);
+      if (b % 8 == 0) bco[b / 8] = pre;
+      if ((col & 31) == 31) ttot[b / kScanTile] = incl;
+    }
+    return;
+  }
   if (b0 < nb) {
     for (uint32_t r = r0; r < r1; r += kBatch) {
       uint4 e[kBatch];
@@ -1618,11 +1741,11 @@ __global__ void __launch_bounds__(1024, 1)
                typename Traits<InT>::K *__restrict__ seg_lo,
                typename Traits<InT>::K *__restrict__ seg_hi, Req *__restrict__ klist,
                uint64_t surv_cap, const uint32_t *__restrict__ bsingle,
-               const typename Traits<InT>::K *__restrict__ bkey) {
+               const typename Traits<InT>::K *__restrict__ bkey, uint64_t dense_at) {
   using K = typename Traits<InT>::K;
   constexpr uint32_t kEnt = sv_entries<K>();
-  constexpr uint32_t kTiles = kMaxNb / kScanTile;
-  static_assert(kTiles < 1024, "a thread per tile and one past the last");
+  constexpr uint32_t kTiles = kDenseKeys / kScanTile;
+  static_assert(kTiles <= 1024 && kMaxNb <= kDenseKeys, "a thread per tile");
   __shared__ uint32_t s_lut[kEnt];
   __shared__ uint32_t s_tile[kTiles + 1];
   __shared__ uint32_t s_b[kPlanFew], s_head[kPlanFew + 1];
@@ -1640,8 +1763,10 @@ __global__ void __launch_bounds__(1024, 1)
 #pragma unroll
   for (uint32_t i = 0; i < (kEnt + 1023) / 1024; ++i)
     e[i] = tid + 1024 * i < kEnt ? __ldcg(lut_g + tid + 1024 * i) : 0u;
-  const uint32_t tt = tid < nb_max / kScanTile ? __ldcg(ttot + tid) : 0u;  // stale past nb
+  uint32_t tt = tid < nb_max / kScanTile ? __ldcg(ttot + tid) : 0u;  // stale past nb
+  const uint32_t dense_lo = ctrl->dense_lo, dense_hi = ctrl->dense_hi;
   if (status & ST_FATAL) return;
+  if (h.dense && tid >= nb_max / kScanTile) tt = __ldcg(ttot + tid);
   const uint32_t nb = h.nb;
   const uint32_t ntile = (nb + kScanTile - 1) / kScanTile;
 #pragma unroll
@@ -1649,9 +1774,11 @@ __global__ void __launch_bounds__(1024, 1)
     if (tid + 1024 * i < kEnt) s_lut[tid + 1024 * i] = e[i];
   uint32_t total;
   const uint32_t tpre = block_excl_scan(tid < ntile ? tt : 0u, s_scan[0], &total);
-  if (tid <= ntile) s_tile[tid] = tpre;
-  // the totals must add up to n (else the input changed under the histogram)
-  if (total != n && tid == 0) atomicOr(&ctrl->status, ST_INTERNAL);
+  if (tid < ntile) s_tile[tid] = tpre;
+  if (tid == 0) s_tile[ntile] = total;
+  // the totals must add up to n (else the input changed under the histogram, or a
+  // dense table's count ran past 16 bits)
+  if (total != n && tid == 0) atomicOr(&ctrl->status, h.dense ? ST_TOPK_MISS : ST_INTERNAL);
   __syncthreads();
   // the request's tile: the last whose prefix is <= the rank (never an empty one)
   uint32_t t = 0;
@@ -1666,12 +1793,32 @@ __global__ void __launch_bounds__(1024, 1)
                                     s_tile[t + 1] - s_tile[t], q.rank - s_tile[t], &pre, &next);
     q.rank -= s_tile[t] + pre;  // now the rank inside the bucket
   }
-  const uint32_t count = next - pre;
+  uint32_t count = next - pre;
+  // a dense table: the lists of the keys below and above its range (at dense_at)
+  // are the segments of the ranks they hold
+  int list = 0;
+  if (mine && h.dense) {
+    if (b == 0 && q.rank < dense_lo) {
+      list = -1;
+      b = kDenseKeys;
+      count = dense_lo;
+    } else if (b + 1 == nb && q.rank >= count - dense_hi) {
+      list = 1;
+      b = kDenseKeys + 1u;
+      q.rank -= count - dense_hi;
+      count = dense_hi;
+    }
+    if (list != 0 && count > kDenseList) atomicOr(&ctrl->status, ST_TOPK_MISS);
+  }
   s_b[tid] = b;
   // the bucket's key range, whether it holds one key, and which
   K klo = 0, khi = 0;
   bool one = false;
-  if (mine) {
+  if (mine && h.dense) {
+    one = list == 0;
+    klo = list < 0 ? K(0) : list > 0 ? h.base + (K)kDenseKeys : h.base + (K)b;
+    khi = list < 0 ? h.base - K(1) : list > 0 ? KeyMax<K>::v : klo;
+  } else if (mine) {
     const uint32_t ents = sv_slices<K>() + 1 + h.low;
     klo = bucket_lo<K>(b, h.base, h.shift, s_lut, ents);
     const K knext = (b + 1 < nb) ? bucket_lo<K>(b + 1, h.base, h.shift, s_lut, ents) : K(0);
@@ -1693,14 +1840,14 @@ __global__ void __launch_bounds__(1024, 1)
   uint32_t slots, surv;
   const uint32_t slot = block_excl_scan(head ? 1u : 0u, s_scan[1], &slots);
   // (the survivors of all slots are at most n elements)
-  const uint32_t off = block_excl_scan(head && !one ? count : 0u, s_scan[2], &surv);
+  const uint32_t off = block_excl_scan(head && !one && list == 0 ? count : 0u, s_scan[2], &surv);
   if (head) s_head[slot] = tid;
   if (tid == 0) s_head[slots] = num_req;
   __syncthreads();
   if (mine) klist[tid] = q;
   if (head) {
     seg_bucket[slot] = b;
-    seg_off[slot] = off;
+    seg_off[slot] = list < 0 ? dense_at : list > 0 ? dense_at + kDenseList : (uint64_t)off;
     seg_size[slot] = one ? 0u : count;
     seg_lo[slot] = klo;
     seg_hi[slot] = khi;

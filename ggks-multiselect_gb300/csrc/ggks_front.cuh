@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kTableThreads, 1)
     k_table(const K *__restrict__ samples, uint32_t S, const K *__restrict__ spans,
             const uint32_t *__restrict__ fine_g, uint64_t n, const __grid_constant__ RankWindows win,
             LutHeader<K> *hdr, uint32_t *__restrict__ lut, uint32_t nb_max, uint32_t cand_cap,
-            uint32_t G, Ctrl *ctrl, const __grid_constant__ ReqCopy sort) {
+            uint32_t G, bool dense_ok, Ctrl *ctrl, const __grid_constant__ ReqCopy sort) {
   pdl_trigger();
   constexpr int kBits = sv_bits<K>();
   constexpr uint32_t nsl = sv_slices<K>();
@@ -296,6 +296,34 @@ __global__ void __launch_bounds__(kTableThreads, 1)
     return m << fold;
   };
   LutHeader<K> h;
+  if constexpr (sizeof(K) == 4) {
+    // a dense table: two keys or more to a bucket otherwise, and no slice of keys
+    // (with six standard deviations and ten samples to spare) that could fill a
+    // CTA's 16-bit count
+    if (dense_ok && bl == 16) {
+      const float c = (float)density(tid);
+      const bool full = (c + 6.0f * sqrtf(c) + 10.0f) * ((float)n / ((float)S * (float)G)) > kDenseFill;
+      if (!__syncthreads_or(full)) {
+        if (tid == 0) {
+          // the range's spare keys, half on each side, within the keys there are
+          const K spare = (kDenseKeys - 1u) - (kmax - kmin), left = min(kmin, spare / 2);
+          const K right = min(KeyMax<K>::v - kmax, spare - left);
+          h.base = kmin - min(kmin, spare - right);
+          h.top = kDenseKeys - 1u;
+          h.shift = 0;
+          h.low = 0;
+          h.nb = kDenseKeys;
+          h.heavy = h.dup = h.spec = h.cand_cap = 0;
+          h.spec_lo[0] = h.spec_lo[1] = 0;
+          h.spec_len[0] = h.spec_len[1] = 0;
+          h.dense = 1;
+          *hdr = h;
+          ctrl->nb = h.nb;
+        }
+        return;
+      }
+    }
+  }
   table_place<K>(h, kmin, shift, nsl);
   const uint32_t nb = build_table<K, SPT>(density, nsl, h.low, shift, bcap, nb_max, lut, tab, ts);
 

@@ -183,7 +183,7 @@ extern "C" int ggks_multiselect_noalloc_f32(const float *d_vec, uint64_t n, cons
   Req *sorted = reinterpret_cast<Req *>(A + kNaSorted);
   const ReqCopy sort{reqs, sorted, few ? num_k : 0u};
   k_table<K><<<1 + sort_ctas(sort.num), kTableThreads, 0, s>>>(samples, S, spans, fine, n, RankWindows{},
-                                                          hdr, lut, kNaNbMax, 0u, G, ctrl, sort);
+                                                          hdr, lut, kNaNbMax, 0u, G, false, ctrl, sort);
   {
     const int smem = (int)(kRepWords * sizeof(uint32_t) + (size_t)kNaNbMax * 4);
     k_hist<float, UNROLL><<<G, 1024, smem, s>>>(d_vec, n, hdr, lut, partials, kNaNbMax, ctrl,
@@ -195,7 +195,7 @@ extern "C" int ggks_multiselect_noalloc_f32(const float *d_vec, uint64_t n, cons
   if (few) {
     k_plan_few<float><<<1, 1024, 0, s>>>(hdr, lut, bpre, bco, ttot, n, sorted, num_k, kNaNbMax, ctrl,
                                          seg_bucket, seg_off, seg_size, kstart, kcnt, fill, seg_lo,
-                                         seg_hi, klist, n, nullptr, nullptr);
+                                         seg_hi, klist, n, nullptr, nullptr, 0);
   } else {
     const int smem = (int)(kLutPadded * sizeof(uint32_t) + (size_t)kNaNbMax * 5);
     k_plan<float, float><<<1, 1024, smem, s>>>(hdr, lut, bpre, ttot, n, reqs, num_k, kNaNbMax,

@@ -154,9 +154,10 @@ static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req) {
     o = align_up(o + elems * esz, A);
   };
   arr(p.sorted, kPlanFew, sizeof(Req));
-  arr(p.bpre, p.nb_max, 4);
-  arr(p.bco, p.nb_max / 8, 4);
-  arr(p.ttot, p.scan_tiles, 4);
+  // (sized for a dense table's buckets)
+  arr(p.bpre, kDenseKeys, 4);
+  arr(p.bco, kDenseKeys / 8, 4);
+  arr(p.ttot, kDenseKeys / kScanTile, 4);
   arr(p.seg_bucket, p.nb_max, 4);
   arr(p.seg_off, p.nb_max, 8);
   arr(p.seg_size, p.nb_max, 4);
@@ -836,6 +837,8 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   };
   // ---- (b) sample + splitter table; the requests
   const bool few = num_req <= kPlanFew;
+  const bool dense_ok = std::is_same<InT, uint32_t>::value && src.h_k && few && !ingest &&
+                        !src.no_dense && ctx.depth == 0 && p.nb_max == kMaxNb;
   {
     PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
     const uint32_t g = front_ctas(p.S);
@@ -848,7 +851,7 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
     const RankWindows win{ci.spec_nwin, {ci.spec_lo[0], ci.spec_lo[1]}, {ci.spec_hi[0], ci.spec_hi[1]}};
     const ReqCopy sort{raw, sorted, few ? num_req : 0u};
     L(launch(k_table<K>, 1 + sort_ctas(sort.num), kTableThreads, 0, s, samples, p.S, spans, fine, n,
-             win, hdr, lut, p.nb_max, p.cand_chunks, p.G, ctrl, sort));
+             win, hdr, lut, p.nb_max, p.cand_chunks, p.G, dense_ok, ctrl, sort));
     rq = few ? sorted : raw;
     ctx.stats.launches += 2;
     ran[GGKS_PASS_SAMPLE] = true;
@@ -899,7 +902,7 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
     if (few)
       L(launch(k_plan_few<InT>, 1, 1024, 0, s, hdr, lut, bpre, bco, ttot, n, rq, num_req, p.nb_max, ctrl,
                seg_bucket, seg_off, seg_size, kstart, kcnt, fill, seg_lo, seg_hi, klist, p.surv_cap,
-               bsingle, bkey));
+               bsingle, bkey, p.surv_half));
     else
       L(launch(k_plan<InT, OutT>, 1, 1024, smem, s, hdr, lut, bpre, ttot, n, rq, num_req, p.nb_max,
                ctrl, seg_bucket, seg_off, seg_size, kstart, kcnt, kcur, fill, seg_lo, seg_hi,
@@ -953,6 +956,13 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
     const Ctrl c = *h_ctrl;
     if (c.status & ST_FATAL) {
       return (c.status & ST_TIMEOUT) ? GGKS_TIMEOUT : GGKS_INTERNAL;
+    }
+    if (dense_ok && (c.status & ST_TOPK_MISS)) {
+      // a dense table that cannot answer: the call again, with an ordinary one
+      ctx.stats.retries++;
+      ReqSource again = src;
+      again.no_dense = true;
+      return select<InT, OutT>(ctx, d_in, n, again, num_req, d_out_user, host_results, s, nullptr);
     }
     if (c.status & ST_OVERFLOW) {
       // survivors did not fit: grow the buffer, re-run compaction + finish
