@@ -230,7 +230,8 @@ template <class K>
 __global__ void __launch_bounds__(kTableThreads, 1)
     k_table(const K *__restrict__ samples, uint32_t S, const K *__restrict__ spans,
             const uint32_t *__restrict__ fine_g, uint64_t n, const __grid_constant__ RankWindows win,
-            LutHeader<K> *hdr, uint32_t *__restrict__ lut, uint32_t nb_max, uint32_t cand_cap,
+            LutHeader<K> *hdr, uint32_t *__restrict__ lut, uint32_t nb_max, uint32_t nb_want,
+            uint32_t cand_cap,
             uint32_t G, bool dense_ok, Ctrl *ctrl, const __grid_constant__ ReqCopy sort) {
   pdl_trigger();
   constexpr int kBits = sv_bits<K>();
@@ -279,6 +280,8 @@ __global__ void __launch_bounds__(kTableThreads, 1)
   const bool far = S >= 256;
   if (dup_cap && far && (uint64_t)far_same * nb_max >= kFarTimes * far_pairs && nb_max > dup_cap)
     nb_max = dup_cap;
+  else
+    nb_max = min(nb_max, nb_want);
   const int bl = bitlen<K>(kmax - kmin);
   const uint32_t shift = bl > kBits ? (uint32_t)(bl - kBits) : 0u;
   const uint32_t fold = shift - sp.shift;  // a slice is 2^fold fine slices

@@ -183,7 +183,7 @@ extern "C" int ggks_multiselect_noalloc_f32(const float *d_vec, uint64_t n, cons
   Req *sorted = reinterpret_cast<Req *>(A + kNaSorted);
   const ReqCopy sort{reqs, sorted, few ? num_k : 0u};
   k_table<K><<<1 + sort_ctas(sort.num), kTableThreads, 0, s>>>(samples, S, spans, fine, n, RankWindows{},
-                                                          hdr, lut, kNaNbMax, 0u, G, false, ctrl, sort);
+                                                          hdr, lut, kNaNbMax, kNaNbMax, 0u, G, false, ctrl, sort);
   {
     const int smem = (int)(kRepWords * sizeof(uint32_t) + (size_t)kNaNbMax * 4);
     k_hist<float, UNROLL><<<G, 1024, smem, s>>>(d_vec, n, hdr, lut, partials, kNaNbMax, ctrl,

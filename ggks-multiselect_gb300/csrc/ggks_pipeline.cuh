@@ -58,7 +58,8 @@ struct Plan {
   uint64_t n = 0;
   uint32_t num_req = 0;
   uint32_t S = 0;
-  uint32_t nb_max = 0;
+  uint32_t nb_max = 0;   // buckets that the rows and arrays hold
+  uint32_t nb_want = 0;  // buckets of a table that tracks no keys
   uint32_t G = 0;           // hist / compact grid
   bool unroll8 = true;      // tiles of 8 (else 4) vectors per thread in hist / compact
   uint32_t scan_tiles = 0;
@@ -87,18 +88,29 @@ static_assert(sizeof(Ctrl) <= 256 && sizeof(Ctrl) % 4 == 0, "the control block's
 // 10 M floats, 257 k's: 96 -> 91 us.)
 constexpr uint32_t kPinOut = 4096;
 
+// The streaming passes' grid and buckets.  A CTA per 16384 elements up to one per
+// SM: below 10 M elements a pass is its CTAs' fixed work and one or two tiles
+// each, so more of them end sooner (65536 elements a CTA: 2^21 floats, 101 k's 63 us
+// a call, now 52; 2^21 doubles 75 -> 60; 2^22 floats 63 -> 57).  A top-k that takes
+// the pipeline keeps 65536 (cta_keys): its speculating passes keep a list per warp.
+// n / 512 buckets, 8192 to kMaxNb, in the table: a CTA writes as many counts
+// (n / 32: 55 us for 52 at 2^21 floats, 60 for 57 at 2^22, 70 for 68 at 10 M); the
+// rows have room for n / 32, as tables that track single keys and dense ones need.
 template <class InT, class OutT>
-static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req) {
+static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req, uint32_t cta_keys = 16384) {
   using K = typename Traits<InT>::K;
   Plan p;
   p.n = n;
   p.num_req = num_req;
   p.S = n <= kFrontSamples ? (uint32_t)n : kFrontSamples;
-  uint64_t want = n / 32;
-  uint32_t nb = 8192;
-  while (nb < kMaxNb && (uint64_t)nb * 2 <= want) nb *= 2;
-  p.nb_max = nb;
-  uint64_t g = (n + 65535) / 65536;
+  auto buckets = [&](uint64_t want) {
+    uint32_t nb = 8192;
+    while (nb < kMaxNb && (uint64_t)nb * 2 <= want) nb *= 2;
+    return nb;
+  };
+  p.nb_max = buckets(n / 32);
+  p.nb_want = buckets(n / 512);
+  const uint64_t g = (n + cta_keys - 1) / cta_keys;
   p.G = (uint32_t)(g < 1 ? 1 : (g > (uint64_t)ctx.sm_count ? ctx.sm_count : g));
   p.scan_tiles = (p.nb_max + kScanTile - 1) / kScanTile;
   // Tiles of 8 vectors per thread stream a little faster than tiles of 4, but
@@ -449,6 +461,9 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   return GGKS_OK;
 }
 
+// smallest vector whose clustered k's go to the window path before the one-launch one
+constexpr uint64_t kWinFirstN = 1ull << 19;
+
 // The window path's choice (ggks_window.cuh): the sample ranks around the
 // requested ascending ranks [rlo, rhi] -- six standard deviations and four ranks
 // outside them, or an open end -- and the candidates to expect.
@@ -724,10 +739,23 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
            OutT *d_out_user, const OutT **host_results, cudaStream_t s, const InT *ingest) {
   using K = typename Traits<InT>::K;
   if (ctx.depth > 12) return GGKS_INTERNAL;
+  // the requests' ranks, where the window path may take them
+  const bool window = ctx.depth == 0 && num_req >= 1 &&
+                      (src.topk ? !src.topk_pipeline : src.h_k && num_req <= kPlanFew);
+  uint64_t rlo = n - num_req, rhi = n - 1;
+  if (window && src.h_k) {
+    const auto mm = std::minmax_element(src.h_k, src.h_k + num_req);
+    rlo = n - *mm.second;
+    rhi = n - *mm.first;
+  }
+  // clustered k's of a vector above 2^19: the window path is the faster one (one k,
+  // 2^19 floats 44 us a call in one launch, 41 by a window; 2^20 53 and 42; 2^20
+  // doubles 65 and 55; 400 K doubles 52 and 54)
+  const bool window_first = window && src.h_k && n > kWinFirstN && rhi - rlo < n / 32;
   // a small device vector with host k's or a top-k: one launch, unless that
   // kernel leaves the case to the pipeline
   if constexpr (std::is_same<InT, OutT>::value) {
-    if (ctx.depth == 0 && !ingest && !src.no_small && (src.h_k || src.topk) && num_req >= 1 &&
+    if (ctx.depth == 0 && !ingest && !src.no_small && !window_first && (src.h_k || src.topk) && num_req >= 1 &&
         num_req <= kSmMaxReq && n <= (src.topk ? kSmMaxTopkN : kSmMaxN)) {
       bool missed = false;
       const int st = select_small<InT, OutT>(ctx, d_in, n, src, num_req, d_out_user,
@@ -745,15 +773,8 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
                                          ingest, &missed);
       if (st != GGKS_OK || !missed) return st;
       ingest = nullptr;  // the filter pass wrote the device copy
-    } else if (ctx.depth == 0 && num_req >= 1 &&
-               (src.topk ? !src.topk_pipeline : src.h_k && num_req <= kPlanFew)) {
+    } else if (window) {
       // clustered ranks: the window path, unless its candidates fall short
-      uint64_t rlo = n - num_req, rhi = n - 1;
-      if (src.h_k) {
-        const auto mm = std::minmax_element(src.h_k, src.h_k + num_req);
-        rlo = n - *mm.second;
-        rhi = n - *mm.first;
-      }
       bool missed = false;
       const uint64_t done = ctx.stats.launches;
       const int st = select_window<InT>(ctx, d_in, n, src, num_req, rlo, rhi, d_out_user,
@@ -762,7 +783,7 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
       if (ctx.stats.launches != done) ingest = nullptr;  // the pass wrote the device copy
     }
   }
-  const Plan p = make_plan<InT, OutT>(ctx, n, num_req);
+  const Plan p = make_plan<InT, OutT>(ctx, n, num_req, src.topk ? 65536u : 16384u);
   cudaError_t e = ensure_arena(ctx, p.total);
   if (e != cudaSuccess) return from_cuda(e);
   e = ensure_surv(ctx, (size_t)p.surv_cap * sizeof(K));
@@ -851,7 +872,7 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
     const RankWindows win{ci.spec_nwin, {ci.spec_lo[0], ci.spec_lo[1]}, {ci.spec_hi[0], ci.spec_hi[1]}};
     const ReqCopy sort{raw, sorted, few ? num_req : 0u};
     L(launch(k_table<K>, 1 + sort_ctas(sort.num), kTableThreads, 0, s, samples, p.S, spans, fine, n,
-             win, hdr, lut, p.nb_max, p.cand_chunks, p.G, dense_ok, ctrl, sort));
+             win, hdr, lut, p.nb_max, p.nb_want, p.cand_chunks, p.G, dense_ok, ctrl, sort));
     rq = few ? sorted : raw;
     ctx.stats.launches += 2;
     ran[GGKS_PASS_SAMPLE] = true;
