@@ -30,7 +30,8 @@
 //   F  the owners check that every CTA's cursor reached its end, then finish
 //      their requested buckets: a warp per bucket of at most small_warp_cap
 //      keys (finish_warp_select for up to four requests, else finish_warp);
-//      the whole CTA for larger ones: a bitonic sort of
+//      the warps also select from the middle ones (kSmSelMax), the whole CTA
+//      takes the larger ones: a bitonic sort of
 //      the segment in shared memory up to small_sort_cap keys, finish_slot
 //      beyond.
 //
@@ -117,6 +118,12 @@ template <class K>
 __host__ __device__ constexpr uint32_t small_warp_cap() {
   return kSmWarpBytes / (uint32_t)sizeof(K);
 }
+// larger segments of at most this many keys with at most kWarpSelReq requests
+// are selected by one warp (finish_warp_select): a CTA's bitonic sort of 512 to
+// 1024 doubles takes 6-8 us, and the CTAs of a distribution's thin end have
+// several (2^20 uniform doubles, 1001 ks: 124-169
+// us a call, now 87-92)
+constexpr uint32_t kSmSelMax = 4096;
 // segments of at most this many keys are sorted whole by the CTA in shared
 // memory (a bitonic network); larger ones go to finish_slot
 template <class K>
@@ -196,10 +203,10 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   __shared__ uint32_t s_pre[kSmThreads];      // global prefix of this CTA's buckets
   __shared__ uint32_t s_kcnt[kSmThreads];     // requests per bucket
   __shared__ uint32_t s_kstart[kSmThreads];   // their lists' starts in s_klist
-  __shared__ uint32_t s_kcur[kSmThreads];
+  __shared__ uint32_t s_kcur[kSmThreads];     // list fill counts; then the buckets that a warp selects
   __shared__ Req s_klist[kSmMaxReq];          // requests by bucket (ranks local to the bucket)
   __shared__ uint32_t s_slot[kSmThreads];     // requested buckets: small ones up, large down
-  __shared__ uint32_t s_nsmall, s_nlarge;
+  __shared__ uint32_t s_nsmall, s_nlarge, s_nmid;
   __shared__ bool s_miss;
 
   GGKS_SMALL_STAMP(0);
@@ -217,6 +224,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   if (tid == 0) {
     s_nsmall = 0;
     s_nlarge = 0;
+    s_nmid = 0;
     s_miss = false;
   }
   {
@@ -349,14 +357,16 @@ __global__ void __launch_bounds__(kSmThreads, 1)
 #pragma unroll
     for (uint32_t c = 0; c < kSmCtas; ++c) cl.map_shared_rank(hc, c)[b] = kInactive;
   }
+  GGKS_SMALL_STAMP(13);
+  cl.sync();  // 3: every cursor is in place
   if (kc) {
     if (tot <= small_warp_cap<K>())
       s_slot[atomicAdd(&s_nsmall, 1u)] = tid;
+    else if (tot <= kSmSelMax && kc <= kWarpSelReq && !h.dup)
+      s_kcur[atomicAdd(&s_nmid, 1u)] = tid;
     else
       s_slot[kSmThreads - 1u - atomicAdd(&s_nlarge, 1u)] = tid;
   }
-  GGKS_SMALL_STAMP(13);
-  cl.sync();  // 3: every cursor is in place
   GGKS_SMALL_STAMP(4);
 
   // ---------------- E: compaction of this CTA's share
@@ -389,7 +399,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   GGKS_SMALL_STAMP(6);
   if (!s_miss) {
     uint32_t *scratch = reinterpret_cast<uint32_t *>(smem_raw);
-    const uint32_t nsmall = s_nsmall, nlarge = s_nlarge;
+    const uint32_t nsmall = s_nsmall, nmid = s_nmid;
     // key range of bucket gb: from its first key to the next bucket's
     auto range = [&](uint32_t gb, K *klo, K *khi) {
       const uint32_t ents = sv_slices<K>() + 1 + h.low;
@@ -401,6 +411,30 @@ __global__ void __launch_bounds__(kSmThreads, 1)
     auto size_of = [&](uint32_t t) {
       return (t + 1 < kSmThreads ? s_pre[t + 1] : coff + ctot) - s_pre[t];
     };
+    K *wbuf = reinterpret_cast<K *>(scratch) + (size_t)warp * small_warp_cap<K>();
+    uint32_t *whist = scratch + (size_t)(kSmThreads / 32) * (kSmWarpBytes / 4) +
+                      (size_t)warp * (kWarpSelBins + kWarpSelReq);
+    // the middle ones first (the longer jobs); one whose needed bins do not fit a
+    // warp's buffer joins the large ones
+    for (uint32_t i = warp; i < nmid + nsmall; i += kSmThreads / 32) {
+      const bool mid = i < nmid;
+      const uint32_t t = mid ? s_kcur[i] : s_slot[i - nmid];
+      K lo, hi;
+      range(r * kSmThreads + t, &lo, &hi);
+      const uint32_t size = size_of(t), m = s_kcnt[t];
+      const Req *rq = s_klist + s_kstart[t];
+      // up to kWarpSelReq requests: radix select, else (or when the needed
+      // bins do not fit) the segment is sorted
+      if (m > kWarpSelReq || !finish_warp_select<K, OutT>(surv + s_pre[t], size, lo, hi, rq, m,
+                                                           wbuf, small_warp_cap<K>(), whist, out)) {
+        if (!mid)
+          finish_warp<K, OutT>(surv + s_pre[t], size, lo, rq, m, wbuf, out);
+        else if (lane == 0)
+          s_slot[kSmThreads - 1u - atomicAdd(&s_nlarge, 1u)] = t;
+      }
+    }
+    __syncthreads();
+    const uint32_t nlarge = s_nlarge;
     for (uint32_t i = 0; i < nlarge; ++i) {
       const uint32_t t = s_slot[kSmThreads - 1u - i];
       const uint32_t size = size_of(t);
@@ -452,22 +486,6 @@ __global__ void __launch_bounds__(kSmThreads, 1)
                                                  small_fin_cap<K>(), scratch, out);
         if (!done && tid == 0) s_miss = true;
       }
-    }
-    __syncthreads();
-    K *wbuf = reinterpret_cast<K *>(scratch) + (size_t)warp * small_warp_cap<K>();
-    uint32_t *whist = scratch + (size_t)(kSmThreads / 32) * (kSmWarpBytes / 4) +
-                      (size_t)warp * (kWarpSelBins + kWarpSelReq);
-    for (uint32_t i = warp; i < nsmall; i += kSmThreads / 32) {
-      const uint32_t t = s_slot[i];
-      K lo, hi;
-      range(r * kSmThreads + t, &lo, &hi);
-      const uint32_t size = size_of(t), m = s_kcnt[t];
-      const Req *rq = s_klist + s_kstart[t];
-      // up to kWarpSelReq requests: radix select, else (or when the needed
-      // bins do not fit) the segment is sorted
-      if (m > kWarpSelReq || !finish_warp_select<K, OutT>(surv + s_pre[t], size, lo, hi, rq, m,
-                                                           wbuf, small_warp_cap<K>(), whist, out))
-        finish_warp<K, OutT>(surv + s_pre[t], size, lo, rq, m, wbuf, out);
     }
   }
   __syncthreads();
