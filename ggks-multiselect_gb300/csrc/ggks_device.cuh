@@ -22,7 +22,8 @@
 //                 without its 4n-byte element-to-bucket array.
 //   (d) totals    k_colsum: sums the per-CTA rows per bucket.  Replaces
 //                 sumCounts (:214-221).
-//   (e) plan      k_plan: one CTA takes the exclusive bucket prefix in shared
+//   (e) plan      k_plan_few (up to kPlanFew requests, in rank order) or k_plan:
+//                 one CTA takes the exclusive bucket prefix in shared
 //                 memory, maps every requested rank to its bucket and local
 //                 rank, answers ranks that fall in single-key buckets
 //                 directly, assigns compact slots to the active buckets and

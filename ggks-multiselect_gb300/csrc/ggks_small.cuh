@@ -1,7 +1,7 @@
 // ggks_small.cuh -- the selection of a small vector in one launch.
 //
-// Below a few million elements the pipeline's seven dependent kernels cost
-// about 70-95 us whatever the size (each pass's fixed latency, not its
+// Below a few million elements the pipeline's eight dependent kernels cost
+// about 50-60 us whatever the size (each pass's fixed latency, not its
 // traffic).  Here one thread-block cluster of kSmCtas CTAs runs the same
 // algorithm -- sample, range-adaptive splitter table, bucket histogram,
 // k -> bucket plan, compaction of the requested buckets, in-shared-memory
@@ -89,8 +89,8 @@ __host__ __device__ constexpr uint32_t small_samples() {
 }
 constexpr uint32_t kSmMaxReq = kSmThreads;        // one request per thread
 // largest vectors taken by this path: multiselects up to 2^20 elements
-// (measured on GB300: 2^20 / 101 k's 80 us against 92 us for the pipeline,
-// even at 2^21); top-k up to 2^18 (the threshold path is faster above)
+// (101 k's: 2^18 floats 42 us against 52 us for the pipeline, 2^19 46 and 53, even
+// at 2^20); top-k up to 2^18 (the threshold path is faster above)
 constexpr uint64_t kSmMaxN = 1ull << 20;
 constexpr uint64_t kSmMaxTopkN = 1ull << 18;
 

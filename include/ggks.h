@@ -65,8 +65,9 @@ typedef struct ggks_opts {
 #define GGKS_FLAG_TOPK_PIPELINE 4u
 /* opts->flags for ggks_multiselect_* / ggks_topk_*: run the pipeline even
  * where the one-launch small-vector path applies (a device vector of at most
- * 2^20 elements -- 2^18 for a top-k -- and at most 1024 k's); the results are
- * the same. */
+ * 2^20 elements -- 2^18 for a top-k -- and at most 1024 k's, unless the k's
+ * span less than n / 32 ranks of more than 2^19 elements); the results are the
+ * same. */
 #define GGKS_FLAG_NO_SMALL 8u
 
 /* ------------------------------------------------------------------------ */
