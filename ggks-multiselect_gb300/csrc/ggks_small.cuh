@@ -9,8 +9,9 @@
 // memory for the exchanges, so nothing of the plan goes through global memory
 // or the host:
 //
-//   A  every CTA samples the same keys (pairs of neighbouring elements at
-//      hashed positions) and builds the same table with build_lut_cta, the
+//   A  the CTAs gather a sixteenth of the sample each (pairs of neighbouring
+//      elements at hashed positions), read each other's parts and build the same
+//      table with build_lut_cta, the
 //      single-vector builder (sv_slices slices, kSmNb buckets): no CTA waits for
 //      another's table.
 //   B  every CTA holds the table's copies and counts its contiguous
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   __shared__ uint32_t s_kcnt[kSmThreads];     // requests per bucket
   __shared__ uint32_t s_kstart[kSmThreads];   // their lists' starts in s_klist
   __shared__ uint32_t s_kcur[kSmThreads];     // list fill counts; then the buckets that a warp selects
-  __shared__ Req s_klist[kSmMaxReq];          // requests by bucket (ranks local to the bucket)
+  __shared__ __align__(16) Req s_klist[kSmMaxReq];          // requests by bucket (ranks local to the bucket)
   __shared__ uint32_t s_slot[kSmThreads];     // requested buckets: small ones up, large down
   __shared__ uint32_t s_nsmall, s_nlarge, s_nmid;
   __shared__ bool s_miss;
@@ -216,9 +217,9 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   q.rank = 0;
   q.out = 0;
   if (tid < num_req) q = reqs[tid];
-  // ---------------- A: sample and table, in every CTA (the same samples and
-  // the same deterministic build give every CTA the same table, so no CTA
-  // waits for another's)
+  // ---------------- A: the sample, gathered by all CTAs together, and the table,
+  // built in every CTA (the same samples and the same deterministic build give
+  // every CTA the same table, so no CTA waits for another's)
   constexpr uint32_t kS = small_samples<K>();
   const uint32_t S = n < kS ? (uint32_t)n : kS;
   if (tid == 0) {
@@ -241,26 +242,40 @@ __global__ void __launch_bounds__(kSmThreads, 1)
       // pairs of neighbouring elements at hashed positions (samples 2q and
       // 2q + 1 are neighbours for the table builder's estimate of lanes
       // sharing a bucket); S / 2 independent positions keep the edge buckets
-      // (keys beyond the sampled extremes) near n / (S / 2) keys.  Every
-      // load of a thread is issued before its keys are used.
-      constexpr uint32_t PER = kS / 2 / kSmThreads;  // pairs per thread
-      K k[2 * PER];
+      // (keys beyond the sampled extremes) near n / (S / 2) keys.  Each CTA
+      // gathers a sixteenth of them and reads the others' from their shared
+      // memory (4096 scattered sectors per CTA took 6.0 us, this 4.0: 2^18 floats, 101
+      // k's 43 -> 41 us a call, 2^20 54 -> 51)
+      constexpr uint32_t kPart = kS / kSmCtas;  // keys gathered by a CTA
+      static_assert(kPart / 2 <= kSmThreads && kPart * sizeof(K) <= sizeof(s_klist), "one pair a thread");
+      K *part = reinterpret_cast<K *>(s_klist);  // (the requests come after barrier 1)
+      if (tid < kPart / 2) {
+        const uint32_t q = r * (kPart / 2) + tid;
+        const uint64_t pos = ((uint64_t)hash32(q * 0x9E3779B9u + 0x5EEDu) * (n - 1)) >> 32;
+        const K k0 = Traits<T>::key(x[pos]), k1 = Traits<T>::key(x[pos + 1]);
+        part[2 * tid] = k0;
+        part[2 * tid + 1] = k1;
+      }
+      cl.sync();  // 0: every part is gathered
+      // 16-byte reads, each CTA beginning at its own part (all 16 reading one
+      // owner at a time queue up there)
+      constexpr uint32_t kVec = 16 / sizeof(K), kVecs = kS / kVec, PER = kVecs / kSmThreads;
+      static_assert(kVecs % kSmThreads == 0, "whole vectors per thread");
+      uint4 v[PER];
 #pragma unroll
       for (uint32_t u = 0; u < PER; ++u) {
-        const uint32_t q = tid + u * kSmThreads;
-        const uint64_t pos = ((uint64_t)hash32(q * 0x9E3779B9u + 0x5EEDu) * (n - 1)) >> 32;
-        k[2 * u] = Traits<T>::key(x[pos]);
-        k[2 * u + 1] = Traits<T>::key(x[pos + 1]);
+        const uint32_t i = (tid + u * kSmThreads + r * (kPart / kVec)) % kVecs;
+        v[u] = reinterpret_cast<const uint4 *>(cl.map_shared_rank(part, i / (kPart / kVec)))[i % (kPart / kVec)];
       }
 #pragma unroll
       for (uint32_t u = 0; u < PER; ++u) {
-        const uint32_t q = tid + u * kSmThreads;
+        const uint32_t i = (tid + u * kSmThreads + r * (kPart / kVec)) % kVecs;
+        reinterpret_cast<uint4 *>(samples)[i] = v[u];
+        const K *k = reinterpret_cast<const K *>(&v[u]);
 #pragma unroll
-        for (uint32_t e = 0; e < 2; ++e) {
-          const K kk = k[2 * u + e];
-          samples[2 * q + e] = kk;
-          lo = kk < lo ? kk : lo;
-          hi = kk > hi ? kk : hi;
+        for (uint32_t e = 0; e < kVec; ++e) {
+          lo = k[e] < lo ? k[e] : lo;
+          hi = k[e] > hi ? k[e] : hi;
         }
       }
     }
