@@ -184,6 +184,10 @@ int select_batch(Context &ctx, const BatchInput &in, T *d_out_user, T *h_out, cu
       const double pl = b.spec_lo / n, ph = (b.spec_hi + 1.0) / n;
       cand_per = ((b.spec_hi - b.spec_lo + 1.0) + (margin(pl) + margin(ph)) * n / S) / n * 1.5;
     }
+    // eight samples a bucket are enough where no window rests on them (8192 for
+    // every problem: the table phase of 4096 vectors 222 us, so 181; 2048 vectors of
+    // 2^17 floats 970 -> 933 us a call)
+    if (!b.spec) b.S = std::min(b.S, std::max(1024u, 8u * nbm));
     b.lut_off = lut_words;
     lut_words += ((1u << nsl_bits) + 2 + 3) & ~3u;
     b.cnt_off = cnt_words;
