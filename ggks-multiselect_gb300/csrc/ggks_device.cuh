@@ -366,18 +366,6 @@ __device__ __forceinline__ void vec_keys(const ulonglong2 &v, uint64_t (&k)[2]) 
 // ---------------------------------------------------------------------------
 // small PTX helpers
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t *p) {
-  uint64_t v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_u64(uint64_t *p, uint64_t v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_volatile_u32(const uint32_t *p) {
-  return *(const volatile uint32_t *)p;
-}
-
 // streaming 128-bit load that does not allocate in L1
 template <class V>
 __device__ __forceinline__ V ldg_stream(const V *p);
@@ -682,7 +670,7 @@ template <class K, int SPT, class D>
 __device__ __forceinline__ uint32_t build_table(D &&density, uint32_t nsl, uint32_t low,
                                                 uint32_t shift, int bcap, uint32_t nb_max,
                                                 uint32_t *lut, uint32_t *tab, TableShared &ts) {
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
   // this thread's slices [SPT tid, SPT tid + SPT)
   uint32_t c[SPT];
   bool prev_nonempty[SPT];
@@ -933,17 +921,6 @@ __device__ __forceinline__ void track_key(uint32_t *hist, K *rep, uint32_t i, K 
     } else if (!(hist[i] & kMixed)) {
       atomicOr(&hist[i], kMixed);
     }
-  }
-}
-
-template <bool HEAVY>
-__device__ __forceinline__ void hist_add(uint32_t *hist, uint32_t b) {
-  if (HEAVY) {
-    const uint32_t peers = __match_any_sync(0xffffffffu, b);
-    const int leader = __ffs(peers) - 1;
-    if ((int)(threadIdx.x & 31) == leader) atomicAdd(&hist[b], (uint32_t)__popc(peers));
-  } else {
-    atomicAdd(&hist[b], 1u);
   }
 }
 
