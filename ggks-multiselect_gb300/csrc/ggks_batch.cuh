@@ -42,7 +42,7 @@
 //              by one warp), then a warp queue over the small slots (at most
 //              warp_cap keys, the common case); after one more grid barrier,
 //              a CTA queue over the mid-size slots whose needed bins did not
-//              fit a warp's buffer.  A batch with fewer than kWselPerCta
+//              fit a warp's buffer.  A batch with fewer than wsel_per_cta
 //              mid-size slots per CTA puts them in the first CTA queue
 //              instead, and skips that barrier.
 //
@@ -363,8 +363,13 @@ constexpr uint32_t kWarpSelBins = 256;  // the select's histogram (one word per 
 constexpr uint32_t kWarpSelMax = 16384;
 // A warp takes about ten times a CTA's time on such a segment, so warps take
 // them only when a batch has at least this many per CTA of the grid (a CTA
-// queue of fewer ends sooner); otherwise they join the CTA queue.
-constexpr uint32_t kWselPerCta = 16;
+// queue of fewer ends sooner); otherwise they join the CTA queue.  Finish phase by
+// CTAs / by warps: 4 vectors of 2^22 floats 9 a CTA 50 / 50 us, 11 58 / 51, 15 73 /
+// 55; of 2^20 doubles 7 a CTA 47 / 33, 11 63 / 36, 15 80 / 39.
+template <class K>
+__host__ __device__ constexpr uint32_t wsel_per_cta() {
+  return sizeof(K) == 4 ? 10u : 6u;
+}
 
 // One warp answers m <= kWarpSelReq requests of a segment of size > 0 keys, all
 // in [lo, hi], by radix select instead of sorting the segment: a histogram of
@@ -1266,7 +1271,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
   // whatever the status: one choice for the grid, and so for the barrier
   // that only the warps' fallback needs.
   const uint32_t n_wsel_all = __ldcg(&ctrl->n_wsel);
-  const bool wsel_warps = n_wsel_all >= kWselPerCta * gridDim.x;
+  const bool wsel_warps = n_wsel_all >= wsel_per_cta<K>() * gridDim.x;
   if (!(st & (ST_FATAL | ST_OVERFLOW))) {
     const uint32_t n_big = __ldcg(&ctrl->n_big), n_small = __ldcg(&ctrl->n_small);
     const uint32_t n_wsel = wsel_warps ? n_wsel_all : 0u;
