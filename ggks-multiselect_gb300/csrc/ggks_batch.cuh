@@ -364,11 +364,13 @@ constexpr uint32_t kWarpSelMax = 16384;
 // A warp takes about ten times a CTA's time on such a segment, so warps take
 // them only when a batch has at least this many per CTA of the grid (a CTA
 // queue of fewer ends sooner); otherwise they join the CTA queue.  Finish phase by
-// CTAs / by warps: 4 vectors of 2^22 floats 9 a CTA 50 / 50 us, 11 58 / 51, 15 73 /
-// 55; of 2^20 doubles 7 a CTA 47 / 33, 11 63 / 36, 15 80 / 39.
+// CTAs / by warps, floats: 4 vectors of 2^22, 9 a CTA 50 / 50 us, 15 73 / 55; 64 of
+// 2^18, 8 a CTA 27 / 31, 12 37 / 35, 16 45 / 37; 256 of 2^16, 12 a CTA 36 / 37, 16
+// 45 / 38.  Doubles differ more: 16 of 2^20, 7 a CTA 47 / 33; 64 of 2^18, 10 a CTA
+// 65 / 67; 256 of 2^16 (needed bins often too large for a warp) 16 a CTA 92 / 120.
 template <class K>
 __host__ __device__ constexpr uint32_t wsel_per_cta() {
-  return sizeof(K) == 4 ? 10u : 6u;
+  return sizeof(K) == 4 ? 12u : 16u;
 }
 
 // One warp answers m <= kWarpSelReq requests of a segment of size > 0 keys, all

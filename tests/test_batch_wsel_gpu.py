@@ -1,5 +1,5 @@
 """Mid-size slots finished by CTAs or by warps, around the count per CTA of the grid
-from which the warps take them (10 for 4-byte keys, 6 for 8-byte ones), with
+from which the warps take them (12 for 4-byte keys, 16 for 8-byte ones), with
 spread keys and with clusters whose bins do not fit a warp's buffer.  Every answer
 equals sorting."""
 import numpy as np
@@ -20,8 +20,8 @@ def g():
     return ggks
 
 
-@pytest.mark.parametrize("dtype,per", [(np.float32, 9), (np.float32, 10), (np.float32, 11), (np.uint32, 10),
-                                       (np.float64, 5), (np.float64, 6), (np.float64, 7)])
+@pytest.mark.parametrize("dtype,per", [(np.float32, 11), (np.float32, 12), (np.float32, 13), (np.uint32, 12),
+                                       (np.float64, 15), (np.float64, 16), (np.float64, 17)])
 @pytest.mark.parametrize("cluster", [False, True])
 def test_around_the_step(g, dtype, per, cluster):
     import torch
