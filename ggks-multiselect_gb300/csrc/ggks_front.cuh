@@ -555,7 +555,8 @@ __global__ void __launch_bounds__(1024)
 // sample), more by a radix select.  A slice of more than kSliceBuf samples gives
 // its smallest sample (list 0) or its largest (list 1): a wider window.  A list
 // of up to 1024 samples comes in one round of loads (with its unused end),
-// through L1; ends with a barrier.
+// through L1.  Ends with a barrier after the last read of sh, so a second call may
+// follow on the same sh.
 template <class K>
 struct RankShared {
   K keys[kSliceBuf];
@@ -590,7 +591,9 @@ __device__ __forceinline__ K rank_key(const SliceOut<K> *out, int w, RankShared<
     }
   }
   __syncthreads();
-  return sh.found;
+  const K found = sh.found;
+  __syncthreads();
+  return found;
 }
 
 }  // namespace ggks

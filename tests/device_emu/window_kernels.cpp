@@ -1,0 +1,117 @@
+// window_kernels.cpp -- the sampled-window kernels on the host CPU (see
+// cuda_on_host.h), as plain C functions for tests/test_window_host.py.
+#include "cuda_on_host.h"
+
+#include "ggks_window.cuh"
+
+using namespace ggks;
+
+namespace {
+
+template <class T>
+struct Front {
+  using K = typename Traits<T>::K;
+  std::vector<K> samples, spans;
+  std::vector<uint32_t> fine;
+  SliceOut<K> slice;
+  Ctrl ctrl;
+};
+
+// k_sample, k_bin, k_slice, k_wfilter over x[0 .. n), n <= kFrontSamples: every
+// element is a sample, so the window's ends are the keys of ranks r0 and r1.
+template <class T>
+int filter(const T *x, uint64_t n, uint32_t r0, uint32_t r1, bool lo_open, bool hi_open,
+           uint32_t grid, typename Traits<T>::K *arr, uint64_t cap, uint32_t *bins, uint64_t *out) {
+  using K = typename Traits<T>::K;
+  static Front<T> f;
+  const uint32_t S = (uint32_t)n, g = front_ctas(S);
+  f.samples.assign(S, 0);
+  f.spans.assign(2 * g, 0);
+  f.fine.assign(kLutIdx, ~0u);
+  std::memset(&f.slice, 0, sizeof(f.slice));
+  WinCtl<K> wc;
+  std::memset(&wc, 0, sizeof(wc));
+  SliceWant want;
+  want.rank[0] = r0;
+  want.rank[1] = r1;
+  const K *samples = f.samples.data(), *spans = f.spans.data();
+  bool ok = emu::launch(g, 1024, 0, [&] {
+    k_sample<T>(x, n, S, 1u, f.samples.data(), f.spans.data(), f.fine.data(), kLutIdx, &f.ctrl,
+                Ctrl{}, ReqCopy{});
+  });
+  ok = ok && emu::launch(g, 1024, 0, [&] { k_bin<K>(samples, S, spans, f.fine.data(), &f.ctrl); });
+  ok = ok && emu::launch(g, 1024, 0, [&] {
+         k_slice<K, 2>(samples, S, spans, f.fine.data(), want, &f.slice);
+       });
+  ok = ok && emu::launch(grid, 1024, wfilter_smem_bytes<K>(), [&] {
+         k_wfilter<T>(x, n, &f.slice, spans, g, lo_open, hi_open, &wc, arr, cap, bins, nullptr);
+       });
+  out[0] = wc.len;
+  out[1] = wc.below;
+  out[2] = wc.lo;
+  out[3] = wc.shift;
+  out[4] = wc.nbins;
+  return ok ? 0 : 1;
+}
+
+// k_wplace over the candidates arr[0 .. len) and the given bin counts.
+template <class K>
+int place(const K *arr, uint32_t len, uint64_t n, uint32_t below, K lo, uint32_t shift,
+          uint32_t nbins, const uint32_t *bins, uint32_t kk, const uint32_t *ranks,
+          uint32_t num_req, uint32_t grid, K *placed, uint64_t placed_cap, uint32_t *status) {
+  WinCtl<K> wc;
+  std::memset(&wc, 0, sizeof(wc));
+  wc.len = len;
+  wc.below = below;
+  wc.lo = lo;
+  wc.shift = shift;
+  wc.nbins = nbins;
+  std::vector<uint32_t> cur(kWinBins, 0), pre(kWinBins, 0);
+  std::vector<unsigned long long> big_lo(kWinBins, 0), big_hi(kWinBins, 0);
+  const uint32_t slots = num_req ? num_req : 1;
+  std::vector<uint64_t> seg_off(slots);
+  std::vector<uint32_t> seg_size(slots), kstart(slots), kcnt(slots);
+  std::vector<K> seg_lo(slots), seg_hi(slots);
+  std::vector<Req> klist(slots), reqs(slots);
+  for (uint32_t i = 0; i < num_req; ++i) {
+    reqs[i].rank = ranks[i];
+    reqs[i].out = i;
+  }
+  WinSlots<K> sl{seg_off.data(), seg_size.data(), kstart.data(), kcnt.data(),
+                 seg_lo.data(),  seg_hi.data(),   klist.data()};
+  Ctrl ctrl{};
+  const bool ok = emu::launch(grid, 1024, 0, [&] {
+    k_wplace<K>(arr, len, n, kk, false, kk != 0, reqs.data(), num_req, &wc, bins, cur.data(),
+                pre.data(), placed, placed_cap, big_lo.data(), big_hi.data(), sl, &ctrl);
+  });
+  *status = ctrl.status;
+  return ok ? 0 : 1;
+}
+
+}  // namespace
+
+extern "C" {
+
+int emu_filter_f32(const float *x, uint64_t n, uint32_t r0, uint32_t r1, int lo_open, int hi_open,
+                   uint32_t grid, uint32_t *arr, uint64_t cap, uint32_t *bins, uint64_t *out) {
+  return filter<float>(x, n, r0, r1, lo_open, hi_open, grid, arr, cap, bins, out);
+}
+int emu_filter_u32(const uint32_t *x, uint64_t n, uint32_t r0, uint32_t r1, int lo_open,
+                   int hi_open, uint32_t grid, uint32_t *arr, uint64_t cap, uint32_t *bins,
+                   uint64_t *out) {
+  return filter<uint32_t>(x, n, r0, r1, lo_open, hi_open, grid, arr, cap, bins, out);
+}
+int emu_filter_f64(const double *x, uint64_t n, uint32_t r0, uint32_t r1, int lo_open,
+                   int hi_open, uint32_t grid, uint64_t *arr, uint64_t cap, uint32_t *bins,
+                   uint64_t *out) {
+  return filter<double>(x, n, r0, r1, lo_open, hi_open, grid, arr, cap, bins, out);
+}
+int emu_place_u32(const uint32_t *arr, uint32_t len, uint64_t n, uint32_t below, uint32_t lo,
+                  uint32_t shift, uint32_t nbins, const uint32_t *bins, uint32_t kk,
+                  const uint32_t *ranks, uint32_t num_req, uint32_t grid, uint32_t *placed,
+                  uint64_t placed_cap, uint32_t *status) {
+  return place<uint32_t>(arr, len, n, below, lo, shift, nbins, bins, kk, ranks, num_req, grid,
+                         placed, placed_cap, status);
+}
+
+}  // extern "C"

@@ -1,0 +1,87 @@
+"""The sampled-window kernels (csrc/ggks_window.cuh) run on the host CPU, one block
+at a time, with thread 0 as far ahead of the other threads as the barriers allow
+(device_emu/cuda_on_host.h): what they write must not depend on how far that is.
+Every element is sampled here, so the window's ends are known exactly."""
+import ctypes
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.join(os.path.dirname(os.path.abspath(__file__)), "device_emu"))
+import build_emu  # noqa: E402
+
+BINS = 8192
+MISS = 32  # ST_TOPK_MISS
+U32 = ctypes.POINTER(ctypes.c_uint32)
+
+
+@pytest.fixture(scope="module")
+def emu(tmp_path_factory):
+    lib = build_emu.build("window_kernels.cpp",
+                          ["ggks_device.cuh", "ggks_front.cuh", "ggks_tiny.cuh", "ggks_window.cuh"],
+                          tmp_path_factory.mktemp("emu"))
+    if lib is None:
+        pytest.skip("no host compiler or CUDA headers")
+    return lib
+
+
+def keys(x):
+    if x.dtype == np.uint32:
+        return x.copy()
+    u = np.dtype(f"u{x.itemsize}").type
+    b, top = x.view(u), u(1 << (8 * x.itemsize - 1))
+    return np.where(b & top, ~b, b | top)
+
+
+def make(dtype, dist, n):
+    r = np.random.default_rng(n)
+    if dist == "few":
+        x = r.integers(0, 5, n) * 100.0
+    elif dist == "spread":
+        x = r.random(n) * 1e9
+    else:
+        x = r.standard_cauchy(n) * 1e4
+    return (np.abs(x) if dtype == np.uint32 else x).clip(-4e9, 4e9).astype(dtype)
+
+
+def run_filter(emu, x, r0, r1, lo_open, hi_open, grid=3):
+    k = keys(x)
+    arr = np.zeros(x.size, k.dtype)
+    bins = np.zeros(BINS, np.uint32)
+    out = np.zeros(5, np.uint64)
+    fn = {np.dtype(np.float32): emu.emu_filter_f32, np.dtype(np.float64): emu.emu_filter_f64,
+          np.dtype(np.uint32): emu.emu_filter_u32}[x.dtype]
+    rc = fn(x.ctypes.data_as(ctypes.c_void_p), ctypes.c_uint64(x.size), r0, r1, int(lo_open),
+            int(hi_open), grid, arr.ctypes.data_as(ctypes.c_void_p), ctypes.c_uint64(x.size),
+            bins.ctypes.data_as(U32), out.ctypes.data_as(ctypes.c_void_p))
+    assert rc == 0
+    return k, arr, bins, [int(v) for v in out]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.uint32])
+@pytest.mark.parametrize("dist", ["spread", "heavy", "few"])
+@pytest.mark.parametrize("ends", ["closed", "low", "high"])
+def test_filter(emu, dtype, dist, ends):
+    n = 5003
+    x = make(dtype, dist, n)
+    r0, r1 = {"closed": (2300, 2700), "low": (0, 300), "high": (n - 400, n - 1)}[ends]
+    lo_open, hi_open = ends == "low", ends == "high"
+    k, arr, bins, (length, below, lo, shift, nbins) = run_filter(emu, x, r0, r1, lo_open, hi_open)
+    s = np.sort(k)
+    keep = np.ones(n, bool)
+    if not lo_open:
+        keep &= k >= s[r0]
+    if not hi_open:
+        keep &= k <= s[r1]
+    want = np.sort(k[keep])
+    assert length == want.size
+    if ends == "closed":
+        assert below == np.count_nonzero(k < s[r0])
+    if ends == "closed" and s[r0] == s[r1]:
+        assert bins[0] == length and not bins[1:].any()  # one key: counted, not kept
+        return
+    assert np.array_equal(np.sort(arr[:length]), want)
+    at = np.array([0 if v < lo else min((v - lo) >> shift, nbins - 1) for v in want.tolist()])
+    assert np.array_equal(bins, np.bincount(at, minlength=BINS))
