@@ -450,7 +450,9 @@ __global__ void __launch_bounds__(kWinSortThreads)
   pdl_start();
   __shared__ uint32_t s_last;
   const uint32_t tid = threadIdx.x, lane = tid & 31;
-  const uint32_t status = ctrl->status;
+  // one value for the whole warp: other CTAs set ST_TOPK_MISS meanwhile, and the
+  // lanes meet in shuffles below
+  const uint32_t status = __shfl_sync(0xffffffffu, ctrl->status, 0);
   if (!(status & (ST_FATAL | ST_TOPK_MISS))) {
     const uint32_t C = wc->len, nbins = wc->nbins, first = wc->first;
     const uint32_t warps = gridDim.x * (kWinSortThreads / 32);

@@ -54,11 +54,13 @@ int filter(const T *x, uint64_t n, uint32_t r0, uint32_t r1, bool lo_open, bool 
   return ok ? 0 : 1;
 }
 
-// k_wplace over the candidates arr[0 .. len) and the given bin counts.
+// k_wplace over the candidates arr[0 .. len) and the given bin counts, and for a
+// top-k (kk > 0, out given) k_wsort.
 template <class K>
 int place(const K *arr, uint32_t len, uint64_t n, uint32_t below, K lo, uint32_t shift,
           uint32_t nbins, const uint32_t *bins, uint32_t kk, const uint32_t *ranks,
-          uint32_t num_req, uint32_t grid, K *placed, uint64_t placed_cap, uint32_t *status) {
+          uint32_t num_req, uint32_t grid, K *placed, uint64_t placed_cap, K *out,
+          uint32_t *status) {
   WinCtl<K> wc;
   std::memset(&wc, 0, sizeof(wc));
   wc.len = len;
@@ -80,11 +82,16 @@ int place(const K *arr, uint32_t len, uint64_t n, uint32_t below, K lo, uint32_t
   WinSlots<K> sl{seg_off.data(), seg_size.data(), kstart.data(), kcnt.data(),
                  seg_lo.data(),  seg_hi.data(),   klist.data()};
   Ctrl ctrl{};
-  const bool ok = emu::launch(grid, 1024, 0, [&] {
+  bool ok = emu::launch(grid, 1024, 0, [&] {
     k_wplace<K>(arr, len, n, kk, false, kk != 0, reqs.data(), num_req, &wc, bins, cur.data(),
                 pre.data(), placed, placed_cap, big_lo.data(), big_hi.data(), sl, &ctrl);
   });
   *status = ctrl.status;
+  if (out)
+    ok = ok && emu::launch(grid, kWinSortThreads, 0, [&] {
+           k_wsort<K, K>(placed, &wc, bins, pre.data(), big_lo.data(), big_hi.data(), kk, out, &ctrl,
+                         status);
+         });
   return ok ? 0 : 1;
 }
 
@@ -109,9 +116,9 @@ int emu_filter_f64(const double *x, uint64_t n, uint32_t r0, uint32_t r1, int lo
 int emu_place_u32(const uint32_t *arr, uint32_t len, uint64_t n, uint32_t below, uint32_t lo,
                   uint32_t shift, uint32_t nbins, const uint32_t *bins, uint32_t kk,
                   const uint32_t *ranks, uint32_t num_req, uint32_t grid, uint32_t *placed,
-                  uint64_t placed_cap, uint32_t *status) {
+                  uint64_t placed_cap, uint32_t *out, uint32_t *status) {
   return place<uint32_t>(arr, len, n, below, lo, shift, nbins, bins, kk, ranks, num_req, grid,
-                         placed, placed_cap, status);
+                         placed, placed_cap, out, status);
 }
 
 }  // extern "C"

@@ -14,6 +14,7 @@ import build_emu  # noqa: E402
 
 BINS = 8192
 MISS = 32  # ST_TOPK_MISS
+EMPTY = 0xABCDEF01
 U32 = ctypes.POINTER(ctypes.c_uint32)
 
 
@@ -85,3 +86,39 @@ def test_filter(emu, dtype, dist, ends):
     assert np.array_equal(np.sort(arr[:length]), want)
     at = np.array([0 if v < lo else min((v - lo) >> shift, nbins - 1) for v in want.tolist()])
     assert np.array_equal(bins, np.bincount(at, minlength=BINS))
+
+
+def place(emu, arr, n, below, lo, shift, nbins, bins, kk, ranks, grid, sort=False):
+    guard = 64
+    placed = np.full(arr.size + guard, EMPTY, np.uint32)
+    out = np.zeros(max(kk, 1), np.uint32)
+    status = ctypes.c_uint32()
+    rc = emu.emu_place_u32(
+        arr.ctypes.data_as(U32), arr.size, ctypes.c_uint64(n), below, lo, shift, nbins,
+        bins.ctypes.data_as(U32), kk, ranks.ctypes.data_as(U32), ranks.size, grid,
+        placed.ctypes.data_as(U32), ctypes.c_uint64(arr.size),
+        out.ctypes.data_as(U32) if sort else None, ctypes.byref(status))
+    assert rc == 0, "threads wait for others that never come"
+    assert np.all(placed[arr.size:] == EMPTY)
+    return placed[:arr.size], out, status.value
+
+
+@pytest.mark.parametrize("big", ["none", "copies", "distinct"])
+def test_topk_bins(emu, big):
+    """Bins that a warp sorts, large bins of one key and large bins of many keys, which
+    the first CTA reports while the others may still read the status."""
+    r = np.random.default_rng(1)
+    n, lo, shift, nbins, kk = 100_000, 5000, 6, 300, 3000
+    arr = (lo + r.integers(0, nbins << shift, 4000)).astype(np.uint32)
+    if big != "none":
+        at = nbins - 40 - np.arange(16) * 2
+        extra = lo + (np.repeat(at, 400) << shift)
+        extra += r.integers(0, 1 << shift, extra.size) if big == "distinct" else 3
+        arr = np.concatenate([arr[~np.isin((arr - lo) >> shift, at)], extra]).astype(np.uint32)
+    bins = np.bincount((arr - lo) >> shift, minlength=BINS).astype(np.uint32)
+    _, out, status = place(emu, arr, n, 0, lo, shift, nbins, bins, kk, np.zeros(0, np.uint32), 3,
+                           sort=True)
+    if big == "distinct":
+        assert status & MISS
+    else:
+        assert status == 0 and np.array_equal(out, np.sort(arr)[::-1][:kk])
