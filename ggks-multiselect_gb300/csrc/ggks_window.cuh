@@ -399,7 +399,9 @@ __global__ void __launch_bounds__(1024, 1)
       for (uint32_t b = tid; b < kWinBins; b += blockDim.x) pre_g[b] = pre[b];
   }
   if (miss || single) return;
-  // whole warps over the candidates, four loads in flight per lane
+  // whole warps over the candidates, four loads in flight per lane; a bin that meets
+  // more keys than it counted keeps its places and the call is a miss
+  bool over = false;
   constexpr uint32_t U = 4;
   const uint32_t step = gridDim.x * 1024 * U;
   for (uint32_t i0 = blockIdx.x * 1024 * U + (tid >> 5) * 32 * U; i0 < C; i0 += step) {
@@ -425,7 +427,11 @@ __global__ void __launch_bounds__(1024, 1)
       if (place && (int)lane == leader) base = atomicAdd(&cur[b], (uint32_t)__popc(peers));
       base = __shfl_sync(0xffffffffu, base, leader);
       if (place) {
-        placed[pre[b] + base + __popc(peers & ((1u << lane) - 1u))] = k[u];
+        const uint32_t at = base + __popc(peers & ((1u << lane) - 1u));
+        if (at < count_of(b))
+          placed[pre[b] + at] = k[u];
+        else
+          over = true;
       } else if (want) {
         // a large bin: does it hold one key?  (the complement of the smallest)
         if ((unsigned long long)~(uint64_t)k[u] > __ldcg(big_lo_inv + b))
@@ -435,6 +441,7 @@ __global__ void __launch_bounds__(1024, 1)
       }
     }
   }
+  if (over) atomicOr(&ctrl->status, ST_TOPK_MISS);
 }
 
 // A top-k's values from the placed bins: a warp per bin from wc->first up, the

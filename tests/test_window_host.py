@@ -122,3 +122,34 @@ def test_topk_bins(emu, big):
         assert status & MISS
     else:
         assert status == 0 and np.array_equal(out, np.sort(arr)[::-1][:kk])
+
+
+@pytest.mark.parametrize("kk", [0, 700])
+@pytest.mark.parametrize("grid", [1, 2])
+def test_place(emu, kk, grid):
+    """Candidates go to the places of their bins; a bin that meets more keys than it
+    counted stores none outside its places, and the call is a miss."""
+    r = np.random.default_rng(grid)
+    n, length, lo, shift, nbins = 100_000, 4500, 1000, 4, 500
+    arr = (lo + r.integers(0, nbins << shift, length)).astype(np.uint32)
+    at = (arr - lo) >> shift
+    true = np.bincount(at, minlength=BINS).astype(np.uint32)
+    first = int(np.searchsorted(np.cumsum(true), length - kk, side="right")) if kk else 0
+    below = n - length if kk else 40_000
+    short = true.copy()  # a needed bin counts two keys too few, a later one two too many
+    short[first] -= 2
+    short[first + 9] += 2
+    ranks = np.zeros(0, np.uint32) if kk else np.array([0, 1000, length - 1], np.uint32) + 40_000
+    for bins in (true, short):
+        placed, _, status = place(emu, arr, n, below, lo, shift, nbins, bins, kk, ranks, grid)
+        assert (status == 0) if bins is true else (status & MISS)
+        pre = np.concatenate([[0], np.cumsum(bins)]).astype(int)
+        need = range(first, nbins) if kk else np.searchsorted(pre, ranks.astype(int) - below, "right") - 1
+        for b in range(nbins):
+            part = placed[pre[b]:pre[b + 1]]
+            if b not in need:
+                assert np.all(part == EMPTY)
+            elif bins is true:
+                assert np.array_equal(np.sort(part), np.sort(arr[at == b]))
+            else:
+                assert np.all((part[part != EMPTY] - lo) >> shift == b)
