@@ -135,6 +135,10 @@ constexpr uint32_t kCandChunksPerWarp = 64;   // chunks one warp's list can hold
 // successor be scheduled at once: it orders nothing, the successor's own wait
 // does.  No kernel of the pipeline waits on other CTAs, so successors that sit
 // resident while waiting cannot hold up the running grid.
+// A kernel is resident while its predecessors still write what it reads, so its
+// parameters for reading carry no __restrict__: a const pointer with it promises
+// data that no one writes while the kernel is there, and the compiler may then
+// move its loads ahead of the wait.
 __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -366,7 +370,10 @@ __device__ __forceinline__ void vec_keys(const ulonglong2 &v, uint64_t (&k)[2]) 
 // ---------------------------------------------------------------------------
 // small PTX helpers
 // ---------------------------------------------------------------------------
-// streaming 128-bit load that does not allocate in L1
+// streaming 128-bit load that does not allocate in L1.  The device copy of a host
+// vector, written by the kernel before, is also read this way: only after the wait
+// (both are volatile, so in this order), when no L1 holds any line of it.  (Without
+// .nc the streaming passes are slower: 2^28 floats, 1001 k's 479 -> 524 us a call.)
 template <class V>
 __device__ __forceinline__ V ldg_stream(const V *p);
 template <>
@@ -1178,8 +1185,8 @@ __device__ __forceinline__ void dense_body(const uint32_t *__restrict__ x, uint6
 // more than one key.
 template <class T, int UNROLL>
 __global__ void __launch_bounds__(1024, 1)
-    k_hist(const T *__restrict__ x, uint64_t n, const LutHeader<typename Traits<T>::K> *hdr,
-           const uint32_t *__restrict__ lut_g, uint32_t *__restrict__ partials, uint32_t nb_max,
+    k_hist(const T *x, uint64_t n, const LutHeader<typename Traits<T>::K> *hdr,
+           const uint32_t *lut_g, uint32_t *__restrict__ partials, uint32_t nb_max,
            Ctrl *ctrl, T *__restrict__ copy_to, typename Traits<T>::K *__restrict__ cand,
            uint32_t *__restrict__ cand_cnt, uint32_t *__restrict__ cand_tab,
            uint32_t *cand_next, typename Traits<T>::K *__restrict__ reps) {
@@ -1284,9 +1291,9 @@ constexpr int kScanTile = 64;  // buckets per CTA
 // row.
 template <class K>
 __global__ void __launch_bounds__(kScanThreads, 4)
-    k_colsum(const uint32_t *__restrict__ partials, uint32_t rows, uint32_t nb_max,
+    k_colsum(const uint32_t *partials, uint32_t rows, uint32_t nb_max,
              const LutHeader<K> *hdr, uint32_t *__restrict__ bpre, uint32_t *__restrict__ bco,
-             uint32_t *__restrict__ ttot, const Ctrl *ctrl, const K *__restrict__ reps, uint32_t *__restrict__ bsingle,
+             uint32_t *__restrict__ ttot, const Ctrl *ctrl, const K *reps, uint32_t *__restrict__ bsingle,
              K *__restrict__ bkey) {
   pdl_start();
   constexpr uint32_t kVecs = kScanTile / 4;              // 16-byte vectors per tile row
@@ -1586,8 +1593,8 @@ static __device__ uint64_t load_prefix(const uint32_t *__restrict__ bpre_g,
 // Bitmap and counts must start at zero.  Shared memory: the bucket prefix
 // (nb_max u32), from the tile prefixes and totals.
 static __global__ void __launch_bounds__(1024)
-    k_reqmap(const uint32_t *__restrict__ bpre_g, const uint32_t *__restrict__ ttot_g,
-             const Ctrl *ctrl, const Req *__restrict__ reqs, uint32_t num_req,
+    k_reqmap(const uint32_t *bpre_g, const uint32_t *ttot_g,
+             const Ctrl *ctrl, const Req *reqs, uint32_t num_req,
              uint32_t *__restrict__ req_bucket, uint32_t *__restrict__ req_local, uint32_t *bits,
              uint32_t *bcount) {
   pdl_start();
@@ -1633,9 +1640,9 @@ static __global__ void __launch_bounds__(1024)
 // klist positions: kstart[slot] + arrival order in the slot (warp-aggregated
 // cursors; kcur starts at zero, set by k_plan).
 static __global__ void __launch_bounds__(1024)
-    k_reqplace(const Ctrl *ctrl, const Req *__restrict__ reqs, uint32_t num_req,
-               const uint32_t *__restrict__ req_bucket, const uint32_t *__restrict__ req_local,
-               const uint32_t *__restrict__ bslot, const uint32_t *__restrict__ kstart,
+    k_reqplace(const Ctrl *ctrl, const Req *reqs, uint32_t num_req,
+               const uint32_t *req_bucket, const uint32_t *req_local,
+               const uint32_t *bslot, const uint32_t *kstart,
                uint32_t *kcur, Req *__restrict__ klist) {
   pdl_start();
   if (ctrl->status & ST_FATAL) return;
@@ -1710,17 +1717,17 @@ __device__ __forceinline__ uint32_t tile_bucket(const uint32_t *__restrict__ p,
 // seg_lo without survivors.  Bound: latency, four rounds of loads.
 template <class InT>
 __global__ void __launch_bounds__(1024, 1)
-    k_plan_few(const LutHeader<typename Traits<InT>::K> *hdr, const uint32_t *__restrict__ lut_g,
-               const uint32_t *__restrict__ bpre, const uint32_t *__restrict__ bco,
-               const uint32_t *__restrict__ ttot, uint64_t n,
-               const Req *__restrict__ reqs, uint32_t num_req, uint32_t nb_max, Ctrl *ctrl,
+    k_plan_few(const LutHeader<typename Traits<InT>::K> *hdr, const uint32_t *lut_g,
+               const uint32_t *bpre, const uint32_t *bco,
+               const uint32_t *ttot, uint64_t n,
+               const Req *reqs, uint32_t num_req, uint32_t nb_max, Ctrl *ctrl,
                uint32_t *__restrict__ seg_bucket, uint64_t *__restrict__ seg_off,
                uint32_t *__restrict__ seg_size, uint32_t *__restrict__ kstart,
                uint32_t *__restrict__ kcnt, uint32_t *__restrict__ fill,
                typename Traits<InT>::K *__restrict__ seg_lo,
                typename Traits<InT>::K *__restrict__ seg_hi, Req *__restrict__ klist,
-               uint64_t surv_cap, const uint32_t *__restrict__ bsingle,
-               const typename Traits<InT>::K *__restrict__ bkey, uint64_t dense_at) {
+               uint64_t surv_cap, const uint32_t *bsingle,
+               const typename Traits<InT>::K *bkey, uint64_t dense_at) {
   using K = typename Traits<InT>::K;
   constexpr uint32_t kEnt = sv_entries<K>();
   constexpr uint32_t kTiles = kDenseKeys / kScanTile;
@@ -1899,9 +1906,9 @@ __device__ __forceinline__ void plan_map_requests(const uint32_t *excl, uint32_t
 // bucket's count.
 template <class InT, class OutT>
 __global__ void __launch_bounds__(1024, 1)
-    k_plan(const LutHeader<typename Traits<InT>::K> *hdr, const uint32_t *__restrict__ lut_g,
-           const uint32_t *__restrict__ bpre, const uint32_t *__restrict__ ttot, uint64_t n,
-           const Req *__restrict__ reqs, uint32_t num_req, uint32_t nb_max, Ctrl *ctrl,
+    k_plan(const LutHeader<typename Traits<InT>::K> *hdr, const uint32_t *lut_g,
+           const uint32_t *bpre, const uint32_t *ttot, uint64_t n,
+           const Req *reqs, uint32_t num_req, uint32_t nb_max, Ctrl *ctrl,
            uint32_t *__restrict__ seg_bucket,
            uint64_t *__restrict__ seg_off, uint32_t *__restrict__ seg_size,
            uint32_t *__restrict__ kstart, uint32_t *__restrict__ kcnt,
@@ -1909,8 +1916,8 @@ __global__ void __launch_bounds__(1024, 1)
            typename Traits<InT>::K *__restrict__ seg_lo,
            typename Traits<InT>::K *__restrict__ seg_hi, uint32_t *__restrict__ req_bucket,
            uint32_t *__restrict__ req_local, Req *__restrict__ klist, uint64_t surv_cap,
-           Premap pm, const uint32_t *__restrict__ bsingle = nullptr,
-           const typename Traits<InT>::K *__restrict__ bkey = nullptr) {
+           Premap pm, const uint32_t *bsingle = nullptr,
+           const typename Traits<InT>::K *bkey = nullptr) {
   pdl_start();
   using K = typename Traits<InT>::K;
   extern __shared__ uint4 smem_raw[];
@@ -2291,13 +2298,13 @@ __host__ __device__ constexpr size_t compact_smem_bytes(uint32_t nb_max) {
 // surv_half, so candidate mode also needs the survivors to end below it.
 template <class T, int UNROLL>
 __global__ void __launch_bounds__(1024, 1)
-    k_compact(const T *__restrict__ x, uint64_t n, const LutHeader<typename Traits<T>::K> *hdr,
-              const uint32_t *__restrict__ lut_g, const uint32_t *__restrict__ seg_bucket,
-              const uint64_t *__restrict__ seg_off, const uint32_t *__restrict__ seg_size,
+    k_compact(const T *x, uint64_t n, const LutHeader<typename Traits<T>::K> *hdr,
+              const uint32_t *lut_g, const uint32_t *seg_bucket,
+              const uint64_t *seg_off, const uint32_t *seg_size,
               uint32_t *__restrict__ rows, uint32_t *__restrict__ fill, uint32_t nb_max,
               typename Traits<T>::K *__restrict__ surv, uint64_t surv_cap, Ctrl *ctrl,
-              const typename Traits<T>::K *__restrict__ cand,
-              const uint32_t *__restrict__ cand_cnt, const uint32_t *__restrict__ cand_tab,
+              const typename Traits<T>::K *cand,
+              const uint32_t *cand_cnt, const uint32_t *cand_tab,
               uint64_t surv_half) {
   // the cursors are cleared ahead of the dependency wait (as in k_hist); after
   // it the control block, the table and each thread's first slot come in one
@@ -2946,10 +2953,10 @@ __device__ bool finish_slot(const K *__restrict__ src, uint32_t size, K lo, K hi
 
 template <class K, class OutT>
 __global__ void __launch_bounds__(kFinThreads)
-    k_finish(const K *__restrict__ surv, Ctrl *ctrl, const uint64_t *__restrict__ seg_off,
-             const uint32_t *__restrict__ seg_size, const K *__restrict__ seg_lo,
-             const K *__restrict__ seg_hi, const uint32_t *__restrict__ kstart,
-             const uint32_t *__restrict__ kcnt, const Req *__restrict__ klist,
+    k_finish(const K *surv, Ctrl *ctrl, const uint64_t *seg_off,
+             const uint32_t *seg_size, const K *seg_lo,
+             const K *seg_hi, const uint32_t *kstart,
+             const uint32_t *kcnt, const Req *klist,
              uint32_t *__restrict__ deferred, uint32_t bcap, OutT *__restrict__ out,
              Ctrl *__restrict__ host_ctrl) {
   pdl_start();

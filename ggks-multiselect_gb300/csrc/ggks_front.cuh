@@ -54,7 +54,7 @@ struct ReqCopy {
 // copy or clearing precedes the call's first kernel.
 template <class T>
 __global__ void __launch_bounds__(1024)
-    k_sample(const T *__restrict__ x, uint64_t n, uint32_t S, uint32_t seed,
+    k_sample(const T *x, uint64_t n, uint32_t S, uint32_t seed,
              typename Traits<T>::K *__restrict__ samples, typename Traits<T>::K *__restrict__ spans,
              uint32_t *__restrict__ zero, uint32_t zero_words, Ctrl *ctrl,
              const __grid_constant__ Ctrl init, const __grid_constant__ ReqCopy req) {
@@ -145,7 +145,7 @@ __device__ __forceinline__ SampleSpan<K> sample_span(const K *__restrict__ spans
 // hold many copies of a key?
 template <class K>
 __global__ void __launch_bounds__(1024)
-    k_bin(const K *__restrict__ samples, uint32_t S, const K *__restrict__ spans, uint32_t *fine,
+    k_bin(const K *samples, uint32_t S, const K *spans, uint32_t *fine,
           Ctrl *ctrl) {
   pdl_trigger();
   __shared__ uint32_t cnt[kLutIdx];
@@ -228,8 +228,8 @@ static __device__ __forceinline__ void sort_requests(const ReqCopy &rc, uint32_t
 
 template <class K>
 __global__ void __launch_bounds__(kTableThreads, 1)
-    k_table(const K *__restrict__ samples, uint32_t S, const K *__restrict__ spans,
-            const uint32_t *__restrict__ fine_g, uint64_t n, const __grid_constant__ RankWindows win,
+    k_table(const K *samples, uint32_t S, const K *spans,
+            const uint32_t *fine_g, uint64_t n, const __grid_constant__ RankWindows win,
             LutHeader<K> *hdr, uint32_t *__restrict__ lut, uint32_t nb_max, uint32_t nb_want,
             uint32_t cand_cap,
             uint32_t G, bool dense_ok, Ctrl *ctrl, const __grid_constant__ ReqCopy sort) {
@@ -495,8 +495,8 @@ constexpr uint32_t kSliceZeroWords = 12;  // words that are zero on entry
 
 template <class K, int W>
 __global__ void __launch_bounds__(1024)
-    k_slice(const K *__restrict__ samples, uint32_t S, const K *__restrict__ spans,
-            const uint32_t *__restrict__ fine_g, const __grid_constant__ SliceWant want,
+    k_slice(const K *samples, uint32_t S, const K *spans,
+            const uint32_t *fine_g, const __grid_constant__ SliceWant want,
             SliceOut<K> *out) {
   pdl_start();
   __shared__ uint32_t s_scan[32];

@@ -157,7 +157,7 @@ __device__ __forceinline__ void filter_body(const T *__restrict__ x, uint64_t n,
 // *len (zero on entry) their count.
 template <class T, int UNROLL>
 __global__ void __launch_bounds__(1024, 1)
-    k_filter(const T *__restrict__ x, uint64_t n, const SliceOut<typename Traits<T>::K> *slice,
+    k_filter(const T *x, uint64_t n, const SliceOut<typename Traits<T>::K> *slice,
              bool open, typename Traits<T>::K *tau, typename Traits<T>::K *__restrict__ arr,
              uint64_t cap, uint32_t *len, T *__restrict__ copy_to, const Ctrl *ctrl) {
   pdl_start();
@@ -222,7 +222,7 @@ __host__ __device__ constexpr size_t pick_smem_bytes() {
 
 template <class K, class OutT>
 __global__ void __launch_bounds__(1024, 1)
-    k_pick(const K *__restrict__ arr, uint64_t cap, const uint32_t *len, const K *tau, uint32_t kk,
+    k_pick(const K *arr, uint64_t cap, const uint32_t *len, const K *tau, uint32_t kk,
            OutT *__restrict__ out, const Ctrl *ctrl, uint32_t *host_status) {
   pdl_start();
   constexpr uint32_t kStage = PickShape<K>::kStage;

@@ -216,8 +216,8 @@ __device__ __forceinline__ uint32_t wfilter_body(const T *__restrict__ x, uint64
 // bins: kWinBins words, zero on entry.
 template <class T>
 __global__ void __launch_bounds__(1024, 1)
-    k_wfilter(const T *__restrict__ x, uint64_t n, const SliceOut<typename Traits<T>::K> *slice,
-              const typename Traits<T>::K *__restrict__ spans, uint32_t parts, bool lo_open,
+    k_wfilter(const T *x, uint64_t n, const SliceOut<typename Traits<T>::K> *slice,
+              const typename Traits<T>::K *spans, uint32_t parts, bool lo_open,
               bool hi_open, WinCtl<typename Traits<T>::K> *wc,
               typename Traits<T>::K *__restrict__ arr, uint64_t cap, uint32_t *__restrict__ bins_g,
               T *__restrict__ copy_to) {
@@ -306,9 +306,9 @@ struct WinSlots {
 // bins' prefix, written by CTA 0 for a top-k.
 template <class K>
 __global__ void __launch_bounds__(1024, 1)
-    k_wplace(const K *__restrict__ arr, uint64_t cap, uint64_t n, uint32_t kk, bool lo_open,
-             bool hi_open, const Req *__restrict__ reqs, uint32_t num_req, WinCtl<K> *wc,
-             const uint32_t *__restrict__ bins_g, uint32_t *cur, uint32_t *__restrict__ pre_g,
+    k_wplace(const K *arr, uint64_t cap, uint64_t n, uint32_t kk, bool lo_open,
+             bool hi_open, const Req *reqs, uint32_t num_req, WinCtl<K> *wc,
+             const uint32_t *bins_g, uint32_t *cur, uint32_t *__restrict__ pre_g,
              K *__restrict__ placed, uint64_t placed_cap, unsigned long long *big_lo_inv,
              unsigned long long *big_hi, WinSlots<K> sl, Ctrl *ctrl) {
   pdl_start();
@@ -450,9 +450,9 @@ __global__ void __launch_bounds__(1024, 1)
 constexpr uint32_t kWinSortThreads = 256;
 template <class K, class OutT>
 __global__ void __launch_bounds__(kWinSortThreads)
-    k_wsort(const K *__restrict__ placed, const WinCtl<K> *wc, const uint32_t *__restrict__ bins_g,
-            const uint32_t *__restrict__ pre_g, const unsigned long long *__restrict__ big_lo_inv,
-            const unsigned long long *__restrict__ big_hi, uint32_t kk, OutT *__restrict__ out,
+    k_wsort(const K *placed, const WinCtl<K> *wc, const uint32_t *bins_g,
+            const uint32_t *pre_g, const unsigned long long *big_lo_inv,
+            const unsigned long long *big_hi, uint32_t kk, OutT *__restrict__ out,
             Ctrl *ctrl, uint32_t *host_status) {
   pdl_start();
   __shared__ uint32_t s_last;
