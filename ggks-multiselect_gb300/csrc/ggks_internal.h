@@ -120,6 +120,7 @@ struct ReqSource {
   bool topk = false;              // ranks n-1 .. n-K into outputs 0 .. K-1
   bool topk_pipeline = false;     // a top-k that does not take the threshold path
   bool no_small = false;          // never the one-launch small-vector path
+  bool no_window = false;         // never the sampled window
   bool no_dense = false;          // never a dense table
 };
 

@@ -740,7 +740,7 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   using K = typename Traits<InT>::K;
   if (ctx.depth > 12) return GGKS_INTERNAL;
   // the requests' ranks, where the window path may take them
-  const bool window = ctx.depth == 0 && num_req >= 1 &&
+  const bool window = ctx.depth == 0 && num_req >= 1 && !src.no_window &&
                       (src.topk ? !src.topk_pipeline : src.h_k && num_req <= kPlanFew);
   uint64_t rlo = n - num_req, rhi = n - 1;
   if (window && src.h_k) {
@@ -752,35 +752,42 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
   // 2^19 floats 44 us a call in one launch, 41 by a window; 2^20 53 and 42; 2^20
   // doubles 65 and 55; 400 K doubles 52 and 54)
   const bool window_first = window && src.h_k && n > kWinFirstN && rhi - rlo < n / 32;
-  // a small device vector with host k's or a top-k: one launch, unless that
-  // kernel leaves the case to the pipeline
   if constexpr (std::is_same<InT, OutT>::value) {
-    if (ctx.depth == 0 && !ingest && !src.no_small && !window_first && (src.h_k || src.topk) && num_req >= 1 &&
-        num_req <= kSmMaxReq && n <= (src.topk ? kSmMaxTopkN : kSmMaxN)) {
-      bool missed = false;
-      const int st = select_small<InT, OutT>(ctx, d_in, n, src, num_req, d_out_user,
-                                             host_results, s, &missed);
+    bool missed = false;
+    auto try_small = [&]() -> int {
+      return select_small<InT, OutT>(ctx, d_in, n, src, num_req, d_out_user, host_results, s, &missed);
+    };
+    // a small device vector with host k's or a top-k: one launch, unless that
+    // kernel leaves the case to the pipeline
+    const bool small = ctx.depth == 0 && !ingest && !src.no_small && (src.h_k || src.topk) &&
+                       num_req >= 1 && num_req <= kSmMaxReq &&
+                       n <= (src.topk ? kSmMaxTopkN : kSmMaxN);
+    if (small && !window_first) {
+      const int st = try_small();
       if (st != GGKS_OK || !missed) return st;
     }
-  }
-  // a top-k of at most kPickMax values from a vector larger than the sample:
-  // the threshold path, unless its candidates fall short
-  if constexpr (std::is_same<InT, OutT>::value) {
     if (src.topk && ctx.depth == 0 && num_req <= kPickMax && n > 65536 &&
         (uint64_t)num_req * 64 <= n && !src.topk_pipeline) {
-      bool missed = false;
+      // a top-k of at most kPickMax values from a vector larger than the sample:
+      // the threshold path, unless its candidates fall short
       const int st = topk_threshold<InT>(ctx, d_in, n, num_req, d_out_user, host_results, s,
                                          ingest, &missed);
       if (st != GGKS_OK || !missed) return st;
       ingest = nullptr;  // the filter pass wrote the device copy
     } else if (window) {
       // clustered ranks: the window path, unless its candidates fall short
-      bool missed = false;
       const uint64_t done = ctx.stats.launches;
       const int st = select_window<InT>(ctx, d_in, n, src, num_req, rlo, rhi, d_out_user,
                                         host_results, s, ingest, &missed);
       if (st != GGKS_OK || !missed) return st;
-      if (ctx.stats.launches != done) ingest = nullptr;  // the pass wrote the device copy
+      if (ctx.stats.launches != done) {
+        ctx.stats.topk_misses++;
+        ingest = nullptr;  // the pass wrote the device copy
+      }
+      if (small && window_first) {
+        const int st2 = try_small();
+        if (st2 != GGKS_OK || !missed) return st2;
+      }
     }
   }
   const Plan p = make_plan<InT, OutT>(ctx, n, num_req, src.topk ? 65536u : 16384u);
@@ -979,10 +986,10 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
       return (c.status & ST_TIMEOUT) ? GGKS_TIMEOUT : GGKS_INTERNAL;
     }
     if (dense_ok && (c.status & ST_TOPK_MISS)) {
-      // a dense table that cannot answer: the call again, with an ordinary one
+      // a dense table that cannot answer: the pipeline again, with an ordinary one
       ctx.stats.retries++;
       ReqSource again = src;
-      again.no_dense = true;
+      again.no_dense = again.no_window = again.no_small = true;
       return select<InT, OutT>(ctx, d_in, n, again, num_req, d_out_user, host_results, s, nullptr);
     }
     if (c.status & ST_OVERFLOW) {

@@ -345,7 +345,7 @@ typedef struct ggks_stats {
   uint64_t spec_ctas;                 /* compaction CTAs that read those candidates
                                          in place of their share of the vector */
   uint64_t topk_threshold_calls;      /* top-k calls answered by the threshold path */
-  uint64_t topk_misses;               /* threshold attempts that fell back to the pipeline */
+  uint64_t topk_misses;               /* threshold and window attempts left to another path */
   uint64_t batch_spec_tiles;          /* batched compaction tiles that read their candidates
                                          in place of their elements */
   uint64_t small_calls;               /* calls answered by the one-launch small-vector path */
