@@ -21,6 +21,8 @@
 // k_sample (15.2 before).
 #pragma once
 
+#include <cstddef>
+
 #include "ggks_device.cuh"
 
 namespace ggks {
@@ -473,25 +475,37 @@ __global__ void __launch_bounds__(kTableThreads, 1)
 // ---------------------------------------------------------------------------
 // The fine slices holding W sample ranks, and their samples.  k_slice: grid of
 // front_ctas(S); every CTA finds the slices for itself from the counts and
-// appends its samples in them to the slices' lists.  rank_key, in the prologue
+// appends its samples in them to the slices' lists.  rank_keys, in the prologue
 // of the kernel that follows, then takes the key of the wanted rank.
 struct SliceWant {
   uint32_t rank[2];  // 0-based among the S samples
 };
-// samples of one list that are ranked (values of 8 bits put 2048 samples into a
-// fine slice; an unranked slice widens the window by its other values)
+// samples of one list (values of 8 bits put 2048 samples into a fine slice).  A
+// slice with more has no list but the counts of its samples in kLutIdx parts:
+// doubles spread their span over every exponent, so that a slice is half a binade
+// and holds up to a quarter of uniform values.
 constexpr uint32_t kSliceBuf = 4096;
 template <class K>
 struct SliceOut {
-  uint32_t at[2];                // list lengths so far (zero on entry)
+  uint32_t at[2];                // list lengths so far (zero on entry, as all down to sub)
   uint32_t pad[2];
   unsigned long long lo_inv[2];  // slices of more than kSliceBuf samples: the
-  unsigned long long hi[2];      // complement of the smallest and the largest (zero on entry)
+  unsigned long long hi[2];      // complement of the smallest and the largest
+  uint32_t sub[2][kLutIdx];      // and their samples per part
   uint32_t cnt[2];               // samples in the slice
   uint32_t rank[2];              // the wanted rank inside the slice
+  uint32_t shift, pad2;          // slices are 2^shift keys wide
+  K base[2];                     // the slice's first key
   K buf[2][kSliceBuf];
 };
-constexpr uint32_t kSliceZeroWords = 12;  // words that are zero on entry
+constexpr uint32_t kSliceZeroWords = 12 + 2 * kLutIdx;  // words that are zero on entry
+static_assert(offsetof(SliceOut<uint64_t>, sub) % 16 == 0 &&
+                  offsetof(SliceOut<uint64_t>, cnt) == kSliceZeroWords * 4,
+              "the counts are read in 16-byte vectors");
+// a slice of 2^shift keys has parts of 2^part_shift(shift) keys
+__device__ __forceinline__ uint32_t part_shift(uint32_t shift) {
+  return shift > (uint32_t)kLutIdxBits ? shift - kLutIdxBits : 0u;
+}
 
 template <class K, int W>
 __global__ void __launch_bounds__(1024)
@@ -542,58 +556,163 @@ __global__ void __launch_bounds__(1024)
         atomicMax(&out->lo_inv[w], (unsigned long long)~(uint64_t)lo);
         atomicMax(&out->hi[w], (unsigned long long)hi);
       }
+      const K o = k - sp.kmin - ((K)s_slice[w] << sp.shift);
+      const uint32_t part = in ? (uint32_t)(o >> part_shift(sp.shift)) : 0xFFFFFFFFu;
+      const uint32_t peers = __match_any_sync(0xffffffffu, part);
+      if (in && (tid & 31) == (uint32_t)__ffs(peers) - 1)
+        atomicAdd(&out->sub[w][part], (uint32_t)__popc(peers));
     }
     if (i == 0) {
       out->rank[w] = s_rank[w];
       out->cnt[w] = s_cnt[w];
+      out->base[w] = sp.kmin + ((K)s_slice[w] << sp.shift);
+      out->shift = sp.shift;
     }
   }
 }
 
-// The key of the wanted rank of list w, by the whole CTA (1024 threads): up to
-// 256 samples are ranked by counting the samples before each (four threads per
-// sample), more by a radix select.  A slice of more than kSliceBuf samples gives
-// its smallest sample (list 0) or its largest (list 1): a wider window.  A list
-// of up to 1024 samples comes in one round of loads (with its unused end),
-// through L1.  Ends with a barrier after the last read of sh, so a second call may
-// follow on the same sh.
+// The keys of the wanted ranks of lists 0 .. W - 1, by the whole CTA (1024 threads;
+// skip: a list that is not wanted).  Up to 256 samples are ranked by counting the
+// samples before each (four threads per sample), more by a radix select.  A list of
+// up to 1024 samples comes in one round of loads (with its unused end), through L1.
+// A slice without a list is narrowed to the part that holds the rank, whose samples
+// are gathered from all S, one reading for both lists; a part of more than
+// kSliceBuf samples is narrowed again by counting.  (Taking the slice's first or
+// last sample instead made the window up to a quarter of the vector, too many
+// candidates: the 30 % quantile of 2^26 normal doubles 360 us a call, against 247 in the
+// pipeline, now 149.)  keys: W * kSliceBuf keys of shared memory, 16-byte
+// aligned, the caller's again afterwards.  One call per sh.
 template <class K>
 struct RankShared {
-  K keys[kSliceBuf];
-  K found;
-  uint32_t cnt[256], sel[2];
+  K found[2];
+  uint32_t cnt[256], sel[2][3], scan[2][32], at[2];
 };
-template <class K>
-__device__ __forceinline__ K rank_key(const SliceOut<K> *out, int w, RankShared<K> &sh) {
-  const uint32_t tid = threadIdx.x;
-  const uint32_t cnt = out->cnt[w], r = out->rank[w];
-  sh.keys[tid] = out->buf[w][tid];
-  if (tid == 0) sh.found = (K)(w == 0 ? ~out->lo_inv[w] : out->hi[w]);
-  if (cnt <= kSliceBuf)
-    for (uint32_t i = 1024 + tid; i < cnt; i += 1024) sh.keys[i] = out->buf[w][i];
+template <int W, class K>
+__device__ __forceinline__ void rank_keys(const SliceOut<K> *out, const K *samples, uint32_t S,
+                                          const bool (&skip)[W], K *keys, RankShared<K> &sh,
+                                          K (&found)[W]) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  uint32_t cnt[W], r[W], shift[W];
+  K base[W], first[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    cnt[w] = out->cnt[w];
+    r[w] = out->rank[w];
+    shift[w] = out->shift;
+    first[w] = out->buf[w][tid];
+    base[w] = out->base[w];
+  }
+  // every sample: fn(key, whether there is one)
+  auto each = [&](auto &&fn) {
+    constexpr uint32_t U = 8;
+    for (uint32_t i0 = 0; i0 < S; i0 += U * 1024) {
+      K k[U];
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        const uint32_t i = i0 + 1024 * u + tid;
+        k[u] = i < S ? __ldcg(samples + i) : K(0);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) fn(k[u], i0 + 1024 * u + tid < S);
+    }
+  };
+  bool rank_it[W], gather = false;  // lists to rank; lists to gather first
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    rank_it[w] = !skip[w];
+    if (skip[w]) continue;
+    K *kw = keys + (size_t)w * kSliceBuf;
+    if (cnt[w] <= kSliceBuf) {
+      kw[tid] = first[w];
+      for (uint32_t i = 1024 + tid; i < cnt[w]; i += 1024) kw[i] = out->buf[w][i];
+      shift[w] = 0xFFFFFFFFu;  // nothing to gather
+      continue;
+    }
+    if ((K)~out->lo_inv[w] == (K)out->hi[w]) {  // copies of one key
+      if (tid == 0) sh.found[w] = (K)out->hi[w];
+      rank_it[w] = false;
+      continue;
+    }
+    uint32_t *hist = reinterpret_cast<uint32_t *>(kw);
+    uint4 c4 = __ldcg(reinterpret_cast<const uint4 *>(out->sub[w]) + tid);
+    for (;;) {
+      const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w}, sub = part_shift(shift[w]);
+      uint32_t all;
+      uint32_t pre = block_excl_scan(c4.x + c4.y + c4.z + c4.w, sh.scan[w], &all);
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        if (c[q] && pre <= r[w] && r[w] < pre + c[q]) {
+          sh.sel[w][0] = 4 * tid + q;
+          sh.sel[w][1] = r[w] - pre;
+          sh.sel[w][2] = c[q];
+        }
+        pre += c[q];
+      }
+      __syncthreads();
+      base[w] += (K)sh.sel[w][0] << sub;
+      r[w] = sh.sel[w][1];
+      cnt[w] = sh.sel[w][2];
+      shift[w] = sub;
+      if (cnt[w] <= kSliceBuf || sub == 0) break;
+      fill_words(hist, kLutIdx, 0u);
+      __syncthreads();  // (also: sel is read)
+      const uint32_t next = part_shift(sub);
+      each([&](K k, bool valid) {
+        const K o = k - base[w];
+        if (valid && k >= base[w] && (o >> sub) == 0) atomicAdd(&hist[(uint32_t)(o >> next)], 1u);
+      });
+      __syncthreads();
+      c4 = reinterpret_cast<const uint4 *>(hist)[tid];
+    }
+    if (cnt[w] > kSliceBuf) {  // a part of one key
+      if (tid == 0) sh.found[w] = base[w];
+      rank_it[w] = false;
+    } else {
+      gather = true;
+    }
+  }
+  if (gather) {
+    if (tid < W) sh.at[tid] = 0;
+    __syncthreads();
+    each([&](K k, bool valid) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        const bool in = rank_it[w] && shift[w] != 0xFFFFFFFFu && valid && k >= base[w] &&
+                        ((k - base[w]) >> shift[w]) == 0;
+        const uint32_t m = __ballot_sync(0xffffffffu, in);
+        if (!m) continue;
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&sh.at[w], (uint32_t)__popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (in && at < kSliceBuf) keys[(size_t)w * kSliceBuf + at] = k;
+      }
+    });
+  }
   __syncthreads();
-  if (cnt <= kSliceBuf && r < cnt) {
-    if (cnt <= 256) {
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    if (!rank_it[w]) continue;
+    const K *kw = keys + (size_t)w * kSliceBuf;
+    if (cnt[w] <= 256) {
       const uint32_t me = tid >> 2;
-      const K mine = sh.keys[me];
+      const K mine = kw[me];
       uint32_t less = 0;
-      if (me < cnt)
-        for (uint32_t i = tid & 3; i < cnt; i += 4) {
-          const K o = sh.keys[i];
+      if (me < cnt[w])
+        for (uint32_t i = tid & 3; i < cnt[w]; i += 4) {
+          const K o = kw[i];
           less += o < mine || (o == mine && i < me) ? 1u : 0u;
         }
       less += __shfl_xor_sync(0xffffffffu, less, 1);
       less += __shfl_xor_sync(0xffffffffu, less, 2);
-      if (me < cnt && less == r && (tid & 3) == 0) sh.found = mine;
+      if (me < cnt[w] && less == r[w] && (tid & 3) == 0) sh.found[w] = mine;
     } else {
-      const K k = cta_select_rank<K>(sh.keys, cnt, r, sh.cnt, sh.sel);
-      if (tid == 0) sh.found = k;
+      const K k = cta_select_rank<K>(kw, cnt[w], r[w], sh.cnt, sh.sel[w]);
+      if (tid == 0) sh.found[w] = k;
     }
   }
   __syncthreads();
-  const K found = sh.found;
-  __syncthreads();
-  return found;
+#pragma unroll
+  for (int w = 0; w < W; ++w) found[w] = sh.found[w];
 }
 
 }  // namespace ggks

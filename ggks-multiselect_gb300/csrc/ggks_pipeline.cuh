@@ -432,7 +432,7 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   {
     PassTimer t(ctx, s, GGKS_PASS_HIST);
     L(launch(p.unroll8 ? k_filter<InT, 8> : k_filter<InT, 4>, p.G, 1024, filt_smem, s,
-             ingest ? ingest : d_in, n, slice, open, tau, arr, arr_cap, &ctrl->cand_next,
+             ingest ? ingest : d_in, n, slice, samples, p.S, open, tau, arr, arr_cap, &ctrl->cand_next,
              ingest ? const_cast<InT *>(d_in) : nullptr, ctrl));
     ran[GGKS_PASS_HIST] = true;
   }
@@ -562,7 +562,7 @@ static int select_window(Context &ctx, const InT *d_in, uint64_t n, const ReqSou
     const int smem = (int)wfilter_smem_bytes<K>();
     L(set_smem_max<k_wfilter<InT>>(smem));
     PassTimer t(ctx, s, GGKS_PASS_HIST);
-    L(launch(k_wfilter<InT>, p.G, 1024, smem, s, ingest ? ingest : d_in, n, slice, spans, g,
+    L(launch(k_wfilter<InT>, p.G, 1024, smem, s, ingest ? ingest : d_in, n, slice, samples, p.S, spans, g,
              w.lo_open, w.hi_open, wc, arr, p.surv_half, bins,
              ingest ? const_cast<InT *>(d_in) : nullptr));
     ran[GGKS_PASS_HIST] = true;

@@ -158,7 +158,7 @@ __device__ __forceinline__ void filter_body(const T *__restrict__ x, uint64_t n,
 template <class T, int UNROLL>
 __global__ void __launch_bounds__(1024, 1)
     k_filter(const T *x, uint64_t n, const SliceOut<typename Traits<T>::K> *slice,
-             bool open, typename Traits<T>::K *tau, typename Traits<T>::K *__restrict__ arr,
+             const typename Traits<T>::K *samples, uint32_t S, bool open, typename Traits<T>::K *tau, typename Traits<T>::K *__restrict__ arr,
              uint64_t cap, uint32_t *len, T *__restrict__ copy_to, const Ctrl *ctrl) {
   pdl_start();
   using K = typename Traits<T>::K;
@@ -167,12 +167,17 @@ __global__ void __launch_bounds__(1024, 1)
   __shared__ uint32_t s_base;
   __shared__ RankShared<K> s_rank;
   const uint32_t status = ctrl->status;
-  const K t = open ? K(0) : rank_key<K>(slice, 0, s_rank);
+  // (the candidates' buffers lend their space)
+  K *bufs = reinterpret_cast<K *>(smem_raw), end[1];
+  static_assert(kCandWarps * kFiltBuf >= kSliceBuf, "the samples around the threshold fit");
+  const bool skip[1] = {open};
+  rank_keys<1, K>(slice, samples, S, skip, bufs, s_rank, end);
+  const K t = open ? K(0) : end[0];
   if (status & ST_FATAL) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) *tau = t;  // for k_pick
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   FiltWarp<K> fw;
-  fw.buf = reinterpret_cast<K *>(smem_raw) + warp * kFiltBuf;
+  fw.buf = bufs + warp * kFiltBuf;
   fw.arr = arr;
   fw.cap = cap;
   fw.len = len;

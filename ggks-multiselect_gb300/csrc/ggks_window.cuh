@@ -38,6 +38,7 @@ constexpr int kWinBinBits = 13;
 constexpr uint32_t kWinBins = 1u << kWinBinBits;
 constexpr uint32_t kWinCol = 16;    // keys of one lane's column (k_wfilter)
 constexpr uint32_t kWinSort = 256;  // keys of a bin that a warp sorts (k_wsort)
+static_assert(1024 * kWinCol >= 2 * kSliceBuf, "the samples around the ends fit the columns");
 
 // The window, its bins and what k_wfilter counted (device; len and below are
 // zero on entry).
@@ -217,6 +218,7 @@ __device__ __forceinline__ uint32_t wfilter_body(const T *__restrict__ x, uint64
 template <class T>
 __global__ void __launch_bounds__(1024, 1)
     k_wfilter(const T *x, uint64_t n, const SliceOut<typename Traits<T>::K> *slice,
+              const typename Traits<T>::K *samples, uint32_t S,
               const typename Traits<T>::K *spans, uint32_t parts, bool lo_open,
               bool hi_open, WinCtl<typename Traits<T>::K> *wc,
               typename Traits<T>::K *__restrict__ arr, uint64_t cap, uint32_t *__restrict__ bins_g,
@@ -231,9 +233,11 @@ __global__ void __launch_bounds__(1024, 1)
   fill_words(bins, kWinBins, 0u);
   pdl_wait();
   const SampleSpan<K> sp = sample_span<K>(spans, parts);
-  const K tlo = lo_open ? K(0) : rank_key<K>(slice, 0, s_rank);
-  const K thi = hi_open ? KeyMax<K>::v : rank_key<K>(slice, 1, s_rank);
-  __syncthreads();  // the cleared bins
+  // (the candidates' columns lend their space)
+  K *cols = reinterpret_cast<K *>(bins + kWinBins), ends[2];
+  const bool open[2] = {lo_open, hi_open};
+  rank_keys<2, K>(slice, samples, S, open, cols, s_rank, ends);
+  const K tlo = lo_open ? K(0) : ends[0], thi = hi_open ? KeyMax<K>::v : ends[1];
   WinWarp<K> ww;
   // at an open end the bins reach a quarter of the range and 64 keys past the
   // sampled extreme, for the keys the sample missed (of 65536 values, 1024 copies
@@ -247,7 +251,7 @@ __global__ void __launch_bounds__(1024, 1)
   const int bl = bitlen<K>(range);
   ww.shift = bl > kWinBinBits ? (uint32_t)(bl - kWinBinBits) : 0u;
   ww.nbins = (uint32_t)(range >> ww.shift) + 1u;
-  ww.col = reinterpret_cast<K *>(bins + kWinBins) + warp * (32 * kWinCol) + lane;
+  ww.col = cols + warp * (32 * kWinCol) + lane;
   ww.arr = arr;
   ww.cap = cap;
   ww.len = &wc->len;

@@ -44,7 +44,7 @@ int filter(const T *x, uint64_t n, uint32_t r0, uint32_t r1, bool lo_open, bool 
          k_slice<K, 2>(samples, S, spans, f.fine.data(), want, &f.slice);
        });
   ok = ok && emu::launch(grid, 1024, wfilter_smem_bytes<K>(), [&] {
-         k_wfilter<T>(x, n, &f.slice, spans, g, lo_open, hi_open, &wc, arr, cap, bins, nullptr);
+         k_wfilter<T>(x, n, &f.slice, samples, S, spans, g, lo_open, hi_open, &wc, arr, cap, bins, nullptr);
        });
   out[0] = wc.len;
   out[1] = wc.below;

@@ -34,3 +34,27 @@ def test_repeated(g, dtype, n):
             assert_same(g.multiselect_ptr(d.ptr, n, dtype, ks, ctx=ctx, small=False), desc[ks - 1],
                         f"call {i}, k's {ks}")
     ctx.close()
+
+
+@pytest.mark.parametrize("dist", ["normal", "uniform", "crowd"])
+def test_crowded_slices(g, dist):
+    """Doubles, whose fine slices of the sample are half a binade wide and hold up to a
+    quarter of it (all of it: "crowd"): the window stays as narrow as the sample allows."""
+    n = 20_000_003
+    r = np.random.default_rng(3)
+    x = r.standard_normal(n) if dist == "normal" else r.random(n) * 2e6 - 1e6
+    if dist == "crowd":
+        x = 1000.0 + x * 1e-9
+        x[r.choice(n, 2000, replace=False)] = r.random(2000) * 1e300
+    desc = np.sort(x)[::-1]
+    d = DeviceArray(x)
+    ctx = g.Context(0)
+    for at in (0.3, 0.45, 0.7, 0.93):
+        ks = np.array([int(n * at)], dtype=np.uint32)
+        assert_same(g.multiselect_ptr(d.ptr, n, np.float64, ks, ctx=ctx), desc[ks - 1], f"{dist} {at}")
+    assert ctx.stats()["topk_misses"] == 0
+    for K in (16, 3000, 20000):
+        assert_same(g.topk_ptr(d.ptr, n, np.float64, K, ctx=ctx), desc[:K], f"{dist} top-{K}")
+    if dist != "crowd":  # (whose top-k's span the gap below the values far out)
+        assert ctx.stats()["topk_misses"] == 0
+    ctx.close()

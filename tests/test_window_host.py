@@ -42,6 +42,11 @@ def make(dtype, dist, n):
         x = r.integers(0, 5, n) * 100.0
     elif dist == "spread":
         x = r.random(n) * 1e9
+    elif dist == "crowd":  # most samples in one fine slice, a few far out
+        x = 1000.0 + r.random(n)
+        x[r.choice(n, 20, replace=False)] = r.random(20) * 1e9
+    elif dist == "same":  # a fine slice of one key
+        x = np.where(r.random(n) < 0.97, 1000.0, r.random(n) * 1e9)
     else:
         x = r.standard_cauchy(n) * 1e4
     return (np.abs(x) if dtype == np.uint32 else x).clip(-4e9, 4e9).astype(dtype)
@@ -62,10 +67,10 @@ def run_filter(emu, x, r0, r1, lo_open, hi_open, grid=3):
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64, np.uint32])
-@pytest.mark.parametrize("dist", ["spread", "heavy", "few"])
+@pytest.mark.parametrize("dist", ["spread", "heavy", "few", "crowd", "same"])
 @pytest.mark.parametrize("ends", ["closed", "low", "high"])
 def test_filter(emu, dtype, dist, ends):
-    n = 5003
+    n = 5003 if dist in ("spread", "heavy", "few") else 9001  # (past 4096 in a slice)
     x = make(dtype, dist, n)
     r0, r1 = {"closed": (2300, 2700), "low": (0, 300), "high": (n - 400, n - 1)}[ends]
     lo_open, hi_open = ends == "low", ends == "high"
