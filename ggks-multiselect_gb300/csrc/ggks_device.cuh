@@ -233,7 +233,7 @@ struct Ctrl {
   uint32_t cand_next;  // candidate chunks handed out (k_hist)
   uint32_t fin_done;   // last-CTA ticket of k_finish
   uint32_t dense_hi;   // keys above a dense table's range (k_hist)
-  uint32_t pad;
+  uint32_t copies;     // copies of a popular threshold (k_filter)
   uint64_t t_ns[16];   // phase stamps of the small-vector kernel (GGKS_SMALL_TIMING builds)
 };
 

@@ -581,16 +581,18 @@ __global__ void __launch_bounds__(1024)
 // last sample instead made the window up to a quarter of the vector, too many
 // candidates: the 30 % quantile of 2^26 normal doubles 360 us a call, against 247 in the
 // pipeline, now 149.)  keys: W * kSliceBuf keys of shared memory, 16-byte
-// aligned, the caller's again afterwards.  One call per sh.
+// aligned, the caller's again afterwards.  same: the samples that hold the key.  One
+// call per sh.
 template <class K>
 struct RankShared {
   K found[2];
+  uint32_t same[2];
   uint32_t cnt[256], sel[2][3], scan[2][32], at[2];
 };
 template <int W, class K>
 __device__ __forceinline__ void rank_keys(const SliceOut<K> *out, const K *samples, uint32_t S,
                                           const bool (&skip)[W], K *keys, RankShared<K> &sh,
-                                          K (&found)[W]) {
+                                          K (&found)[W], uint32_t (&same)[W]) {
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   uint32_t cnt[W], r[W], shift[W];
   K base[W], first[W];
@@ -599,7 +601,7 @@ __device__ __forceinline__ void rank_keys(const SliceOut<K> *out, const K *sampl
     cnt[w] = out->cnt[w];
     r[w] = out->rank[w];
     shift[w] = out->shift;
-    first[w] = out->buf[w][tid];
+    first[w] = skip[w] ? K(0) : out->buf[w][tid];
     base[w] = out->base[w];
   }
   // every sample: fn(key, whether there is one)
@@ -617,6 +619,10 @@ __device__ __forceinline__ void rank_keys(const SliceOut<K> *out, const K *sampl
     }
   };
   bool rank_it[W], gather = false;  // lists to rank; lists to gather first
+  if (tid == 0) {  // (which alone writes same before the barrier ahead of the ranking)
+#pragma unroll
+    for (int w = 0; w < W; ++w) sh.same[w] = sh.at[w] = 0;
+  }
 #pragma unroll
   for (int w = 0; w < W; ++w) {
     rank_it[w] = !skip[w];
@@ -629,7 +635,10 @@ __device__ __forceinline__ void rank_keys(const SliceOut<K> *out, const K *sampl
       continue;
     }
     if ((K)~out->lo_inv[w] == (K)out->hi[w]) {  // copies of one key
-      if (tid == 0) sh.found[w] = (K)out->hi[w];
+      if (tid == 0) {
+        sh.found[w] = (K)out->hi[w];
+        sh.same[w] = cnt[w];
+      }
       rank_it[w] = false;
       continue;
     }
@@ -665,14 +674,16 @@ __device__ __forceinline__ void rank_keys(const SliceOut<K> *out, const K *sampl
       c4 = reinterpret_cast<const uint4 *>(hist)[tid];
     }
     if (cnt[w] > kSliceBuf) {  // a part of one key
-      if (tid == 0) sh.found[w] = base[w];
+      if (tid == 0) {
+        sh.found[w] = base[w];
+        sh.same[w] = cnt[w];
+      }
       rank_it[w] = false;
     } else {
       gather = true;
     }
   }
   if (gather) {
-    if (tid < W) sh.at[tid] = 0;
     __syncthreads();
     each([&](K k, bool valid) {
 #pragma unroll
@@ -696,23 +707,43 @@ __device__ __forceinline__ void rank_keys(const SliceOut<K> *out, const K *sampl
     if (cnt[w] <= 256) {
       const uint32_t me = tid >> 2;
       const K mine = kw[me];
-      uint32_t less = 0;
+      uint32_t less = 0, eq = 0;
       if (me < cnt[w])
         for (uint32_t i = tid & 3; i < cnt[w]; i += 4) {
           const K o = kw[i];
           less += o < mine || (o == mine && i < me) ? 1u : 0u;
+          eq += o == mine ? 1u : 0u;
         }
       less += __shfl_xor_sync(0xffffffffu, less, 1);
       less += __shfl_xor_sync(0xffffffffu, less, 2);
-      if (me < cnt[w] && less == r[w] && (tid & 3) == 0) sh.found[w] = mine;
+      eq += __shfl_xor_sync(0xffffffffu, eq, 1);
+      eq += __shfl_xor_sync(0xffffffffu, eq, 2);
+      if (me < cnt[w] && less == r[w] && (tid & 3) == 0) {
+        sh.found[w] = mine;
+        sh.same[w] = eq;
+      }
     } else {
       const K k = cta_select_rank<K>(kw, cnt[w], r[w], sh.cnt, sh.sel[w]);
+      uint32_t eq = 0;
+      for (uint32_t i = tid; i < cnt[w]; i += 1024) eq += kw[i] == k ? 1u : 0u;
+      eq = __reduce_add_sync(0xffffffffu, eq);
+      if (lane == 0 && eq) atomicAdd(&sh.same[w], eq);
       if (tid == 0) sh.found[w] = k;
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < W; ++w) found[w] = sh.found[w];
+  for (int w = 0; w < W; ++w) {
+    found[w] = sh.found[w];
+    same[w] = sh.same[w];
+  }
 }
+
+// Whether copies of a key that `same` of S samples hold are counted rather than kept
+// as candidates: more than one key in 128.  (A window that kept the copies of its
+// two end keys held up to the whole of a few-valued vector: of ten values in 2^26
+// floats, the median took 264 us a call by a miss, now 87; of two values 267, now 87;
+// 179 and 133 in the pipeline.)
+__host__ __device__ constexpr bool popular(uint32_t same, uint32_t S) { return same * 128u > S; }
 
 }  // namespace ggks

@@ -80,10 +80,11 @@ struct FiltWarp {
   }
 };
 
-template <class T, int UNROLL, bool INGEST>
-__device__ __forceinline__ void filter_body(const T *__restrict__ x, uint64_t n,
-                                            typename Traits<T>::K t, T *__restrict__ copy_to,
-                                            FiltWarp<typename Traits<T>::K> &fw) {
+// COPIES: copies of the threshold are counted (returned, per thread), not kept.
+template <class T, int UNROLL, bool INGEST, bool COPIES>
+__device__ __forceinline__ uint32_t filter_body(const T *__restrict__ x, uint64_t n,
+                                                typename Traits<T>::K t, T *__restrict__ copy_to,
+                                                FiltWarp<typename Traits<T>::K> &fw) {
   using K = typename Traits<T>::K;
   using V = typename Traits<T>::Vec;
   constexpr int PV = Traits<T>::kPerVec;
@@ -92,6 +93,8 @@ __device__ __forceinline__ void filter_body(const T *__restrict__ x, uint64_t n,
   V *cv = reinterpret_cast<V *>(copy_to + sp.head);
   const uint64_t tile_v = (uint64_t)blockDim.x * UNROLL;
   const uint64_t ntiles = sp.nvec / tile_v;
+  uint32_t copies = 0;
+  auto kept = [&](K k) { return COPIES ? k > t : k >= t; };
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const uint64_t off = tile * tile_v + threadIdx.x;
     V v[UNROLL];
@@ -108,11 +111,14 @@ __device__ __forceinline__ void filter_body(const T *__restrict__ x, uint64_t n,
       vec_keys<T>(v[u], k);
       bool any = false;
 #pragma unroll
-      for (int e = 0; e < PV; ++e) any |= k[e] >= t;
+      for (int e = 0; e < PV; ++e) {
+        any |= kept(k[e]);
+        if (COPIES) copies += k[e] == t ? 1u : 0u;
+      }
       // one vote per vector; the per-key votes only when a lane keeps one
       if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
-        for (int e = 0; e < PV; ++e) fw.put(k[e], k[e] >= t);
+        for (int e = 0; e < PV; ++e) fw.put(k[e], kept(k[e]));
       }
     }
   }
@@ -130,7 +136,10 @@ __device__ __forceinline__ void filter_body(const T *__restrict__ x, uint64_t n,
       K k[PV];
       vec_keys<T>(vv, k);
 #pragma unroll
-      for (int e = 0; e < PV; ++e) fw.put(k[e], valid && k[e] >= t);
+      for (int e = 0; e < PV; ++e) {
+        if (COPIES) copies += valid && k[e] == t ? 1u : 0u;
+        fw.put(k[e], valid && kept(k[e]));
+      }
     }
     auto scalar = [&](uint64_t e0, uint64_t e1) {
       for (uint64_t eb = e0; eb < e1; eb += blockDim.x) {
@@ -142,24 +151,28 @@ __device__ __forceinline__ void filter_body(const T *__restrict__ x, uint64_t n,
           if (INGEST) copy_to[e] = v;
           k = Traits<T>::key(v);
         }
-        fw.put(k, valid && k >= t);
+        if (COPIES) copies += valid && k == t ? 1u : 0u;
+        fw.put(k, valid && kept(k));
       }
     };
     scalar(0, sp.head);
     scalar(sp.tail0, n);
   }
+  return copies;
 }
 
 // The threshold is the key of slice's list 0, or 0 (open: the rank reaches the
 // smallest sample, every key is a candidate).  Grid and tiles as k_hist; 1024
 // threads; dynamic shared memory
 // kCandWarps * kFiltBuf keys.  arr[0 .. cap) receives the candidates and
-// *len (zero on entry) their count.
+// *len (zero on entry) their count.  Copies of a popular threshold are counted in
+// ctrl->copies instead (two values in 3 M floats, top-16: half the vector was
+// candidates, which one CTA of k_pick read, 493 us a call, now 35).
 template <class T, int UNROLL>
 __global__ void __launch_bounds__(1024, 1)
     k_filter(const T *x, uint64_t n, const SliceOut<typename Traits<T>::K> *slice,
              const typename Traits<T>::K *samples, uint32_t S, bool open, typename Traits<T>::K *tau, typename Traits<T>::K *__restrict__ arr,
-             uint64_t cap, uint32_t *len, T *__restrict__ copy_to, const Ctrl *ctrl) {
+             uint64_t cap, uint32_t *len, T *__restrict__ copy_to, Ctrl *ctrl) {
   pdl_start();
   using K = typename Traits<T>::K;
   extern __shared__ uint4 smem_raw[];
@@ -171,7 +184,8 @@ __global__ void __launch_bounds__(1024, 1)
   K *bufs = reinterpret_cast<K *>(smem_raw), end[1];
   static_assert(kCandWarps * kFiltBuf >= kSliceBuf, "the samples around the threshold fit");
   const bool skip[1] = {open};
-  rank_keys<1, K>(slice, samples, S, skip, bufs, s_rank, end);
+  uint32_t same[1];
+  rank_keys<1, K>(slice, samples, S, skip, bufs, s_rank, end, same);
   const K t = open ? K(0) : end[0];
   if (status & ST_FATAL) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) *tau = t;  // for k_pick
@@ -181,10 +195,16 @@ __global__ void __launch_bounds__(1024, 1)
   fw.arr = arr;
   fw.cap = cap;
   fw.len = len;
-  if (copy_to)
-    filter_body<T, UNROLL, true>(x, n, t, copy_to, fw);
-  else
-    filter_body<T, UNROLL, false>(x, n, t, nullptr, fw);
+  if (!open && popular(same[0], S)) {
+    uint32_t copies = copy_to ? filter_body<T, UNROLL, true, true>(x, n, t, copy_to, fw)
+                              : filter_body<T, UNROLL, false, true>(x, n, t, nullptr, fw);
+    copies = __reduce_add_sync(0xffffffffu, copies);
+    if (lane == 0 && copies) atomicAdd(&ctrl->copies, copies);
+  } else if (copy_to) {
+    filter_body<T, UNROLL, true, false>(x, n, t, copy_to, fw);
+  } else {
+    filter_body<T, UNROLL, false, false>(x, n, t, nullptr, fw);
+  }
   // what the warps hold: one atomic for the CTA
   if (lane == 0) s_wcnt[warp] = fw.cnt;
   __syncthreads();
@@ -211,7 +231,7 @@ __global__ void __launch_bounds__(1024, 1)
 // copied into shared memory once and every later pass reads them there.
 // Dynamic shared memory: the histogram and the bins' offsets (kPickBins words
 // each), the stage and the sort buffer (kPickCap keys).  out[i] = the (i + 1)-th
-// largest, i < kk.  The call's status (ctrl's, with ST_TOPK_MISS on a miss) goes
+// largest, i < want.  The call's status (ctrl's, with ST_TOPK_MISS on a miss) goes
 // to *host_status, in host memory, as the outputs may: the host reads both after
 // the stream's synchronisation, no copy follows.
 template <class K>
@@ -227,7 +247,7 @@ __host__ __device__ constexpr size_t pick_smem_bytes() {
 
 template <class K, class OutT>
 __global__ void __launch_bounds__(1024, 1)
-    k_pick(const K *arr, uint64_t cap, const uint32_t *len, const K *tau, uint32_t kk,
+    k_pick(const K *arr, uint64_t cap, const uint32_t *len, const K *tau, uint32_t want,
            OutT *__restrict__ out, const Ctrl *ctrl, uint32_t *host_status) {
   pdl_start();
   constexpr uint32_t kStage = PickShape<K>::kStage;
@@ -246,10 +266,14 @@ __global__ void __launch_bounds__(1024, 1)
   const uint32_t C = __ldcg(len);
   const K t = *tau;
   for (uint32_t b = tid; b < kPickBins; b += nt) hist[b] = 0;
-  if ((uint64_t)C > cap || C < kk) {  // candidates lost past the capacity, or too few
+  // candidates lost past the capacity, or too few with the threshold's copies
+  if ((uint64_t)C > cap || (C < want && want - C > __ldcg(&ctrl->copies))) {
     if (tid == 0) *host_status = status | ST_TOPK_MISS;
     return;
   }
+  const uint32_t kk = want < C ? want : C;  // from the candidates; copies for the rest
+  for (uint32_t i = kk + tid; i < want; i += nt) out[i] = Traits<OutT>::value(t);
+  if (kk == 0) return;
   const bool staged = C <= kStage;
   // every candidate once: fn(key); eight loads per thread in flight
   auto each = [&](auto &&fn) {

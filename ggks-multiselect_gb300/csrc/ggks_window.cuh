@@ -40,32 +40,50 @@ constexpr uint32_t kWinCol = 16;    // keys of one lane's column (k_wfilter)
 constexpr uint32_t kWinSort = 256;  // keys of a bin that a warp sorts (k_wsort)
 static_assert(1024 * kWinCol >= 2 * kSliceBuf, "the samples around the ends fit the columns");
 
-// The window, its bins and what k_wfilter counted (device; len and below are
-// zero on entry).
+// The window's bins: [copies of key_lo] [inner equal-width bins] [copies of key_hi].
+// The two one-key bins exist where the window's closed ends are counted rather than
+// kept (popular()): their copies are no candidates, and what lies between is never
+// more than the window's ranks.
+template <class K>
+struct WinMap {
+  K lo;                   // bin(k) = has_lo + (k - lo) >> shift, clamped to the inner bins
+  K key_lo, key_hi;
+  uint32_t shift, inner;  // inner may be 0 (counted ends with no key between them)
+  bool has_lo, has_hi, lo_open, hi_open;
+  __device__ __forceinline__ uint32_t nbins() const { return inner + has_lo + has_hi; }
+  // bin of a candidate; keys outside [lo, ...] (beyond the sampled extremes, at an open
+  // end) go to the end bins
+  __device__ __forceinline__ uint32_t bin(K k) const {
+    const K j = (k - lo) >> shift;
+    return has_lo + (k < lo ? 0u : j < (K)inner ? (uint32_t)j : inner - 1u);
+  }
+  // bins one key wide; an end bin at an open end also holds the keys beyond the
+  // sampled extremes
+  __device__ __forceinline__ bool one_key(uint32_t b) const {
+    return (has_lo && b == 0) || (has_hi && b + 1 == nbins()) ||
+           (shift == 0 && !(lo_open && b == 0) && !(hi_open && b + 1 == nbins()));
+  }
+  // such a bin's key
+  __device__ __forceinline__ K key(uint32_t b) const {
+    return has_lo && b == 0 ? key_lo : has_hi && b + 1 == nbins() ? key_hi : lo + (K)(b - has_lo);
+  }
+};
+
+// The map and what k_wfilter counted (device; len and below are zero on entry).
 template <class K>
 struct WinCtl {
   uint32_t len;    // candidates
   uint32_t below;  // keys below the window
+  uint32_t total;  // keys in all bins: the candidates and the counted ends (k_wplace)
   uint32_t first;  // first bin that a top-k needs (k_wplace)
   uint32_t big;    // needed bins of more than kWinSort keys exist (k_wplace)
-  K lo;            // smallest key of bin 1's left end: bin(k) = (k - lo) >> shift, clamped
-  uint32_t shift, nbins;
+  uint32_t ends;   // 1: has_lo, 2: has_hi
+  K lo, key_lo, key_hi;
+  uint32_t shift, inner;
+  __device__ __forceinline__ WinMap<K> map(bool lo_open, bool hi_open) const {
+    return {lo, key_lo, key_hi, shift, inner, (ends & 1u) != 0, (ends & 2u) != 0, lo_open, hi_open};
+  }
 };
-
-// bin of a candidate; keys outside [lo, ...] (beyond the sampled extremes, at an
-// open end) go to the end bins
-template <class K>
-__device__ __forceinline__ uint32_t win_bin(K k, K lo, uint32_t shift, uint32_t nbins) {
-  const K j = (k - lo) >> shift;
-  return k < lo ? 0u : j < (K)nbins ? (uint32_t)j : nbins - 1u;
-}
-
-// bins one key wide hold copies of lo + b; an end bin at an open end also holds
-// the keys beyond the sampled extremes
-__device__ __forceinline__ bool win_one_key(uint32_t b, uint32_t shift, uint32_t nbins, bool lo_open,
-                                            bool hi_open) {
-  return shift == 0 && !(lo_open && b == 0) && !(hi_open && b + 1 == nbins);
-}
 
 // One warp's candidates: each lane keeps its own in a column of shared memory --
 // a predicated store and increment per key, no votes -- and when a column could
@@ -81,8 +99,7 @@ struct WinWarp {
   uint64_t cap;
   uint32_t *len;
   uint32_t *bins;  // the CTA's
-  K lo;
-  uint32_t shift, nbins;
+  WinMap<K> map;
   __device__ __forceinline__ void put(K k, bool keep) {
     if (keep) col[32 * cnt++] = k;
   }
@@ -102,7 +119,7 @@ struct WinWarp {
       const uint32_t m = __ballot_sync(0xffffffffu, have);
       if (have) {
         const K k = col[32 * c];
-        atomicAdd(&bins[win_bin(k, lo, shift, nbins)], 1u);
+        atomicAdd(&bins[map.bin(k)], 1u);
         const uint64_t at = (uint64_t)base + __popc(m & ((1u << lane) - 1u));
         if (at < cap) arr[at] = k;
       }
@@ -117,18 +134,22 @@ __host__ __device__ constexpr size_t wfilter_smem_bytes() {
   return kWinBins * 4 + (size_t)1024 * kWinCol * sizeof(K);
 }
 
-// Grid and tiles as k_hist; 1024 threads.  COUNT: the keys below the window are
-// counted (neither end open: a window that is open below has none, one that is
-// open above has all keys that are not candidates).  A window of one key (a
-// value that a good part of the vector holds) keeps nothing: *same counts its
-// copies.  copy_to: as in k_filter.
-template <class T, bool COUNT, bool INGEST>
-__device__ __forceinline__ uint32_t wfilter_body(const T *__restrict__ x, uint64_t n,
-                                                 typename Traits<T>::K tlo,
-                                                 typename Traits<T>::K width,
-                                                 T *__restrict__ copy_to,
-                                                 WinWarp<typename Traits<T>::K> &ww,
-                                                 uint32_t *same) {
+// What a thread counted: keys below the window (COUNT: neither end open -- a window
+// that is open below has none, one that is open above has all keys outside it),
+// and copies of its end keys (ENDS).
+struct WinCount {
+  uint32_t below = 0, lo = 0, hi = 0;
+};
+
+// Grid and tiles as k_hist; 1024 threads.  Keeps the keys of [in, in + width] (ENDS:
+// none at all where `none`).  copy_to: as in k_filter.
+template <class T, bool COUNT, bool ENDS, bool INGEST>
+__device__ __forceinline__ void wfilter_body(const T *__restrict__ x, uint64_t n,
+                                             typename Traits<T>::K tlo, typename Traits<T>::K thi,
+                                             typename Traits<T>::K in,
+                                             typename Traits<T>::K width, bool none,
+                                             T *__restrict__ copy_to,
+                                             WinWarp<typename Traits<T>::K> &ww, WinCount &wcnt) {
   using K = typename Traits<T>::K;
   using V = typename Traits<T>::Vec;
   constexpr int PV = Traits<T>::kPerVec;
@@ -138,8 +159,15 @@ __device__ __forceinline__ uint32_t wfilter_body(const T *__restrict__ x, uint64
   V *cv = reinterpret_cast<V *>(copy_to + sp.head);
   const uint64_t tile_v = (uint64_t)blockDim.x * UNROLL;
   const uint64_t ntiles = sp.nvec / tile_v;
-  uint32_t below = 0, equal = 0;
-  const bool single = width == 0;  // one key: its copies are only counted
+  uint32_t below = 0, at_lo = 0, at_hi = 0;
+  auto one = [&](K k, bool valid) {
+    if (COUNT || ENDS) below += valid && k < tlo ? 1u : 0u;
+    if (ENDS) {
+      at_lo += valid && k == tlo ? 1u : 0u;
+      at_hi += valid && k == thi ? 1u : 0u;
+    }
+    ww.put(k, valid && !(ENDS && none) && (K)(k - in) <= width);
+  };
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const uint64_t off = tile * tile_v + threadIdx.x;
     V v[UNROLL];
@@ -154,31 +182,13 @@ __device__ __forceinline__ uint32_t wfilter_body(const T *__restrict__ x, uint64
     for (int u = 0; u < UNROLL; ++u) {
       K k[PV];
       vec_keys<T>(v[u], k);
-      if (COUNT && single) {
 #pragma unroll
-        for (int e = 0; e < PV; ++e) {
-          below += k[e] < tlo ? 1u : 0u;
-          equal += k[e] == tlo ? 1u : 0u;
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < PV; ++e) {
-          if (COUNT) below += k[e] < tlo ? 1u : 0u;
-          ww.put(k[e], (K)(k[e] - tlo) <= width);
-        }
-        ww.check();
-      }
+      for (int e = 0; e < PV; ++e) one(k[e], true);
+      ww.check();
     }
   }
   // leftover vectors and the scalar head / tail: every lane runs every round
   if (blockIdx.x == (uint32_t)(ntiles % gridDim.x)) {
-    auto one = [&](K k, bool valid) {
-      if (COUNT) below += valid && k < tlo ? 1u : 0u;
-      if (COUNT && single)
-        equal += valid && k == tlo ? 1u : 0u;
-      else
-        ww.put(k, valid && (K)(k - tlo) <= width);
-    };
     for (uint64_t vb = ntiles * tile_v; vb < sp.nvec; vb += blockDim.x) {
       const uint64_t vi = vb + threadIdx.x;
       const bool valid = vi < sp.nvec;
@@ -210,8 +220,9 @@ __device__ __forceinline__ uint32_t wfilter_body(const T *__restrict__ x, uint64
     scalar(0, sp.head);
     scalar(sp.tail0, n);
   }
-  *same = equal;
-  return below;
+  wcnt.below = below;
+  wcnt.lo = at_lo;
+  wcnt.hi = at_hi;
 }
 
 // bins: kWinBins words, zero on entry.
@@ -236,59 +247,81 @@ __global__ void __launch_bounds__(1024, 1)
   // (the candidates' columns lend their space)
   K *cols = reinterpret_cast<K *>(bins + kWinBins), ends[2];
   const bool open[2] = {lo_open, hi_open};
-  rank_keys<2, K>(slice, samples, S, open, cols, s_rank, ends);
+  uint32_t same[2];
+  rank_keys<2, K>(slice, samples, S, open, cols, s_rank, ends, same);
   const K tlo = lo_open ? K(0) : ends[0], thi = hi_open ? KeyMax<K>::v : ends[1];
+  // counted ends: all closed ones, where one is popular or both are the same key
+  const bool counted = (!lo_open && popular(same[0], S)) || (!hi_open && popular(same[1], S)) ||
+                       tlo == thi;
   WinWarp<K> ww;
+  WinMap<K> &map = ww.map;
+  map.has_lo = counted && !lo_open;
+  map.has_hi = counted && !hi_open && !(map.has_lo && thi == tlo);
+  map.lo_open = lo_open;
+  map.hi_open = hi_open;
+  map.key_lo = tlo;
+  map.key_hi = thi;
+  // the kept keys [in, out], if any
+  const K in = map.has_lo ? tlo + 1 : tlo, out = map.has_hi ? thi - 1 : thi;
+  const bool none = in > out || (map.has_lo && in == 0) || (map.has_hi && thi == 0);
   // at an open end the bins reach a quarter of the range and 64 keys past the
   // sampled extreme, for the keys the sample missed (of 65536 values, 1024 copies
   // each, it misses the largest in one vector of three)
-  K lo = lo_open ? sp.kmin : tlo, hi = hi_open ? sp.kmax : thi;
+  K lo = lo_open ? sp.kmin : in, hi = hi_open ? sp.kmax : out;
   const K more = (hi > lo ? hi - lo : K(0)) / 4 + 64;
   if (lo_open) lo = lo > more ? lo - more : K(0);
   if (hi_open) hi = hi < KeyMax<K>::v - more ? hi + more : KeyMax<K>::v;
-  ww.lo = lo;
+  map.lo = lo;
   const K range = hi > lo ? hi - lo : K(0);
   const int bl = bitlen<K>(range);
-  ww.shift = bl > kWinBinBits ? (uint32_t)(bl - kWinBinBits) : 0u;
-  ww.nbins = (uint32_t)(range >> ww.shift) + 1u;
+  map.shift = bl > kWinBinBits ? (uint32_t)(bl - kWinBinBits) : 0u;
+  if (counted && (range >> map.shift) + 1 > (K)(kWinBins - 2)) map.shift++;  // room for the ends
+  map.inner = none ? 0u : (uint32_t)(range >> map.shift) + 1u;
   ww.col = cols + warp * (32 * kWinCol) + lane;
   ww.arr = arr;
   ww.cap = cap;
   ww.len = &wc->len;
   ww.bins = bins;
   if (blockIdx.x == 0 && tid == 0) {
-    wc->lo = ww.lo;
-    wc->shift = ww.shift;
-    wc->nbins = ww.nbins;
+    wc->lo = map.lo;
+    wc->key_lo = map.key_lo;
+    wc->key_hi = map.key_hi;
+    wc->shift = map.shift;
+    wc->inner = map.inner;
+    wc->ends = (map.has_lo ? 1u : 0u) | (map.has_hi ? 2u : 0u);
   }
-  const K width = thi - tlo;
-  uint32_t below = 0, same = 0;
+  const K width = out - in;
+  WinCount wcnt;
   if (copy_to) {
-    if (lo_open || hi_open)
-      wfilter_body<T, false, true>(x, n, tlo, width, copy_to, ww, &same);
+    if (counted)
+      wfilter_body<T, false, true, true>(x, n, tlo, thi, in, width, none, copy_to, ww, wcnt);
+    else if (lo_open || hi_open)
+      wfilter_body<T, false, false, true>(x, n, tlo, thi, in, width, none, copy_to, ww, wcnt);
     else
-      below = wfilter_body<T, true, true>(x, n, tlo, width, copy_to, ww, &same);
+      wfilter_body<T, true, false, true>(x, n, tlo, thi, in, width, none, copy_to, ww, wcnt);
+  } else if (counted) {
+    wfilter_body<T, false, true, false>(x, n, tlo, thi, in, width, none, nullptr, ww, wcnt);
   } else if (lo_open || hi_open) {
-    wfilter_body<T, false, false>(x, n, tlo, width, nullptr, ww, &same);
+    wfilter_body<T, false, false, false>(x, n, tlo, thi, in, width, none, nullptr, ww, wcnt);
   } else {
-    below = wfilter_body<T, true, false>(x, n, tlo, width, nullptr, ww, &same);
+    wfilter_body<T, true, false, false>(x, n, tlo, thi, in, width, none, nullptr, ww, wcnt);
   }
   ww.flush();
-  below = __reduce_add_sync(0xffffffffu, below);
-  same = __reduce_add_sync(0xffffffffu, same);
+  const uint32_t nbins = map.nbins();
+  const uint32_t below = __reduce_add_sync(0xffffffffu, wcnt.below);
+  const uint32_t at_lo = __reduce_add_sync(0xffffffffu, wcnt.lo);
+  const uint32_t at_hi = __reduce_add_sync(0xffffffffu, wcnt.hi);
   if (lane == 0) {
     s_below[warp] = below;
-    if (same) {
-      atomicAdd(&bins[0], same);
-      atomicAdd(&wc->len, same);
-    }
+    if (map.has_lo && at_lo) atomicAdd(&bins[0], at_lo);
+    if (map.has_hi && at_hi) atomicAdd(&bins[nbins - 1], at_hi);
   }
   __syncthreads();
-  for (uint32_t b = tid; b < ww.nbins; b += blockDim.x)
+  for (uint32_t b = tid; b < nbins; b += blockDim.x)
     if (bins[b]) atomicAdd(&bins_g[b], bins[b]);
   if (warp == 0) {
-    below = __reduce_add_sync(0xffffffffu, s_below[lane]);
-    if (lane == 0 && below) atomicAdd(&wc->below, below);
+    const uint32_t all = __reduce_add_sync(0xffffffffu, s_below[lane]);
+    if (lane == 0 && all) atomicAdd(&wc->below, all);
   }
 }
 
@@ -321,11 +354,9 @@ __global__ void __launch_bounds__(1024, 1)
   __shared__ uint32_t s_scan[32];
   __shared__ bool s_miss;
   const uint32_t tid = threadIdx.x, lane = tid & 31;
-  const uint32_t C = wc->len, nbins = wc->nbins, shift = wc->shift;
-  const K lo = wc->lo;
-  // keys below the window: none below an open low end, all that are no
-  // candidates below an open high end, else counted
-  const uint64_t below = lo_open ? 0u : hi_open ? n - C : wc->below;
+  const uint32_t C = wc->len;
+  const WinMap<K> map = wc->map(lo_open, hi_open);
+  const uint32_t nbins = map.nbins();
   constexpr uint32_t kPer = kWinBins / 1024;
   uint32_t c[kPer], sum = 0;
 #pragma unroll
@@ -335,9 +366,7 @@ __global__ void __launch_bounds__(1024, 1)
     sum += v.x + v.y + v.z + v.w;
   }
   if (tid < kWinBins / 32) need[tid] = 0;
-  // a window of one key: its copies were counted, not kept
-  const bool single = nbins == 1 && shift == 0 && !lo_open && !hi_open;
-  if (tid == 0) s_miss = ((uint64_t)C > cap && !single) || (kk && (C < kk || !hi_open));
+  if (tid == 0) s_miss = false;
   uint32_t total;
   uint32_t run = block_excl_scan(sum, s_scan, &total);
   bool big = false;
@@ -347,7 +376,18 @@ __global__ void __launch_bounds__(1024, 1)
     run += c[q];
   }
   __syncthreads();
-  // the last bin whose prefix is <= r, for r < C (never an empty one)
+  auto count_of = [&](uint32_t b) -> uint32_t {
+    return (b + 1 < kWinBins ? pre[b + 1] : total) - pre[b];
+  };
+  // the counted ends' copies take no places: a bin's begin at pre - off
+  const uint32_t off = map.has_lo ? count_of(0) : 0u;
+  const uint32_t copies = off + (map.has_hi ? count_of(nbins - 1) : 0u);
+  // keys below the window: none below an open low end, all outside the window below an
+  // open high end, else counted
+  const uint64_t below = lo_open ? 0u : hi_open ? n - total : wc->below;
+  const bool bad = (uint64_t)C > cap || (uint64_t)C > placed_cap || total - copies != C ||
+                   (kk && (total < kk || !hi_open));
+  // the last bin whose prefix is <= r, for r < total (never an empty one)
   auto bin_at = [&](uint32_t r) -> uint32_t {
     uint32_t b = 0;
 #pragma unroll
@@ -355,31 +395,28 @@ __global__ void __launch_bounds__(1024, 1)
       if (pre[b + step] <= r && b + step < nbins) b += step;
     return b;
   };
-  auto count_of = [&](uint32_t b) -> uint32_t {
-    return (b + 1 < kWinBins ? pre[b + 1] : total) - pre[b];
-  };
-  // bins one key wide (but the end bins at open ends): their key is known
-  auto one_key = [&](uint32_t b) -> bool { return win_one_key(b, shift, nbins, lo_open, hi_open); };
   uint32_t first = 0;
-  if (!s_miss && kk) {
-    first = bin_at(C - kk);
+  if (!bad && kk) {
+    first = bin_at(total - kk);
 #pragma unroll
     for (uint32_t q = 0; q < kPer; ++q) big |= tid * kPer + q >= first && c[q] > kWinSort;
   }
   big = __syncthreads_or(big);
-  if (!s_miss && !kk && tid < num_req) {
+  if (!bad && !kk && tid < num_req) {
     const Req q = reqs[tid];
-    if (q.rank < below || q.rank - below >= C) {
+    if (q.rank < below || q.rank - below >= total) {
       s_miss = true;
     } else {
       const uint32_t r = (uint32_t)(q.rank - below), b = bin_at(r);
-      if (!one_key(b)) atomicOr(&need[b >> 5], 1u << (b & 31));
+      const bool one = map.one_key(b);
+      if (!one) atomicOr(&need[b >> 5], 1u << (b & 31));
       if (blockIdx.x == 0) {
-        sl.seg_off[tid] = pre[b];
-        sl.seg_size[tid] = one_key(b) ? 0u : count_of(b);  // 0: a flat slot, answered from seg_lo
+        const uint32_t j = b - map.has_lo;  // among the inner bins
+        sl.seg_off[tid] = pre[b] - off;
+        sl.seg_size[tid] = one ? 0u : count_of(b);  // 0: a flat slot, answered from seg_lo
         // an end bin also holds the keys beyond the sampled extremes
-        sl.seg_lo[tid] = b == 0 && lo_open ? K(0) : lo + ((K)b << shift);
-        sl.seg_hi[tid] = b + 1 >= nbins ? KeyMax<K>::v : lo + (((K)b + 1) << shift) - K(1);
+        sl.seg_lo[tid] = one ? map.key(b) : b == 0 && lo_open ? K(0) : map.lo + ((K)j << map.shift);
+        sl.seg_hi[tid] = j + 1 >= map.inner ? KeyMax<K>::v : map.lo + (((K)j + 1) << map.shift) - K(1);
         sl.kstart[tid] = tid;
         sl.kcnt[tid] = 1;
         Req e;
@@ -390,19 +427,20 @@ __global__ void __launch_bounds__(1024, 1)
     }
   }
   __syncthreads();
-  const bool miss = s_miss || ((uint64_t)total > placed_cap && !single);
+  const bool miss = bad || s_miss;
   if (blockIdx.x == 0) {
     if (tid == 0) {
       if (miss) atomicOr(&ctrl->status, ST_TOPK_MISS);
       ctrl->num_slots = num_req;
       ctrl->total_surv = C;
+      wc->total = total;
       wc->first = first;
       wc->big = big ? 1u : 0u;
     }
     if (kk)
       for (uint32_t b = tid; b < kWinBins; b += blockDim.x) pre_g[b] = pre[b];
   }
-  if (miss || single) return;
+  if (miss) return;
   // whole warps over the candidates, four loads in flight per lane; a bin that meets
   // more keys than it counted keeps its places and the call is a miss
   bool over = false;
@@ -418,9 +456,9 @@ __global__ void __launch_bounds__(1024, 1)
 #pragma unroll
     for (uint32_t u = 0; u < U; ++u) {
       const bool valid = i0 + 32 * u + lane < C;
-      const uint32_t b = win_bin(k[u], lo, shift, nbins);
+      const uint32_t b = map.bin(k[u]);
       const bool want =
-          valid && (kk ? b >= first && !one_key(b) : ((need[b >> 5] >> (b & 31)) & 1u) != 0u);
+          valid && (kk ? b >= first && !map.one_key(b) : ((need[b >> 5] >> (b & 31)) & 1u) != 0u);
       const uint32_t m = __ballot_sync(0xffffffffu, want);
       if (!m) continue;
       // lanes of one bin take one atomic
@@ -433,7 +471,7 @@ __global__ void __launch_bounds__(1024, 1)
       if (place) {
         const uint32_t at = base + __popc(peers & ((1u << lane) - 1u));
         if (at < count_of(b))
-          placed[pre[b] + at] = k[u];
+          placed[pre[b] - off + at] = k[u];
         else
           over = true;
       } else if (want) {
@@ -465,9 +503,11 @@ __global__ void __launch_bounds__(kWinSortThreads)
   // lanes meet in shuffles below
   const uint32_t status = __shfl_sync(0xffffffffu, ctrl->status, 0);
   if (!(status & (ST_FATAL | ST_TOPK_MISS))) {
-    const uint32_t C = wc->len, nbins = wc->nbins, first = wc->first;
+    const uint32_t C = wc->total, first = wc->first;
+    const WinMap<K> map = wc->map(false, true);
+    const uint32_t nbins = map.nbins(), off = map.has_lo ? bins_g[0] : 0u;
     const uint32_t warps = gridDim.x * (kWinSortThreads / 32);
-    // position p of the candidates' order is the (C - p)-th largest
+    // position p of the window's order is the (C - p)-th largest
     auto put = [&](uint32_t p, K k) {
       const uint32_t i = C - 1 - p;
       if (i < kk) out[i] = Traits<OutT>::value(k);
@@ -477,20 +517,17 @@ __global__ void __launch_bounds__(kWinSortThreads)
       K v[R];
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        v[r] = r * 32 + lane < c ? __ldcg(placed + p0 + r * 32 + lane) : KeyMax<K>::v;
+        v[r] = r * 32 + lane < c ? __ldcg(placed + p0 - off + r * 32 + lane) : KeyMax<K>::v;
       warp_bitonic_regs<K, R>(v);
 #pragma unroll
       for (int r = 0; r < R; ++r)
         if (r * 32 + lane < c) put(p0 + r * 32 + lane, v[r]);
     };
-    const K lo = wc->lo;
-    const uint32_t shift = wc->shift;
-    auto one_key = [&](uint32_t b) -> bool { return win_one_key(b, shift, nbins, false, true); };
     for (uint32_t b = first + blockIdx.x * (kWinSortThreads / 32) + (tid >> 5); b < nbins; b += warps) {
       const uint32_t c = bins_g[b], p0 = pre_g[b];
       if (c == 0) continue;
-      if (one_key(b)) {
-        for (uint32_t j = lane; c <= kWinSort && j < c; j += 32) put(p0 + j, lo + (K)b);
+      if (map.one_key(b)) {
+        for (uint32_t j = lane; c <= kWinSort && j < c; j += 32) put(p0 + j, map.key(b));
       } else if (c <= 32)
         sorted(std::integral_constant<int, 1>{}, p0, c);
       else if (c <= 64)
@@ -508,7 +545,7 @@ __global__ void __launch_bounds__(kWinSortThreads)
         for (uint32_t step = kWinBins / 2; step; step >>= 1)
           if (b + step < nbins && pre_g[b + step] <= p) b += step;
         if (bins_g[b] > kWinSort)
-          out[i] = Traits<OutT>::value(one_key(b) ? lo + (K)b : (K)big_hi[b]);
+          out[i] = Traits<OutT>::value(map.one_key(b) ? map.key(b) : (K)big_hi[b]);
       }
     }
   }

@@ -50,7 +50,10 @@ int filter(const T *x, uint64_t n, uint32_t r0, uint32_t r1, bool lo_open, bool 
   out[1] = wc.below;
   out[2] = wc.lo;
   out[3] = wc.shift;
-  out[4] = wc.nbins;
+  out[4] = wc.inner;
+  out[5] = wc.ends;
+  out[6] = wc.key_lo;
+  out[7] = wc.key_hi;
   return ok ? 0 : 1;
 }
 
@@ -67,7 +70,7 @@ int place(const K *arr, uint32_t len, uint64_t n, uint32_t below, K lo, uint32_t
   wc.below = below;
   wc.lo = lo;
   wc.shift = shift;
-  wc.nbins = nbins;
+  wc.inner = nbins;
   std::vector<uint32_t> cur(kWinBins, 0), pre(kWinBins, 0);
   std::vector<unsigned long long> big_lo(kWinBins, 0), big_hi(kWinBins, 0);
   const uint32_t slots = num_req ? num_req : 1;

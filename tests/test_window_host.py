@@ -38,6 +38,13 @@ def keys(x):
 
 def make(dtype, dist, n):
     r = np.random.default_rng(n)
+    if dist == "limits":  # the smallest and the largest key, 40 % of the vector each
+        u = np.dtype(f"u{np.dtype(dtype).itemsize}")
+        top = u.type(-1 % (1 << 8 * u.itemsize)) >> u.type(dtype != np.uint32)
+        b = (r.random(n) * 1e9).astype(dtype).view(u)
+        p = r.random(n)
+        return np.where(p < 0.4, u.type(0 if dtype == np.uint32 else -1 % (1 << 8 * u.itemsize)),
+                        np.where(p < 0.8, top, b)).astype(u).view(dtype)
     if dist == "few":
         x = r.integers(0, 5, n) * 100.0
     elif dist == "spread":
@@ -56,7 +63,7 @@ def run_filter(emu, x, r0, r1, lo_open, hi_open, grid=3):
     k = keys(x)
     arr = np.zeros(x.size, k.dtype)
     bins = np.zeros(BINS, np.uint32)
-    out = np.zeros(5, np.uint64)
+    out = np.zeros(8, np.uint64)
     fn = {np.dtype(np.float32): emu.emu_filter_f32, np.dtype(np.float64): emu.emu_filter_f64,
           np.dtype(np.uint32): emu.emu_filter_u32}[x.dtype]
     rc = fn(x.ctypes.data_as(ctypes.c_void_p), ctypes.c_uint64(x.size), r0, r1, int(lo_open),
@@ -67,30 +74,40 @@ def run_filter(emu, x, r0, r1, lo_open, hi_open, grid=3):
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64, np.uint32])
-@pytest.mark.parametrize("dist", ["spread", "heavy", "few", "crowd", "same"])
+@pytest.mark.parametrize("dist", ["spread", "heavy", "few", "crowd", "same", "limits"])
 @pytest.mark.parametrize("ends", ["closed", "low", "high"])
 def test_filter(emu, dtype, dist, ends):
-    n = 5003 if dist in ("spread", "heavy", "few") else 9001  # (past 4096 in a slice)
+    n = 5003 if dist not in ("crowd", "same") else 9001  # (past 4096 in a slice)
     x = make(dtype, dist, n)
     r0, r1 = {"closed": (2300, 2700), "low": (0, 300), "high": (n - 400, n - 1)}[ends]
     lo_open, hi_open = ends == "low", ends == "high"
-    k, arr, bins, (length, below, lo, shift, nbins) = run_filter(emu, x, r0, r1, lo_open, hi_open)
+    k, arr, bins, (length, below, lo, shift, inner, counted, key_lo, key_hi) = run_filter(
+        emu, x, r0, r1, lo_open, hi_open)
     s = np.sort(k)
+    has_lo, has_hi = counted & 1, counted >> 1
+    share = {e: np.count_nonzero(k == s[r]) / n for e, r in (("lo", r0), ("hi", r1))}
+    popular = (not lo_open and share["lo"] > 1 / 128) or (not hi_open and share["hi"] > 1 / 128)
+    same = ends == "closed" and s[r0] == s[r1]
+    assert bool(counted) == (popular or same)
     keep = np.ones(n, bool)
     if not lo_open:
-        keep &= k >= s[r0]
+        keep &= k > s[r0] if has_lo else k >= s[r0]
     if not hi_open:
-        keep &= k <= s[r1]
+        keep &= k < s[r1] if has_hi else k <= s[r1]
     want = np.sort(k[keep])
     assert length == want.size
     if ends == "closed":
         assert below == np.count_nonzero(k < s[r0])
-    if ends == "closed" and s[r0] == s[r1]:
-        assert bins[0] == length and not bins[1:].any()  # one key: counted, not kept
-        return
     assert np.array_equal(np.sort(arr[:length]), want)
-    at = np.array([0 if v < lo else min((v - lo) >> shift, nbins - 1) for v in want.tolist()])
-    assert np.array_equal(bins, np.bincount(at, minlength=BINS))
+    at = [has_lo + (0 if v < lo else min((v - lo) >> shift, inner - 1)) for v in want.tolist()]
+    expect = np.bincount(np.array(at, int), minlength=BINS)
+    if has_lo:
+        assert key_lo == s[r0]
+        expect[0] += np.count_nonzero(k == s[r0])
+    if has_hi:
+        assert key_hi == s[r1]
+        expect[has_lo + inner] += np.count_nonzero(k == s[r1])
+    assert np.array_equal(bins, expect)
 
 
 def place(emu, arr, n, below, lo, shift, nbins, bins, kk, ranks, grid, sort=False):
