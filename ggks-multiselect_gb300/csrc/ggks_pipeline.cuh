@@ -45,13 +45,13 @@ constexpr int kPlanSmemMax = (int)(kLutPadded * sizeof(uint32_t) + (size_t)kMaxN
                                    kPlanSlotBytes);
 
 // The words after the fine counts, cleared by k_sample with them where a path
-// uses them: the window path's bins, cursors, large bins' extreme keys (64-bit)
-// and counters, then the sample keys around thresholds (SliceOut, whose first
+// uses them: the window path's bins, cursors, large bins' first keys (64-bit) and
+// flags, and counters, then the sample keys around thresholds (SliceOut, whose first
 // words are cleared too).
 constexpr uint32_t kWinBinsAt = kLutIdx, kWinCurAt = kWinBinsAt + kWinBins,
-                   kWinLoAt = kWinCurAt + kWinBins, kWinHiAt = kWinLoAt + 2 * kWinBins,
-                   kWinCtlAt = kWinHiAt + 2 * kWinBins, kFineWords = kWinCtlAt + 16;
-static_assert(sizeof(WinCtl<uint64_t>) <= 64 && kWinLoAt % 2 == 0 && kFineWords % 4 == 0,
+                   kWinFirstAt = kWinCurAt + kWinBins, kWinMixedAt = kWinFirstAt + 2 * kWinBins,
+                   kWinCtlAt = kWinMixedAt + kWinBins, kFineWords = kWinCtlAt + 16;
+static_assert(sizeof(WinCtl<uint64_t>) <= 64 && kWinFirstAt % 2 == 0 && kFineWords % 4 == 0,
               "the counters' place and alignment");
 
 struct Plan {
@@ -461,6 +461,12 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   return GGKS_OK;
 }
 
+// A top-k selects again from one large bin of distinct keys at most, and for at most
+// kWinMaxAgain values; else the pipeline answers (2^24 floats, 0.1 % of them one value
+// far out, top-20000: 222 us a call by the pipeline after the window, 134 with 3300
+// values of one bin selected again; 3 M floats, 17000 values: 163 and 203).
+constexpr uint32_t kWinMaxDefer = 1;
+constexpr uint32_t kWinMaxAgain = 4096;
 // smallest vector whose clustered k's go to the window path before the one-launch one
 constexpr uint64_t kWinFirstN = 1ull << 19;
 
@@ -518,18 +524,20 @@ static int select_window(Context &ctx, const InT *d_in, uint64_t n, const ReqSou
   K *spans = reinterpret_cast<K *>(A + p.spans);
   uint32_t *fine = reinterpret_cast<uint32_t *>(A + p.fine);
   uint32_t *bins = fine + kWinBinsAt, *cur = fine + kWinCurAt;
-  auto *big_lo = reinterpret_cast<unsigned long long *>(fine + kWinLoAt);
-  auto *big_hi = reinterpret_cast<unsigned long long *>(fine + kWinHiAt);
+  const BigBins big{reinterpret_cast<unsigned long long *>(fine + kWinFirstAt), fine + kWinMixedAt};
   WinCtl<K> *wc = reinterpret_cast<WinCtl<K> *>(fine + kWinCtlAt);
   SliceOut<K> *slice = reinterpret_cast<SliceOut<K> *>(fine + kFineWords);
   uint32_t *wpre = reinterpret_cast<uint32_t *>(A + p.wpre);
   K *arr = reinterpret_cast<K *>(ctx.surv), *placed = arr + p.surv_half;
-  // pinned: [out | control block | requests]
+  // pinned: [out | control block | requests | large bins]
   const bool want_host = host_results != nullptr;
   const size_t out_span = p.ctrl - p.out;
-  e = ensure_pin(ctx, out_span + 256 + (src.h_k ? (size_t)num_req * sizeof(Req) : 0));
+  const uint32_t room = src.h_k ? num_req : kWinMaxDefer;
+  const size_t big_at = align_up(out_span + 256 + (src.h_k ? (size_t)num_req * sizeof(Req) : 0), 16);
+  e = ensure_pin(ctx, big_at + room * sizeof(WinDefer));
   if (e != cudaSuccess) return from_cuda(e);
   Ctrl *h_ctrl = reinterpret_cast<Ctrl *>(ctx.pin + out_span);
+  WinDefer *h_big = reinterpret_cast<WinDefer *>(ctx.pin + big_at);
   // results in place: at most kPlanFew of a k list, and a top-k's warps write
   // neighbouring ones (65536 uint32: 4 us a call less than by a copy)
   static_assert(kPlanFew <= kPinOut, "results of a k list");
@@ -570,47 +578,96 @@ static int select_window(Context &ctx, const InT *d_in, uint64_t n, const ReqSou
   WinSlots<K> sl;
   sl.seg_off = reinterpret_cast<uint64_t *>(A + p.seg_off);
   sl.seg_size = reinterpret_cast<uint32_t *>(A + p.seg_size);
-  sl.kstart = reinterpret_cast<uint32_t *>(A + p.kstart);
-  sl.kcnt = reinterpret_cast<uint32_t *>(A + p.kcnt);
+  sl.bin = reinterpret_cast<uint32_t *>(A + p.kstart);
   sl.seg_lo = reinterpret_cast<K *>(A + p.seg_lo);
   sl.seg_hi = reinterpret_cast<K *>(A + p.seg_hi);
   sl.klist = reinterpret_cast<Req *>(A + p.klist);
   {
     PassTimer t(ctx, s, GGKS_PASS_COMPACT);
     const uint32_t grid = (uint32_t)std::min<double>(ctx.sm_count, 1.0 + w.expect / 4096.0);
-    L(launch(k_wplace<K>, grid, 1024, 0, s, arr, p.surv_half, n, src.topk ? num_req : 0u, w.lo_open,
-             w.hi_open, reqs, num_req, wc, bins, cur, wpre, placed, p.surv_cap - p.surv_half, big_lo,
-             big_hi, sl, ctrl));
+    L(set_smem_max<k_wplace<K>>((int)(kWinBins * 4)));
+    L(launch(k_wplace<K>, grid, 1024, kWinBins * 4, s, arr, p.surv_half, n, src.topk ? num_req : 0u, w.lo_open,
+             w.hi_open, reqs, num_req, wc, bins, cur, wpre, placed, p.surv_cap - p.surv_half, big, sl,
+             ctrl));
     ran[GGKS_PASS_COMPACT] = true;
   }
   Ctrl *h_ctrl_dev = reinterpret_cast<Ctrl *>(ctx.pin_dev + out_span);
+  WinDefer *deferred = reinterpret_cast<WinDefer *>(ctx.pin_dev + big_at);
   {
     PassTimer t(ctx, s, GGKS_PASS_FINISH);
     if (src.topk) {
       L(launch(k_wsort<K, InT>, 2u * (uint32_t)ctx.sm_count, kWinSortThreads, 0, s, placed, wc, bins,
-               wpre, big_lo, big_hi, num_req, d_out, ctrl, &h_ctrl_dev->status));
+               wpre, big, num_req, deferred, room, d_out, ctrl, h_ctrl_dev));
     } else {
       const int smem = finish_smem_bytes<InT>();
-      L(set_smem_max<k_finish<K, InT>>(smem));
-      L(launch(k_finish<K, InT>, num_req, kFinThreads, smem, s, placed, ctrl, sl.seg_off,
-               sl.seg_size, sl.seg_lo, sl.seg_hi, sl.kstart, sl.kcnt, sl.klist,
-               reinterpret_cast<uint32_t *>(A + p.deferred), p.cap_keys, d_out, h_ctrl_dev));
+      L(set_smem_max<k_wfinish<K, InT>>(smem));
+      L(launch(k_wfinish<K, InT>, num_req, kFinThreads, smem, s, placed, sl, big, deferred,
+               p.cap_keys, d_out, ctrl, h_ctrl_dev));
     }
     ran[GGKS_PASS_FINISH] = true;
   }
   e = le != cudaSuccess ? le : cudaGetLastError();
   if (e != cudaSuccess) return from_cuda(e);
-  if (want_host && d_out_user)
-    e = cudaMemcpyAsync(ctx.pin, d_out, (size_t)num_req * sizeof(InT), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  auto pull = [&]() -> cudaError_t {  // results to host memory, and the synchronisation
+    cudaError_t r = cudaSuccess;
+    if (want_host && d_out_user)
+      r = cudaMemcpyAsync(ctx.pin, d_out, (size_t)num_req * sizeof(InT), cudaMemcpyDeviceToHost, s);
+    return r == cudaSuccess ? cudaStreamSynchronize(s) : r;
+  };
+  e = pull();
   if (e != cudaSuccess) return from_cuda(e);
   collect_pass_times(ctx, ran);
   const uint32_t status = *reinterpret_cast<const volatile uint32_t *>(&h_ctrl->status);
   if (status & ST_FATAL) return (status & ST_TIMEOUT) ? GGKS_TIMEOUT : GGKS_INTERNAL;
-  // a miss, or a slot that needs a recursive level: the pipeline answers (the
-  // streaming pass has written the device copy of an ingested vector)
-  *missed = (status & (ST_TOPK_MISS | ST_DEFERRED)) != 0;
+  // a miss: the pipeline answers (the streaming pass has written the device copy of an
+  // ingested vector)
+  const uint32_t D = (status & ST_DEFERRED) ? h_ctrl->deferred_count : 0u;
+  *missed = (status & ST_TOPK_MISS) != 0 ||
+            (src.topk && (D > kWinMaxDefer ||
+                          (D && std::min(h_big[0].size, num_req - h_big[0].above) > kWinMaxAgain)));
   if (*missed) return GGKS_OK;
+  if (D) {
+    // large bins of distinct keys: select from each again, on its keys
+    int st = GGKS_OK;
+    Context *ch = child_of(ctx, &st);
+    if (!ch) return st;
+    if (src.topk) {
+      // a bin's largest keys are the outputs from the number of keys above it on (many
+      // results: through the arena, see kPinOut)
+      for (uint32_t i = 0; i < D; ++i) {
+        const WinDefer &d = h_big[i];
+        const uint32_t m = std::min(d.size, num_req - d.above);
+        InT *o = (d_out_user ? d_out : reinterpret_cast<InT *>(A + p.out)) + d.above;
+        ReqSource cs;
+        cs.topk = true;
+        ctx.stats.recursions++;
+        st = select<K, InT>(*ch, placed + d.off, d.size, cs, m, o, nullptr, s, nullptr);
+        if (st != GGKS_OK) return st;
+        if (!d_out_user)
+          e = cudaMemcpyAsync(ctx.pin + (size_t)d.above * sizeof(InT), o, (size_t)m * sizeof(InT),
+                              cudaMemcpyDeviceToHost, s);
+        if (e != cudaSuccess) return from_cuda(e);
+      }
+    } else {
+      // the requests of one bin together, in the call's pinned requests (all read by now)
+      std::sort(h_big, h_big + D, [](const WinDefer &a, const WinDefer &b) { return a.off < b.off; });
+      Req *hr = reinterpret_cast<Req *>(ctx.pin + out_span + 256);
+      const Req *dr = reinterpret_cast<const Req *>(ctx.pin_dev + out_span + 256);
+      for (uint32_t i = 0; i < D; ++i) hr[i] = {h_big[i].rank, h_big[i].slot};
+      for (uint32_t i = 0, j; i < D; i = j) {
+        for (j = i + 1; j < D && h_big[j].off == h_big[i].off; ++j) {
+        }
+        ReqSource cs;
+        cs.d_reqs = dr + i;
+        ctx.stats.recursions++;
+        st = select<K, InT>(*ch, placed + h_big[i].off, h_big[i].size, cs, j - i, d_out, nullptr, s,
+                            nullptr);
+        if (st != GGKS_OK) return st;
+      }
+    }
+    e = pull();
+    if (e != cudaSuccess) return from_cuda(e);
+  }
   ctx.stats.spec_calls++;
   ctx.stats.spec_ctas += p.G;
   if (want_host) *host_results = reinterpret_cast<const InT *>(ctx.pin);

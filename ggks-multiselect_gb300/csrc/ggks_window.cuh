@@ -16,17 +16,16 @@
 //             requested ranks, and the candidates of those bins go to the
 //             places of their ranks (bin by bin, unordered inside a bin);
 //   k_wsort   (top-k) a warp per bin sorts and writes its values, descending; or
-//   k_finish  (requests) a CTA per request selects inside its bin.
+//   k_wfinish (requests) a CTA per request selects inside its bin;
+//   large bins hold copies of one key, or the host selects from their keys again.
 // No second read of the vector, no splitter table, no bucket atomics per key:
 // the pass does two or three compares per key and is bound by HBM, where the
 // speculating histogram pass (ggks_device.cuh) did a table lookup, a shared
 // atomic and a vote: 50 M floats, their median: 81 us, now 43; the call 132 ->
 // 77 us.
 // Correctness never rests on the prediction: k_wplace checks that the candidates
-// were all kept and hold every requested rank, and k_wsort that a bin too large
-// to sort holds copies of one key; else the call reports ST_TOPK_MISS (or a slot
-// that k_finish would leave to a recursive level) and the caller runs the
-// pipeline.
+// were all kept, fill their bins exactly and hold every requested rank; else the
+// call reports ST_TOPK_MISS and the caller runs the pipeline.
 #pragma once
 
 #include "ggks_front.cuh"
@@ -38,6 +37,18 @@ constexpr int kWinBinBits = 13;
 constexpr uint32_t kWinBins = 1u << kWinBinBits;
 constexpr uint32_t kWinCol = 16;    // keys of one lane's column (k_wfilter)
 constexpr uint32_t kWinSort = 256;  // keys of a bin that a warp sorts (k_wsort)
+// Large bins of requests: more keys than kWinFlat may be copies of one key (a value's,
+// in few-valued vectors), which needs no selection: 256 values in 2^26 floats, their
+// median 287 us a call by selecting from the copies, now 108.  More than win_slot_max
+// distinct ones (a gap in the distribution puts all candidates on one side into one
+// bin) take one CTA longer than a recursive level, about 50 us: 2^26 floats in
+// +-[1, 2), median: 505 us a call by one CTA and then the pipeline, now 155; 169 in
+// the pipeline.
+constexpr uint32_t kWinFlat = 2048;
+template <class K>
+__host__ __device__ constexpr uint32_t win_slot_max() {
+  return (256u << 10) / (uint32_t)sizeof(K);
+}
 static_assert(1024 * kWinCol >= 2 * kSliceBuf, "the samples around the ends fit the columns");
 
 // The window's bins: [copies of key_lo] [inner equal-width bins] [copies of key_hi].
@@ -325,34 +336,49 @@ __global__ void __launch_bounds__(1024, 1)
   }
 }
 
-// The slots that k_finish reads, one per request (k_wplace).
+// Whether a large bin holds one key: first[b] is one of its keys (big_first), mixed[b]
+// is set when another one is met (also by the largest 8-byte key, which first[]
+// cannot tell from no key).  Zero on entry.
+struct BigBins {
+  unsigned long long *first;
+  uint32_t *mixed;
+};
+__device__ __forceinline__ unsigned long long big_first(uint32_t k) { return (1ull << 32) | k; }
+__device__ __forceinline__ unsigned long long big_first(uint64_t k) { return ~k; }
+template <class K>
+__device__ __forceinline__ K big_key(unsigned long long f) {
+  return sizeof(K) == 4 ? (K)f : (K)~f;
+}
+
+// The slots that k_wfinish reads, one per request (k_wplace).
 template <class K>
 struct WinSlots {
   uint64_t *seg_off;
-  uint32_t *seg_size, *kstart, *kcnt;
+  uint32_t *seg_size, *bin;
   K *seg_lo, *seg_hi;
   Req *klist;
 };
 
 // Bins that hold requested ranks: their candidates go to placed[prefix of the bin
 // ...), which holds the keys of local ranks (rank - below) prefix ... .  kk > 0:
-// a top-k (every bin from the one of the kk-th largest up; bins of more than
-// kWinSort keys are not placed, the complement of their smallest key and their
-// largest key go to big_lo_inv / big_hi); else num_req requests, whose slots CTA
-// 0 writes.  cur, big_lo_inv, big_hi: kWinBins entries, zero on entry; pre_g: the
+// a top-k (every bin from the one of the kk-th largest up); else num_req requests,
+// whose slots CTA 0 writes.  Large bins (of more than kWinSort or kWinFlat keys): also
+// whether they hold one key, in big.  cur: kWinBins entries, zero on entry; pre_g: the
 // bins' prefix, written by CTA 0 for a top-k.
 template <class K>
 __global__ void __launch_bounds__(1024, 1)
     k_wplace(const K *arr, uint64_t cap, uint64_t n, uint32_t kk, bool lo_open,
              bool hi_open, const Req *reqs, uint32_t num_req, WinCtl<K> *wc,
              const uint32_t *bins_g, uint32_t *cur, uint32_t *__restrict__ pre_g,
-             K *__restrict__ placed, uint64_t placed_cap, unsigned long long *big_lo_inv,
-             unsigned long long *big_hi, WinSlots<K> sl, Ctrl *ctrl) {
+             K *__restrict__ placed, uint64_t placed_cap, BigBins big_bins, WinSlots<K> sl,
+             Ctrl *ctrl) {
   pdl_start();
+  extern __shared__ uint4 smem_raw[];
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(smem_raw);  // the CTA's keys per bin, then their place
   __shared__ __align__(16) uint32_t pre[kWinBins];
-  __shared__ uint32_t need[kWinBins / 32];
+  __shared__ uint32_t need[kWinBins / 32], mix[kWinBins / 32];  // needed bins; bins of several keys
   __shared__ uint32_t s_scan[32];
-  __shared__ bool s_miss;
+  __shared__ bool s_miss, s_any;
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   const uint32_t C = wc->len;
   const WinMap<K> map = wc->map(lo_open, hi_open);
@@ -365,8 +391,9 @@ __global__ void __launch_bounds__(1024, 1)
     c[4 * q] = v.x; c[4 * q + 1] = v.y; c[4 * q + 2] = v.z; c[4 * q + 3] = v.w;
     sum += v.x + v.y + v.z + v.w;
   }
-  if (tid < kWinBins / 32) need[tid] = 0;
-  if (tid == 0) s_miss = false;
+  if (tid < kWinBins / 32) need[tid] = mix[tid] = 0;
+  if (tid == 0) s_miss = s_any = false;
+  fill_words(cnt, kWinBins, 0u);
   uint32_t total;
   uint32_t run = block_excl_scan(sum, s_scan, &total);
   bool big = false;
@@ -399,7 +426,11 @@ __global__ void __launch_bounds__(1024, 1)
   if (!bad && kk) {
     first = bin_at(total - kk);
 #pragma unroll
-    for (uint32_t q = 0; q < kPer; ++q) big |= tid * kPer + q >= first && c[q] > kWinSort;
+    for (uint32_t q = 0; q < kPer; ++q) {
+      const uint32_t b = tid * kPer + q;
+      big |= b >= first && c[q] > kWinSort;
+      if (b >= first && c[q] && !map.one_key(b)) s_any = true;
+    }
   }
   big = __syncthreads_or(big);
   if (!bad && !kk && tid < num_req) {
@@ -409,7 +440,10 @@ __global__ void __launch_bounds__(1024, 1)
     } else {
       const uint32_t r = (uint32_t)(q.rank - below), b = bin_at(r);
       const bool one = map.one_key(b);
-      if (!one) atomicOr(&need[b >> 5], 1u << (b & 31));
+      if (!one) {
+        atomicOr(&need[b >> 5], 1u << (b & 31));
+        s_any = true;
+      }
       if (blockIdx.x == 0) {
         const uint32_t j = b - map.has_lo;  // among the inner bins
         sl.seg_off[tid] = pre[b] - off;
@@ -417,8 +451,7 @@ __global__ void __launch_bounds__(1024, 1)
         // an end bin also holds the keys beyond the sampled extremes
         sl.seg_lo[tid] = one ? map.key(b) : b == 0 && lo_open ? K(0) : map.lo + ((K)j << map.shift);
         sl.seg_hi[tid] = j + 1 >= map.inner ? KeyMax<K>::v : map.lo + (((K)j + 1) << map.shift) - K(1);
-        sl.kstart[tid] = tid;
-        sl.kcnt[tid] = 1;
+        sl.bin[tid] = b;
         Req e;
         e.rank = r - pre[b];
         e.out = q.out;
@@ -440,67 +473,139 @@ __global__ void __launch_bounds__(1024, 1)
     if (kk)
       for (uint32_t b = tid; b < kWinBins; b += blockDim.x) pre_g[b] = pre[b];
   }
-  if (miss) return;
-  // whole warps over the candidates, four loads in flight per lane; a bin that meets
-  // more keys than it counted keeps its places and the call is a miss
+  if (miss || !s_any) return;
+  // The candidates of needed bins: a key's place among the CTA's in its bin by one
+  // shared atomic, the CTA's places in the bin by one global atomic per bin and round.
+  // (Few-valued vectors put hundreds of thousands of keys into a handful of bins;
+  // warps that took their places with an atomic each queued on them: clustered k's
+  // of 256 values in 2^26 floats 171 us a call, now 130.)  A bin that meets more keys
+  // than it counted keeps its places and the call is a miss.
   bool over = false;
-  constexpr uint32_t U = 4;
-  const uint32_t step = gridDim.x * 1024 * U;
-  for (uint32_t i0 = blockIdx.x * 1024 * U + (tid >> 5) * 32 * U; i0 < C; i0 += step) {
+  constexpr uint32_t U = 8;
+  for (uint32_t i0 = blockIdx.x * 1024 * U; i0 < C; i0 += gridDim.x * 1024 * U) {
     K k[U];
 #pragma unroll
     for (uint32_t u = 0; u < U; ++u) {
-      const uint32_t i = i0 + 32 * u + lane;
+      const uint32_t i = i0 + 1024 * u + tid;
       k[u] = i < C ? __ldcg(arr + i) : K(0);
     }
+    uint32_t at[U];  // place in the CTA's part of the bin; kNoSlot: not needed
 #pragma unroll
     for (uint32_t u = 0; u < U; ++u) {
-      const bool valid = i0 + 32 * u + lane < C;
       const uint32_t b = map.bin(k[u]);
-      const bool want =
-          valid && (kk ? b >= first && !map.one_key(b) : ((need[b >> 5] >> (b & 31)) & 1u) != 0u);
-      const uint32_t m = __ballot_sync(0xffffffffu, want);
-      if (!m) continue;
-      // lanes of one bin take one atomic
-      const uint32_t peers = __match_any_sync(0xffffffffu, want ? b : 0xFFFFFFFFu);
-      const int leader = __ffs(peers) - 1;
-      const bool place = want && !(kk && count_of(b) > kWinSort);
-      uint32_t base = 0;
-      if (place && (int)lane == leader) base = atomicAdd(&cur[b], (uint32_t)__popc(peers));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (place) {
-        const uint32_t at = base + __popc(peers & ((1u << lane) - 1u));
-        if (at < count_of(b))
-          placed[pre[b] - off + at] = k[u];
-        else
-          over = true;
-      } else if (want) {
-        // a large bin: does it hold one key?  (the complement of the smallest)
-        if ((unsigned long long)~(uint64_t)k[u] > __ldcg(big_lo_inv + b))
-          atomicMax(big_lo_inv + b, (unsigned long long)~(uint64_t)k[u]);
-        if ((unsigned long long)k[u] > __ldcg(big_hi + b))
-          atomicMax(big_hi + b, (unsigned long long)k[u]);
+      const bool want = i0 + 1024 * u + tid < C &&
+                        (kk ? b >= first && !map.one_key(b) : ((need[b >> 5] >> (b & 31)) & 1u) != 0u);
+      at[u] = want ? atomicAdd(&cnt[b], 1u) : kNoSlot;
+      // the first key of a large bin, taken by one lane for all of a bin's lanes
+      const bool large = want && count_of(b) > (kk ? kWinSort : kWinFlat);
+      if (!__any_sync(0xffffffffu, large)) continue;
+      unsigned long long one = large ? __ldcg(big_bins.first + b) : 1ull;
+      const unsigned long long mine = big_first(k[u]);
+      for (uint32_t round = 0; round < 32; ++round) {  // (each settles a lane at least)
+        const uint32_t none = __ballot_sync(0xffffffffu, one == 0);
+        if (!none) break;
+        const int leader = __ffs(none) - 1;
+        unsigned long long got = 0;
+        if ((int)lane == leader) {
+          got = atomicCAS(big_bins.first + b, 0ull, mine);
+          got = got ? got : mine ? mine : ~0ull;  // (the largest 8-byte key: no first key)
+        }
+        got = __shfl_sync(0xffffffffu, got, leader);
+        const uint32_t bin = __shfl_sync(0xffffffffu, b, leader);
+        if (one == 0 && b == bin) one = got;
       }
+      const uint32_t bit = 1u << (b & 31);
+      if (large && one != mine && !(mix[b >> 5] & bit)) atomicOr(&mix[b >> 5], bit);
+    }
+    __syncthreads();
+    for (uint32_t b = tid; b < nbins; b += 1024) {
+      if (cnt[b]) cnt[b] = atomicAdd(&cur[b], cnt[b]);
+      if (mix[b >> 5] & (1u << (b & 31))) big_bins.mixed[b] = 1u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      if (at[u] == kNoSlot) continue;
+      const uint32_t b = map.bin(k[u]), p = cnt[b] + at[u];
+      if (p < count_of(b))
+        placed[pre[b] - off + p] = k[u];
+      else
+        over = true;
+    }
+    if (i0 + gridDim.x * 1024 * U < C) {  // another round
+      __syncthreads();
+      fill_words(cnt, kWinBins, 0u);
+      __syncthreads();
     }
   }
   if (over) atomicOr(&ctrl->status, ST_TOPK_MISS);
 }
 
+// A large bin of distinct keys, left to a recursive level: its places, and for a
+// request its slot and rank, for a top-k the number of keys above the bin.
+struct WinDefer {
+  uint64_t off;
+  uint32_t size, slot, rank, above;
+};
+// (one thread calls this; list: host memory, the first `room` are kept)
+__device__ __forceinline__ void win_defer(Ctrl *ctrl, WinDefer *list, uint32_t room,
+                                          const WinDefer &d) {
+  const uint32_t at = atomicAdd(&ctrl->deferred_count, 1u);
+  if (at < room) list[at] = d;
+  atomicOr(&ctrl->status, ST_DEFERRED);
+}
+
+// The last CTA leaves the call's status and its large bins' number in host memory.
+// Every thread calls this last.
+__device__ __forceinline__ void win_leave(Ctrl *ctrl, Ctrl *host_ctrl) {
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(&ctrl->fin_done, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  host_ctrl->deferred_count = __ldcg(&ctrl->deferred_count);
+  host_ctrl->status = __ldcg(&ctrl->status);
+}
+
+// Requests' values from their bins, a CTA per request.  Large bins of one key need no
+// selection, those of more than win_slot_max distinct ones go to a recursive level.
+template <class K, class OutT>
+__global__ void __launch_bounds__(kFinThreads)
+    k_wfinish(const K *placed, WinSlots<K> sl, BigBins big_bins, WinDefer *__restrict__ deferred,
+              uint32_t bcap, OutT *__restrict__ out, Ctrl *ctrl, Ctrl *__restrict__ host_ctrl) {
+  pdl_start();
+  extern __shared__ uint4 smem_raw[];
+  const uint32_t i = blockIdx.x;
+  // (only ST_DEFERRED is set meanwhile)
+  if (!(ctrl->status & (ST_FATAL | ST_TOPK_MISS))) {
+    const uint32_t size = sl.seg_size[i], b = sl.bin[i];
+    const bool done =
+        size > kWinFlat && !big_bins.mixed[b]
+            ? finish_slot<K, OutT>(placed, 0u, big_key<K>(big_bins.first[b]), K(0), sl.klist + i, 1u,
+                                   bcap, reinterpret_cast<uint32_t *>(smem_raw), out)
+            : size <= win_slot_max<K>() &&
+                  finish_slot<K, OutT>(placed + sl.seg_off[i], size, sl.seg_lo[i], sl.seg_hi[i],
+                                       sl.klist + i, 1u, bcap,
+                                       reinterpret_cast<uint32_t *>(smem_raw), out);
+    if (!done && threadIdx.x == 0)
+      win_defer(ctrl, deferred, gridDim.x, {sl.seg_off[i], size, i, sl.klist[i].rank, 0u});
+  }
+  win_leave(ctrl, host_ctrl);
+}
+
 // A top-k's values from the placed bins: a warp per bin from wc->first up, the
-// values in descending order to out[0 .. kk).  The last CTA leaves the call's
-// status in *host_status.
+// values in descending order to out[0 .. kk).  A large bin of distinct keys is left
+// to a recursive level.
 constexpr uint32_t kWinSortThreads = 256;
 template <class K, class OutT>
 __global__ void __launch_bounds__(kWinSortThreads)
     k_wsort(const K *placed, const WinCtl<K> *wc, const uint32_t *bins_g,
-            const uint32_t *pre_g, const unsigned long long *big_lo_inv,
-            const unsigned long long *big_hi, uint32_t kk, OutT *__restrict__ out,
-            Ctrl *ctrl, uint32_t *host_status) {
+            const uint32_t *pre_g, BigBins big_bins, uint32_t kk, WinDefer *__restrict__ deferred,
+            uint32_t room, OutT *__restrict__ out, Ctrl *ctrl, Ctrl *__restrict__ host_ctrl) {
   pdl_start();
-  __shared__ uint32_t s_last;
   const uint32_t tid = threadIdx.x, lane = tid & 31;
-  // one value for the whole warp: other CTAs set ST_TOPK_MISS meanwhile, and the
-  // lanes meet in shuffles below
+  // (one value for the whole warp, whose lanes meet in shuffles below, whatever other
+  // CTAs set meanwhile)
   const uint32_t status = __shfl_sync(0xffffffffu, ctrl->status, 0);
   if (!(status & (ST_FATAL | ST_TOPK_MISS))) {
     const uint32_t C = wc->total, first = wc->first;
@@ -534,8 +639,8 @@ __global__ void __launch_bounds__(kWinSortThreads)
         sorted(std::integral_constant<int, 2>{}, p0, c);
       else if (c <= kWinSort)
         sorted(std::integral_constant<int, (int)(kWinSort / 32)>{}, p0, c);
-      else if (lane == 0 && ~big_lo_inv[b] != big_hi[b])
-        atomicOr(&ctrl->status, ST_TOPK_MISS);  // too many distinct keys: the pipeline
+      else if (lane == 0 && big_bins.mixed[b])
+        win_defer(ctrl, deferred, room, {p0 - off, c, b, 0u, C - p0 - c});
     }
     // copies of one key: every thread writes its share of the outputs in large bins
     if (wc->big) {
@@ -544,18 +649,12 @@ __global__ void __launch_bounds__(kWinSortThreads)
         uint32_t b = 0;
         for (uint32_t step = kWinBins / 2; step; step >>= 1)
           if (b + step < nbins && pre_g[b + step] <= p) b += step;
-        if (bins_g[b] > kWinSort)
-          out[i] = Traits<OutT>::value(map.one_key(b) ? map.key(b) : (K)big_hi[b]);
+        if (bins_g[b] > kWinSort && (map.one_key(b) || !big_bins.mixed[b]))
+          out[i] = Traits<OutT>::value(map.one_key(b) ? map.key(b) : big_key<K>(big_bins.first[b]));
       }
     }
   }
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    s_last = atomicAdd(&ctrl->fin_done, 1u) == gridDim.x - 1 ? 1u : 0u;
-    __threadfence();
-    if (s_last) *host_status = __ldcg(&ctrl->status);
-  }
+  win_leave(ctrl, host_ctrl);
 }
 
 }  // namespace ggks

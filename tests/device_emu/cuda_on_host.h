@@ -144,7 +144,7 @@ inline void fiber_main() {
 inline uint4 *dynamic_smem() { return reinterpret_cast<uint4 *>(engine().smem.data()); }
 
 // Runs body once per thread of every block of the grid; false when threads wait
-// for others that never come.
+// for others that never come, or without end.
 inline bool launch(unsigned grid, unsigned block, size_t smem, const std::function<void()> &body) {
   Engine &e = engine();
   gridDim = dim3(grid);
@@ -171,13 +171,15 @@ inline bool launch(unsigned grid, unsigned block, size_t smem, const std::functi
       makecontext(&e.fiber[t], fiber_main, 0);
     }
     bool ran = true;
+    uint64_t left = 1ull << 26;  // resumptions: a loop that never ends fails the launch
     while (e.live && ran) {
       ran = false;
       for (unsigned t = 0; t < block; ++t) {
         if (e.done[t] || (e.wait_at[t] && *e.wait_at[t] == e.wait_old[t])) continue;
         set_thread(t);
         swapcontext(&e.sched, &e.fiber[t]);
-        ran = true;
+        ran = --left != 0;
+        if (!ran) return false;
       }
     }
     if (e.live) return false;

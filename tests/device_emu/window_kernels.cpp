@@ -57,8 +57,8 @@ int filter(const T *x, uint64_t n, uint32_t r0, uint32_t r1, bool lo_open, bool 
   return ok ? 0 : 1;
 }
 
-// k_wplace over the candidates arr[0 .. len) and the given bin counts, and for a
-// top-k (kk > 0, out given) k_wsort.
+// k_wplace over the candidates arr[0 .. len) and the given bin counts, and, with out
+// given, k_wsort (a top-k, kk > 0) or k_wfinish.
 template <class K>
 int place(const K *arr, uint32_t len, uint64_t n, uint32_t below, K lo, uint32_t shift,
           uint32_t nbins, const uint32_t *bins, uint32_t kk, const uint32_t *ranks,
@@ -72,29 +72,37 @@ int place(const K *arr, uint32_t len, uint64_t n, uint32_t below, K lo, uint32_t
   wc.shift = shift;
   wc.inner = nbins;
   std::vector<uint32_t> cur(kWinBins, 0), pre(kWinBins, 0);
-  std::vector<unsigned long long> big_lo(kWinBins, 0), big_hi(kWinBins, 0);
+  std::vector<unsigned long long> first(kWinBins, 0);
+  std::vector<uint32_t> mixed(kWinBins, 0);
+  const BigBins big{first.data(), mixed.data()};
   const uint32_t slots = num_req ? num_req : 1;
   std::vector<uint64_t> seg_off(slots);
-  std::vector<uint32_t> seg_size(slots), kstart(slots), kcnt(slots);
+  std::vector<uint32_t> seg_size(slots), bin(slots);
+  std::vector<WinDefer> deferred(kWinBins);
   std::vector<K> seg_lo(slots), seg_hi(slots);
   std::vector<Req> klist(slots), reqs(slots);
   for (uint32_t i = 0; i < num_req; ++i) {
     reqs[i].rank = ranks[i];
     reqs[i].out = i;
   }
-  WinSlots<K> sl{seg_off.data(), seg_size.data(), kstart.data(), kcnt.data(),
+  WinSlots<K> sl{seg_off.data(), seg_size.data(), bin.data(),
                  seg_lo.data(),  seg_hi.data(),   klist.data()};
-  Ctrl ctrl{};
-  bool ok = emu::launch(grid, 1024, 0, [&] {
+  Ctrl ctrl{}, host_ctrl{};
+  bool ok = emu::launch(grid, 1024, kWinBins * 4, [&] {
     k_wplace<K>(arr, len, n, kk, false, kk != 0, reqs.data(), num_req, &wc, bins, cur.data(),
-                pre.data(), placed, placed_cap, big_lo.data(), big_hi.data(), sl, &ctrl);
+                pre.data(), placed, placed_cap, big, sl, &ctrl);
   });
-  *status = ctrl.status;
-  if (out)
+  if (out && kk)
     ok = ok && emu::launch(grid, kWinSortThreads, 0, [&] {
-           k_wsort<K, K>(placed, &wc, bins, pre.data(), big_lo.data(), big_hi.data(), kk, out, &ctrl,
-                         status);
+           k_wsort<K, K>(placed, &wc, bins, pre.data(), big, kk,
+                         deferred.data(), 4u, out, &ctrl, &host_ctrl);
          });
+  else if (out)
+    ok = ok && emu::launch(num_req, kFinThreads, finish_smem_for<K>(4096), [&] {
+           k_wfinish<K, K>(placed, sl, big, deferred.data(), 4096u, out,
+                           &ctrl, &host_ctrl);
+         });
+  *status = out ? host_ctrl.status : ctrl.status;
   return ok ? 0 : 1;
 }
 

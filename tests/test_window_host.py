@@ -13,7 +13,7 @@ sys.path.insert(0, os.path.join(os.path.dirname(os.path.abspath(__file__)), "dev
 import build_emu  # noqa: E402
 
 BINS = 8192
-MISS = 32  # ST_TOPK_MISS
+DEFERRED, MISS = 2, 32  # ST_DEFERRED, ST_TOPK_MISS
 EMPTY = 0xABCDEF01
 U32 = ctypes.POINTER(ctypes.c_uint32)
 
@@ -113,7 +113,7 @@ def test_filter(emu, dtype, dist, ends):
 def place(emu, arr, n, below, lo, shift, nbins, bins, kk, ranks, grid, sort=False):
     guard = 64
     placed = np.full(arr.size + guard, EMPTY, np.uint32)
-    out = np.zeros(max(kk, 1), np.uint32)
+    out = np.full(max(kk, ranks.size), EMPTY, np.uint32)
     status = ctypes.c_uint32()
     rc = emu.emu_place_u32(
         arr.ctypes.data_as(U32), arr.size, ctypes.c_uint64(n), below, lo, shift, nbins,
@@ -128,7 +128,7 @@ def place(emu, arr, n, below, lo, shift, nbins, bins, kk, ranks, grid, sort=Fals
 @pytest.mark.parametrize("big", ["none", "copies", "distinct"])
 def test_topk_bins(emu, big):
     """Bins that a warp sorts, large bins of one key and large bins of many keys, which
-    the first CTA reports while the others may still read the status."""
+    the first CTA leaves to a recursive level while others may still read the status."""
     r = np.random.default_rng(1)
     n, lo, shift, nbins, kk = 100_000, 5000, 6, 300, 3000
     arr = (lo + r.integers(0, nbins << shift, 4000)).astype(np.uint32)
@@ -140,10 +140,31 @@ def test_topk_bins(emu, big):
     bins = np.bincount((arr - lo) >> shift, minlength=BINS).astype(np.uint32)
     _, out, status = place(emu, arr, n, 0, lo, shift, nbins, bins, kk, np.zeros(0, np.uint32), 3,
                            sort=True)
-    if big == "distinct":
-        assert status & MISS
-    else:
-        assert status == 0 and np.array_equal(out, np.sort(arr)[::-1][:kk])
+    want = np.sort(arr)[::-1][:kk]
+    assert status == (DEFERRED if big == "distinct" else 0)
+    later = np.isin((want - lo) >> shift, at) if big == "distinct" else np.zeros(kk, bool)
+    assert np.array_equal(out[~later], want[~later]) and np.all(out[later] == EMPTY)
+
+
+@pytest.mark.parametrize("big", ["none", "copies", "distinct"])
+def test_request_bins(emu, big):
+    r = np.random.default_rng(2)
+    n, lo, shift, nbins, below = 1_000_000, 5000, 20, 50, 400_000
+    arr = (lo + r.integers(0, nbins << shift, 6000)).astype(np.uint32)
+    b = 17
+    if big != "none":
+        extra = lo + (b << shift) + (r.integers(0, 1 << shift, 66_000) if big == "distinct" else 7)
+        arr = np.concatenate([arr[(arr - lo) >> shift != b], np.broadcast_to(extra, 66_000)])
+        arr = r.permutation(arr.astype(np.uint32))
+    s = np.sort(arr)
+    bins = np.bincount((arr - lo) >> shift, minlength=BINS).astype(np.uint32)
+    local = np.array([0, 3000, 3001, arr.size // 2, arr.size - 1, 3000])
+    _, out, status = place(emu, arr, n, below, lo, shift, nbins, bins, 0,
+                           (local + below).astype(np.uint32), 2, sort=True)
+    want = s[local]
+    assert status == (DEFERRED if big == "distinct" else 0)
+    later = (want - lo) >> shift == b if big == "distinct" else np.zeros(local.size, bool)
+    assert np.array_equal(out[~later], want[~later]) and np.all(out[later] == EMPTY)
 
 
 @pytest.mark.parametrize("kk", [0, 700])
