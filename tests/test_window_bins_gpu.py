@@ -88,3 +88,20 @@ def test_topk_over_a_gap(g, dtype, far):
         ks = np.array([far, far + 1, far + 9000], dtype=np.uint32)
         assert_same(g.multiselect_ptr(d.ptr, n, dtype, ks, ctx=ctx), desc[ks - 1], str(ks))
         ctx.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("dist", ["normal", "cauchy"])
+def test_topk_tail(g, dtype, dist):
+    """The few hundred keys past the sample's largest spread over the open end's bins."""
+    n = 40_000_003
+    r = np.random.default_rng(14)
+    x = (100 + r.standard_normal(n) if dist == "normal" else r.standard_cauchy(n)).astype(dtype)
+    top = np.sort(np.partition(x, n - 30_000)[-30_000:])[::-1]
+    d = DeviceArray(x)
+    ctx = g.Context(0)
+    for K in (4500, 9000, 20_000, 30_000):
+        assert_same(g.topk_ptr(d.ptr, n, dtype, K, ctx=ctx), top[:K], f"{dist} top-{K}")
+    st = ctx.stats()
+    assert st["topk_misses"] == 0 and st["recursions"] == 0
+    ctx.close()
