@@ -2861,11 +2861,25 @@ __device__ bool finish_slot(const K *__restrict__ src, uint32_t size, K lo, K hi
     return true;
   }
   // a needed bin that does not fit, or so many needed keys that the rounds
-  // would read the segment more than kFinMaxRounds times: the caller
-  // re-selects this slot on its keys
+  // would read the segment more than kFinMaxRounds times: a segment that fits the
+  // buffer is sorted whole, else the caller re-selects this slot on its keys.
+  // (The bucket around zero of a vector of doubles spans a thousand binades, its keys
+  // the last few: 65536 k's of 2^24 normal doubles re-selected 1864 keys, 1159 us a
+  // call, now 1030.)
   if (s_maxneed > tcap || V > kFinMaxRounds * bcap) {
     __syncthreads();
-    return false;
+    if (size > bcap) return false;
+    uint32_t P = 64;
+    while (P < size) P <<= 1;  // (bcap is a power of two)
+    for (uint32_t i = tid; i < P; i += blockDim.x) B[i] = i < size ? __ldcg(src + i) : KeyMax<K>::v;
+    __syncthreads();
+    bitonic_sort_smem(B, P);
+    for (uint32_t j = tid; j < m; j += blockDim.x) {
+      const Req e = req_at(j);
+      out[e.out] = Traits<OutT>::value(B[e.rank]);
+    }
+    __syncthreads();
+    return true;
   }
   (void)fits;
 
