@@ -96,6 +96,12 @@ constexpr uint32_t kPinOut = 4096;
 // n / 512 buckets, 8192 to kMaxNb, in the table: a CTA writes as many counts
 // (n / 32: 55 us for 52 at 2^21 floats, 60 for 57 at 2^22, 70 for 68 at 10 M); the
 // rows have room for n / 32, as tables that track single keys and dense ones need.
+// Half as many, down to 8192, where there are more requests than buckets (above 2^25
+// elements: n / 2^25 times as many, as survivors then cost more than slots): nearly
+// every bucket holds one, whatever their number, and the plan and the finisher work
+// by the slot (65536 k's of 2^24 floats / doubles 827 / 1041 us a call with 32768
+// buckets, 479 / 721 with 8192; 20000 k's of 2^23 doubles 408 and 344 with 16384 and
+// 8192; but 33000 k's of 2^27 doubles 3546 with 32768, 4292 with 8192).
 template <class InT, class OutT>
 static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req, uint32_t cta_keys = 16384) {
   using K = typename Traits<InT>::K;
@@ -110,6 +116,8 @@ static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req, uint32_t
   };
   p.nb_max = buckets(n / 32);
   p.nb_want = buckets(n / 512);
+  const uint64_t many = std::max<uint64_t>(1, n >> 25);
+  while (p.nb_want > 8192 && num_req >= p.nb_want * many) p.nb_want /= 2;
   const uint64_t g = (n + cta_keys - 1) / cta_keys;
   p.G = (uint32_t)(g < 1 ? 1 : (g > (uint64_t)ctx.sm_count ? ctx.sm_count : g));
   p.scan_tiles = (p.nb_max + kScanTile - 1) / kScanTile;
