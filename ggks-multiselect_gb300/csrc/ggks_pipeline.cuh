@@ -88,7 +88,8 @@ static_assert(sizeof(Ctrl) <= 256 && sizeof(Ctrl) % 4 == 0, "the control block's
 // 10 M floats, 257 k's: 96 -> 91 us.)
 constexpr uint32_t kPinOut = 4096;
 
-// The streaming passes' grid and buckets.  A CTA per 16384 elements up to one per
+// The streaming passes' grid and buckets, and the arena's layout (rows: with the
+// histogram's rows, up to 60 MB, which only the pipeline reads).  A CTA per 16384 elements up to one per
 // SM: below 10 M elements a pass is its CTAs' fixed work and one or two tiles
 // each, so more of them end sooner (65536 elements a CTA: 2^21 floats, 101 k's 63 us
 // a call, now 52; 2^21 doubles 75 -> 60; 2^22 floats 63 -> 57).  A top-k that takes
@@ -103,7 +104,8 @@ constexpr uint32_t kPinOut = 4096;
 // buckets, 479 / 721 with 8192; 20000 k's of 2^23 doubles 408 and 344 with 16384 and
 // 8192; but 33000 k's of 2^27 doubles 3546 with 32768, 4292 with 8192).
 template <class InT, class OutT>
-static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req, uint32_t cta_keys = 16384) {
+static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req, uint32_t cta_keys = 16384,
+                      bool rows = true) {
   using K = typename Traits<InT>::K;
   Plan p;
   p.n = n;
@@ -168,7 +170,7 @@ static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req, uint32_t
   p.wpre = o;
   o = align_up(o + kWinBins * sizeof(uint32_t), A);
   p.partials = o;
-  o = align_up(o + (size_t)p.G * p.nb_max * sizeof(uint32_t), A);
+  o = align_up(o + (rows ? (size_t)p.G * p.nb_max * sizeof(uint32_t) : 0), A);
   auto arr = [&](size_t &off, size_t elems, size_t esz) {
     off = o;
     o = align_up(o + elems * esz, A);
@@ -201,7 +203,7 @@ static Plan make_plan(const Context &ctx, uint64_t n, uint32_t num_req, uint32_t
   arr(p.cand_tab, (size_t)p.G * kCandWarps * kCandChunksPerWarp, 4);
   // single-key tracking of tables whose keys repeat often: each CTA's key per
   // bucket, and per bucket whether the vector holds one key there and which
-  arr(p.reps, (size_t)p.G * p.nb_max, sizeof(K));
+  arr(p.reps, rows ? (size_t)p.G * p.nb_max : 0, sizeof(K));
   arr(p.bsingle, p.nb_max, 4);
   arr(p.bkey, p.nb_max, sizeof(K));
   p.total = o;
@@ -386,7 +388,7 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
                           bool *missed) {
   using Kt = typename Traits<InT>::K;
   *missed = false;
-  const Plan p = make_plan<InT, InT>(ctx, n, K);
+  const Plan p = make_plan<InT, InT>(ctx, n, K, 16384u, false);
   cudaError_t e = ensure_arena(ctx, p.total);
   if (e != cudaSuccess) return from_cuda(e);
   e = ensure_surv(ctx, (size_t)p.surv_cap * sizeof(Kt));
@@ -518,7 +520,7 @@ static int select_window(Context &ctx, const InT *d_in, uint64_t n, const ReqSou
                          bool *missed) {
   using K = typename Traits<InT>::K;
   *missed = true;
-  const Plan p = make_plan<InT, InT>(ctx, n, num_req);
+  const Plan p = make_plan<InT, InT>(ctx, n, num_req, 16384u, false);
   const WindowPlan w = plan_window(p, rlo, rhi, src.topk);
   if (!w.ok) return GGKS_OK;
   cudaError_t e = ensure_arena(ctx, p.total);
