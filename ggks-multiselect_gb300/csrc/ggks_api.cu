@@ -325,11 +325,18 @@ static int api_topk(const T *vec, uint64_t n, uint32_t K, T *out, const ggks_opt
 // batched selection
 // ---------------------------------------------------------------------------
 // Autotuner candidates: bucket divisor (elements per bucket, roughly) x tile
-// size (elements per work item).  Results do not depend on the choice.
-static const BatchTune kTuneCandidates[] = {
-    {256, 1u << 16},  {256, 1u << 18},  {256, 1u << 20},  {1024, 1u << 16}, {1024, 1u << 18},
-    {1024, 1u << 20}, {4096, 1u << 16}, {4096, 1u << 18}, {4096, 1u << 20},
+// size (elements per work item), the choice of untuned calls among them.  Results
+// do not depend on the choice.
+static constexpr BatchTune kTuneCandidates[] = {
+    {256, 1u << 16},  {256, 1u << 18},  {256, 1u << 20},  {256, 1u << 21},  {1024, 1u << 16},
+    {1024, 1u << 18}, {1024, 1u << 20}, {4096, 1u << 16}, {4096, 1u << 18}, {4096, 1u << 20},
 };
+static constexpr bool default_is_candidate() {
+  for (const BatchTune &c : kTuneCandidates)
+    if (c.div == BatchTune{}.div && c.tile == BatchTune{}.tile) return true;
+  return false;
+}
+static_assert(default_is_candidate(), "tuning cannot choose worse than no tuning");
 
 static inline uint32_t log2_round(uint64_t v) {
   uint32_t r = 0;
