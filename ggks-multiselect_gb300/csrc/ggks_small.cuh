@@ -444,6 +444,17 @@ __global__ void __launch_bounds__(kSmThreads, 1)
         __syncwarp();
         continue;
       }
+      // few-valued input: copies of one key need no selection (120000 floats of 256
+      // values, one k: 66 us a call, now 46)
+      if (h.dup) {
+        const K first = __ldcg(surv + s_pre[t]);
+        bool same = true;
+        for (uint32_t j = lane; j < size; j += 32) same = same && __ldcg(surv + s_pre[t] + j) == first;
+        if (__all_sync(0xffffffffu, same)) {
+          for (uint32_t j = lane; j < m; j += 32) out[rq[j].out] = Traits<OutT>::value(first);
+          continue;
+        }
+      }
       K lo, hi;
       range(r * kSmThreads + t, &lo, &hi);
       // up to kWarpSelReq requests: radix select, else (or when the needed
