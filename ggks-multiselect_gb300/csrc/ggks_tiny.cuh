@@ -288,7 +288,9 @@ __global__ void __launch_bounds__(kTinyThreads, 1)
     } else if (c <= 64) {
       warp_sort_smem<K, 2>(a, c);
     } else if (!warp_sort_runs<K>(a, c)) {
-      if (c <= 256)
+      if (c <= 128)
+        warp_sort_smem<K, 4>(a, c);
+      else if (c <= 256)
         warp_sort_smem<K, 8>(a, c);
       else if (c <= 512 && tiny_bin<K>() >= 512)
         warp_sort_smem<K, 16>(a, c);
