@@ -11,7 +11,8 @@
 //   1 table    queue over problems: up to kBMaxS keys sampled into shared
 //              memory, the problem's splitter table built by build_lut_cta
 //              (the single-vector builder) with 2^nsl_bits slices, nsl_bits <= b_slice_bits;
-//              the tile phases hold it in shared memory once per bank.
+//              the tile phases hold it in shared memory in several copies (4-byte
+//              keys: once per bank; 8-byte keys: four).
 //   2 hist     queue over (problem, tile) items: a tile is a contiguous range
 //              of one problem; its shared-memory histogram becomes one row of
 //              counts (rows of a problem's tiles are consecutive).  Tiles of a

@@ -22,10 +22,11 @@
 //                 without its 4n-byte element-to-bucket array.
 //   (d) totals    k_colsum: sums the per-CTA rows per bucket.  Replaces
 //                 sumCounts (:214-221).
-//   (e) plan      k_plan_few (up to kPlanFew requests, in rank order) or k_plan:
-//                 one CTA takes the exclusive bucket prefix in shared
-//                 memory, maps every requested rank to its bucket and local
-//                 rank, answers ranks that fall in single-key buckets
+//   (e) plan      k_plan_few (up to kPlanFew requests, in rank order: a search
+//                 over the totals of the 64-bucket tiles, then inside one tile) or
+//                 k_plan (the exclusive bucket prefix in shared memory): one
+//                 CTA maps every requested rank to its bucket and local rank,
+//                 answers ranks that fall in single-key buckets
 //                 directly, assigns compact slots to the active buckets and
 //                 groups the requests by slot.  Replaces the host walk of findKBuckets
 //                 (:87-111), the host reindex loop and reindexCounts
@@ -1663,7 +1664,7 @@ static __global__ void __launch_bounds__(1024)
   }
 }
 
-constexpr uint32_t kPlanFew = 1024;  // requests of k_plan_few, sorted by rank (bring_requests)
+constexpr uint32_t kPlanFew = 1024;  // requests of k_plan_few, sorted by rank (k_table)
 
 // The last of a tile's 64 bucket prefixes (p[0 .. m) are in use, p[0] = 0) that
 // is <= r, found from every eighth of them (q[0 .. 8), the largest value past

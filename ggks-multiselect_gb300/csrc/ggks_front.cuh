@@ -4,8 +4,8 @@
 //   k_sample  kFrontSamples keys at hashed positions, gathered by the whole GPU
 //   k_bin     the sample counted in 4096 fine slices of its span
 //   k_table   the splitter table (LUT) of the pipeline, by one CTA
-//   k_slice   the samples of the fine slices that hold given sample ranks
-//             (thresholds of a top-k, ggks_topk.cuh)
+//   k_slice   the samples of the fine slices that hold given sample ranks (a
+//             top-k's threshold, a window's ends)
 //
 // Workspace: [fine counts kLutIdx words][window path's bins and counters][SliceOut].
 //

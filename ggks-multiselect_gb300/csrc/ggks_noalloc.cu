@@ -20,8 +20,8 @@
 // that device current on the first call there, which also sets the kernels'
 // shared-memory limits on that device (so the first call on a device must
 // come before any stream capture).  Every call shares the one array, which
-// keeps the last call's contents; each call clears the control block and the
-// slice counts, the only parts that must start at zero.  Calls whose work
+// keeps the last call's contents; each call's first kernel (k_sample) sets the
+// control block and clears the slice counts, the only parts that must start at zero.  Calls whose work
 // overlaps on the GPU (different streams, or several host threads) race and
 // must be serialised by the caller.
 #include <mutex>
@@ -38,8 +38,7 @@ constexpr uint32_t kNaMaxG = 64;     // histogram / compaction CTAs
 constexpr uint32_t kNaS = 65536;     // sample size
 
 constexpr size_t na_align(size_t v) { return (v + 255) / 256 * 256; }
-// scratch layout (byte offsets); the control block and the slice counts are
-// zeroed together at the start of each call
+// scratch layout (byte offsets)
 constexpr size_t kNaCtrl = 0;
 constexpr size_t kNaReqs = na_align(kNaCtrl + sizeof(Ctrl));
 constexpr size_t kNaSorted = na_align(kNaReqs + kNaMaxK * sizeof(Req));

@@ -252,7 +252,7 @@ static cudaError_t launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem
 }
 
 // Launches k_small as one cluster of kSmCtas CTAs, plainly (no programmatic
-// serialization: it follows a copy).
+// serialization: it is the call's first kernel).
 template <class... P, class... A>
 static cudaError_t launch_small(void (*kern)(P...), cudaStream_t s, A &&...args) {
   cudaLaunchAttribute at[1];

@@ -97,8 +97,8 @@ constexpr uint64_t kSmMaxTopkN = 1ull << 18;
 
 // dynamic shared memory: the table's copies, then one word per bucket --
 // its count after the histogram phase, its compaction cursor after the plan
-// (inactive cursors carry bit 31).  CTA 0's samples (phase A) lie over the
-// bucket words; the finishers' scratch (phase F) over both.
+// (inactive cursors carry bit 31).  Every CTA's copy of the sample (phase A) lies
+// over the bucket words; the finishers' scratch (phase F) over both.
 constexpr size_t kSmHcOff = (size_t)kRepWords * 4;
 constexpr size_t kSmBytes = kSmHcOff + (size_t)kSmNb * 4;
 // a warp finisher's buffer: a warp sorts at most 512 four-byte or 256 eight-byte

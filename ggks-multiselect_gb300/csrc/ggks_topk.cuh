@@ -15,14 +15,15 @@
 //             about Binomial(S, 1 - K / n): six standard deviations and four
 //             ranks below its mean), and
 //             streams the vector once: each key >= tau is appended to one
-//             contiguous candidate array, nothing else is written;
+//             contiguous candidate array, nothing else is written (copies of
+//             a tau that much of the vector holds are counted instead);
 //   k_pick    one CTA: a 4096-bin histogram of the candidates over their key
 //             range, the bin holding the K-th largest, a gather of every
 //             candidate from that bin up into shared memory, a bitonic sort,
 //             and the K largest out in descending order.
 // Correctness never rests on the prediction: k_pick checks that every
-// candidate was kept and that there are at least K, and that the gathered
-// keys fit; else it reports ST_TOPK_MISS and the caller runs the pipeline.
+// candidate was kept and that there are at least K with tau's copies, and that
+// the gathered keys fit; else it reports ST_TOPK_MISS and the caller runs the pipeline.
 #pragma once
 
 #include <type_traits>

@@ -11,7 +11,8 @@
 //             deviations and four ranks outside the requests' extreme ranks (an
 //             end past the sample is open) and streams the vector once: keys
 //             inside go to one contiguous candidate array and are counted in
-//             kWinBins equal-width bins, keys below are counted;
+//             kWinBins equal-width bins, keys below are counted, and so are
+//             the copies of end keys that much of the vector holds;
 //   k_wplace  every CTA takes the bins' prefix, finds the bins that hold the
 //             requested ranks, and the candidates of those bins go to the
 //             places of their ranks (bin by bin, unordered inside a bin);
