@@ -2557,6 +2557,43 @@ __device__ __forceinline__ void bitonic_sort_smem(K *s, uint32_t P) {
   }
 }
 
+// Sorts a[0, c) (shared memory, any length) in place, ascending, by the whole CTA
+// (whole warps): 32-key runs in registers, then merges whose first step compares
+// mirrored positions, so that every run ascends and positions past the end, which
+// would hold the largest key, need not exist.  Ends with a barrier.
+template <class K>
+__device__ void cta_sort_any(K *a, uint32_t c) {
+  const uint32_t tid = threadIdx.x, nt = blockDim.x;
+  for (uint32_t i = tid; (i & ~31u) < c; i += nt) {
+    const K v = warp_bitonic32(i < c ? a[i] : KeyMax<K>::v);
+    if (i < c) a[i] = v;
+  }
+  __syncthreads();
+  auto step = [&](uint32_t lo, uint32_t hi) {
+    if (hi >= c) return;
+    const K x = a[lo], y = a[hi];
+    if (x > y) {
+      a[lo] = y;
+      a[hi] = x;
+    }
+  };
+  for (uint32_t k = 64; (k >> 1) < c; k <<= 1) {
+    const uint32_t half = k >> 1, pairs = (c + k - 1) / k * half;
+    for (uint32_t i = tid; i < pairs; i += nt) {
+      const uint32_t lo = ((i & ~(half - 1)) << 1) | (i & (half - 1));
+      step(lo, lo ^ (k - 1));
+    }
+    __syncthreads();
+    for (uint32_t j = k >> 2; j > 0; j >>= 1) {
+      for (uint32_t i = tid; i < pairs; i += nt) {
+        const uint32_t lo = ((i & ~(j - 1)) << 1) | (i & (j - 1));
+        step(lo, lo + j);
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // last bin with start[bin] <= r (start is an exclusive scan, start[0] = 0)
 __device__ __forceinline__ uint32_t bin_of_rank(const uint32_t *start, uint32_t nbins, uint32_t r) {
   uint32_t lo = 0, hi = nbins;

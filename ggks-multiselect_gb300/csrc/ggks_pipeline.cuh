@@ -735,20 +735,16 @@ static int select_small(Context &ctx, const InT *d_in, uint64_t n, const ReqSour
     }
     return GGKS_OK;
   };
-  // A vector that fits the registers of one CTA: one CTA, unless a requested
-  // bin holds too many keys.
+  // A vector that fits the registers of one CTA: one CTA.
   if (n <= tiny_max<K>()) {
     const int smem = (int)tiny_smem_bytes<K>(n);
     e = set_smem_max<k_tiny<InT, OutT>>((int)tiny_smem_bytes<K>(tiny_max<K>()));
     if (e != cudaSuccess) return from_cuda(e);
     {
       PassTimer t(ctx, s, GGKS_PASS_SAMPLE);
-      k_tiny<InT, OutT><<<1, kTinyThreads, smem, s>>>(d_in, (uint32_t)n, d_reqs, num_req, d_out,
-                                                      d_status);
+      k_tiny<InT, OutT><<<1, kTinyThreads, smem, s>>>(d_in, (uint32_t)n, d_reqs, num_req, d_out);
     }
-    bool miss = false;
-    const int st = finish(1, &miss);
-    if (st != GGKS_OK || !miss) return st;
+    return finish(0, missed);
   }
   if (!small_ready<InT, OutT>()) {
     *missed = true;

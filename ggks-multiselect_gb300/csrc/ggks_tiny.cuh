@@ -16,15 +16,14 @@
 //   place   each request finds its bin; the keys of requested bins go to the
 //           positions of their bin's ranks in shared memory;
 //   sort    a warp per requested bin, in registers (at most tiny_bin<K> keys) or,
-//           when it holds few distinct keys, by counting their copies;
+//           when it holds few distinct keys, by counting their copies; the
+//           CTA together for a larger one;
 //   answer  each request reads its own rank.
 //
 // Bound: latency, about eight block barriers.  A call's device time at 5003
 // floats, 11 k's: about 6 us, against 31 us for the cluster kernel
 // (ggks_small.cuh), whose sampling, table build and cluster barriers cost the
 // same at every size.
-// A requested bin of more than tiny_bin<K> keys, too many of them distinct, reports
-// ST_SMALL_MISS, and the caller runs the cluster kernel.
 #pragma once
 
 #include "ggks_device.cuh"
@@ -40,6 +39,13 @@ constexpr uint32_t kTinyBins = 1u << kTinyBinBits;
 template <class K>
 __host__ __device__ constexpr uint32_t tiny_bin() {
   return sizeof(K) == 4 ? 1024u : 256u;
+}
+// larger bins are sorted by the CTA, one after the other (616 doubles, most of them within
+// 1e-7 of one value: by the cluster kernel after this one 89 us a call, now 29; 53 by the
+// cluster kernel alone): at most so many
+template <class K>
+__host__ __device__ constexpr uint32_t tiny_big() {
+  return sizeof(K) == 4 ? 32u : 64u;
 }
 constexpr uint32_t kTinyMaxReq = kTinyThreads;
 
@@ -139,8 +145,8 @@ __device__ __forceinline__ bool warp_sort_runs(K *a, uint32_t c) {
     above = g;
     seen += cnt;
     ++runs;
-    // more runs to come than the bin's size pays for: two passes tell
-    if (runs == 2 && seen * 16 < c && c <= tiny_bin<K>()) return false;
+    // more than 32 runs to come: two passes tell
+    if (runs == 2 && seen * 16 < c) return false;
   }
   uint32_t at = 0;
   for (uint32_t i = 0; i < runs; ++i) {
@@ -154,13 +160,12 @@ __device__ __forceinline__ bool warp_sort_runs(K *a, uint32_t c) {
 
 // x: device vector of n elements, 1 <= n <= tiny_max<K>(); reqs: num_req
 // requests (ascending 0-based rank below n, output index; num_req <=
-// kTinyMaxReq); out: outputs; *host_status: 0 or ST_SMALL_MISS (then no output
-// is written).  reqs, out and host_status may lie in host memory.  One CTA of
+// kTinyMaxReq); out: outputs.  reqs and out may lie in host memory.  One CTA of
 // kTinyThreads threads, tiny_smem_bytes<K>(n) of shared memory.
 template <class T, class OutT>
 __global__ void __launch_bounds__(kTinyThreads, 1)
     k_tiny(const T *__restrict__ x, uint32_t n, const Req *__restrict__ reqs, uint32_t num_req,
-           OutT *__restrict__ out, uint32_t *__restrict__ host_status) {
+           OutT *__restrict__ out) {
   using K = typename Traits<T>::K;
   constexpr uint32_t kPer = tiny_per<K>();
   // the keys of -0.0 and +0.0: kMid and kMid + 1
@@ -172,8 +177,8 @@ __global__ void __launch_bounds__(kTinyThreads, 1)
   __shared__ uint32_t s_w[33];
   __shared__ uint32_t s_need[kTinyBins / 32];  // requested bins
   __shared__ uint32_t s_off[kTinyMaxReq], s_cnt[kTinyMaxReq];  // their segments of buf
-  __shared__ uint32_t s_nbin;
-  __shared__ bool s_miss;
+  static_assert(tiny_max<K>() / (tiny_bin<K>() + 1) < tiny_big<K>(), "every large bin");
+  __shared__ uint32_t s_nbin, s_nbig, s_big[tiny_big<K>()];  // requested bins; the large ones
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   Req q;
@@ -190,7 +195,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1)
   if (tid < kTinyBins / 32) s_need[tid] = 0;
   if (tid == 0) {
     s_nbin = 0;
-    s_miss = false;
+    s_nbig = 0;
   }
   // the occupied ranges [lo[h], hi[h]] below and above the two middle keys
   K lo[2] = {KeyMax<K>::v, KeyMax<K>::v}, hi[2] = {0, 0};
@@ -296,14 +301,13 @@ __global__ void __launch_bounds__(kTinyThreads, 1)
         warp_sort_smem<K, 16>(a, c);
       else if (c <= tiny_bin<K>())
         warp_sort_smem<K, (int)(tiny_bin<K>() / 32)>(a, c);
-      else
-        s_miss = true;
+      else if (lane == 0)
+        s_big[atomicAdd(&s_nbig, 1u)] = i;
     }
   }
   __syncthreads();
-  const bool miss = s_miss;
-  if (!miss && tid < num_req) out[q.out] = Traits<OutT>::value(buf[q.rank]);
-  if (tid == 0) *host_status = miss ? ST_SMALL_MISS : 0u;
+  for (uint32_t i = 0; i < s_nbig; ++i) cta_sort_any<K>(buf + s_off[s_big[i]], s_cnt[s_big[i]]);
+  if (tid < num_req) out[q.out] = Traits<OutT>::value(buf[q.rank]);
 }
 
 }  // namespace ggks

@@ -110,6 +110,10 @@ int place(const K *arr, uint32_t len, uint64_t n, uint32_t below, K lo, uint32_t
 
 extern "C" {
 
+int emu_sort_u64(uint64_t *a, uint32_t c, uint32_t threads) {
+  return emu::launch(1, threads, 0, [&] { cta_sort_any<uint64_t>(a, c); }) ? 0 : 1;
+}
+
 int emu_filter_f32(const float *x, uint64_t n, uint32_t r0, uint32_t r1, int lo_open, int hi_open,
                    uint32_t grid, uint32_t *arr, uint64_t cap, uint32_t *bins, uint64_t *out) {
   return filter<float>(x, n, r0, r1, lo_open, hi_open, grid, arr, cap, bins, out);

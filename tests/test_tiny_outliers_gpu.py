@@ -1,5 +1,6 @@
 """Tiny vectors whose keys crowd into few of the bins because some values lie far
-out: bins just below and above what a warp sorts, answered by the one-CTA kernel."""
+out: bins just below and above what a warp sorts, and most of the vector in one bin,
+answered by the one-CTA kernel."""
 import numpy as np
 import pytest
 
@@ -48,3 +49,25 @@ def test_one_bin(g, crowd):
     d = DeviceArray(x)
     got = g.multiselect_ptr(d.ptr, x.size, np.uint32, ks)
     assert_same(got, desc[ks - 1])
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.uint32])
+@pytest.mark.parametrize("n", [40, 616, 5563, 16_384, 32_768])
+def test_crowd(g, dtype, n):
+    """Nine tenths of the vector within a sliver of its range, in one bin or two."""
+    if n > 16_384 and dtype == np.float64:
+        n = 16_384
+    r = np.random.default_rng(n)
+    x = (1e6 + r.random(n) * 30_000).astype(dtype) if dtype == np.uint32 else (1000 + r.random(n) * 0.05).astype(dtype)
+    at = r.random(n) < 0.1
+    x[at] = (r.random(np.count_nonzero(at)) * (4e9 if dtype == np.uint32 else 1e30)).astype(dtype)
+    desc = np.sort(x)[::-1]
+    d = DeviceArray(x, pad_front=1)
+    ctx = g.Context(0)
+    for ks in (r.integers(1, n + 1, 1000), [1], [n], [n // 2], np.linspace(1, n, 30).astype(int)):
+        ks = np.array(ks, dtype=np.uint32)
+        assert_same(g.multiselect_ptr(d.ptr, n, dtype, ks, ctx=ctx), desc[ks - 1])
+    assert_same(g.topk_ptr(d.ptr, n, dtype, min(n, 1024), ctx=ctx), desc[:1024])
+    st = ctx.stats()
+    ctx.close()
+    assert st["small_calls"] == 6 and st["launches"] == 6

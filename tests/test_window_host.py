@@ -196,3 +196,16 @@ def test_place(emu, kk, grid):
                 assert np.array_equal(np.sort(part), np.sort(arr[at == b]))
             else:
                 assert np.all((part[part != EMPTY] - lo) >> shift == b)
+
+
+@pytest.mark.parametrize("threads", [64, 1024])
+@pytest.mark.parametrize("c", [1, 2, 31, 32, 33, 63, 64, 65, 127, 129, 500, 1000, 1024, 1025, 3000])
+def test_sort_any_length(emu, threads, c):
+    r = np.random.default_rng(c)
+    guard = 40
+    for hi in (3, 1 << 60):
+        a = r.integers(0, hi, c + guard).astype(np.uint64)
+        a[r.integers(0, c)] = ~np.uint64(0)
+        want = np.concatenate([np.sort(a[:c]), a[c:]])
+        assert emu.emu_sort_u64(a.ctypes.data_as(ctypes.c_void_p), c, threads) == 0
+        assert np.array_equal(a, want)
