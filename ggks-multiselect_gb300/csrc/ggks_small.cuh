@@ -480,13 +480,14 @@ __global__ void __launch_bounds__(kSmThreads, 1)
       if (h.dup) {
         const K first = __ldcg(surv + s_pre[t]);
         bool same = true;
-        for (uint32_t j0 = tid; j0 < size; j0 += 4 * kSmThreads) {
-          K v[4];
+        constexpr int U = (int)(64 / sizeof(K));  // 64 KB in flight
+        for (uint32_t j0 = tid; j0 < size; j0 += U * kSmThreads) {
+          K v[U];
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
+          for (int u = 0; u < U; ++u)
             v[u] = j0 + u * kSmThreads < size ? __ldcg(surv + s_pre[t] + j0 + u * kSmThreads) : first;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) same = same && v[u] == first;
+          for (int u = 0; u < U; ++u) same = same && v[u] == first;
         }
         if (__syncthreads_and(same)) {
           for (uint32_t j = tid; j < m; j += kSmThreads) out[rq[j].out] = Traits<OutT>::value(first);
