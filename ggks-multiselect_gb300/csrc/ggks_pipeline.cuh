@@ -471,11 +471,13 @@ static int topk_threshold(Context &ctx, const InT *d_in, uint64_t n, uint32_t K,
   return GGKS_OK;
 }
 
-// A top-k selects again from one large bin of distinct keys at most, and for at most
-// kWinMaxAgain values; else the pipeline answers (2^24 floats, 0.1 % of them one value
-// far out, top-20000: 222 us a call by the pipeline after the window, 134 with 3300
-// values of one bin selected again; 3 M floats, 17000 values: 163 and 203).
-constexpr uint32_t kWinMaxDefer = 1;
+// A top-k's large bins of distinct keys: up to kWinMaxDefer that a CTA can sort are
+// (k_wbig); else one bin is selected from again for at most kWinMaxAgain values, or the
+// pipeline answers.  (786000 values, most of them 0 to 2, some up to 150000, top-20000:
+// 151 us a call by the pipeline after the window, now 75; 110 by the pipeline alone.  2^24
+// floats, 0.1 % of them one value far out, top-20000: 222, by a recursive level 134, now
+// 105; 3 M such floats, 17000 values of one bin: 163, by a recursive level 203, now 98.)
+constexpr uint32_t kWinMaxDefer = 64;
 constexpr uint32_t kWinMaxAgain = 4096;
 // smallest vector whose clustered k's go to the window path before the one-launch one
 constexpr uint64_t kWinFirstN = 1ull << 19;
@@ -632,11 +634,22 @@ static int select_window(Context &ctx, const InT *d_in, uint64_t n, const ReqSou
   // a miss: the pipeline answers (the streaming pass has written the device copy of an
   // ingested vector)
   const uint32_t D = (status & ST_DEFERRED) ? h_ctrl->deferred_count : 0u;
+  bool sort = src.topk && D && D <= kWinMaxDefer;  // large bins that k_wbig can sort
+  for (uint32_t i = 0; sort && i < D; ++i) sort = h_big[i].size <= win_big_max<K>();
   *missed = (status & ST_TOPK_MISS) != 0 ||
-            (src.topk && (D > kWinMaxDefer ||
-                          (D && std::min(h_big[0].size, num_req - h_big[0].above) > kWinMaxAgain)));
+            (src.topk && !sort &&
+             (D > 1 || (D && std::min(h_big[0].size, num_req - h_big[0].above) > kWinMaxAgain)));
   if (*missed) return GGKS_OK;
-  if (D) {
+  if (sort) {
+    const int smem = (int)wbig_smem_bytes<K>();
+    e = set_smem_max<k_wbig<K, InT>>(smem);
+    if (e != cudaSuccess) return from_cuda(e);
+    k_wbig<K, InT><<<D, 1024, smem, s>>>(placed, deferred, num_req, d_out);
+    ctx.stats.launches++;
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = pull();
+    if (e != cudaSuccess) return from_cuda(e);
+  } else if (D) {
     // large bins of distinct keys: select from each again, on its keys
     int st = GGKS_OK;
     Context *ch = child_of(ctx, &st);

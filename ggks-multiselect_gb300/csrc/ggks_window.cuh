@@ -596,9 +596,88 @@ __global__ void __launch_bounds__(kFinThreads)
   win_leave(ctrl, host_ctrl);
 }
 
+// A top-k's large bins of distinct keys (win_big_max keys at most), a CTA of 1024
+// threads each; launched only where k_wsort left some.  A bin's keys go to the places
+// of 4096 parts of their range in shared memory, and one thread sorts each part; where
+// a part holds more than kWinPart keys (another gap) the whole bin is sorted by the
+// CTA's network (about 1 us a step: 22000 of 3 M floats, the call 226 us, by parts 98).
+constexpr uint32_t kWinParts = 4096, kWinPart = 32;
+template <class K>
+__host__ __device__ constexpr uint32_t win_big_max() {
+  return (128u << 10) / (uint32_t)sizeof(K);
+}
+template <class K>
+__host__ __device__ constexpr size_t wbig_smem_bytes() {
+  return 2 * kWinParts * 4 + (size_t)win_big_max<K>() * sizeof(K);
+}
+template <class K, class OutT>
+__global__ void __launch_bounds__(1024, 1)
+    k_wbig(const K *placed, const WinDefer *list, uint32_t kk, OutT *__restrict__ out) {
+  extern __shared__ uint4 smem_raw[];
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(smem_raw), *start = cnt + kWinParts;
+  K *a = reinterpret_cast<K *>(start + kWinParts);
+  __shared__ K s_key[33];
+  __shared__ uint32_t s_scan[32];
+  const WinDefer d = list[blockIdx.x];
+  const uint32_t tid = threadIdx.x, c = d.size;
+  if (c > win_big_max<K>()) return;
+  auto each = [&](auto &&fn) {
+    constexpr uint32_t U = 8;
+    for (uint32_t i0 = tid; i0 < c; i0 += U * 1024) {
+      K k[U];
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) k[u] = i0 + 1024 * u < c ? __ldcg(placed + d.off + i0 + 1024 * u) : K(0);
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u)
+        if (i0 + 1024 * u < c) fn(i0 + 1024 * u, k[u]);
+    }
+  };
+  fill_words(cnt, kWinParts, 0u);
+  K lo = KeyMax<K>::v, hi = 0;
+  each([&](uint32_t, K k) {
+    lo = k < lo ? k : lo;
+    hi = k > hi ? k : hi;
+  });
+  lo = block_reduce(lo, [](K u, K v) { return u < v ? u : v; }, s_key);
+  hi = block_reduce(hi, [](K u, K v) { return u > v ? u : v; }, s_key);
+  const int bl = bitlen<K>(hi - lo);
+  const uint32_t sh = bl > 12 ? (uint32_t)(bl - 12) : 0u;
+  each([&](uint32_t, K k) { atomicAdd(&cnt[(uint32_t)((k - lo) >> sh)], 1u); });
+  __syncthreads();
+  const uint4 c4 = reinterpret_cast<const uint4 *>(cnt)[tid];
+  uint32_t all;
+  const uint32_t pre = block_excl_scan(c4.x + c4.y + c4.z + c4.w, s_scan, &all);
+  reinterpret_cast<uint4 *>(start)[tid] = make_uint4(pre, pre + c4.x, pre + c4.x + c4.y, pre + c4.x + c4.y + c4.z);
+  // (parts one key wide need no sort)
+  const bool crowded = __syncthreads_or(sh && max(max(c4.x, c4.y), max(c4.z, c4.w)) > kWinPart);
+  if (crowded) {
+    each([&](uint32_t i, K k) { a[i] = k; });
+    __syncthreads();
+    cta_sort_any<K>(a, c);
+  } else {
+    each([&](uint32_t, K k) {
+      const uint32_t b = (uint32_t)((k - lo) >> sh);
+      a[start[b] + atomicSub(&cnt[b], 1u) - 1u] = k;
+    });
+    __syncthreads();
+    for (uint32_t b = tid; sh && b < kWinParts; b += 1024) {
+      const uint32_t p0 = start[b], p1 = b + 1 < kWinParts ? start[b + 1] : c;
+      for (uint32_t p = p0 + 1; p < p1; ++p) {
+        const K v = a[p];
+        uint32_t r = p;
+        for (; r > p0 && a[r - 1] > v; --r) a[r] = a[r - 1];
+        a[r] = v;
+      }
+    }
+    __syncthreads();
+  }
+  for (uint32_t i = tid; i < c && d.above + i < kk; i += 1024)
+    out[d.above + i] = Traits<OutT>::value(a[c - 1 - i]);
+}
+
 // A top-k's values from the placed bins: a warp per bin from wc->first up, the
 // values in descending order to out[0 .. kk).  A large bin of distinct keys is left
-// to a recursive level.
+// to k_wbig or a recursive level.
 constexpr uint32_t kWinSortThreads = 256;
 template <class K, class OutT>
 __global__ void __launch_bounds__(kWinSortThreads)

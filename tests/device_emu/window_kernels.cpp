@@ -110,6 +110,14 @@ int place(const K *arr, uint32_t len, uint64_t n, uint32_t below, K lo, uint32_t
 
 extern "C" {
 
+int emu_big_u32(const uint32_t *placed, uint64_t off, uint32_t size, uint32_t above, uint32_t kk,
+                uint32_t *out) {
+  const WinDefer d{off, size, 0, 0, above};
+  return emu::launch(1, 1024, wbig_smem_bytes<uint32_t>(),
+                     [&] { k_wbig<uint32_t, uint32_t>(placed, &d, kk, out); })
+             ? 0
+             : 1;
+}
 int emu_sort_u64(uint64_t *a, uint32_t c, uint32_t threads) {
   return emu::launch(1, threads, 0, [&] { cta_sort_any<uint64_t>(a, c); }) ? 0 : 1;
 }

@@ -209,3 +209,23 @@ def test_sort_any_length(emu, threads, c):
         want = np.concatenate([np.sort(a[:c]), a[c:]])
         assert emu.emu_sort_u64(a.ctypes.data_as(ctypes.c_void_p), c, threads) == 0
         assert np.array_equal(a, want)
+
+
+@pytest.mark.parametrize("kind", ["spread", "crowd", "narrow", "full"])
+@pytest.mark.parametrize("size", [257, 1000, 4097, 20_000, 32_768])
+def test_big_bin(emu, kind, size):
+    """One large bin of a top-k: parts that a thread sorts, a crowded part, parts one key wide."""
+    r = np.random.default_rng(size)
+    off, above = 37, 100
+    keys = {"spread": lambda: r.integers(1 << 20, 1 << 30, size),
+            "crowd": lambda: np.append(r.integers(0, 5000, size - 1), 0xFFFFFFFF),
+            "narrow": lambda: 7 + r.integers(0, 4000, size),
+            "full": lambda: r.permutation(size) * 131}[kind]().astype(np.uint32)
+    placed = np.concatenate([np.zeros(off, np.uint32), keys])
+    for kk in (above + size, above + size // 3, above + 1):
+        out = np.full(above + size + 8, EMPTY, np.uint32)
+        rc = emu.emu_big_u32(placed.ctypes.data_as(U32), ctypes.c_uint64(off), size, above, kk,
+                             out.ctypes.data_as(U32))
+        assert rc == 0
+        assert np.array_equal(out[above:kk], np.sort(keys)[::-1][:kk - above])
+        assert np.all(out[:above] == EMPTY) and np.all(out[kk:] == EMPTY)
