@@ -130,7 +130,7 @@ struct alignas(16) BHdr {  // (load_hdr reads it in 16-byte vectors)
   uint32_t spec_ok;  // phase 3: every slot's bucket lies strictly inside it
   uint32_t low;      // 1: the table has a low entry
   uint64_t tau_lo, tau_hi;  // keys; tau_lo 0 / tau_hi the largest key: open end
-  uint64_t top;      // position of the table's top entry
+  uint64_t lo, hi;   // the table's clamps
 };
 
 // one (problem, tile) work item (host-written)
@@ -297,7 +297,8 @@ __device__ __forceinline__ BHdr load_hdr(const BHdr *h) {
   r.spec_on = w2.y;
   r.spec_ok = w2.z;
   r.low = w2.w;
-  r.top = ldcg_u(&h->top);
+  r.lo = ldcg_u(&h->lo);
+  r.hi = ldcg_u(&h->hi);
   r.tau_lo = ldcg_u(&h->tau_lo);
   r.tau_hi = ldcg_u(&h->tau_hi);
   return r;
@@ -724,7 +725,8 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
     if (tid == 0) {
       BHdr h;
       h.base = s_hdr.base;
-      h.top = s_hdr.top;
+      h.lo = s_hdr.lo;
+      h.hi = s_hdr.hi;
       h.surv_off = 0;
       h.shift = s_hdr.shift;
       h.nb = s_hdr.nb;
@@ -772,7 +774,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       if (tid == 0) s_ccnt = 0;
       __syncthreads();
       if (tid == 0) s_cur = tl.prob;
-      const KeyTable<K> kt((K)H.base, (K)H.top, H.shift);
+      const KeyTable<K> kt((K)H.base, (K)H.lo, (K)H.hi, H.shift);
       if (H.dup) {
         // count, and keep the bucket's first key; a second distinct key (or
         // the largest key, which marks an empty entry) sets the mixed bit
@@ -981,7 +983,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       // speculation holds when every slot with survivors lies strictly between
       // the buckets of the window's ends (an open end bounds nothing)
       const bool lo_open = H.tau_lo == 0, hi_open = (K)H.tau_hi == KeyMax<K>::v;
-      const KeyTable<K> kt((K)H.base, (K)H.top, H.shift);
+      const KeyTable<K> kt((K)H.base, (K)H.lo, (K)H.hi, H.shift);
       const uint32_t ents = nsl + 1 + H.low;
       const uint32_t b_tlo = lo_open ? 0u : bucket_of<K>((K)H.tau_lo, kt, lut);
       const uint32_t b_thi = hi_open ? 0u : bucket_of<K>((K)H.tau_hi, kt, lut);
@@ -1177,7 +1179,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch(BArgs A) {
       // and every store inside the buffer (see compact_one)
       const uint64_t room = A.surv_cap - H.surv_off;
       const uint32_t cap = (uint32_t)(room < (uint64_t)kInactive ? room : kInactive);
-      const KeyTable<K> kt((K)H.base, (K)H.top, H.shift);
+      const KeyTable<K> kt((K)H.base, (K)H.lo, (K)H.hi, H.shift);
       const uint32_t ncand = H.spec_ok ? __ldcg(A.cand_cnt + t) : 0xFFFFFFFFu;
       if (H.spec_ok && ncand <= tl.cand_cap) {
         // the tile's complete candidate list holds every key of its slots'

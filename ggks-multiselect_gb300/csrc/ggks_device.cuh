@@ -241,8 +241,9 @@ struct Ctrl {
 template <class K>
 struct LutHeader {
   K base;          // the table's first key: one slice below the smallest sampled key
-                   // (low == 1), or that key itself where no slice fits below it
-  K top;           // position of the top entry: one slice past the sampled span
+                   // (low == 1; modulo the key width), or that key itself
+  K lo, hi;        // keys are clamped to [lo, hi]: hi lies in the top entry, one slice
+                   // past the sampled span
   uint32_t shift;  // entry of a key: its position (table_pos) >> shift
   uint32_t low;    // 1: entry 0 is the keys below the smallest sampled one
   uint32_t nb;     // number of buckets
@@ -433,7 +434,7 @@ __device__ __forceinline__ uint32_t hash32(uint32_t a) {
 // bucket function: slice lookup + sub-bucket by the next bits of the key
 // ---------------------------------------------------------------------------
 // A key's position is the key clamped to the table's range, less its first key:
-//   d = min(max(key, base) - base, top),
+//   d = min(max(key, lo), hi) - base,
 // and its entry is d >> shift: [low] slices 0 .. nsl - 1, [top].  lut[j] =
 // (C_j << 7) | rs_j; for an entry with first bucket B_j cut into 2^b_j
 // sub-buckets rs_j = shift - b_j and C_j = B_j - (j << b_j) modulo 2^25.  Then
@@ -441,8 +442,12 @@ __device__ __forceinline__ uint32_t hash32(uint32_t a) {
 // since d >> rs_j = (j << b_j) + sub-bucket.  Empty slices of one run share a
 // bucket (b = 0); the low and top entries are buckets too (b = 0): keys below the
 // smallest sampled one reach the low entry, those further below by the clamp,
-// and keys above the sampled span the top one.  Without a low entry (fewer than
-// 2^shift keys below) they share the first slice's first bucket.
+// and keys above the sampled span the top one.  The low entry's slice may begin
+// below key 0 (base wraps, lo is 0): without it the keys below shared a bucket with the
+// smallest sampled key, which much of the vector may hold (3.2 M integers, 454000 copies
+// of their tenth percentile: one bucket of two keys, 867 us a call for 101 k's, now 224).
+// There is none where no key lies below, or where the table would reach past the key
+// width.
 //
 // For 4-byte keys the bucket's byte offset in an array of words takes three
 // operations after the lookup: x = d >> rs (a shift by the entry's low five
@@ -453,15 +458,14 @@ __device__ __forceinline__ uint32_t hash32(uint32_t a) {
 // 101 ks: 56 -> 53 us a call).
 template <class K>
 struct KeyTable {
-  K base, top;
+  K base, lo, hi;
   uint32_t shift;
-  __device__ __forceinline__ KeyTable(K b, K t, uint32_t s) : base(b), top(t), shift(s) {}
+  __device__ __forceinline__ KeyTable(K b, K l, K h, uint32_t s) : base(b), lo(l), hi(h), shift(s) {}
   __device__ __forceinline__ explicit KeyTable(const LutHeader<K> &h)
-      : base(h.base), top(h.top), shift(h.shift) {}
+      : base(h.base), lo(h.lo), hi(h.hi), shift(h.shift) {}
   __device__ __forceinline__ K pos(K key) const {
-    const K c = key > base ? key : base;
-    const K d = c - base;
-    return d < top ? d : top;
+    const K c = key > lo ? key : lo;
+    return (c < hi ? c : hi) - base;
   }
 };
 
@@ -776,14 +780,23 @@ __device__ __forceinline__ uint32_t build_table(D &&density, uint32_t nsl, uint3
   return low + total + (top_run_start ? 1u : 0u);
 }
 
-// The table's place around a sampled span: its first key and the position of its
-// top entry (see bucket_of).
+// The table's place around a sampled span: its first key, the clamps and whether it
+// has a low entry (see bucket_of).
 template <class K>
-__device__ __forceinline__ void table_place(LutHeader<K> &h, K kmin, uint32_t shift, uint32_t nsl) {
-  h.low = kmin >= ((K)1 << shift) ? 1u : 0u;
-  h.base = h.low ? kmin - ((K)1 << shift) : kmin;
+__device__ __forceinline__ void table_place(LutHeader<K> &h, K kmin, K kmax, uint32_t shift,
+                                            uint32_t nsl) {
+  const K width = (K)1 << shift;
+  const K under = kmin < width ? width - kmin : K(0);  // how far below key 0 the low entry begins
+  h.low = kmin > 0 && kmax <= KeyMax<K>::v - under ? 1u : 0u;
+  h.base = h.low ? kmin - width : kmin;
+  h.lo = h.low && kmin < width ? K(0) : h.base;
+  // the top entry's position, if it lies within the key width
   const K ents = (K)(nsl + h.low);
-  h.top = ents > (KeyMax<K>::v >> shift) ? KeyMax<K>::v : ents << shift;
+  const K top = ents > (KeyMax<K>::v >> shift) ? KeyMax<K>::v : ents << shift;
+  if (h.low && under)
+    h.hi = top - under;
+  else
+    h.hi = top > KeyMax<K>::v - h.base ? KeyMax<K>::v : h.base + top;
   h.shift = shift;
   h.dense = 0;
 }
@@ -822,7 +835,7 @@ __device__ void build_lut_cta(const K *samples, uint32_t S, K kmin, K kmax, uint
   }
   __syncthreads();
   LutHeader<K> h;
-  table_place<K>(h, kmin, shift, nsl);
+  table_place<K>(h, kmin, kmax, shift, nsl);
   const uint32_t nb = build_table<K, SPT>([&](uint32_t j) { return cnt[j]; }, nsl, h.low, shift, bcap,
                                           nb_max, lut, tab, ts);
   __syncthreads();

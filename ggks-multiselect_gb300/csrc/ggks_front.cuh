@@ -314,7 +314,8 @@ __global__ void __launch_bounds__(kTableThreads, 1)
           const K spare = (kDenseKeys - 1u) - (kmax - kmin), left = min(kmin, spare / 2);
           const K right = min(KeyMax<K>::v - kmax, spare - left);
           h.base = kmin - min(kmin, spare - right);
-          h.top = kDenseKeys - 1u;
+          h.lo = h.base;
+          h.hi = h.base + (K)(kDenseKeys - 1u);
           h.shift = 0;
           h.low = 0;
           h.nb = kDenseKeys;
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(kTableThreads, 1)
       }
     }
   }
-  table_place<K>(h, kmin, shift, nsl);
+  table_place<K>(h, kmin, kmax, shift, nsl);
   const uint32_t nb = build_table<K, SPT>(density, nsl, h.low, shift, bcap, nb_max, lut, tab, ts);
 
   // Candidate windows.  The number of samples below the element of rank r is

@@ -1,5 +1,6 @@
-// window_kernels.cpp -- the sampled-window kernels on the host CPU (see
-// cuda_on_host.h), as plain C functions for tests/test_window_host.py.
+// window_kernels.cpp -- the sampled-window kernels and the splitter table on the host
+// CPU (see cuda_on_host.h), as plain C functions for tests/test_window_host.py and
+// tests/test_table_host.py.
 #include "cuda_on_host.h"
 
 #include "ggks_window.cuh"
@@ -57,6 +58,38 @@ int filter(const T *x, uint64_t n, uint32_t r0, uint32_t r1, bool lo_open, bool 
   return ok ? 0 : 1;
 }
 
+// The table of x[0 .. n), n <= kFrontSamples (every element is a sample), and where it
+// puts each of keys[0 .. m): the bucket and that bucket's smallest key.
+template <class T>
+int table(const T *x, uint64_t n, uint32_t nb_max, const typename Traits<T>::K *keys, uint32_t m,
+          uint32_t *bucket, typename Traits<T>::K *first, uint32_t *nb) {
+  using K = typename Traits<T>::K;
+  const uint32_t S = (uint32_t)n, g = front_ctas(S);
+  std::vector<K> samples(S), spans(2 * g);
+  std::vector<uint32_t> fine(kLutIdx, ~0u), lut(kLutPadded, 0);
+  LutHeader<K> h;
+  Ctrl ctrl{};
+  bool ok = emu::launch(g, 1024, 0, [&] {
+    k_sample<T>(x, n, S, 1u, samples.data(), spans.data(), fine.data(), kLutIdx, &ctrl, Ctrl{},
+                ReqCopy{});
+  });
+  ok = ok && emu::launch(g, 1024, 0, [&] {
+         k_bin<K>(samples.data(), S, spans.data(), fine.data(), &ctrl);
+       });
+  ok = ok && emu::launch(1, kTableThreads, 0, [&] {
+         k_table<K>(samples.data(), S, spans.data(), fine.data(), n, RankWindows{}, &h, lut.data(),
+                    nb_max, nb_max, 0u, 1u, false, &ctrl, ReqCopy{});
+       });
+  if (!ok) return 1;
+  const KeyTable<K> kt(h);
+  for (uint32_t i = 0; i < m; ++i) {
+    bucket[i] = bucket_of<K>(keys[i], kt, lut.data());
+    first[i] = bucket_lo<K>(bucket[i], h.base, h.shift, lut.data(), sv_slices<K>() + 1 + h.low);
+  }
+  *nb = h.nb;
+  return 0;
+}
+
 // k_wplace over the candidates arr[0 .. len) and the given bin counts, and, with out
 // given, k_wsort (a top-k, kk > 0) or k_wfinish.
 template <class K>
@@ -110,6 +143,14 @@ int place(const K *arr, uint32_t len, uint64_t n, uint32_t below, K lo, uint32_t
 
 extern "C" {
 
+int emu_table_u32(const uint32_t *x, uint64_t n, uint32_t nb_max, const uint32_t *keys, uint32_t m,
+                  uint32_t *bucket, uint32_t *first, uint32_t *nb) {
+  return table<uint32_t>(x, n, nb_max, keys, m, bucket, first, nb);
+}
+int emu_table_f64(const double *x, uint64_t n, uint32_t nb_max, const uint64_t *keys, uint32_t m,
+                  uint32_t *bucket, uint64_t *first, uint32_t *nb) {
+  return table<double>(x, n, nb_max, keys, m, bucket, first, nb);
+}
 int emu_big_u32(const uint32_t *placed, uint64_t off, uint32_t size, uint32_t above, uint32_t kk,
                 uint32_t *out) {
   const WinDefer d{off, size, 0, 0, above};
