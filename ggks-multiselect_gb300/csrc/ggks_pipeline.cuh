@@ -35,6 +35,12 @@ static inline int finish_smem_bytes() {
   return (int)finish_smem_for<K>(cap_keys_for<T>());
 }
 
+// Shared memory asked for when there are no more slots than SMs: a CTA per SM.  The CTAs
+// start as the ones of k_compact end, and with their own need four of them shared
+// the first SM to be free (7.5 M few-valued floats, 11 slots of 28000 keys: 245 us a
+// call, now 151; 40 to 150 of them on other vectors: the same).
+constexpr int kFinAlone = 120 << 10;
+
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // k_plan's shared memory: the table, the bucket prefix and flags for the
@@ -1032,8 +1038,8 @@ int select(Context &ctx, const InT *d_in, uint64_t n, const ReqSource &src, uint
       ran[GGKS_PASS_COMPACT] = true;
     }
     {
-      const int smem = finish_smem_bytes<InT>();
-      L(set_smem_max<k_finish<K, OutT>>(smem));
+      const int smem = p.fin_grid <= (uint32_t)ctx.sm_count ? kFinAlone : finish_smem_bytes<InT>();
+      L(set_smem_max<k_finish<K, OutT>>(kFinAlone));
       PassTimer t(ctx, s, GGKS_PASS_FINISH);
       L(launch(k_finish<K, OutT>, p.fin_grid, kFinThreads, smem, s, surv, ctrl, seg_off, seg_size,
                seg_lo, seg_hi, kstart, kcnt, klist, deferred, p.cap_keys, d_out, h_ctrl_dev));
