@@ -38,7 +38,7 @@ static inline int finish_smem_bytes() {
 // Shared memory asked for when there are no more slots than SMs: a CTA per SM.  The CTAs
 // start as the ones of k_compact end, and with their own need four of them shared
 // the first SM to be free (7.5 M few-valued floats, 11 slots of 28000 keys: 245 us a
-// call, now 151; 40 to 150 of them on other vectors: the same).
+// call, now 151; 3 to 150 small slots: the same).
 constexpr int kFinAlone = 120 << 10;
 
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
