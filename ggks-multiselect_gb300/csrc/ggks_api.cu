@@ -411,6 +411,8 @@ static int api_batch(const T *const *vecs, const uint64_t *n, uint32_t P, const 
     // whole calls are timed: planning, launches, re-runs and recursion
     double best = -1.0;
     for (const BatchTune &c : kTuneCandidates) {
+      // fewer than two tiles of 2^21 per resident CTA: halved, they are those of 2^20
+      if (c.tile > (1u << 20) && elems / c.tile < 4ull * (uint32_t)ctx->sm_count) continue;
       const auto t0 = std::chrono::steady_clock::now();
       st = select_batch<T>(*ctx, in, out_dev ? out : nullptr, nullptr, s, c, nullptr);
       const double dt = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
