@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
     hi = block_reduce(hi, [](K u, K v) { return u > v ? u : v; }, redk);
     GGKS_SMALL_STAMP(1);
     build_lut_cta<K, (int)((sv_slices<K>() + kSmThreads - 1) / kSmThreads)>(
-        samples, S, lo, hi, kSmNb, s_tab, s_tab, &s_hdr, sv_bits<K>());
+        samples, S, lo, hi, kSmNb, s_tab, s_tab, &s_hdr, sv_bits<K>(), false);
   }
   __syncthreads();
   GGKS_SMALL_STAMP(2);
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   for (uint32_t i = tid; i < sv_entries<K>() * sv_copies<K>(); i += kSmThreads)
     rep[i] = s_tab[i >> sv_copy_bits<K>()];
   const LutHeader<K> h = s_hdr;
-  const KeyTable<K> kt(h);
+  const KeyTableUp<K> kt(h);
   const uint64_t a0 = n * r / kSmCtas, a1 = n * (r + 1) / kSmCtas;
   const uint32_t *lut = sv_lane_table<K>(rep);
   __syncthreads();
